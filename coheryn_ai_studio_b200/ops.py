@@ -1071,6 +1071,8 @@ def recurrent():
     global _recurrent
     if _recurrent is None:
         lib = build.recurrent_library()
+        lib.coheryn_delta_chunk_floats.restype = ctypes.c_long
+        lib.chunk_from, lib.chunk_tokens = int(lib.coheryn_chunk_from()), int(lib.coheryn_chunk_tokens())
         lib.coheryn_last_error.restype = ctypes.c_char_p
         lib.coheryn_launch_count.restype = ctypes.c_ulonglong
         _recurrent = lib
@@ -1088,6 +1090,20 @@ def _scan_scratch(T: int, B: int, heads: int, dv: int, extra: int, device):
     if dv <= 64 or B * heads > 74 or T < 64 * B:
         return None
     return torch.empty(T * heads * dv + extra, dtype=torch.float32, device=device)
+
+
+def _chunked_runs(lib, step, T: int):
+    """(chunks, runs that are cut into chunks, whether others are left) of a step whose long runs go chunk by chunk.  From the
+    host's copy of the runs' lengths where the step has one, else the most that T tokens of so many requests can be."""
+    first, size, B = lib.chunk_from, lib.chunk_tokens, step.num_requests
+    if T < first:
+        return 0, 0, True
+    lens = getattr(step, "q_lens", None)
+    if lens is not None and len(lens) == B:
+        long = [n for n in lens if n >= first]
+        return sum(-(-n // size) for n in long), len(long), len(long) < B
+    runs = min(B, T // first)
+    return T // size + runs, runs, True
 
 
 def short_conv_silu(x: torch.Tensor, taps: torch.Tensor, state: torch.Tensor, step, update_state: bool = True) -> torch.Tensor:
@@ -1128,7 +1144,12 @@ def gated_delta_scan(q, k, v, beta, step_pre, step_bias, rate_log, state, step, 
     gate_code = {"sigmoid": 0, "silu": 1}[gate_activation]
     assert state.shape[1] == heads * dk * dv and out.shape == (q.shape[0], heads * dv) and out.stride(1) == 1
     lib = recurrent()
-    scratch = _scan_scratch(q.shape[0], step.num_requests, heads, dv, q.shape[0] * (2 * kv_heads * dk + heads * dk + heads), q.device)
+    chunks, runs, rest = _chunked_runs(lib, step, q.shape[0])
+    floats = int(lib.coheryn_delta_chunk_floats(c_int(chunks), c_int(heads), c_int(dk), c_int(dv))) if chunks else 0
+    if floats:
+        scratch = torch.empty(floats, dtype=torch.float32, device=q.device)
+    else:
+        scratch = _scan_scratch(q.shape[0], step.num_requests, heads, dv, q.shape[0] * (2 * kv_heads * dk + heads * dk + heads), q.device)
     _check(lib, lib.coheryn_gated_delta_scan(
         _ptr(q), _ptr(k), _ptr(v), c_long(q.stride(0)), _ptr(beta), c_long(beta.stride(0)), _ptr(step_pre),
         c_long(step_pre.stride(0)), _ptr(step_bias), c_int(_code(step_bias)), _ptr(rate_log), c_int(_code(rate_log)),
@@ -1136,7 +1157,7 @@ def gated_delta_scan(q, k, v, beta, step_pre, step_bias, rate_log, state, step, 
         c_int(heads), c_int(kv_heads), c_int(dk), c_int(dv), _ptr(out), c_int(_code(out)), c_long(out.stride(0)),
         _ptr(norm_weight), c_int(_code(norm_weight)), c_int(0), _ptr(gate), c_long(gate.stride(0)), c_float(eps),
         c_float(out_scale), c_int(q.shape[0]), _ptr(scratch), c_long(scratch.numel() if scratch is not None else 0),
-        c_int(dc), c_int(gate_code), _stream()))
+        c_int(dc), c_int(gate_code), c_int(chunks if floats else 0), c_int(runs), c_int(1 if rest else 0), _stream()))
 
 
 def matrix_memory_scan(q, k, v, gate_i, gate_f, bias_i, bias_f, cap: float, state, step, heads: int, dk: int, dv: int,

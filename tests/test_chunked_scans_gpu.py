@@ -1,0 +1,125 @@
+"""The gated delta rule in chunks of 64 tokens (csrc/delta_chunks.cu) against the recurrence written token by token in float64,
+at the edges of the runs it takes, of its chunks, blocks and tiles, and beside runs that stay with the scan."""
+import types
+
+import numpy as np
+import pytest
+import torch
+
+import plain_kapudra as plain
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+
+def dev(a, dtype=torch.float32):
+    return torch.as_tensor(np.asarray(a)).to(DEV, dtype)
+
+
+def step_of(lengths, slots, host=True):
+    cu = np.concatenate([[0], np.cumsum(lengths)])
+    st = types.SimpleNamespace(num_requests=len(lengths), num_tokens=int(cu[-1]), cu_q=dev(cu, torch.int32),
+                               token_req=dev(np.repeat(np.arange(len(lengths)), lengths), torch.int32), state_slots=dev(slots, torch.int32))
+    if host:
+        st.q_lens = list(lengths)
+    return st
+
+
+def delta_inputs(rng, n, heads, groups, dk, dv, channel):
+    f = lambda *s: rng.normal(size=s)
+    return dict(q=f(n, groups * dk), k=f(n, groups * dk), v=f(n, heads * dv), beta=f(n, heads), step=f(n, heads * (dk if channel else 1)),
+                gate=f(n, heads * dv))
+
+
+def run_delta(parts, state, slots, bias, rate_log, weight, heads, groups, dk, dv, channel, act, host):
+    from coheryn_ai_studio_b200 import ops
+    cat = lambda key: dev(np.concatenate([d[key] for d in parts]))
+    step = step_of([len(d["q"]) for d in parts], slots, host)
+    qkv, G = torch.cat([cat("q"), cat("k"), cat("v")], dim=1), groups * dk
+    out = torch.empty((step.num_tokens, heads * dv), device=DEV)
+    ops.gated_delta_scan(qkv[:, :G], qkv[:, G:2 * G], qkv[:, 2 * G:], cat("beta"), cat("step"), dev(bias), dev(rate_log), state, step, heads,
+                         groups, dk, dv, out, dev(weight), cat("gate"), 1e-5, decay_per_channel=channel, gate_activation=act)
+    return out.cpu().numpy()
+
+
+# The bounds are those of the token-by-token kernel's own test (2e-4 of the largest value): the chunks add the same float32
+# products in another order.
+@pytest.mark.parametrize("lens", [[47, 48], [64, 2, 65], [130, 1, 63], [257]])
+@pytest.mark.parametrize("heads,groups,dk,dv,channel,act,host", [
+    (4, 2, 20, 30, True, "sigmoid", True), (2, 1, 64, 64, False, "silu", True), (2, 2, 65, 72, True, "silu", False),
+    (2, 1, 128, 128, True, "sigmoid", True), (1, 1, 128, 256, False, "sigmoid", False), (3, 1, 96, 144, True, "sigmoid", True)])
+def test_gated_delta_rule_in_chunks(lens, heads, groups, dk, dv, channel, act, host):
+    rng = np.random.default_rng(dk + dv + lens[0])
+    parts = [delta_inputs(rng, n, heads, groups, dk, dv, channel) for n in lens]
+    dc = dk if channel else 1
+    # decays from nearly one to nothing: a chunk's product leaves float32's range in some channels and not in others
+    bias, rate_log, weight = rng.uniform(-7, 3, size=heads * dc), rng.normal(size=heads), rng.normal(size=dv)
+    slots = list(rng.permutation(len(lens) + 1)[:len(lens)])
+    first = rng.normal(size=(len(lens) + 1, heads * dk * dv)) * 0.1
+    state = dev(first)
+    got = run_delta(parts, state, slots, bias, rate_log, weight, heads, groups, dk, dv, channel, act, host)
+    after, at = state.cpu().numpy(), 0
+    for d, slot in zip(parts, slots):
+        n = len(d["q"])
+        q = d["q"].reshape(n, groups, dk); k = d["k"].reshape(n, groups, dk)
+        q = q / np.sqrt((q * q).sum(-1, keepdims=True) + 1e-6) * dk ** -0.5
+        k = k / np.sqrt((k * k).sum(-1, keepdims=True) + 1e-6)
+        decay = np.exp(-np.exp(rate_log)[None, :, None] * plain.softplus(d["step"] + bias).reshape(n, heads, dc))
+        o = np.zeros((n, heads, dv))
+        for h in range(heads):
+            S, g = first[slot].reshape(heads, dk, dv)[h].copy(), h // (heads // groups)
+            for t in range(n):
+                S = decay[t, h][:, None] * S
+                u = plain.sigmoid(d["beta"][t, h]) * (d["v"].reshape(n, heads, dv)[t, h] - S.T @ k[t, g])
+                S = S + np.outer(k[t, g], u)
+                o[t, h] = S.T @ q[t, g]
+            end = after[slot].reshape(heads, dk, dv)[h]
+            assert np.abs(end - S).max() <= 2e-4 * max(1.0, np.abs(S).max()), (slot, h)
+        z = d["gate"].reshape(n, heads, dv)
+        want = (plain.rms(o, 1e-5) * weight * plain.sigmoid(z) * (z if act == "silu" else 1.0)).reshape(n, heads * dv)
+        assert np.abs(got[at:at + n] - want).max() <= 2e-4 * max(1.0, np.abs(want).max()), slot
+        at += n
+    untouched = [s for s in range(len(lens) + 1) if s not in slots]
+    assert np.array_equal(after[untouched], dev(first[untouched]).cpu().numpy())
+
+
+def test_a_runs_rows_do_not_depend_on_the_other_runs():
+    """Bit for bit: alone, beside a run that goes chunk by chunk and beside one that goes token by token."""
+    rng = np.random.default_rng(5)
+    heads, groups, dk, dv = 2, 1, 64, 48
+    parts = [delta_inputs(rng, n, heads, groups, dk, dv, True) for n in (100, 9, 47, 64)]
+    bias, rate_log, weight = rng.normal(size=heads * dk), rng.normal(size=heads), rng.normal(size=dv)
+    args = (bias, rate_log, weight, heads, groups, dk, dv, True, "sigmoid", True)
+    state = torch.zeros((4, heads * dk * dv), device=DEV)
+    both, at = run_delta(parts, state, [2, 0, 3, 1], *args), 0
+    for d in parts:
+        n = len(d["q"])
+        alone = run_delta([d], torch.zeros((1, heads * dk * dv), device=DEV), [0], *args)
+        assert np.array_equal(alone, both[at:at + n]), n
+        at += n
+
+
+@pytest.mark.parametrize("taps,channels,offset", [(2, 40, 0), (3, 36, 3), (4, 1028, 4), (4, 130, 1), (5, 24, 0)])
+def test_short_convolution_by_runs_of_tokens(taps, channels, offset):
+    """Runs shorter and longer than the taps and than a thread's tokens, aligned and unaligned columns, states of strided rows."""
+    from coheryn_ai_studio_b200 import ops
+    rng = np.random.default_rng(taps + channels)
+    lens = [1, 2, 40, 3, 17]
+    n = sum(lens)
+    wide = dev(rng.normal(size=(n, channels + 12)))
+    x = wide[:, offset:offset + channels]
+    w = dev(rng.normal(size=(channels, taps)))
+    keep = taps - 1
+    state = dev(rng.normal(size=(6, 8 + keep * channels)))[:, 8:]
+    slots = [4, 0, 5, 2, 1]
+    before = state.double().cpu().numpy().reshape(6, keep, channels)
+    y = ops.short_conv_silu(x, w, state, step_of(lens, slots)).double().cpu().numpy()
+    xs, ws, at = x.double().cpu().numpy(), w.double().cpu().numpy(), 0
+    after = state.cpu().numpy().reshape(6, keep, channels)
+    for m, slot in zip(lens, slots):
+        rows = np.concatenate([before[slot], xs[at:at + m]])
+        want = plain.silu(sum(rows[j:j + m] * ws[:, j] for j in range(taps)))
+        # a sum of `taps` products and the activation in float32
+        assert np.abs(y[at:at + m] - want).max() <= 1e-5 * max(1.0, np.abs(want).max())
+        assert np.array_equal(after[slot], rows[-keep:].astype(np.float32))
+        at += m
