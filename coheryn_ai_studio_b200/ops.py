@@ -1071,7 +1071,7 @@ def recurrent():
     global _recurrent
     if _recurrent is None:
         lib = build.recurrent_library()
-        lib.coheryn_delta_chunk_floats.restype = ctypes.c_long
+        lib.coheryn_delta_chunk_floats.restype = lib.coheryn_memory_chunk_floats.restype = ctypes.c_long
         lib.chunk_from, lib.chunk_tokens = int(lib.coheryn_chunk_from()), int(lib.coheryn_chunk_tokens())
         lib.coheryn_last_error.restype = ctypes.c_char_p
         lib.coheryn_launch_count.restype = ctypes.c_ulonglong
@@ -1176,14 +1176,16 @@ def matrix_memory_scan(q, k, v, gate_i, gate_f, bias_i, bias_f, cap: float, stat
     assert norm_weight.numel() == heads * dv
     assert state.shape[1] == heads * (dk * dv + dk + 1) and out.shape == (q.shape[0], heads * dv) and out.stride(1) == 1
     lib = recurrent()
-    scratch = _scan_scratch(q.shape[0], step.num_requests, heads, dv, step.num_requests * heads * (dk + 1), q.device)
+    chunks, runs, rest = _chunked_runs(lib, step, q.shape[0])
+    floats = int(lib.coheryn_memory_chunk_floats(c_int(chunks), c_int(heads), c_int(dk), c_int(dv))) if chunks else 0
+    scratch = torch.empty(floats, dtype=torch.float32, device=q.device) if floats else None
     _check(lib, lib.coheryn_matrix_memory_scan(
         _ptr(q), _ptr(k), _ptr(v), c_long(q.stride(0)), _ptr(gate_i), _ptr(gate_f), c_long(gate_i.stride(0)), _ptr(bias_i),
         _ptr(bias_f), c_int(_code(bias_i)), c_float(cap), _ptr(state), c_long(state.stride(0)), _ptr(step.cu_q),
         _ptr(step.state_slots), c_int(step.num_requests), c_int(heads), c_int(dk), c_int(dv), _ptr(out), c_int(_code(out)),
         c_long(out.stride(0)), _ptr(norm_weight), c_int(_code(norm_weight)), c_int(dv), _ptr(gate), c_long(gate.stride(0)),
-        c_float(eps), c_float(out_scale), c_int(q.shape[0]), _ptr(scratch), c_long(scratch.numel() if scratch is not None else 0),
-        _stream()))
+        c_float(eps), c_float(out_scale), _ptr(scratch), c_long(floats),
+        c_int(chunks if floats else 0), c_int(runs), c_int(1 if rest else 0), _stream()))
 
 
 def qk_norm_kv_write(q, k, v, q_weight, k_weight, eps: float, slots, k_cache, v_cache, num_heads: int, num_kv_heads: int,

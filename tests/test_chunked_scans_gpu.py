@@ -1,4 +1,4 @@
-"""The gated delta rule in chunks of 64 tokens (csrc/delta_chunks.cu) against the recurrence written token by token in float64,
+"""The gated delta rule and the matrix memory in chunks of 64 tokens (csrc/delta_chunks.cu, csrc/memory_chunks.cu) against the recurrences written token by token in float64,
 at the edges of the runs it takes, of its chunks, blocks and tiles, and beside runs that stay with the scan."""
 import types
 
@@ -123,3 +123,49 @@ def test_short_convolution_by_runs_of_tokens(taps, channels, offset):
         assert np.abs(y[at:at + m] - want).max() <= 1e-5 * max(1.0, np.abs(want).max())
         assert np.array_equal(after[slot], rows[-keep:].astype(np.float32))
         at += m
+
+
+# The bound is that of the token-by-token kernel's own test: a float32 recurrence is itself up to 5e-4 from float64 where a row's
+# output nearly cancels before its norm.
+@pytest.mark.parametrize("lens", [[47, 48], [64, 2, 65], [130, 1, 63], [257]])
+@pytest.mark.parametrize("heads,dk,dv,cap,open_gate,host", [
+    (3, 20, 30, 9.0, False, True), (2, 64, 128, 15.0, True, True), (2, 72, 130, 8.0, False, False), (1, 128, 256, 15.0, True, False),
+    (1, 256, 144, 12.0, False, True)])
+def test_matrix_memory_in_chunks(lens, heads, dk, dv, cap, open_gate, host):
+    from coheryn_ai_studio_b200 import ops
+    rng = np.random.default_rng(dk + dv + lens[0])
+    f = lambda *s: rng.normal(size=s)
+    parts = [dict(q=f(n, heads * dk), k=f(n, heads * dk), v=f(n, heads * dv), gi=f(n, heads) * 3, gf=f(n, heads) * 3 + (6.0 if open_gate else -6.0),
+                  gate=f(n, heads * dv)) for n in lens]       # forget gates held open, or shut: exponents from 0 to hundreds in a chunk
+    bi, bf, weight = f(heads), f(heads), f(heads * dv)
+    size = heads * (dk * dv + dk + 1)
+    slots = list(rng.permutation(len(lens) + 1)[:len(lens)])
+    first = f(len(lens) + 1, size) * 0.3
+    state, step = dev(first), step_of(lens, slots, host)
+    cat = lambda key: dev(np.concatenate([d[key] for d in parts]))
+    qkv, gates = torch.cat([cat("q"), cat("k"), cat("v")], dim=1), torch.cat([cat("gi"), cat("gf")], dim=1)
+    out = torch.empty((step.num_tokens, heads * dv), device=DEV)
+    ops.matrix_memory_scan(qkv[:, :heads * dk], qkv[:, heads * dk:2 * heads * dk], qkv[:, 2 * heads * dk:], gates[:, :heads], gates[:, heads:],
+                           dev(bi), dev(bf), cap, state, step, heads, dk, dv, out, dev(weight), cat("gate"), 1e-5)
+    got, after, at = out.cpu().numpy(), state.cpu().numpy(), 0
+    for d, slot in zip(parts, slots):
+        n = len(d["q"])
+        li = cap * np.tanh((d["gi"] + bi) / cap)
+        lf = plain.log_sigmoid(cap * np.tanh((d["gf"] + bf) / cap))
+        o = np.zeros((n, heads, dv))
+        for h in range(heads):
+            S = first[slot][:heads * dk * dv].reshape(heads, dk, dv)[h].copy()
+            nn = first[slot][heads * dk * dv:heads * dk * (dv + 1)].reshape(heads, dk)[h].copy()
+            m = first[slot][heads * dk * (dv + 1) + h]
+            q, k, v = d["q"].reshape(n, heads, dk)[:, h] * dk ** -0.5, d["k"].reshape(n, heads, dk)[:, h], d["v"].reshape(n, heads, dv)[:, h]
+            for t in range(n):
+                m_new = max(lf[t, h] + m, li[t, h])
+                a, b, m = np.exp(lf[t, h] + m - m_new), np.exp(li[t, h] - m_new), m_new
+                S, nn = a * S + b * np.outer(k[t], v[t]), a * nn + b * k[t]
+                o[t, h] = (S.T @ q[t]) / (max(abs(nn @ q[t]), np.exp(-m)) + 1e-6)
+            assert np.abs(after[slot][:heads * dk * dv].reshape(heads, dk, dv)[h] - S).max() <= 2e-4 * max(1.0, np.abs(S).max())
+            assert np.abs(after[slot][heads * dk * dv:heads * dk * (dv + 1)].reshape(heads, dk)[h] - nn).max() <= 2e-4 * max(1.0, np.abs(nn).max())
+            assert abs(after[slot][heads * dk * (dv + 1) + h] - m) <= 2e-5 * max(1.0, abs(m))
+        want = plain.rms(o, 1e-5).reshape(n, heads * dv) * weight * plain.sigmoid(d["gate"])
+        assert np.abs(got[at:at + n] - want).max() <= 1e-3 * max(1.0, np.abs(want).max()), slot
+        at += n
