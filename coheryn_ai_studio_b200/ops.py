@@ -44,6 +44,7 @@ def core():
         lib.coheryn_launch_count.restype = ctypes.c_ulonglong
         lib.coheryn_argmax_scratch_slots.restype = ctypes.c_long
         lib.coheryn_gemm_tc_workspace_floats.restype = ctypes.c_long
+        lib.coheryn_gemm_simt_workspace_floats.restype = ctypes.c_long
         _core = lib
     return _core
 
@@ -467,6 +468,11 @@ def qkv_rope_parts(x: torch.Tensor, w_qkv: torch.Tensor, b_qkv: Optional[torch.T
     return q
 
 
+@functools.lru_cache(maxsize=4096)
+def _simt_workspace_floats(M: int, N: int, K: int) -> int:
+    return int(core().coheryn_gemm_simt_workspace_floats(c_int(M), c_int(N), c_int(K)))
+
+
 def gemm_simt(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor], out: torch.Tensor, act: int = 0) -> None:
     """out = x @ w.T (+ bias), passed through the plain activation ``act`` (see ``PLAIN_ACTIVATIONS``), with float32 FMA
     accumulation (no tensor cores)."""
@@ -478,10 +484,12 @@ def gemm_simt(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor], ou
     if bias is not None:
         assert bias.shape == (N,) and bias.is_contiguous()
     lib = core()
+    floats = _simt_workspace_floats(M, N, K)      # > 0: K is shared out over CTAs
+    workspace = torch.empty(floats, dtype=torch.float32, device=x.device) if floats else None
     _check(lib, lib.coheryn_gemm_simt(
         _ptr(x), c_int(_code(x)), _ptr(w), c_int(_code(w)), _ptr(bias),
         c_int(_code(bias) if bias is not None else F32), _ptr(out), c_int(_code(out)), c_int(M),
-        c_int(N), c_int(K), c_long(x.stride(0)), c_long(out.stride(0)), c_int(act), _stream()))
+        c_int(N), c_int(K), c_long(x.stride(0)), c_long(out.stride(0)), c_int(act), _ptr(workspace), c_long(floats), _stream()))
 
 
 def attention_simple(q: torch.Tensor, out: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor,
