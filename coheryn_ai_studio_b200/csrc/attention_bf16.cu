@@ -1069,13 +1069,13 @@ CO_EXPORT long coheryn_attn_scratch_floats(int B, int nkv, int max_kv_len) {
 
 // q: [T, nh*HD] rows of stride q_stride; out likewise.  Caches: [page][kv head][slot][HD].
 // cu_q [B+1], kv_lens [B] on the device.  Host hints: max_rows = the largest q_len*G of the
-// batch, any_small / any_large = whether some request has <= 16 / > 16 rows, max_kv_len,
+// batch, any_small = whether some request has <= 16 rows, large = how many have > 16 (at most), max_kv_len,
 // total_tokens = T, num_pages = pages per cache tensor; settled = whether the positions before each
 // request's new tokens were written by EARLIER steps (the decode kernel then reads them ahead of time).
 CO_EXPORT int coheryn_attention_bf16(const void* q, long q_stride, void* out, long out_stride, const void* k_cache,
                                      const void* v_cache, const int* block_tables, int max_blocks, const int* cu_q,
                                      const int* kv_lens, int B, int nh, int nkv, int page_size, int window,
-                                     float scale, int max_rows, int any_small, int any_large, int max_kv_len,
+                                     float scale, int max_rows, int any_small, int large, int max_kv_len,
                                      float* scratch, long scratch_floats, int* status, int total_tokens,
                                      int num_pages, int settled, cudaStream_t stream) {
   if (B <= 0) return 0;
@@ -1090,12 +1090,12 @@ CO_EXPORT int coheryn_attention_bf16(const void* q, long q_stride, void* out, lo
   (void)status;
   const bool split_path = any_small && G <= 16 &&
                           (max_kv_len + SPLIT_MIN - 1) / SPLIT_MIN + 1 <= 512;   // attn_combine keeps 512 factors
-  if (any_large || (any_small && !split_path)) {
+  if (large || (any_small && !split_path)) {
     // Prompt portions: the tcgen05 kernel where it takes the shape, else the mma.sync one.
     if (!t_slopes_log2 && status && coheryn_attention_tc_takes(nh, nkv, page_size) && ((uintptr_t)out & 7) == 0) {
       if (coheryn_attention_tc_launch(q, q_stride, total_tokens, out, out_stride, k_cache, v_cache, num_pages, block_tables,
                                       max_blocks, cu_q, kv_lens, B, nh, nkv, page_size, window, scale_log2, max_rows, max_kv_len,
-                                      split_path ? 1 : 0, status, stream))
+                                      split_path ? 1 : 0, split_path ? large : B, status, stream))
         return -1;
     } else {
       static bool configured = false;
@@ -1122,12 +1122,12 @@ CO_EXPORT int coheryn_attention_bf16(const void* q, long q_stride, void* out, lo
 CO_EXPORT int coheryn_attention_bf16_biased(const void* q, long q_stride, void* out, long out_stride, const void* k_cache,
                                             const void* v_cache, const int* block_tables, int max_blocks, const int* cu_q,
                                             const int* kv_lens, int B, int nh, int nkv, int page_size, int window,
-                                            float scale, int max_rows, int any_small, int any_large, int max_kv_len,
+                                            float scale, int max_rows, int any_small, int large, int max_kv_len,
                                             float* scratch, long scratch_floats, int* status, int total_tokens,
                                             int num_pages, int settled, const float* slopes_log2, cudaStream_t stream) {
   t_slopes_log2 = slopes_log2;
   const int rc = coheryn_attention_bf16(q, q_stride, out, out_stride, k_cache, v_cache, block_tables, max_blocks, cu_q, kv_lens,
-                                        B, nh, nkv, page_size, window, scale, max_rows, any_small, any_large, max_kv_len,
+                                        B, nh, nkv, page_size, window, scale, max_rows, any_small, large, max_kv_len,
                                         scratch, scratch_floats, status, total_tokens, num_pages, settled, stream);
   t_slopes_log2 = nullptr;
   return rc;

@@ -145,6 +145,21 @@ __device__ __forceinline__ void load_box(void* dst, const CUtensorMap* map, int 
   if constexpr (OPTIONS) tma_load_3d(dst, map, col, row, opt.dense ? kvh : 0, full);
   else tma_load_2d(dst, map, col, row, full);
 }
+// The request that stands at place `want` among those of more than `skip_rows` rows per kv head (-1: there are not so many).
+// A mixed step holds a few portions of prompts among many one-token requests: a grid over all requests times the row tiles of
+// the longest would be mostly CTAs that start, find nothing and leave, at one CTA of this size per SM.  Measured on a B200
+// (28 heads in 4 groups, portions of 1,337, 403 and 96 tokens beside 37 one-token requests): 128 -> 66 us.
+__device__ __forceinline__ int nth_request(const int* cu_q, int n_req, int G, int skip_rows, int want) {
+  const int lane = threadIdx.x & 31;
+  for (int r0 = 0; r0 < n_req; r0 += 32) {
+    const int r = r0 + lane;
+    const unsigned mask = __ballot_sync(0xffffffffu, r < n_req && (cu_q[min(r, n_req - 1) + 1] - cu_q[min(r, n_req - 1)]) * G > skip_rows);
+    const int n = __popc(mask);
+    if (want < n) return r0 + (int)__fns(mask, 0, want + 1);
+    want -= n;
+  }
+  return -1;
+}
 constexpr int XLD = VDP + 4;                      // row stride (floats) of a CTA's published accumulator
 constexpr int MAX_CLUSTER = 8;
 static_assert(!SUPPORTED || (size_t)(128 * XLD + 256) * 4 <= (size_t)Q_BYTES + (size_t)NST * (K_BYTES + V_BYTES), "a published accumulator fits the tiles");
@@ -154,8 +169,8 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
                const __grid_constant__ CUtensorMap map_v, bf16* __restrict__ out, long out_stride,
                const int* __restrict__ block_tables, int max_blocks, const int* __restrict__ cu_q,
                const int* __restrict__ kv_lens, int nh, int nkv, int page_size, int cache_rows, int window,
-               float scale_log2, int skip_rows, int rows_per_box, int* __restrict__ status, int n_req, int n_units,
-               AttnOptions opt) {
+               float scale_log2, int skip_rows, int rows_per_box, int* __restrict__ status, int n_req, int n_listed,
+               int n_units, AttnOptions opt) {
   extern __shared__ unsigned char smem_raw[];
   unsigned char* tiles = (unsigned char*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   unsigned char* q_s = tiles;                                   // [KCH][128 rows][128 B]
@@ -196,12 +211,14 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
   // in the order of their index).  The CTAs of a cluster (consecutive indices) share a row tile and
   // split its key tiles among them; the last one merges.
   const int csize = (int)cluster_size(), crank = (int)cluster_rank();
-  const int unit = (int)(blockIdx.x / csize), heads_reqs = nkv * n_req;
-  const int b = (unit % heads_reqs) / nkv, kvh = unit % nkv, rt = n_units - 1 - unit / heads_reqs;
+  const int unit = (int)(blockIdx.x / csize), heads_reqs = nkv * n_listed;
+  const int kvh = unit % nkv, rt = n_units - 1 - unit / heads_reqs;
   const int G = nh / nkv, TOK = 128 / G, RT = TOK * G;
+  const int place = (unit % heads_reqs) / nkv, listed = n_listed < n_req ? nth_request(cu_q, n_req, G, skip_rows, place) : place;
+  const int b = max(listed, 0);
   const int tok0 = cu_q[b], q_len = cu_q[b + 1] - tok0, kv_len = kv_lens[b];
   const int rows = q_len * G;
-  const bool active = rt * RT < rows && rows > skip_rows;
+  const bool active = listed >= 0 && rt * RT < rows && rows > skip_rows;
   const int base_pos = kv_len - q_len;
   const int row_first = rt * RT, row_last = min(rows, row_first + RT) - 1;
   const int pos_lo = base_pos + row_first / G, pos_hi = base_pos + row_last / G;
@@ -515,8 +532,8 @@ attn_tc2_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
                 const __grid_constant__ CUtensorMap map_v, bf16* __restrict__ out, long out_stride,
                 const int* __restrict__ block_tables, int max_blocks, const int* __restrict__ cu_q,
                 const int* __restrict__ kv_lens, int nh, int nkv, int page_size, int cache_rows, int window,
-                float scale_log2, int skip_rows, int rows_per_box, int* __restrict__ status, int n_req, int n_units,
-               AttnOptions opt) {
+                float scale_log2, int skip_rows, int rows_per_box, int* __restrict__ status, int n_req, int n_listed,
+               int n_units, AttnOptions opt) {
   extern __shared__ unsigned char smem_raw[];
   unsigned char* tiles = (unsigned char*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   unsigned char* q_s = tiles;                                   // [tile][KCH][128 rows][128 B]
@@ -556,12 +573,14 @@ attn_tc2_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
 
   // Late rows see the most keys: their pairs of tiles are started first, for all (request, kv head)
   // pairs before any earlier pair of tiles (one-dimensional grid, the pair of tiles its slowest index).
-  const int unit = (int)blockIdx.x, heads_reqs = nkv * n_req;
-  const int b = (unit % heads_reqs) / nkv, kvh = unit % nkv, pair = n_units - 1 - unit / heads_reqs;
+  const int unit = (int)blockIdx.x, heads_reqs = nkv * n_listed;
+  const int kvh = unit % nkv, pair = n_units - 1 - unit / heads_reqs;
   const int G = nh / nkv, TOK = 128 / G, RT = TOK * G;
+  const int place = (unit % heads_reqs) / nkv, listed = n_listed < n_req ? nth_request(cu_q, n_req, G, skip_rows, place) : place;
+  const int b = max(listed, 0);
   const int tok0 = cu_q[b], q_len = cu_q[b + 1] - tok0, kv_len = kv_lens[b];
   const int rows = q_len * G;
-  const bool active_a = 2 * pair * RT < rows && rows > skip_rows;
+  const bool active_a = listed >= 0 && 2 * pair * RT < rows && rows > skip_rows;
   const bool active_b = active_a && (2 * pair + 1) * RT < rows;
   const int base_pos = kv_len - q_len;
   const int first_a = 2 * pair * RT, first_b = first_a + RT;
@@ -830,12 +849,13 @@ bool coheryn_attention_tc_takes(int nh, int nkv, int page_size) {
   return page_size >= 8 && (BN % page_size == 0 || page_size % BN == 0);   // a box is whole pages of >= 1024 bytes
 }
 
-// The launch behind both interfaces.  skip_rows: requests with at most this many rows per kv head are left out.
+// The launch behind both interfaces.  skip_rows: requests with at most this many rows per kv head are left out; n_listed: how
+// many are not (at most).
 static int attention_tc_launch(const void* q, long q_stride, int total_tokens, void* out, long out_stride,
                                 const void* k_cache, const void* v_cache, int num_pages, const int* block_tables,
                                 int max_blocks, const int* cu_q, const int* kv_lens, int B, int nh, int nkv,
                                 int page_size, int window, float scale_log2, int max_rows, int max_kv_len, int skip_rows,
-                                int* status, const AttnOptions& opt, cudaStream_t stream) {
+                                int n_listed, int* status, const AttnOptions& opt, cudaStream_t stream) {
   if (!SUPPORTED) CO_FAIL("attention_tc: head sizes %d and %d are not built", HD, VD);
   const int G = nh / nkv, TOK = 128 / G, RT = TOK * G;
   const int rows_per_box = opt.dense || page_size >= BN ? BN : page_size;
@@ -870,7 +890,10 @@ static int attention_tc_launch(const void* q, long q_stride, int total_tokens, v
   // CTA's fixed cost is several key tiles' worth, so a batch that fills the GPU stays unsplit.
   // COHERYN_ATTN_TC_CLUSTER in the environment or coheryn_attention_tc_set_cluster fixes it.
   const int row_tiles = (max_rows + RT - 1) / RT;
-  const long ctas = (long)row_tiles * nkv * B;
+  if (n_listed < 1 || n_listed > B) n_listed = B;
+  // how many of the grid's CTAs have a row tile: no more than the step's rows make
+  const long most = ((long)total_tokens * G + RT - 1) / RT + n_listed;
+  const long ctas = nkv * ((long)row_tiles * n_listed < most ? (long)row_tiles * n_listed : most);
   const int key_tiles = (max_kv_len + BN - 1) / BN;
   if (g_forced_cluster < 0) g_forced_cluster = getenv("COHERYN_ATTN_TC_CLUSTER") ? atoi(getenv("COHERYN_ATTN_TC_CLUSTER")) : 0;
   const int forced = g_forced_cluster;
@@ -884,7 +907,8 @@ static int attention_tc_launch(const void* q, long q_stride, int total_tokens, v
   // A portion at the end of a long context has few row tiles and many key tiles each; there the pairs
   // pay from somewhat over half the SMs on (2,048 tokens after 14,336: 98 CTAs, 331 against 405 us;
   // 40 heads in 8 groups, 512 tokens after 15,872: 88 CTAs, 326 against 448; but 60 CTAs: 317 against 227).
-  const long pair_ctas = (long)((row_tiles + 1) / 2) * nkv * B;
+  const long most_pairs = ((long)total_tokens * G + 2 * RT - 1) / (2 * RT) + n_listed, grid_pairs = (long)((row_tiles + 1) / 2) * n_listed;
+  const long pair_ctas = nkv * (grid_pairs < most_pairs ? grid_pairs : most_pairs);
   const bool pairs_pay = pair_ctas >= 185 || (pair_ctas >= 84 && key_tiles >= 48);
   if (TWO_OK && cluster == 1 && row_tiles >= 2 && (g_two_tiles == 1 || (g_two_tiles == 2 && pairs_pay))) {
     static bool configured2 = false;
@@ -894,20 +918,21 @@ static int attention_tc_launch(const void* q, long q_stride, int total_tokens, v
       configured2 = true;
     }
     const int pairs = (row_tiles + 1) / 2;
-    if (pair_ctas >= (1L << 31)) CO_FAIL("attention_tc: %ld CTAs", pair_ctas);
-    dim3 grid2((unsigned)pair_ctas);
+    if (grid_pairs * nkv >= (1L << 31)) CO_FAIL("attention_tc: %ld CTAs", grid_pairs * nkv);
+    dim3 grid2((unsigned)(grid_pairs * nkv));
     cudaError_t le2 = co_launch(attn_tc2_kernel, grid2, dim3(320), (size_t)SMEM2_BYTES, stream, mq, mk, mv, (bf16*)out, out_stride,
                                 block_tables, max_blocks, cu_q, kv_lens, nh, nkv, page_size, (int)cache_rows, window, scale_log2,
-                                skip_rows, rows_per_box, status, B, pairs, opt);
+                                skip_rows, rows_per_box, status, B, n_listed, pairs, opt);
     if (le2 != cudaSuccess) CO_FAIL("attention_tc: launch failed: %s", cudaGetErrorString(le2));
     CO_CHECK_LAUNCH("attn_tc2");
     return 0;
   }
-  if (ctas * cluster >= (1L << 31)) CO_FAIL("attention_tc: %ld CTAs", ctas * cluster);
-  dim3 grid((unsigned)(ctas * cluster));
+  const long grid_ctas = (long)row_tiles * n_listed * nkv * cluster;
+  if (grid_ctas >= (1L << 31)) CO_FAIL("attention_tc: %ld CTAs", grid_ctas);
+  dim3 grid((unsigned)grid_ctas);
   cudaError_t le = co_launch_cluster(cluster, attn_tc_kernel, grid, dim3(320), (size_t)SMEM_BYTES, stream, mq, mk, mv, (bf16*)out,
                                      out_stride, block_tables, max_blocks, cu_q, kv_lens, nh, nkv, page_size, (int)cache_rows,
-                                     window, scale_log2, skip_rows, rows_per_box, status, B, row_tiles, opt);
+                                     window, scale_log2, skip_rows, rows_per_box, status, B, n_listed, row_tiles, opt);
   if (le != cudaSuccess) CO_FAIL("attention_tc: launch failed: %s", cudaGetErrorString(le));
   CO_CHECK_LAUNCH("attn_tc");
   return 0;
@@ -918,10 +943,10 @@ int coheryn_attention_tc_launch(const void* q, long q_stride, int total_tokens, 
                                 const void* k_cache, const void* v_cache, int num_pages, const int* block_tables,
                                 int max_blocks, const int* cu_q, const int* kv_lens, int B, int nh, int nkv,
                                 int page_size, int window, float scale_log2, int max_rows, int max_kv_len, int skip_small,
-                                int* status, cudaStream_t stream) {
+                                int n_listed, int* status, cudaStream_t stream) {
   return attention_tc_launch(q, q_stride, total_tokens, out, out_stride, k_cache, v_cache, num_pages, block_tables, max_blocks,
                              cu_q, kv_lens, B, nh, nkv, page_size, window, scale_log2, max_rows, max_kv_len, skip_small ? 16 : 0,
-                             status, AttnOptions{}, stream);
+                             n_listed, status, AttnOptions{}, stream);
 }
 #else
 CO_EXPORT void coheryn_attention_options_shape(int* dk, int* dv) { *dk = HD; *dv = VD; }
@@ -949,7 +974,7 @@ CO_EXPORT int coheryn_attention_options(const void* q, long q_stride, int total_
   if (!status) CO_FAIL("attention_options: a status word is required");
   const AttnOptions opt{keep, dense, sink, sink_scores, gates, gates_ld, factor};
   return attention_tc_launch(q, q_stride, total_tokens, out, out_stride, k_cache, v_cache, num_pages, block_tables, max_blocks, cu_q,
-                             kv_lens, B, nh, nkv, page_size, window, scale * 1.4426950408889634f, max_rows, max_kv_len, nh / nkv, status,
+                             kv_lens, B, nh, nkv, page_size, window, scale * 1.4426950408889634f, max_rows, max_kv_len, nh / nkv, B, status,
                              opt, stream);
 }
 #endif

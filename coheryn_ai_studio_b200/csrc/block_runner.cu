@@ -54,7 +54,7 @@ int coheryn_gemm_bf16_tc_few(const void* x, const void* w, const void* bias, int
 typedef int (*co_attention_fn)(const void* q, long q_stride, void* out, long out_stride, const void* k_cache,
                                const void* v_cache, const int* block_tables, int max_blocks, const int* cu_q,
                                const int* kv_lens, int B, int nh, int nkv, int page_size, int window, float scale,
-                               int max_rows, int any_small, int any_large, int max_kv_len, float* scratch,
+                               int max_rows, int any_small, int large, int max_kv_len, float* scratch,
                                long scratch_floats, int* status, int total_tokens, int num_pages, int settled,
                                cudaStream_t stream);
 typedef int (*co_attention_oproj_fn)(const void* q, long q_stride, const void* k_cache, const void* v_cache,
@@ -84,6 +84,7 @@ struct CoBlockStep {
   int* tc_status;
   cudaStream_t stream;
   int T, B, min_q_len, max_q_len, max_kv_len, settled;
+  int longer_than[17];    // [n]: requests of more than n tokens
 };
 
 // ops.py's thresholds, as they stand when the step is run.
@@ -320,7 +321,8 @@ int block_pass(const CoBlockLayer& L, const CoBlockStep& S, const CoBlockTuning&
   } else {
     if (Nq % 4) return CO_BLOCK_UNSUPPORTED;
     const int max_rows = S.max_q_len * G;
-    const int any_small = S.min_q_len * G <= 16, any_large = max_rows > 16;
+    const int any_small = S.min_q_len * G <= 16;
+    const int large = G <= 16 ? S.longer_than[16 / G] : B;      // requests of more than 16 rows per kv head
     long floats = 0;
     float* as = nullptr;
     if (any_small && G <= 16) {
@@ -329,7 +331,7 @@ int block_pass(const CoBlockLayer& L, const CoBlockStep& S, const CoBlockTuning&
     }
     void* o = A.take((size_t)T * Nq * 2);
     RUN_ATTENTION(L.attention(q, q_stride, o, Nq, io.k_cache, io.v_cache, io.block_tables, io.max_blocks, S.cu_q, S.kv_lens,
-                              B, nh, nkv, io.page_size, L.window, L.scale, max_rows, any_small, any_large, S.max_kv_len, as,
+                              B, nh, nkv, io.page_size, L.window, L.scale, max_rows, any_small, large, S.max_kv_len, as,
                               floats, S.tc_status, T, io.num_pages, S.settled, stream));
     const Route r = R.linear(T, H, Nq, Nq, o, L.w_o, L.mixer_partial != 0, &mixed_splits);
     plan->o_route = r;

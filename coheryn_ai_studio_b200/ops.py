@@ -920,7 +920,7 @@ def attention_rows(q, out, k_cache, v_cache, block_tables, token_req, positions,
     B = len(q_lens)
     rows = [n * G for n in q_lens]
     any_small = any(r <= 16 for r in rows)
-    any_large = any(r > 16 for r in rows)
+    large = sum(1 for r in rows if r > 16)
     lib = attention_lib(head_dim)
     scratch, floats = None, 0
     if any_small and G <= 16:
@@ -929,7 +929,7 @@ def attention_rows(q, out, k_cache, v_cache, block_tables, token_req, positions,
     args = (_ptr(q), c_long(q.stride(0)), _ptr(out), c_long(out.stride(0)), _ptr(k_cache), _ptr(v_cache),
             _ptr(block_tables), c_int(block_tables.shape[1]), _ptr(cu_q), _ptr(kv_lens), c_int(B),
             c_int(num_heads), c_int(num_kv_heads), c_int(page_size), c_int(window or 0), c_float(scale),
-            c_int(max(rows)), c_int(1 if any_small else 0), c_int(1 if any_large else 0), c_int(max_kv_len),
+            c_int(max(rows)), c_int(1 if any_small else 0), c_int(large), c_int(max_kv_len),
             _ptr(scratch), c_long(floats), _ptr(tc_status(q.device)), c_int(q.shape[0]), c_int(k_cache.shape[0]),
             c_int(1 if settled else 0))
     if slopes_log2 is not None:     # a score that loses a slope per head times the distance
