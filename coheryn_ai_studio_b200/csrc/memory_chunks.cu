@@ -7,7 +7,7 @@
 //   S_t = a_t S_0 + sum_{s <= t} w_ts k_s v_s^T,            n_t likewise with k_s alone
 //   o_t = (a_t S_0^T q_t + sum_{s <= t} w_ts (q_t . k_s) v_s) / (max(|n_t . q_t|, exp(-m_t)) + 1e-6)
 //
-//   memory_gates_kernel   a warp per (run, head): F, i, m of every token and m_0 of every chunk;
+//   memory_gates_kernel   a CTA per (run, head): F, i, m of every token and m_0 of every chunk;
 //   memory_sum_kernel     a CTA per (chunk, head, 64 key channels, 128 value channels): what the chunk adds to S and n;
 //   memory_carry_kernel   over a run's chunks, element by element: the S_0 and n_0 of every chunk; the last ones are kept;
 //   memory_out_kernel     a CTA per (chunk, head): the outputs and the norm, weight and gate behind them.
@@ -18,7 +18,7 @@
 // What bounds it: the scan token by token is a chain of dependent multiply-adds and shuffles on a CTA per (head, 64 value
 // channels): 0.65 us per token with 32 of 148 SMs at work.  Here only the carry is a chain, of one multiply-add per chunk and
 // element; the rest are products over all chunks at once.  Measured on a B200 (8 heads of 128 x 256, one request of 2,048
-// tokens): 30 + 38 + 16 + 125 us in place of 1,350 us (1,850 with the kernels behind the scan launched ahead and waiting beside it).
+// tokens): 14 + 38 + 16 + 94 us in place of 1,350 us (1,850 with the kernels behind the scan launched ahead and waiting beside it).
 //
 // A run of fewer than CHUNK_FROM tokens is left to the scan (recurrent.cu), request by request, so that a row's order of
 // additions depends on its place in its own request's run only.
@@ -66,69 +66,96 @@ struct Area {
   }
 };
 
-// grid (runs, heads), a warp: two tokens per lane of every chunk.
-__global__ void __launch_bounds__(32) memory_gates_kernel(MemoryIn P, int B, Area A) {
+// grid (runs, heads), GATE_WARPS warps.  A warp takes every GATE_WARPS-th chunk, two tokens per lane; what the chunks hand to one
+// another is the running maximum alone, a chain of one step per chunk that one thread walks between the two passes (a warp per
+// head that walked the chunks from beginning to end took 30 us for 32 of them).
+constexpr int GATE_WARPS = 16;
+__global__ void __launch_bounds__(32 * GATE_WARPS) memory_gates_kernel(MemoryIn P, int B, Area A) {
   co_pdl_launch_dependents();
   co_pdl_wait();
-  const int h = blockIdx.y, lane = threadIdx.x;
+  const int h = blockIdx.y, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   Run R;
   if (!find_run(P.cu_q, B, blockIdx.x, true, R)) return;
   float* m_state = P.state + (size_t)P.state_slots[R.r] * P.state_stride + (size_t)P.heads * P.dk * P.dv + (size_t)P.heads * P.dk + h;
   const float bi = co_load_any(P.bias_i, P.bias_dtype, h), bf = co_load_any(P.bias_f, P.bias_dtype, h);
-  float m0 = *m_state;
   const int chunks = (R.len + CH - 1) / CH;
-  float zi[2], zf[2];
-  auto fetch = [&](int c) {
+  // the largest i_s - F_s up to and with this lane's tokens
+  auto best_of = [&](const double (&F)[2], const float (&li)[2], int nt, double (&best)[2]) {
+    const double p0 = 2 * lane < nt ? (double)li[0] - F[0] : -1e300, p1 = fmax(p0, 2 * lane + 1 < nt ? (double)li[1] - F[1] : -1e300);
+    double x = p1;
 #pragma unroll
-    for (int u = 0; u < 2; ++u) {
-      const int t = c * CH + 2 * lane + u;
-      const size_t row = (size_t)(R.start + min(t, R.len - 1));
-      zi[u] = P.gi[row * P.ld_gate + h]; zf[u] = P.gf[row * P.ld_gate + h];
+    for (int o = 1; o < 32; o <<= 1) {
+      const double y = __shfl_up_sync(0xffffffffu, x, o);
+      if (lane >= o) x = fmax(x, y);
     }
+    const double before = __shfl_up_sync(0xffffffffu, x, 1);
+    best[0] = fmax(lane ? before : -1e300, p0);
+    best[1] = x;
   };
-  fetch(0);
-  for (int c = 0; c < chunks; ++c) {
+  for (int c = warp; c < chunks; c += GATE_WARPS) {
     const int nt = min(CH, R.len - c * CH);
     float li[2];
-    double lf[2];
+    double F[2];
 #pragma unroll
     for (int u = 0; u < 2; ++u) {
-      li[u] = P.cap * tanhf((zi[u] + bi) / P.cap);
-      const float z = P.cap * tanhf((zf[u] + bf) / P.cap);
-      lf[u] = 2 * lane + u < nt ? (double)-rc_softplus(-z) : 0.0;
+      const size_t row = (size_t)(R.start + min(c * CH + 2 * lane + u, R.len - 1));
+      li[u] = P.cap * tanhf((P.gi[row * P.ld_gate + h] + bi) / P.cap);
+      const float z = P.cap * tanhf((P.gf[row * P.ld_gate + h] + bf) / P.cap);
+      F[u] = 2 * lane + u < nt ? (double)-rc_softplus(-z) : 0.0;       // log sigmoid; tokens beyond the last add nothing
     }
-    if (c + 1 < chunks) fetch(c + 1);
-    double x = lf[0] + lf[1];                       // sums up to and with this lane's tokens
+    const double second = F[1];
+    double x = F[0] + F[1];                         // sums up to and with this lane's tokens
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
       const double y = __shfl_up_sync(0xffffffffu, x, o);
       if (lane >= o) x += y;
     }
-    const double F[2] = {x - lf[1], x};
-    const bool in0 = 2 * lane < nt, in1 = 2 * lane + 1 < nt;
-    const double p0 = in0 ? (double)li[0] - F[0] : -1e300, p1 = fmax(p0, in1 ? (double)li[1] - F[1] : -1e300);
-    double best = p1;                               // the largest i_s - F_s up to and with this lane's tokens
+    F[0] = x - second;
+    F[1] = x;
+    double best[2];
+    best_of(F, li, nt, best);
+    const size_t at = (size_t)(R.first + c) * P.heads + h;
 #pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const double y = __shfl_up_sync(0xffffffffu, best, o);
-      if (lane >= o) best = fmax(best, y);
+    for (int u = 0; u < 2; ++u) { A.f[at * CH + 2 * lane + u] = F[u]; A.i[at * CH + 2 * lane + u] = li[u]; }
+    if (lane == 31) {
+      *reinterpret_cast<double*>(A.m0 + at * 4) = best[1];
+      *reinterpret_cast<double*>(A.m0 + at * 4 + 2) = F[1];
     }
-    const double before = __shfl_up_sync(0xffffffffu, best, 1);
-    const double b0 = fmax(lane ? before : -1e300, p0);
-    const float m[2] = {(float)(F[0] + fmax((double)m0, b0)), (float)(F[1] + fmax((double)m0, best))};
-    const size_t at = ((size_t)(R.first + c) * P.heads + h);
-#pragma unroll
-    for (int u = 0; u < 2; ++u) {
-      A.f[at * CH + 2 * lane + u] = F[u];
-      A.i[at * CH + 2 * lane + u] = li[u];
-      A.m[at * CH + 2 * lane + u] = m[u];
-    }
-    const float m1 = __shfl_sync(0xffffffffu, m[1], 31);      // the tokens beyond the last add nothing to F and to the maximum
-    if (lane == 0) { A.m0[at * 4] = m0; A.m0[at * 4 + 1] = m1; }
-    if (lane == 31) *reinterpret_cast<double*>(A.m0 + at * 4 + 2) = F[1];
-    m0 = m1;
   }
-  if (lane == 0) *m_state = m0;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    float m0 = *m_state;
+    for (int c0 = 0; c0 < chunks; c0 += 8) {
+      double best[8], end[8];
+#pragma unroll
+      for (int i = 0; i < 8; ++i)
+        if (c0 + i < chunks) {
+          const float* p = A.m0 + ((size_t)(R.first + c0 + i) * P.heads + h) * 4;
+          best[i] = *reinterpret_cast<const double*>(p);
+          end[i] = *reinterpret_cast<const double*>(p + 2);
+        }
+#pragma unroll
+      for (int i = 0; i < 8; ++i)
+        if (c0 + i < chunks) {
+          float* p = A.m0 + ((size_t)(R.first + c0 + i) * P.heads + h) * 4;
+          const float m1 = (float)(end[i] + fmax((double)m0, best[i]));
+          p[0] = m0; p[1] = m1;
+          m0 = m1;
+        }
+    }
+    *m_state = m0;
+  }
+  __syncthreads();
+  for (int c = warp; c < chunks; c += GATE_WARPS) {
+    const size_t at = (size_t)(R.first + c) * P.heads + h;
+    const double F[2] = {A.f[at * CH + 2 * lane], A.f[at * CH + 2 * lane + 1]};
+    const float li[2] = {A.i[at * CH + 2 * lane], A.i[at * CH + 2 * lane + 1]};
+    const double m0 = (double)A.m0[at * 4];
+    double best[2];
+    best_of(F, li, min(CH, R.len - c * CH), best);
+#pragma unroll
+    for (int u = 0; u < 2; ++u) A.m[at * CH + 2 * lane + u] = (float)(F[u] + fmax(m0, best[u]));
+  }
 }
 
 // acc rows 4 la + i and 32 + 4 la + i of a 64-row product, four neighbouring columns: acc[t][c] += left[k][t] right[k][c].
@@ -259,7 +286,7 @@ size_t out_smem(int W, int dk, int dvp) {
 }
 
 template <int W>
-__global__ void __launch_bounds__(2 * W) memory_out_kernel(MemoryIn P, HeadOut E, int B, Area A, int first_floats) {
+__global__ void __launch_bounds__(2 * W, 512 / W) memory_out_kernel(MemoryIn P, HeadOut E, int B, Area A, int first_floats) {
   constexpr int THREADS = 2 * W;
   extern __shared__ __align__(16) float sm[];
   const int dk = P.dk, dv = P.dv, dvp = A.dvp, dkp = (dk + SLICE - 1) / SLICE * SLICE;
@@ -283,6 +310,7 @@ __global__ void __launch_bounds__(2 * W) memory_out_kernel(MemoryIn P, HeadOut E
   const float* gm = A.m + at * CH;
   // a warp takes eight tokens by four channels at a time: sectors of 32 bytes are read whole, and the transposed stores fall on
   // different banks
+#pragma unroll 8
   for (int e = tid; e < dkp * CH; e += THREADS) {
     const int d = (e & 7) + 8 * (e / (8 * CH)), t = (e >> 3) % CH;
     Qt[d * TP + t] = t < nt && d < dk ? P.q[(size_t)(row0 + t) * P.ld + (size_t)h * dk + d] * q_scale : 0.f;
@@ -295,6 +323,7 @@ __global__ void __launch_bounds__(2 * W) memory_out_kernel(MemoryIn P, HeadOut E
     for (int d0 = 0; d0 < dk; d0 += 64) {
       const int n = min(64, dk - d0);
       if (d0) __syncthreads();
+#pragma unroll
       for (int e = tid; e < 64 * CH; e += THREADS) {
         const int d = (e & 7) + 8 * (e / (8 * CH)), t = (e >> 3) % CH;
         if (d < n) area[d * TP + t] = t < nt ? P.k[(size_t)(row0 + t) * P.ld + (size_t)h * dk + d0 + d] : 0.f;
@@ -397,7 +426,7 @@ long co_memory_chunk_floats(int chunks, int heads, int dk, int dv) { return (lon
 int co_memory_chunks(const MemoryIn& P, const HeadOut& E, int B, int chunks, int runs, float* scratch, cudaStream_t stream) {
   const int dvp = padded(P.dv);
   const Area A(scratch, chunks, P.heads, P.dk, dvp);
-  co_launch(memory_gates_kernel, dim3(runs, P.heads), dim3(32), 0, stream, P, B, A);
+  co_launch(memory_gates_kernel, dim3(runs, P.heads), dim3(32 * GATE_WARPS), 0, stream, P, B, A);
   CO_CHECK_LAUNCH("memory_gates");
   const size_t sum_smem = sizeof(float) * (CH * 64 + CH * 128 + CH);
   cudaFuncSetAttribute(memory_sum_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sum_smem);
