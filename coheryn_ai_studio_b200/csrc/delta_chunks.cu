@@ -19,7 +19,7 @@
 //
 // What bounds it: the scan token by token is a chain of dependent multiply-adds and shuffles, 0.55 us per token whatever the
 // chip could do beside it.  Here the chain is two products of 64 x 128 x 16 per chunk; measured on a B200 (12 heads of 128 x
-// 128, one request of 2,048 tokens) the four kernels take 287 us in place of 1,150 us for the scan with its preparation.
+// 128, one request of 2,048 tokens) the four kernels take 271 us in place of 1,150 us for the scan with its preparation.
 //
 // A run of fewer than CHUNK_FROM tokens is left to the scan (recurrent.cu), request by request, so that a row's order of
 // additions depends on its place in its own request's run only.
@@ -107,23 +107,29 @@ __device__ __forceinline__ void mac4(float (&acc)[4][4], const float4 a, const f
 }
 
 // ---------------------------------------------------------------------------------
-// A chunk of a head by itself: A, B and the scaled rows.  grid (chunks, heads).  Three tiles of 64 tokens by all channels are
-// what a CTA keeps, so that two fit an SM (with the inverse and its products in the same kernel one did: 163 us for what the
-// two kernels now do in 122 us; every phase waits for shared memory, and warps are what hides that).
+// A chunk of a head by itself: A, B and the scaled rows.  grid (chunks, heads).  A CTA keeps three tiles of 64 tokens by 64
+// channels and takes 128 channels in two passes (everything here is by channel, except the norms of q and k, taken first, and
+// the sums A and B, which go from pass to pass): three CTAs fit an SM.  With tiles of 128 channels two did, 384 CTAs were 1.3
+// rounds of them and took 86 us (with the inverse and its products in the same kernel one CTA did, and took 163 us); every phase
+// waits for shared memory, and warps are what hides that.  Measured on a B200 (2,048 tokens, 12 heads): 70 us.
 // ---------------------------------------------------------------------------------
-template <int DK>
-constexpr size_t chunk_smem() { return sizeof(float) * (3 * CH * (DK + 4) + 4 * DK + 2 * CH); }
+constexpr int CW = 64, CP = CW + 4;      // channels of a pass, pitch of its tiles
+constexpr size_t CHUNK_SMEM = sizeof(float) * (3 * CH * CP + 4 * CW + 4 * CH + 2 * CH * 17);
 
 template <int DK>
-__global__ void __launch_bounds__(THREADS, 2) delta_chunk_kernel(DeltaIn P, int B, float* __restrict__ scratch, int dvp) {
-  constexpr int DKP = DK + 4, NV = DK / 32;
+__global__ void __launch_bounds__(THREADS, 3) delta_chunk_kernel(DeltaIn P, int B, float* __restrict__ scratch, int dvp) {
+  constexpr int PASSES = DK / CW;
   extern __shared__ __align__(16) float sm[];
-  float* Qs = sm;                       // [64][DKP] q, then q E
-  float* Ks = Qs + CH * DKP;            // [64][DKP] k, then k E
-  float* Gs = Ks + CH * DKP;            // [64][DKP] decays, then k times the decays behind it
-  float* Dm = Gs + CH * DKP;            // [4][DK] decay of a whole block
-  float* betas = Dm + 4 * DK;           // [64]
+  float* Qs = sm;                       // [64][CP] q, then q E
+  float* Ks = Qs + CH * CP;             // [64][CP] k, then k E
+  float* Gs = Ks + CH * CP;             // [64][CP] decays, then k times the decays behind it
+  float* Dm = Gs + CH * CP;             // [4][CW] decay of a whole block
+  float* betas = Dm + 4 * CW;           // [64]
   float* ones = betas + CH;             // [64] the decays of a head that has one for all its channels
+  float* iqs = ones + CH;               // [64] what q and k are multiplied by
+  float* iks = iqs + CH;
+  float* As = iks + CH;                 // [64][17] the sums of A inside the blocks, of B
+  float* Bs = As + CH * 17;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   co_pdl_launch_dependents();
   co_pdl_wait();
@@ -134,26 +140,24 @@ __global__ void __launch_bounds__(THREADS, 2) delta_chunk_kernel(DeltaIn P, int 
   const int g = h / (P.heads / P.kv_heads);
   const float rate = expf(co_load_any(P.rate_log, P.rate_log_dtype, h));
   const bool per_head = P.decay_channels == 1;
-
-#pragma unroll 8
-  for (int e = tid; e < CH * DK; e += THREADS) {
-    const int i = e / DK, d = e % DK;
-    float qv = 0.f, kv = 0.f, gv = 1.f;
-    if (i < nt && d < dk) {
-      const size_t row = (size_t)(row0 + i);
-      qv = P.q[row * P.ld_qkv + (size_t)g * dk + d];
-      kv = P.k[row * P.ld_qkv + (size_t)g * dk + d];
-      if (!per_head) {
-        const size_t sc = (size_t)h * dk + d;
-        gv = expf(-rate * rc_softplus(P.step[row * P.ld_step + sc] + co_load_any(P.step_bias, P.step_bias_dtype, sc)));
-      }
-    }
-    Qs[i * DKP + d] = qv; Ks[i * DKP + d] = kv;
-    if (!per_head) Gs[i * DKP + d] = gv;
-  }
   const Piece<DK> out(scratch, (size_t)blockIdx.x * P.heads + h, dvp);
   float* Nm = out.n;                    // [t][s] beta_t A_ts, written for s < t only
   float* Bt = out.qb + DK * CH;         // [s][t] B, transposed; zero for s > t
+
+  // q and k become unit vectors (q also divided by sqrt(dk))
+  const float q_scale = 1.0f / sqrtf((float)dk);
+#pragma unroll 4
+  for (int i = warp; i < CH; i += THREADS / 32) {
+    float sq = 0.f, sk = 0.f;
+    const size_t row = (size_t)(row0 + min(i, nt - 1)) * P.ld_qkv + (size_t)g * dk;
+#pragma unroll
+    for (int d = lane; d < DK; d += 32) {
+      const float qv = d < dk ? P.q[row + d] : 0.f, kv = d < dk ? P.k[row + d] : 0.f;
+      sq = fmaf(qv, qv, sq); sk = fmaf(kv, kv, sk);
+    }
+    sq = co_warp_sum(sq); sk = co_warp_sum(sk);
+    if (lane == 0) { iqs[i] = q_scale / sqrtf(sq + 1e-6f); iks[i] = 1.0f / sqrtf(sk + 1e-6f); }
+  }
   for (int e = tid; e < CH * CH; e += THREADS)
     if (e / CH > e % CH) Bt[e] = 0.f;
   if (tid < CH) {
@@ -162,136 +166,152 @@ __global__ void __launch_bounds__(THREADS, 2) delta_chunk_kernel(DeltaIn P, int 
       ones[tid] = tid < nt ? expf(-rate * rc_softplus(P.step[(size_t)(row0 + tid) * P.ld_step + h] + co_load_any(P.step_bias, P.step_bias_dtype, h))) : 1.f;
   }
   __syncthreads();
-  if (per_head)
-    for (int e = tid; e < CH * DK; e += THREADS) Gs[(e / DK) * DKP + e % DK] = ones[e / DK];
-  const float q_scale = 1.0f / sqrtf((float)dk);
-  for (int i = warp; i < nt; i += THREADS / 32) {      // q and k become unit vectors (q also divided by sqrt(dk))
-    float sq = 0.f, sk = 0.f;
-#pragma unroll
-    for (int d = lane; d < DK; d += 32) {
-      sq = fmaf(Qs[i * DKP + d], Qs[i * DKP + d], sq); sk = fmaf(Ks[i * DKP + d], Ks[i * DKP + d], sk);
-    }
-    sq = co_warp_sum(sq); sk = co_warp_sum(sk);
-    const float iq = q_scale / sqrtf(sq + 1e-6f), ik = 1.0f / sqrtf(sk + 1e-6f);
-#pragma unroll
-    for (int d = lane; d < DK; d += 32) { Qs[i * DKP + d] *= iq; Ks[i * DKP + d] *= ik; }
-  }
-  __syncthreads();
 
-  // A and B inside the blocks of 16: eight lanes share a row, which walks back through its block with k_t and q_t decaying
-  // token by token.  A warp takes a row of every block, then the row that makes all warps' walks equally long.
-  {
-    const int blk = lane >> 3, l8 = lane & 7;
+  // between blocks i > j: a warp takes a pair of blocks, half of it the rows of k and half those of q, 4 x 4 a lane
+  const int bi = warp < 1 ? 1 : (warp < 3 ? 2 : 3), bj = warp < 1 ? 0 : (warp < 3 ? warp - 1 : warp - 3);
+  float acc[4][4];
+#pragma unroll
+  for (int a = 0; a < 4; ++a) acc[a][0] = acc[a][1] = acc[a][2] = acc[a][3] = 0.f;
+
 #pragma unroll 1
-    for (int half = 0; half < 2; ++half) {
-      const int r = half ? 15 - warp : warp, t = BL * blk + r;
-      float4 wk[NV], wq[NV];
+  for (int pass = 0; pass < PASSES; ++pass) {
+    const int ch0 = pass * CW;
+    if (pass) __syncthreads();          // the tiles of the pass before are stored
+#pragma unroll 8
+    for (int e = tid; e < CH * CW; e += THREADS) {
+      const int i = e / CW, d = e % CW, ch = ch0 + d;
+      float qv = 0.f, kv = 0.f, gv = 1.f;
+      if (i < nt && ch < dk) {
+        const size_t row = (size_t)(row0 + i);
+        qv = P.q[row * P.ld_qkv + (size_t)g * dk + ch] * iqs[i];
+        kv = P.k[row * P.ld_qkv + (size_t)g * dk + ch] * iks[i];
+        if (!per_head) {
+          const size_t sc = (size_t)h * dk + ch;
+          gv = expf(-rate * rc_softplus(P.step[row * P.ld_step + sc] + co_load_any(P.step_bias, P.step_bias_dtype, sc)));
+        }
+      }
+      Qs[i * CP + d] = qv; Ks[i * CP + d] = kv;
+      Gs[i * CP + d] = per_head ? ones[i] : gv;
+    }
+    __syncthreads();
+    // A and B inside the blocks of 16: eight lanes share a row, which walks back through its block with k_t and q_t decaying
+    // token by token.  A warp takes a row of every block, then the row that makes all warps' walks equally long.
+    {
+      const int blk = lane >> 3, l8 = lane & 7;
+#pragma unroll 1
+      for (int half = 0; half < 2; ++half) {
+        const int r = half ? 15 - warp : warp, t = BL * blk + r;
+        float4 wk[2], wq[2];
 #pragma unroll
-      for (int j = 0; j < NV; ++j) { wk[j] = ld4(Ks + t * DKP + 32 * j + 4 * l8); wq[j] = ld4(Qs + t * DKP + 32 * j + 4 * l8); }
-      for (int s = r; s >= 0; --s) {
-        const int row = BL * blk + s;
-        float a = 0.f, b = 0.f;
+        for (int j = 0; j < 2; ++j) { wk[j] = ld4(Ks + t * CP + 32 * j + 4 * l8); wq[j] = ld4(Qs + t * CP + 32 * j + 4 * l8); }
+        for (int s = r; s >= 0; --s) {
+          const int row = BL * blk + s;
+          float a = 0.f, b = 0.f;
 #pragma unroll
-        for (int j = 0; j < NV; ++j) {
-          if (s < r) {
-            const float4 gg = ld4(Gs + (row + 1) * DKP + 32 * j + 4 * l8);
-            wk[j].x *= gg.x; wk[j].y *= gg.y; wk[j].z *= gg.z; wk[j].w *= gg.w;
-            wq[j].x *= gg.x; wq[j].y *= gg.y; wq[j].z *= gg.z; wq[j].w *= gg.w;
+          for (int j = 0; j < 2; ++j) {
+            if (s < r) {
+              const float4 gg = ld4(Gs + (row + 1) * CP + 32 * j + 4 * l8);
+              wk[j].x *= gg.x; wk[j].y *= gg.y; wk[j].z *= gg.z; wk[j].w *= gg.w;
+              wq[j].x *= gg.x; wq[j].y *= gg.y; wq[j].z *= gg.z; wq[j].w *= gg.w;
+            }
+            const float4 kk = ld4(Ks + row * CP + 32 * j + 4 * l8);
+            a = fmaf(wk[j].x, kk.x, a); a = fmaf(wk[j].y, kk.y, a); a = fmaf(wk[j].z, kk.z, a); a = fmaf(wk[j].w, kk.w, a);
+            b = fmaf(wq[j].x, kk.x, b); b = fmaf(wq[j].y, kk.y, b); b = fmaf(wq[j].z, kk.z, b); b = fmaf(wq[j].w, kk.w, b);
           }
-          const float4 kk = ld4(Ks + row * DKP + 32 * j + 4 * l8);
-          a = fmaf(wk[j].x, kk.x, a); a = fmaf(wk[j].y, kk.y, a); a = fmaf(wk[j].z, kk.z, a); a = fmaf(wk[j].w, kk.w, a);
-          b = fmaf(wq[j].x, kk.x, b); b = fmaf(wq[j].y, kk.y, b); b = fmaf(wq[j].z, kk.z, b); b = fmaf(wq[j].w, kk.w, b);
-        }
 #pragma unroll
-        for (int o = 4; o > 0; o >>= 1) { a += __shfl_xor_sync(0xffffffffu, a, o); b += __shfl_xor_sync(0xffffffffu, b, o); }
-        if (l8 == 0) {
-          if (s < r) Nm[t * CH + row] = betas[t] * a;
-          Bt[row * CH + t] = b;
+          for (int o = 4; o > 0; o >>= 1) { a += __shfl_xor_sync(0xffffffffu, a, o); b += __shfl_xor_sync(0xffffffffu, b, o); }
+          if (l8 == 0) {
+            if (pass) { a += As[t * 17 + s]; b += Bs[t * 17 + s]; }
+            if (pass + 1 < PASSES) { As[t * 17 + s] = a; Bs[t * 17 + s] = b; }
+            else {
+              if (s < r) Nm[t * CH + row] = betas[t] * a;
+              Bt[row * CH + t] = b;
+            }
+          }
         }
       }
     }
-  }
-  __syncthreads();
-  // Rows scaled inside their block: q and k by the decays up to and with their token, k also by those behind it.
-  for (int e = tid; e < 4 * DK; e += THREADS) {
-    const int d = e % DK, blk = e / DK, at = BL * blk * DKP + d;
-    float kr[BL], gr[BL];
+    __syncthreads();
+    // Rows scaled inside their block: q and k by the decays up to and with their token, k also by those behind it.
+    {
+      const int d = tid % CW, blk = tid / CW, at = BL * blk * CP + d;
+      float kr[BL], gr[BL];
 #pragma unroll
-    for (int r = 0; r < BL; ++r) { kr[r] = Ks[at + r * DKP]; gr[r] = Gs[at + r * DKP]; }
-    float p = 1.f;
+      for (int r = 0; r < BL; ++r) { kr[r] = Ks[at + r * CP]; gr[r] = Gs[at + r * CP]; }
+      float p = 1.f;
 #pragma unroll
-    for (int r = 0; r < BL; ++r) {
-      p *= gr[r];
-      Ks[at + r * DKP] = kr[r] * p;
-      Qs[at + r * DKP] *= p;
+      for (int r = 0; r < BL; ++r) {
+        p *= gr[r];
+        Ks[at + r * CP] = kr[r] * p;
+        Qs[at + r * CP] *= p;
+      }
+      Dm[blk * CW + d] = p;
+      p = 1.f;
+#pragma unroll
+      for (int r = BL - 1; r >= 0; --r) { Gs[at + r * CP] = kr[r] * p; p *= gr[r]; }
     }
-    Dm[blk * DK + d] = p;
-    p = 1.f;
-#pragma unroll
-    for (int r = BL - 1; r >= 0; --r) { Gs[at + r * DKP] = kr[r] * p; p *= gr[r]; }
-  }
-  __syncthreads();
-  // A and B between blocks i > j: a warp takes a pair of blocks, half of it the rows of k and half those of q, 4 x 4 a lane.
-  if (warp < 6) {
-    const int i = warp < 1 ? 1 : (warp < 3 ? 2 : 3), j = warp < 1 ? 0 : (warp < 3 ? warp - 1 : warp - 3);
-    const float* L = (lane < 16 ? Ks : Qs) + (BL * i + ((lane >> 2) & 3)) * DKP;      // rows +0, +4, +8, +12
-    const float* Rt = Gs + (BL * j + (lane & 3)) * DKP;
-    const float* d1 = Dm + (j + 1) * DK;      // read where a block lies between the two
-    const float* d2 = Dm + (j + 2) * DK;
-    float acc[4][4];
-#pragma unroll
-    for (int a = 0; a < 4; ++a) acc[a][0] = acc[a][1] = acc[a][2] = acc[a][3] = 0.f;
+    __syncthreads();
+    if (warp < 6) {
+      const float* L = (lane < 16 ? Ks : Qs) + (BL * bi + ((lane >> 2) & 3)) * CP;      // rows +0, +4, +8, +12
+      const float* Rt = Gs + (BL * bj + (lane & 3)) * CP;
+      const float* d1 = Dm + (bj + 1) * CW;      // read where a block lies between the two
+      const float* d2 = Dm + (bj + 2) * CW;
 #pragma unroll 4
-    for (int d = 0; d < DK; d += 4) {
-      float4 x[4], y[4];
+      for (int d = 0; d < CW; d += 4) {
+        float4 x[4], y[4];
 #pragma unroll
-      for (int a = 0; a < 4; ++a) { x[a] = ld4(L + 4 * a * DKP + d); y[a] = ld4(Rt + 4 * a * DKP + d); }
-      if (i - j > 1) {
-        float4 w = ld4(d1 + d);
-        if (i - j > 2) { const float4 z = ld4(d2 + d); w.x *= z.x; w.y *= z.y; w.z *= z.z; w.w *= z.w; }
+        for (int a = 0; a < 4; ++a) { x[a] = ld4(L + 4 * a * CP + d); y[a] = ld4(Rt + 4 * a * CP + d); }
+        if (bi - bj > 1) {
+          float4 w = ld4(d1 + d);
+          if (bi - bj > 2) { const float4 z = ld4(d2 + d); w.x *= z.x; w.y *= z.y; w.z *= z.z; w.w *= z.w; }
 #pragma unroll
-        for (int a = 0; a < 4; ++a) { y[a].x *= w.x; y[a].y *= w.y; y[a].z *= w.z; y[a].w *= w.w; }
-      }
-#pragma unroll
-      for (int a = 0; a < 4; ++a)
-#pragma unroll
-        for (int b = 0; b < 4; ++b) {
-          acc[a][b] = fmaf(x[a].x, y[b].x, acc[a][b]); acc[a][b] = fmaf(x[a].y, y[b].y, acc[a][b]);
-          acc[a][b] = fmaf(x[a].z, y[b].z, acc[a][b]); acc[a][b] = fmaf(x[a].w, y[b].w, acc[a][b]);
+          for (int a = 0; a < 4; ++a) { y[a].x *= w.x; y[a].y *= w.y; y[a].z *= w.z; y[a].w *= w.w; }
         }
+#pragma unroll
+        for (int a = 0; a < 4; ++a)
+#pragma unroll
+          for (int b = 0; b < 4; ++b) {
+            acc[a][b] = fmaf(x[a].x, y[b].x, acc[a][b]); acc[a][b] = fmaf(x[a].y, y[b].y, acc[a][b]);
+            acc[a][b] = fmaf(x[a].z, y[b].z, acc[a][b]); acc[a][b] = fmaf(x[a].w, y[b].w, acc[a][b]);
+          }
+      }
     }
+    __syncthreads();
+    // From the block to the chunk: q and k of block i by the decays of the blocks before it, the other k by those behind it.
+    {
+      const int d = tid % CW, blk = tid / CW, at = BL * blk * CP + d;
+      float before = 1.f, behind = 1.f;
+      for (int m = 0; m < blk; ++m) before *= Dm[m * CW + d];
+      for (int m = blk + 1; m < 4; ++m) behind *= Dm[m * CW + d];
+#pragma unroll
+      for (int r = 0; r < BL; ++r) { Ks[at + r * CP] *= before; Qs[at + r * CP] *= before; Gs[at + r * CP] *= behind; }
+    }
+    __syncthreads();
+#pragma unroll
+    for (int e = tid; e < CH * CW / 4; e += THREADS) {
+      const int t = e / (CW / 4), d = 4 * (e % (CW / 4));
+      st4(out.kh + t * DK + ch0 + d, ld4(Gs + t * CP + d));
+      st4(out.wt + t * DK + ch0 + d, ld4(Ks + t * CP + d));       // K~, which delta_solve_kernel replaces by W^T
+    }
+#pragma unroll
+    for (int e = tid; e < CH * CW / 4; e += THREADS) {       // sixteen channels by two groups of four tokens per warp
+      const int d = (e >> 1) % CW, t = 4 * ((e & 1) + 2 * (e / (2 * CW)));
+      st4(out.qb + (ch0 + d) * CH + t, make_float4(Qs[t * CP + d], Qs[(t + 1) * CP + d], Qs[(t + 2) * CP + d], Qs[(t + 3) * CP + d]));
+    }
+    if (tid < CW) out.dec[ch0 + tid] = ((Dm[tid] * Dm[CW + tid]) * Dm[2 * CW + tid]) * Dm[3 * CW + tid];
+  }
+  if (warp < 6) {
 #pragma unroll
     for (int a = 0; a < 4; ++a) {
-      const int t = BL * i + ((lane >> 2) & 3) + 4 * a;
+      const int t = BL * bi + ((lane >> 2) & 3) + 4 * a;
 #pragma unroll
       for (int b = 0; b < 4; ++b) {
-        const int s = BL * j + (lane & 3) + 4 * b;
+        const int s = BL * bj + (lane & 3) + 4 * b;
         if (lane < 16) Nm[t * CH + s] = betas[t] * acc[a][b];
         else Bt[s * CH + t] = acc[a][b];
       }
     }
   }
-  __syncthreads();
-  // From the block to the chunk: q and k of block i by the decays of the blocks before it, the other k by those behind it.
-  for (int e = tid; e < 4 * DK; e += THREADS) {
-    const int d = e % DK, blk = e / DK, at = BL * blk * DKP + d;
-    float before = 1.f, behind = 1.f;
-    for (int m = 0; m < blk; ++m) before *= Dm[m * DK + d];
-    for (int m = blk + 1; m < 4; ++m) behind *= Dm[m * DK + d];
-#pragma unroll
-    for (int r = 0; r < BL; ++r) { Ks[at + r * DKP] *= before; Qs[at + r * DKP] *= before; Gs[at + r * DKP] *= behind; }
-  }
-  __syncthreads();
-  for (int e = tid; e < CH * DK / 4; e += THREADS) {
-    const int t = e / (DK / 4), d = 4 * (e % (DK / 4));
-    st4(out.kh + t * DK + d, ld4(Gs + t * DKP + d));
-    st4(out.wt + t * DK + d, ld4(Ks + t * DKP + d));       // K~, which delta_solve_kernel replaces by W^T
-  }
-  for (int e = tid; e < CH * DK / 4; e += THREADS) {       // sixteen channels by two groups of four tokens per warp
-    const int d = (e >> 1) % DK, t = 4 * ((e & 1) + 2 * (e / (2 * DK)));
-    st4(out.qb + d * CH + t, make_float4(Qs[t * DKP + d], Qs[(t + 1) * DKP + d], Qs[(t + 2) * DKP + d], Qs[(t + 3) * DKP + d]));
-  }
-  for (int d = tid; d < DK; d += THREADS) out.dec[d] = ((Dm[d] * Dm[DK + d]) * Dm[2 * DK + d]) * Dm[3 * DK + d];
 }
 
 // ---------------------------------------------------------------------------------
@@ -586,8 +606,8 @@ int padded(int dv) { return (dv + VS - 1) / VS * VS; }
 template <int DK>
 int launch(const DeltaIn& P, const HeadOut& E, int B, int chunks, int runs, float* scratch, cudaStream_t stream) {
   const int dvp = padded(P.dv);
-  cudaFuncSetAttribute(delta_chunk_kernel<DK>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)chunk_smem<DK>());
-  co_launch(delta_chunk_kernel<DK>, dim3(chunks, P.heads), dim3(THREADS), chunk_smem<DK>(), stream, P, B, scratch, dvp);
+  cudaFuncSetAttribute(delta_chunk_kernel<DK>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)CHUNK_SMEM);
+  co_launch(delta_chunk_kernel<DK>, dim3(chunks, P.heads), dim3(THREADS), CHUNK_SMEM, stream, P, B, scratch, dvp);
   CO_CHECK_LAUNCH("delta_chunk");
   cudaFuncSetAttribute(delta_solve_kernel<DK>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)solve_smem<DK>());
   co_launch(delta_solve_kernel<DK>, dim3(chunks, P.heads), dim3(THREADS), solve_smem<DK>(), stream, P, B, scratch, dvp);
@@ -605,7 +625,7 @@ int launch(const DeltaIn& P, const HeadOut& E, int B, int chunks, int runs, floa
 
 }  // namespace
 
-// Up to 128 key channels three tiles of 64 tokens by all channels fit an SM; beyond that the scan stays.
+// Up to 128 key channels the state kernel's stages fit an SM; beyond that the scan stays.
 bool co_delta_chunks_take(int dk, int dv) { return dk >= 1 && dk <= 128 && dv >= 1 && dv <= 256; }
 
 long co_delta_chunk_floats(int chunks, int heads, int dk, int dv) {
