@@ -59,7 +59,8 @@ __device__ __forceinline__ void store_out(TO* out, size_t at, float v, const voi
 template <typename TX, typename TW, typename TO, int BM, int BN, int BK, int TM, int TN, bool VEC, bool MULTI>
 __global__ void __launch_bounds__((BM / TM) * (BN / TN), MULTI ? 2 : 3)
 gemm_simt_kernel(const TX* __restrict__ x, const TW* __restrict__ w, const void* __restrict__ bias, int bias_dtype, TO* __restrict__ out,
-                 float* __restrict__ apart, int M, int N, int K, long ldx, long ldo, int act, int stretch) {
+                 float* __restrict__ apart, int M, int N, int K, long ldx, long ldo, int act, int stretch, int n_split,
+                 int k_split) {
   constexpr int THREADS = (BM / TM) * (BN / TN), PM = BM + 4, PN = BN + 4, XV = BM * BK / 4;
   constexpr int XL = (XV + THREADS - 1) / THREADS, WL = BN * BK / 4 / THREADS;      // 16-byte vectors of a tile per thread
   static_assert(WL * THREADS * 4 == BN * BK && TM % 4 == 0 && TN % 4 == 0, "whole vectors per thread");
@@ -68,7 +69,9 @@ gemm_simt_kernel(const TX* __restrict__ x, const TW* __restrict__ w, const void*
   const int tid = threadIdx.x;
   const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
   const int tm = (tid / (BN / TN)) * 4, tn = (tid % (BN / TN)) * 4;
-  const int k_from = apart ? blockIdx.z * stretch : 0, k_to = apart ? min(K, k_from + stretch) : K;
+  // (a block-diagonal weight: a tile on one side of n_split reads its own columns of x alone)
+  const int k_from = apart ? blockIdx.z * stretch : (n_split > 0 && n0 >= n_split ? k_split : 0);
+  const int k_to = apart ? min(K, k_from + stretch) : (n0 + BN <= n_split ? k_split : K);
   float4 xr[XL], wr[WL];
   auto fetch = [&](int k0) {
 #pragma unroll
@@ -197,9 +200,10 @@ int stretches_apart(int M, int N, int K) {
 
 template <typename TX, typename TW, typename TO>
 int run(const TX* x, const TW* w, const void* bias, int bias_dtype, TO* out, int M, int N, int K, long ldx, long ldo, int act,
-        float* workspace, long floats, cudaStream_t stream) {
-  const bool vec = K % 4 == 0 && ldx % 4 == 0 && (uintptr_t)x % (4 * sizeof(TX)) == 0 && (uintptr_t)w % (4 * sizeof(TW)) == 0;
+        float* workspace, long floats, int n_split, int k_split, cudaStream_t stream) {
+  const bool vec = K % 4 == 0 && k_split % 4 == 0 && ldx % 4 == 0 && (uintptr_t)x % (4 * sizeof(TX)) == 0 && (uintptr_t)w % (4 * sizeof(TW)) == 0;
   int n = stretches_apart(M, N, K);
+  if (n > 1 || K > stretch_of(N)) n_split = 0;       // the stretches are those of a full row
   if (n > 1 && (!workspace || floats < (long)n * M * N)) n = 1;
   float* apart = n > 1 ? workspace : nullptr;
   const bool few = M <= ROWS_FEW;
@@ -207,7 +211,7 @@ int run(const TX* x, const TW* w, const void* bias, int bias_dtype, TO* out, int
   const int stretch = stretch_of(N);
 #define GO(BM, BN, BK, T, VEC, MULTI)                                                                                       \
   gemm_simt_kernel<TX, TW, TO, BM, BN, BK, T, T, VEC, MULTI><<<grid, (BM / T) * (BN / T), 0, stream>>>(                     \
-      x, w, bias, bias_dtype, out, apart, M, N, K, ldx, ldo, act, stretch)
+      x, w, bias, bias_dtype, out, apart, M, N, K, ldx, ldo, act, stretch, n_split, k_split)
 #define BY_ROWS(VEC, MULTI) if (few) GO(16, 64, 64, 4, VEC, MULTI); else GO(64, 128, 16, 8, VEC, MULTI)
   if (n == 1 && K > stretch) { if (vec) { BY_ROWS(true, true); } else { BY_ROWS(false, true); } }
   else { if (vec) { BY_ROWS(true, false); } else { BY_ROWS(false, false); } }
@@ -231,13 +235,16 @@ CO_EXPORT long coheryn_gemm_simt_workspace_floats(int M, int N, int K) {
 
 // x: [M, K] with row stride ldx; w: [N, K] contiguous; out: [M, N] with row stride ldo.
 // act 0: the (biased) product; CO_ACT_GELU: its exact GELU.  workspace may be absent: one CTA then takes all of k.
+// n_split > 0: w is block-diagonal, its first n_split rows are zero from k_split on and the others zero up to there; tiles on
+// one side then leave the zeros out.
 CO_EXPORT int coheryn_gemm_simt(const void* x, int x_dtype, const void* w, int w_dtype, const void* bias,
                                 int bias_dtype, void* out, int out_dtype, int M, int N, int K, long ldx,
-                                long ldo, int act, float* workspace, long floats, cudaStream_t stream) {
+                                long ldo, int act, float* workspace, long floats, int n_split, int k_split, cudaStream_t stream) {
   if (M <= 0 || N <= 0) return 0;
   if (K <= 0) CO_FAIL("gemm_simt: K must be positive");
   if (act != 0 && act != CO_ACT_GELU) CO_FAIL("gemm_simt: unknown activation %d", act);
-#define RUN(TX, TW, TO) return run((const TX*)x, (const TW*)w, bias, bias_dtype, (TO*)out, M, N, K, ldx, ldo, act, workspace, floats, stream)
+  if (n_split < 0 || n_split > N || (n_split && (k_split <= 0 || k_split >= K))) CO_FAIL("gemm_simt: blocks of %d rows and %d columns", n_split, k_split);
+#define RUN(TX, TW, TO) return run((const TX*)x, (const TW*)w, bias, bias_dtype, (TO*)out, M, N, K, ldx, ldo, act, workspace, floats, n_split, k_split, stream)
   if (x_dtype == CO_F32 && w_dtype == CO_F32 && out_dtype == CO_F32) RUN(float, float, float);
   if (x_dtype == CO_BF16 && w_dtype == CO_BF16 && out_dtype == CO_BF16) RUN(__nv_bfloat16, __nv_bfloat16, __nv_bfloat16);
   if (x_dtype == CO_BF16 && w_dtype == CO_BF16 && out_dtype == CO_F32) RUN(__nv_bfloat16, __nv_bfloat16, float);

@@ -473,9 +473,10 @@ def _simt_workspace_floats(M: int, N: int, K: int) -> int:
     return int(core().coheryn_gemm_simt_workspace_floats(c_int(M), c_int(N), c_int(K)))
 
 
-def gemm_simt(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor], out: torch.Tensor, act: int = 0) -> None:
+def gemm_simt(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor], out: torch.Tensor, act: int = 0, blocks=None) -> None:
     """out = x @ w.T (+ bias), passed through the plain activation ``act`` (see ``PLAIN_ACTIVATIONS``), with float32 FMA
-    accumulation (no tensor cores)."""
+    accumulation (no tensor cores).  ``blocks`` = (rows, columns): w is block-diagonal, zero but for its first rows by its first
+    columns and the other rows by the other columns."""
     _dev(x, w, bias, out)
     M, K = x.shape
     N = w.shape[0]
@@ -489,7 +490,8 @@ def gemm_simt(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor], ou
     _check(lib, lib.coheryn_gemm_simt(
         _ptr(x), c_int(_code(x)), _ptr(w), c_int(_code(w)), _ptr(bias),
         c_int(_code(bias) if bias is not None else F32), _ptr(out), c_int(_code(out)), c_int(M),
-        c_int(N), c_int(K), c_long(x.stride(0)), c_long(out.stride(0)), c_int(act), _ptr(workspace), c_long(floats), _stream()))
+        c_int(N), c_int(K), c_long(x.stride(0)), c_long(out.stride(0)), c_int(act), _ptr(workspace), c_long(floats),
+        c_int(blocks[0] if blocks else 0), c_int(blocks[1] if blocks else 0), _stream()))
 
 
 def attention_simple(q: torch.Tensor, out: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor,

@@ -191,7 +191,7 @@ class GatedDeltaRule(_StateMixer):
         both = torch.zeros((a2.shape[0] + g2.shape[0], a2.shape[1] + g2.shape[1]), dtype=a2.dtype, device=a2.device)
         both[:a2.shape[0], :a2.shape[1]] = a2
         both[a2.shape[0]:, a2.shape[1]:] = g2
-        self.w_second = both.contiguous()
+        self.w_second, self.second_blocks = both.contiguous(), tuple(a2.shape)
 
     def output_weights(self):
         return [self.w_o]
@@ -207,7 +207,9 @@ class GatedDeltaRule(_StateMixer):
         G, H, dk, dv = self.num_kv_heads, self.num_heads, self.dk, self.dv
         qkv = ops.short_conv_silu(st.cut(proj, "q", "v"), self.conv_w, state[:, self.memory:], step)
         if self.low_rank:
-            second = ops.linear(st.cut(proj, "a1", "g1"), self.w_second, out_dtype=torch.float32)
+            second = torch.empty((x.shape[0], self.w_second.shape[0]), dtype=torch.float32, device=x.device)
+            if x.shape[0]:
+                ops.gemm_simt(st.cut(proj, "a1", "g1"), self.w_second, None, second, blocks=self.second_blocks)
             step_pre, gate = second[:, :self.decay_size], second[:, self.decay_size:]
         else:
             step_pre, gate = st.cut(proj, "a"), st.cut(proj, "g")

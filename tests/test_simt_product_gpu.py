@@ -38,3 +38,16 @@ def test_a_row_does_not_depend_on_the_other_rows(N, K):
     whole = product(x, w, None, torch.float32)
     for at, n in ((0, 1), (5, 16), (100, 17), (300, 400)):
         assert torch.equal(product(x[at:at + n], w, None, torch.float32), whole[at:at + n]), (at, n)
+
+
+@pytest.mark.parametrize("M,rows,cols,N,K", [(5, 130, 24, 300, 48), (70, 256, 64, 512, 128), (65, 1, 3, 400, 10), (33, 128, 100, 200, 700)])
+def test_block_diagonal_weight(M, rows, cols, N, K):
+    """Leaving the zero blocks out changes no bit."""
+    from coheryn_ai_studio_b200 import ops
+    g = torch.Generator(device=DEV).manual_seed(N)
+    x, w = torch.randn((M, K), device=DEV, generator=g), torch.randn((N, K), device=DEV, generator=g)
+    w[:rows, cols:] = 0.0
+    w[rows:, :cols] = 0.0
+    out = torch.empty((M, N), device=DEV)
+    ops.gemm_simt(x, w, None, out, blocks=(rows, cols))
+    assert torch.equal(out, product(x, w, None, torch.float32))
