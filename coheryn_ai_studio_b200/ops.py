@@ -1638,8 +1638,7 @@ def gemm_bf16_tc_grouped(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, ro
     assert rows.tile_rows == int(lib.coheryn_gemm_tc_grouped_tile_rows())
     _check(lib, lib.coheryn_gemm_bf16_tc_grouped(
         _ptr(a), _ptr(w), _ptr(out), c_int(_code(out)), c_int(rows.n), c_int(N), c_int(K), c_int(G), c_long(a.stride(0)),
-        c_long(out.stride(0)), c_int(int(epilogue)), _ptr(rows.tile_group), _ptr(rows.tile_row0), _ptr(rows.offsets),
-        _ptr(rows.n_tiles), c_int(rows.max_tiles), _ptr(tc_status(a.device)), _stream()))
+        c_long(out.stride(0)), c_int(int(epilogue)), _ptr(rows.offsets), _ptr(tc_status(a.device)), _stream()))
 
 
 def grouped_linear(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, rows: Optional[RoutedRows] = None,
