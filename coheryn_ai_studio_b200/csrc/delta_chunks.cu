@@ -432,6 +432,9 @@ __global__ void __launch_bounds__(THREADS, 3) delta_solve_kernel(DeltaIn P, int 
 template <int DK>
 constexpr size_t state_smem() { return sizeof(float) * (2 * (2 * CH * DK + CH * VS + DK) + DK * VS + CH * VS + 8 * CH * VS); }
 constexpr int STATE_THREADS = 512;
+// Where a row of the parts lies: neighbouring groups of four rows swap odd and even, so that the eight lanes that store a
+// 16-byte piece each of two such groups fall on all banks.
+__device__ __forceinline__ int slot_of(int row) { return row ^ ((row >> 2) & 1); }
 
 template <int DK>
 __global__ void __launch_bounds__(STATE_THREADS, 1) delta_state_kernel(DeltaIn P, int B, float* __restrict__ scratch, int dvp) {
@@ -485,15 +488,15 @@ __global__ void __launch_bounds__(STATE_THREADS, 1) delta_state_kernel(DeltaIn P
         mac4(acc, ld4(wt + d * CH + t), ld4(S + d * VS + lb));
       }
 #pragma unroll
-      for (int i = 0; i < 4; ++i) st4(part + (slice * CH + t + i) * VS + lb, make_float4(acc[i][0], acc[i][1], acc[i][2], acc[i][3]));
+      for (int i = 0; i < 4; ++i) st4(part + (slice * CH + slot_of(t + i)) * VS + lb, make_float4(acc[i][0], acc[i][1], acc[i][2], acc[i][3]));
     }
     __syncthreads();
     if (tid < CH * VS / 4) {
       const int t = tid >> 2, c4 = 4 * (tid & 3);
-      float4 w = ld4(part + t * VS + c4);
+      float4 w = ld4(part + slot_of(t) * VS + c4);
 #pragma unroll
       for (int p = 1; p < 8; ++p) {
-        const float4 x = ld4(part + (p * CH + t) * VS + c4);
+        const float4 x = ld4(part + (p * CH + slot_of(t)) * VS + c4);
         w.x += x.x; w.y += x.y; w.z += x.z; w.w += x.w;
       }
       float4 u = ld4(uv + t * VS + c4);
@@ -513,15 +516,16 @@ __global__ void __launch_bounds__(STATE_THREADS, 1) delta_state_kernel(DeltaIn P
         mac4(acc, ld4(kh + t * DK + d), ld4(U + t * VS + lb));
       }
 #pragma unroll
-      for (int i = 0; i < 4; ++i) st4(part + (kg * DK + d + i) * VS + lb, make_float4(acc[i][0], acc[i][1], acc[i][2], acc[i][3]));
+      for (int i = 0; i < 4; ++i) st4(part + (kg * DK + slot_of(d + i)) * VS + lb, make_float4(acc[i][0], acc[i][1], acc[i][2], acc[i][3]));
     }
     __syncthreads();
     for (int e = tid; e < DK * VS / 4; e += STATE_THREADS) {
       const float f = dec[e >> 2];
-      float4 s = ld4(S + 4 * e), x = ld4(part + 4 * e);
+      const int at = slot_of(e >> 2) * VS + 4 * (e & 3);
+      float4 s = ld4(S + 4 * e), x = ld4(part + at);
 #pragma unroll
       for (int p = 1; p < KG; ++p) {
-        const float4 y = ld4(part + p * DK * VS + 4 * e);
+        const float4 y = ld4(part + p * DK * VS + at);
         x.x += y.x; x.y += y.y; x.z += y.z; x.w += y.w;
       }
       s.x = fmaf(f, s.x, x.x); s.y = fmaf(f, s.y, x.y); s.z = fmaf(f, s.z, x.z); s.w = fmaf(f, s.w, x.w);
