@@ -410,7 +410,7 @@ gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_x, const __gri
   const int tiles_m = (M + BM - 1) / BM, tiles_n = (N + BN - 1) / BN;
   const int num_tiles = tiles_m * tiles_n;
   const int k_tiles = (K + BK - 1) / BK;
-  constexpr int TMEM_COLS = 2 * BN < 32 ? 32 : 2 * BN;
+  constexpr int TMEM_COLS = 2 * BN <= 32 ? 32 : (2 * BN <= 64 ? 64 : (2 * BN <= 128 ? 128 : (2 * BN <= 256 ? 256 : 512)));
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < STAGES; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
@@ -1087,6 +1087,21 @@ static int splits_for(int M, int N, int K, int bn) {
   return s < 2 ? 1 : s;
 }
 
+// The tile width of the persistent kernel: the one whose rounds over the SMs cost least, rounds times columns (a last round of
+// 256 columns that is nearly empty is paid for like a full one).  Measured on a B200, alone, L2 flushed, M x N x K with 256 columns
+// and with the width chosen: 2048 x 4748 x 1536 51.2 -> 47.1 us (192), 1873 x 3584 x 18944 233 -> 215 (192), 1560 x 4620 x 1536
+// 41.0 -> 36.9 (224), 1100 x 4864 x 1536 34.8 -> 29.5 (160), 2560 x 2600 x 1536 39.7 -> 33.6 (192).
+static int persistent_width(int M, int N) {
+  const long tiles_m = (M + BM - 1) / BM;
+  int best = 256;
+  long cost = 0;
+  for (int bn = 256; bn >= 160; bn -= 32) {
+    const long c = (tiles_m * ((N + bn - 1) / bn) + 147) / 148 * bn;
+    if (bn == 256 || c * 20 < cost * 19) { best = bn; cost = c; }      // by a twentieth at least: narrow tiles read more per product
+  }
+  return best;
+}
+
 // Floats of workspace with which coheryn_gemm_bf16_tc splits K over several CTAs (0: this
 // shape is not split).  Without the workspace the product runs unsplit.
 CO_EXPORT long coheryn_gemm_tc_workspace_floats(int M, int N, int K) {
@@ -1119,12 +1134,18 @@ CO_EXPORT int coheryn_gemm_bf16_tc(const void* x, const void* w, const void* bia
   const long tiles_m = (M + BM - 1) / BM;
   int splits = splits_for(M, N, K, bn);
   if (splits > 1 && (!workspace || workspace_floats < (long)splits * M * N)) splits = 1;
+  const bool persistent = bn == 256 && g_stages != 1 && tiles_m * ((N + 255) / 256) > 148;
+  const int width = persistent ? persistent_width(M, N) : bn;
   CUtensorMap mx, mw;
-  if (!make_map(&mx, x, M, K, ldx, BM) || !make_map(&mw, w, N, K, K, bn))
+  if (!make_map(&mx, x, M, K, ldx, BM) || !make_map(&mw, w, N, K, K, width))
     CO_FAIL("gemm_bf16_tc: cuTensorMapEncodeTiled failed (M=%d N=%d K=%d ldx=%ld)", M, N, K, ldx);
 #define GO(BN_, ST_) return launch_tc<BN_, ST_>(mx, mw, bias, bias_dtype, out, out_dtype, M, N, K, ldo, epilogue, status, stream, workspace, splits)
-  if (bn == 256 && g_stages != 1 && tiles_m * ((N + 255) / 256) > 148)
-    return launch_tc_persistent<256, 4>(mx, mw, bias, bias_dtype, out, out_dtype, M, N, K, ldo, epilogue, status, stream);
+#define GO_PERSISTENT(BN_, ST_) return launch_tc_persistent<BN_, ST_>(mx, mw, bias, bias_dtype, out, out_dtype, M, N, K, ldo, epilogue, status, stream)
+  if (persistent && width == 160) GO_PERSISTENT(160, 6);
+  if (persistent && width == 192) GO_PERSISTENT(192, 5);
+  if (persistent && width == 224) GO_PERSISTENT(224, 5);
+  if (persistent) GO_PERSISTENT(256, 4);
+#undef GO_PERSISTENT
   if (bn == 256 && g_stages == 2) GO(256, 2);
   if (bn == 256 && g_stages == 3) GO(256, 3);
   if (bn == 128 && g_stages == 3) GO(128, 3);
