@@ -10,7 +10,13 @@
 // of them.  TWO passes over the key tiles: the first finds every row's maximum and sum per map (scores only), the
 // second computes the scores again (the same instructions, hence the same bits), forms
 // w = e_0 / l_0 - lambda e_1 / l_1 in float32 and accumulates w V once.  No accumulator is ever rescaled, two maps
-// cost one accumulator, and the difference of the maps is taken before anything is rounded.
+// cost one accumulator, and the difference of the maps is taken before anything is rounded.  With two maps of up to 64
+// channels and values of up to 128 two warps share the 16 rows, a map and half of the value channels each.  Bound by the
+// latency of a warp's chain (copies, scores, maxima, exponentials, products) over the key tiles of the longest row tiles, at
+// two or three warps a scheduler: hence short chains, many warps, one barrier per key tile and row tiles in the order of their
+// length.  Measured on a B200 (2,048 tokens, 12 heads over 2, two maps of 64 channels, values of 128, chunks of 1,024):
+// 118 us with one warp per 16 rows (28 % of the issue slots), 98 us with two, 87 us with a ring of three key tiles and no
+// barrier at a tile's end; three CTAs per SM at 80 registers spill and take 124 us, tiles of 64 keys with one CTA 102 us.
 //
 // Decoding (`maps_decode_kernel` + `maps_combine_kernel`): the rows of a tile are (up to sixteen of) the query heads of
 // ONE key/value head for one token, the visible keys are cut into at most sixteen splits at absolute multiples of the split size,
@@ -69,6 +75,8 @@ struct MapsArgs {
   const int* block_tables; int max_blocks;
   const int* cu_q; const int* kv_lens;
   int nh, nkv, page_size, window, chunk, keep, sink, head_norm, skip_single;
+  int page_shift;       // page_size is two to this power (-1: no power of two)
+  int requests;         // of the prompt kernel's grid
   int table_cache;      // block-table entries a CTA of the prompt kernel may keep in shared memory
   float scale_log2, lambda, eps, out_scale;
   const float* sink_scores;     // [heads]: the sink's score per head (null: 0)
@@ -142,10 +150,11 @@ __device__ __forceinline__ void load_keys(bf16* ks, bf16* vs, const MapsArgs& A,
   for (int row = tid / TPR; row < BN; row += ROWS) {
     const int j = key0 + row;
     int page = -1;
-    if (j < kv_len) page = table[j / A.page_size];
+    const int at_page = A.page_shift >= 0 ? j >> A.page_shift : j / A.page_size;
+    if (j < kv_len) page = table[at_page];
     const bool ok = page >= 0;
     const int bytes = ok ? 16 : 0;
-    const size_t at = ok ? ((size_t)page * A.nkv + kvh) * A.page_size + (size_t)(j % A.page_size) : 0;
+    const size_t at = ok ? ((size_t)page * A.nkv + kvh) * A.page_size + (size_t)(j - at_page * A.page_size) : 0;
     const bf16* ksrc = A.k_cache + at * KROW;
     bf16* kdst = ks + row * KS;
 #pragma unroll
@@ -177,9 +186,30 @@ __device__ __forceinline__ void scores(float (&s)[NT][4], const bf16* qs, const 
   }
 }
 
-// o += w V for the 16 x BN weights w (float32, in the accumulator layout of `scores`) and the BN x DV values of vs:
-// every weight as hi + lo in bfloat16.
-__device__ __forceinline__ void weights_times_values(float (&o)[OT][4], const float (&w)[NT][4], const bf16* vs, int lane) {
+// The same with a map's rows already in registers, as load_rows leaves them.
+__device__ __forceinline__ void load_rows(unsigned (&a)[DK / 16][4], const bf16* qs, int m, int lane) {
+#pragma unroll
+  for (int k = 0; k < DK / 16; ++k) ldsm_x4(a[k], qs + (lane & 15) * KS + m * DK + k * 16 + (lane >> 4) * 8);
+}
+__device__ __forceinline__ void scores_of(float (&s)[NT][4], const unsigned (&a)[DK / 16][4], const bf16* ks, int m, int lane) {
+#pragma unroll
+  for (int nt = 0; nt < NT; ++nt) s[nt][0] = s[nt][1] = s[nt][2] = s[nt][3] = 0.f;
+#pragma unroll
+  for (int k = 0; k < DK / 16; ++k) {
+#pragma unroll
+    for (int nt = 0; nt < NT; nt += 2) {
+      unsigned b[4];
+      ldsm_x4(b, ks + (nt * 8 + (lane & 7) + (lane >> 4) * 8) * KS + m * DK + k * 16 + ((lane >> 3) & 1) * 8);
+      mma16816(s[nt], a[k], b[0], b[1]);
+      mma16816(s[nt + 1], a[k], b[2], b[3]);
+    }
+  }
+}
+
+// o += w V for the 16 x BN weights w (float32, in the accumulator layout of `scores`) and 8 x TILES value channels of the BN
+// rows of vs: every weight as hi + lo in bfloat16.
+template <int TILES>
+__device__ __forceinline__ void weights_times_values(float (&o)[TILES][4], const float (&w)[NT][4], const bf16* vs, int lane) {
 #pragma unroll
   for (int kb = 0; kb < NT / 2; ++kb) {
     unsigned hi[4], lo[4];
@@ -191,12 +221,12 @@ __device__ __forceinline__ void weights_times_values(float (&o)[OT][4], const fl
       lo[i] = pack2(x - __low2float(h), y - __high2float(h));
     }
 #pragma unroll
-    for (int nt = 0; nt < OT; nt += 2) {
+    for (int nt = 0; nt < TILES; nt += 2) {
       unsigned b[4];
       ldsm_x4_t(b, vs + (kb * 16 + (lane & 7) + ((lane >> 3) & 1) * 8) * VS + nt * 8 + (lane >> 4) * 8);
       mma16816(o[nt], hi, b[0], b[1]);
-      mma16816(o[nt], lo, b[0], b[1]);
       mma16816(o[nt + 1], hi, b[2], b[3]);
+      mma16816(o[nt], lo, b[0], b[1]);
       mma16816(o[nt + 1], lo, b[2], b[3]);
     }
   }
@@ -223,29 +253,48 @@ __device__ __forceinline__ void scale_only(float (&s)[NT][4], float scale_log2) 
 }
 
 // ---------------------------------------------------------------------------------
-// Prompt portions.  grid: (row tiles of the longest request, requests, query heads).
+// Prompt portions.  grid: row tiles of the longest request x requests x query heads, in
+// the order that the kernel's first lines give.
 // ---------------------------------------------------------------------------------
+// Two maps (PAIRED; wider heads leave no registers and shared memory for two CTAs of 256 threads): two warps share 16 rows.
+// Each makes the scores, maxima, sums and exponentials of ONE map; they show one another their map's share of the weights
+// through shared memory, and each multiplies the weights by one half of the value channels.
+constexpr bool PAIRED = MAPS == 2 && KROW <= 128 && DV <= 128 && DV % 32 == 0;
+constexpr int TW = PAIRED ? 2 * WARPS : WARPS;             // warps of a CTA
+constexpr int OWN = PAIRED ? 1 : MAPS;                     // maps that a warp works on
+constexpr int OC = PAIRED ? DVC / 2 : DVC, OTW = OC / 8;   // value channels of a warp
+constexpr int STAGES = PAIRED ? 3 : 2;                     // key tiles in shared memory
+constexpr int SHOWN = PAIRED ? TW * 32 * NT * 4 : 0;       // floats of shared memory for what the warps show one another
 #ifndef CO_MAPS_MIN_CTAS
-#define CO_MAPS_MIN_CTAS ((DV <= 128 && KROW <= 128) ? 3 : 1)      // the registers of wider heads allow one
+#define CO_MAPS_MIN_CTAS (PAIRED ? 2 : (DV <= 128 && KROW <= 128) ? 3 : 1)      // the registers of wider heads allow one
 #endif
-__global__ void __launch_bounds__(WARPS * 32, CO_MAPS_MIN_CTAS) maps_tiles_kernel(MapsArgs A) {
+__device__ __forceinline__ void pair_wait(int id) { asm volatile("bar.sync %0, 64;" ::"r"(id) : "memory"); }
+__global__ void __launch_bounds__(TW * 32, CO_MAPS_MIN_CTAS) maps_tiles_kernel(MapsArgs A) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   bf16* qs = reinterpret_cast<bf16*>(smem_raw);        // [BM][KS]
-  bf16* ks = qs + BM * KS;                             // [2][BN][KS]
-  bf16* vs = ks + 2 * BN * KS;                         // [2][BN][VS]
-  int* tbl = reinterpret_cast<int*>(vs + 2 * BN * VROW); // [table_cache]
+  bf16* ks = qs + BM * KS;                             // [STAGES][BN][KS]
+  bf16* vs = ks + STAGES * BN * KS;                    // [STAGES][BN][VS]
+  float4* shown = reinterpret_cast<float4*>(vs + STAGES * BN * VROW);    // [TW][NT][32]
+  int* tbl = reinterpret_cast<int*>(vs + STAGES * BN * VROW) + SHOWN;    // [table_cache]
   co_pdl_launch_dependents();
   co_pdl_wait();
-  const int r = blockIdx.y, h = blockIdx.z;
+  // The row tiles that see the most keys start first, for all heads and requests: the last ones, or with a mask by chunks the
+  // last one of every chunk, then the ones before them.
+  const int place = (int)blockIdx.x, others = A.nh * A.requests, tiles = (int)gridDim.x / others;
+  const int r = place % others / A.nh, h = place % A.nh;
+  int tile = tiles - 1 - place / others;
+  if (A.chunk >= BM) {
+    const int per = A.chunk / BM, chunks = tiles / per, i = place / others;
+    tile = i < chunks * per ? i % chunks * per + per - 1 - i / chunks : i;
+  }
   const int q0 = A.cu_q[r], q_len = A.cu_q[r + 1] - q0, kv_len = A.kv_lens[r];
-  const int tile = (int)gridDim.x - 1 - (int)blockIdx.x;          // later rows see more keys: their CTAs start first
   if (tile * BM >= q_len || (A.skip_single && q_len == 1)) return;
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int tid = threadIdx.x, lane = tid & 31, warp = (tid >> 5) % WARPS, own = PAIRED ? (tid >> 5) / WARPS : 0;
   const int kvh = h / (A.nh / A.nkv);
   const int* table = A.block_tables + (size_t)r * A.max_blocks;
   const int rows = min(BM, q_len - tile * BM);
   const int pos_lo = kv_len - q_len + tile * BM, pos_hi = pos_lo + rows - 1;
-  for (int c = tid; c < BM * (KROW / 8); c += WARPS * 32) {       // the queries of the tile; rows beyond the portion are zeros
+  for (int c = tid; c < BM * (KROW / 8); c += TW * 32) {       // the queries of the tile; rows beyond the portion are zeros
     const int row = c / (KROW / 8), ch = c % (KROW / 8);
     const bool ok = row < rows;
     cp_async16(qs + row * KS + ch * 8, A.q + (size_t)(q0 + tile * BM + (ok ? row : 0)) * A.ldq + (size_t)h * KROW + ch * 8, ok ? 16 : 0);
@@ -258,7 +307,7 @@ __global__ void __launch_bounds__(WARPS * 32, CO_MAPS_MIN_CTAS) maps_tiles_kerne
     const int e0 = (t_lo * BN) / A.page_size, e1 = min(t_hi * BN + BN - 1, kv_len - 1) / A.page_size;
     const int kept = n_kept > 0 ? (n_kept * BN - 1) / A.page_size + 1 : 0;
     if (e1 - e0 + 1 + kept <= A.table_cache) {
-      for (int i = tid; i < kept + e1 - e0 + 1; i += WARPS * 32) tbl[i] = table[i < kept ? i : e0 + i - kept];
+      for (int i = tid; i < kept + e1 - e0 + 1; i += TW * 32) tbl[i] = table[i < kept ? i : e0 + i - kept];
       __syncthreads();
       kept_table = tbl;
       table = tbl + kept - e0;
@@ -280,26 +329,38 @@ __global__ void __launch_bounds__(WARPS * 32, CO_MAPS_MIN_CTAS) maps_tiles_kerne
   auto unseen_tile = [&](int key0) { return warp * 16 >= rows || key0 > wp_hi || (key0 + BN - 1 < wf_lo && key0 >= A.keep); };
   auto open_tile = [&](int key0) { return whole_warp && key0 + BN - 1 <= wp_lo && (key0 >= wf_hi || key0 + BN <= A.keep); };
 
-  // pass 1: maximum and sum of every row, per map
-  float mx[MAPS][2], sum[MAPS][2];
-#pragma unroll
-  for (int m = 0; m < MAPS; ++m) { mx[m][0] = mx[m][1] = -INFINITY; sum[m][0] = sum[m][1] = 0.f; }
-  load_keys<WARPS * 32>(ks, nullptr, A, n_kept ? kept_table : table, kvh, first_key(0), kv_len, tid);
-  cp_commit();
-  for (int i = 0; i < n_tiles; ++i) {
-    if (i + 1 < n_tiles)
-      load_keys<WARPS * 32>(ks + ((i + 1) & 1) * BN * KS, nullptr, A, i + 1 < n_kept ? kept_table : table, kvh, first_key(i + 1), kv_len, tid);
+  unsigned qf[DK / 16][4];       // PAIRED: the warp's rows of its map, once their copies (the first group to land) are here
+  auto tile_scores = [&](float (&s)[NT][4], const bf16* kt, int m) {
+    if (PAIRED) scores_of(s, qf, kt, m, lane);
+    else scores(s, qw, kt, m, lane);
+  };
+
+  // Tile i into its place in the ring, as a group of copies of its own (an empty one beyond the last tile).
+  auto fetch = [&](int i, bool values) {
+    if (i < n_tiles)
+      load_keys<TW * 32>(ks + (i % STAGES) * BN * KS, values ? vs + (i % STAGES) * BN * VS : nullptr, A, i < n_kept ? kept_table : table, kvh,
+                         first_key(i), kv_len, tid);
     cp_commit();
-    cp_wait<1>();
-    __syncthreads();
-    const bf16* kt = ks + (i & 1) * BN * KS;
+  };
+
+  // pass 1: maximum and sum of every row, per map (own + m: the map)
+  float mx[OWN][2], sum[OWN][2];
+#pragma unroll
+  for (int m = 0; m < OWN; ++m) { mx[m][0] = mx[m][1] = -INFINITY; sum[m][0] = sum[m][1] = 0.f; }
+  for (int i = 0; i < STAGES - 1; ++i) fetch(i, false);
+  for (int i = 0; i < n_tiles; ++i) {
+    cp_wait<STAGES - 2>();
+    __syncthreads();                             // tile i is here, and tile i - 1 is read no more
+    fetch(i + STAGES - 1, false);
+    if (PAIRED && i == 0) load_rows(qf, qw, own, lane);
+    const bf16* kt = ks + (i % STAGES) * BN * KS;
     const int key0 = first_key(i);
     const bool unseen = unseen_tile(key0), open = open_tile(key0);
 #pragma unroll
-    for (int m = 0; m < MAPS; ++m) {
+    for (int m = 0; m < OWN; ++m) {
       if (unseen) break;
       float s[NT][4];
-      scores(s, qw, kt, m, lane);
+      tile_scores(s, kt, own + m);
       if (open) scale_only(s, A.scale_log2);
       else mask_scale(s, key0, lane, pos, first, A.keep, A.scale_log2);
 #pragma unroll
@@ -318,11 +379,10 @@ __global__ void __launch_bounds__(WARPS * 32, CO_MAPS_MIN_CTAS) maps_tiles_kerne
         }
       }
     }
-    __syncthreads();
   }
-  float inv[MAPS][2];
+  float inv[OWN][2];
 #pragma unroll
-  for (int m = 0; m < MAPS; ++m)
+  for (int m = 0; m < OWN; ++m)
 #pragma unroll
     for (int rr = 0; rr < 2; ++rr) {
       float l = quad_sum(sum[m][rr]), M = mx[m][rr];
@@ -339,62 +399,85 @@ __global__ void __launch_bounds__(WARPS * 32, CO_MAPS_MIN_CTAS) maps_tiles_kerne
 
   // pass 2: the weights, and their product with the values (once per chunk of value channels)
   for (int vc = 0; vc < NCH; ++vc) {
-  if (vc) __syncthreads();                       // the last tile of the chunk before is read no more
-  float o[OT][4];
+  cp_wait<0>();
+  __syncthreads();                               // the last tiles of the pass before are read no more
+  float o[OTW][4];
 #pragma unroll
-  for (int nt = 0; nt < OT; ++nt) o[nt][0] = o[nt][1] = o[nt][2] = o[nt][3] = 0.f;
-  load_keys<WARPS * 32>(ks, vs, A, n_kept ? kept_table : table, kvh, first_key(0), kv_len, tid);
-  cp_commit();
+  for (int nt = 0; nt < OTW; ++nt) o[nt][0] = o[nt][1] = o[nt][2] = o[nt][3] = 0.f;
+  for (int i = 0; i < STAGES - 1; ++i) fetch(i, true);
   for (int i = 0; i < n_tiles; ++i) {
-    if (i + 1 < n_tiles)
-      load_keys<WARPS * 32>(ks + ((i + 1) & 1) * BN * KS, vs + ((i + 1) & 1) * BN * VS, A, i + 1 < n_kept ? kept_table : table, kvh,
-                            first_key(i + 1), kv_len, tid);
-    cp_commit();
-    cp_wait<1>();
+    cp_wait<STAGES - 2>();
     __syncthreads();
-    const bf16* kt = ks + (i & 1) * BN * KS;
+    fetch(i + STAGES - 1, true);
+    const bf16* kt = ks + (i % STAGES) * BN * KS;
     const int key0 = first_key(i);
     const bool unseen = unseen_tile(key0), open = open_tile(key0);
     if (!unseen) {
     float w[NT][4];
     {
       float s[NT][4];
-      scores(s, qw, kt, 0, lane);
+      tile_scores(s, kt, own);
       if (open) scale_only(s, A.scale_log2);
       else mask_scale(s, key0, lane, pos, first, A.keep, A.scale_log2);
 #pragma unroll
       for (int nt = 0; nt < NT; ++nt)
 #pragma unroll
         for (int e = 0; e < 4; ++e) w[nt][e] = ex2(s[nt][e] - mx[0][e >> 1]) * inv[0][e >> 1];
-      if (MAPS == 2) {
+      if constexpr (PAIRED) {
+        float4* mine = shown + ((own * WARPS + warp) * NT) * 32 + lane;
+#pragma unroll
+        for (int nt = 0; nt < NT; ++nt) mine[nt * 32] = make_float4(w[nt][0], w[nt][1], w[nt][2], w[nt][3]);
+        pair_wait(1 + warp);
+        const float4* other = shown + (((own ^ 1) * WARPS + warp) * NT) * 32 + lane;
+#pragma unroll
+        for (int nt = 0; nt < NT; ++nt) {
+          const float4 x = other[nt * 32];
+          const float y[4] = {x.x, x.y, x.z, x.w};
+#pragma unroll
+          for (int e = 0; e < 4; ++e) w[nt][e] = own ? y[e] - A.lambda * w[nt][e] : w[nt][e] - A.lambda * y[e];
+        }
+      } else if constexpr (MAPS == 2) {
         scores(s, qw, kt, MAPS - 1, lane);
         if (open) scale_only(s, A.scale_log2);
         else mask_scale(s, key0, lane, pos, first, A.keep, A.scale_log2);
 #pragma unroll
         for (int nt = 0; nt < NT; ++nt)
 #pragma unroll
-          for (int e = 0; e < 4; ++e) w[nt][e] -= A.lambda * (ex2(s[nt][e] - mx[MAPS - 1][e >> 1]) * inv[MAPS - 1][e >> 1]);
+          for (int e = 0; e < 4; ++e) w[nt][e] -= A.lambda * (ex2(s[nt][e] - mx[OWN - 1][e >> 1]) * inv[OWN - 1][e >> 1]);
       }
     }
-    weights_times_values(o, w, (V_IN_K ? kt : vs + (i & 1) * BN * VS) + vc * DVC, lane);
+    weights_times_values(o, w, (V_IN_K ? kt : vs + (i % STAGES) * BN * VS) + vc * DVC + own * OC, lane);
     }
-    __syncthreads();
+  }
+  float squares[2];
+  if (A.head_norm) {                             // (the launcher refuses it for values in several chunks)
+#pragma unroll
+    for (int rr = 0; rr < 2; ++rr) {
+      float ss = 0.f;
+#pragma unroll
+      for (int nt = 0; nt < OTW; ++nt) ss += o[nt][2 * rr] * o[nt][2 * rr] + o[nt][2 * rr + 1] * o[nt][2 * rr + 1];
+      squares[rr] = quad_sum(ss);
+    }
+    if constexpr (PAIRED) {                      // the sums of both halves, the first half's first
+      float2* half = reinterpret_cast<float2*>(shown) + warp * 32 + lane;
+      pair_wait(1 + warp);                       // the other warp has read the last tile's weights
+      half[own * WARPS * 32] = make_float2(squares[0], squares[1]);
+      pair_wait(1 + warp);
+      const float2 a = half[0], b = half[WARPS * 32];
+      squares[0] = a.x + b.x;
+      squares[1] = a.y + b.y;
+    }
   }
 #pragma unroll
   for (int rr = 0; rr < 2; ++rr) {
     const int row = warp * 16 + (lane >> 2) + 8 * rr;
     float factor = A.out_scale;
-    if (A.head_norm) {                           // (the launcher refuses it for values in several chunks)
-      float ss = 0.f;
-#pragma unroll
-      for (int nt = 0; nt < OT; ++nt) ss += o[nt][2 * rr] * o[nt][2 * rr] + o[nt][2 * rr + 1] * o[nt][2 * rr + 1];
-      factor *= 1.0f / sqrtf(quad_sum(ss) / (float)DV + A.eps);
-    }
+    if (A.head_norm) factor *= 1.0f / sqrtf(squares[rr] / (float)DV + A.eps);
     if (row < rows) {
       factor *= gate_of(A, (size_t)(q0 + tile * BM + row), h);
-      bf16* orow = A.out + (size_t)(q0 + tile * BM + row) * A.ldo + (size_t)h * DV + vc * DVC + 2 * (lane & 3);
+      bf16* orow = A.out + (size_t)(q0 + tile * BM + row) * A.ldo + (size_t)h * DV + vc * DVC + own * OC + 2 * (lane & 3);
 #pragma unroll
-      for (int nt = 0; nt < OT; ++nt)
+      for (int nt = 0; nt < OTW; ++nt)
         *reinterpret_cast<__nv_bfloat162*>(orow + nt * 8) = __floats2bfloat162_rn(o[nt][2 * rr] * factor, o[nt][2 * rr + 1] * factor);
     }
   }
@@ -613,16 +696,19 @@ CO_EXPORT int coheryn_attention_maps_bf16(const void* q, long ldq, void* out, lo
   if (head_norm && NCH > 1) CO_FAIL("attention_maps_bf16: a normalised output needs values of at most 256 channels (%d)", DV);
   const int blocks = (nh / nkv + 15) / 16;             // of query heads per kv head
   const bool decode = any_single != 0;
+  const int page_shift = (page_size & (page_size - 1)) == 0 ? __builtin_ctz((unsigned)page_size) : -1;
   MapsArgs A{(const bf16*)q, ldq, (bf16*)out, ldo, (const bf16*)k_cache, (const bf16*)v_cache, block_tables, max_blocks, cu_q,
-             kv_lens, nh, nkv, page_size, window, chunk, keep, sink, head_norm, decode ? 1 : 0, 0,
+             kv_lens, nh, nkv, page_size, window, chunk, keep, sink, head_norm, decode ? 1 : 0, page_shift, B, 0,
              scale * 1.4426950408889634f, lambda, eps, out_scale, sink_scores, gates, gates_ld};
   if (any_longer || !decode) {
     const int visible = most_visible(max_kv_len, window, chunk, keep);      // the most keys a row can see
     const long entries = ((long)visible + BM + 3 * BN) / page_size + 3;
     A.table_cache = entries <= 4096 ? (int)entries : 0;    // a longer table is read from global memory
-    const size_t smem = ((size_t)BM * KS + (size_t)2 * BN * KS + (size_t)2 * BN * VROW) * sizeof(bf16) + (size_t)A.table_cache * sizeof(int);
+    const size_t smem = ((size_t)BM * KS + (size_t)STAGES * BN * (KS + VROW)) * sizeof(bf16) + (size_t)(SHOWN + A.table_cache) * sizeof(int);
     if (smem > 48 * 1024) cudaFuncSetAttribute(maps_tiles_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    co_launch(maps_tiles_kernel, dim3((max_q_len + BM - 1) / BM, B, nh), dim3(WARPS * 32), smem, stream, A);
+    const long ctas = (long)((max_q_len + BM - 1) / BM) * B * nh;
+    if (ctas > 0x7fffffffL) CO_FAIL("attention_maps_bf16: %ld row tiles are too many", ctas);
+    co_launch(maps_tiles_kernel, dim3((unsigned)ctas), dim3(TW * 32), smem, stream, A);
     CO_CHECK_LAUNCH("maps_tiles");
   }
   if (decode) {
