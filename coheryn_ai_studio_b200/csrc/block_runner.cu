@@ -84,7 +84,7 @@ struct CoBlockStep {
   int* tc_status;
   cudaStream_t stream;
   int T, B, min_q_len, max_q_len, max_kv_len, settled;
-  int longer_than[17];    // [n]: requests of more than n tokens
+  const int* q_lens;      // on the host: tokens of every request (null: not counted)
 };
 
 // ops.py's thresholds, as they stand when the step is run.
@@ -322,7 +322,11 @@ int block_pass(const CoBlockLayer& L, const CoBlockStep& S, const CoBlockTuning&
     if (Nq % 4) return CO_BLOCK_UNSUPPORTED;
     const int max_rows = S.max_q_len * G;
     const int any_small = S.min_q_len * G <= 16;
-    const int large = G <= 16 ? S.longer_than[16 / G] : B;      // requests of more than 16 rows per kv head
+    int large = max_rows > 16 ? B : 0;      // requests of more than 16 rows per kv head (at most)
+    if (large && S.q_lens) {
+      large = 0;
+      for (int r = 0; r < B; ++r) large += S.q_lens[r] * G > 16;
+    }
     long floats = 0;
     float* as = nullptr;
     if (any_small && G <= 16) {

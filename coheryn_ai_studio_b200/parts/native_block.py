@@ -12,7 +12,6 @@ cover) takes the parts' own path: ``run`` returns None.
 """
 from __future__ import annotations
 
-import bisect
 import ctypes
 from ctypes import c_float, c_int, c_long, c_void_p
 from typing import Optional
@@ -34,8 +33,7 @@ class CoBlockLayer(ctypes.Structure):
 
 class CoBlockStep(ctypes.Structure):
     _fields_ = [(n, P) for n in ("positions", "cu_q", "kv_lens", "tc_status", "stream")] + \
-               [(n, c_int) for n in ("T", "B", "min_q_len", "max_q_len", "max_kv_len", "settled")] + \
-               [("longer_than", c_int * 17)]
+               [(n, c_int) for n in ("T", "B", "min_q_len", "max_q_len", "max_kv_len", "settled")] + [("q_lens", P)]
 
 
 class CoBlockTuning(ctypes.Structure):
@@ -98,14 +96,6 @@ def _entry_point():
     return _entry
 
 
-def _longer_than(q_lens):
-    """For n from 0 to 16 how many requests bring more than n tokens."""
-    if max(q_lens) == 1:
-        return [len(q_lens)] + [0] * 16
-    ordered = sorted(q_lens)
-    return [len(ordered) - bisect.bisect_right(ordered, n) for n in range(17)]
-
-
 class StepNative:
     """What every block of one step shares: the step's description and thresholds as the library
     reads them, the pointers of each cache group's tables, and per kind of layer the plan (kind of
@@ -118,10 +108,14 @@ class StepNative:
                 or not (_i32(step.positions) and _i32(step.cu_q) and _i32(step.kv_lens))):
             return
         device = step.positions.device
+        # The requests' lengths, for the grid of the prompts' attention, where short requests may be many beside longer ones.
+        # Elsewhere the grid covers every request: to hand the lengths over costs the host 1 us of the 55 that a block takes.
+        n, shortest, longest = len(q_lens), min(q_lens), max(q_lens)
+        self.q_lens = (c_int * n)(*q_lens) if n > 3 and shortest <= 16 < longest else None
         self.step = CoBlockStep(step.positions.data_ptr(), step.cu_q.data_ptr(), step.kv_lens.data_ptr(),
-                                ops.tc_status(device).data_ptr(), ops._stream().value or 0, step.num_tokens, len(q_lens),
-                                min(q_lens), max(q_lens), step.max_kv_len, 1 if step.prior_positions_settled else 0,
-                                (c_int * 17)(*_longer_than(q_lens)))
+                                ops.tc_status(device).data_ptr(), ops._stream().value or 0, step.num_tokens, n,
+                                shortest, longest, step.max_kv_len, 1 if step.prior_positions_settled else 0,
+                                ctypes.addressof(self.q_lens) if self.q_lens is not None else None)
         self.tuning = CoBlockTuning(ops.SMALL_WEIGHT_ELEMENTS, ops.FEW_LARGE_WEIGHT, ops.ATTN_OPROJ_MERGE_BYTES, ops.FEW_M,
                                     ops.FEW_DEFER_M, ops.FEW_HEAD_M, ops.SMALL_M, ops.SMALL_M_SHORT, ops.DEFER_MIN_K,
                                     ops.DEFER_MIN_K_WIDE, ops.QKV_ROPE_M, ops.QKV_PARTS_M, ops.QKV_PARTS_FEW_FROM,
