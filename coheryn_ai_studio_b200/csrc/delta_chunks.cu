@@ -19,7 +19,7 @@
 //
 // What bounds it: the scan token by token is a chain of dependent multiply-adds and shuffles, 0.55 us per token whatever the
 // chip could do beside it.  Here the chain is two products of 64 x 128 x 16 per chunk; measured on a B200 (12 heads of 128 x
-// 128, one request of 2,048 tokens) the four kernels take 271 us in place of 1,150 us for the scan with its preparation.
+// 128, one request of 2,048 tokens) the four kernels take 264 us (70, 36, 100 and 58) in place of 1,150 us for the scan with its preparation.
 //
 // A run of fewer than CHUNK_FROM tokens is left to the scan (recurrent.cu), request by request, so that a row's order of
 // additions depends on its place in its own request's run only.

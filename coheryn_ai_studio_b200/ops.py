@@ -1614,7 +1614,8 @@ def route_sort(ids: torch.Tensor, experts: int, wide_tiles: bool = False) -> Rou
     return r
 
 
-# Pairs per expert (on average) from which the routed products take the TMA + tcgen05 kernel: its row tiles are 128 rows.
+# Pairs per expert (on average) from which the routed products take the TMA + tcgen05 kernel: pairs of CTAs over 256 features
+# and up to 256 rows of one expert.
 GROUPED_TC_MIN_ROWS = int(os.environ.get("COHERYN_GROUPED_TC_MIN_ROWS", "48"))
 
 

@@ -21,7 +21,7 @@ that every token uses; with ``gate`` its output is multiplied by sigmoid(w . x),
 
 The pairs (token, choice) that name a real expert are ordered by expert on the device, each expert's rows meet its
 matrices in one grouped product (gate and up interleaved, the activation in the epilogue; then down; with many rows per
-expert the products are the TMA + tcgen05 kernel of the dense layers over row tiles of 128, with fewer the kernel of
+expert the products are a TMA + tcgen05 kernel over pairs of CTAs (256 features, up to 256 rows of an expert), with fewer the kernel of
 ``csrc/routed.cu`` over tiles of 64, which reads the tokens' rows through the index), and a last kernel
 adds a token's weighted rows in the order of its choices, so a token's result does not depend on the other tokens of the
 step.  Nothing is read back to the host: the part can be captured in a CUDA graph.
