@@ -265,6 +265,12 @@ constexpr int OWN = PAIRED ? 1 : MAPS;                     // maps that a warp w
 constexpr int OC = PAIRED ? DVC / 2 : DVC, OTW = OC / 8;   // value channels of a warp
 constexpr int STAGES = PAIRED ? 3 : 2;                     // key tiles in shared memory
 constexpr int SHOWN = PAIRED ? TW * 32 * NT * 4 : 0;       // floats of shared memory for what the warps show one another
+// Where a warp shows its weights (in float4, from the area's beginning) and where a pair exchanges its sums of squares: inside
+// the place of its own first warp's weights.  Between the last key tile and the sums only the pair itself is waited for, and
+// another pair may still read its weights of that tile.
+constexpr int weights_at(int own, int warp) { return (own * WARPS + warp) * NT * 32; }
+constexpr int squares_at(int own, int warp) { return weights_at(0, warp) + own * 16; }      // 32 float2
+static_assert(squares_at(1, WARPS - 1) + 16 <= weights_at(0, WARPS - 1) + NT * 32, "a pair's sums lie inside its own weights");
 #ifndef CO_MAPS_MIN_CTAS
 #define CO_MAPS_MIN_CTAS (PAIRED ? 2 : (DV <= 128 && KROW <= 128) ? 3 : 1)      // the registers of wider heads allow one
 #endif
@@ -424,11 +430,11 @@ __global__ void __launch_bounds__(TW * 32, CO_MAPS_MIN_CTAS) maps_tiles_kernel(M
 #pragma unroll
         for (int e = 0; e < 4; ++e) w[nt][e] = ex2(s[nt][e] - mx[0][e >> 1]) * inv[0][e >> 1];
       if constexpr (PAIRED) {
-        float4* mine = shown + ((own * WARPS + warp) * NT) * 32 + lane;
+        float4* mine = shown + weights_at(own, warp) + lane;
 #pragma unroll
         for (int nt = 0; nt < NT; ++nt) mine[nt * 32] = make_float4(w[nt][0], w[nt][1], w[nt][2], w[nt][3]);
         pair_wait(1 + warp);
-        const float4* other = shown + (((own ^ 1) * WARPS + warp) * NT) * 32 + lane;
+        const float4* other = shown + weights_at(own ^ 1, warp) + lane;
 #pragma unroll
         for (int nt = 0; nt < NT; ++nt) {
           const float4 x = other[nt * 32];
@@ -459,11 +465,11 @@ __global__ void __launch_bounds__(TW * 32, CO_MAPS_MIN_CTAS) maps_tiles_kernel(M
       squares[rr] = quad_sum(ss);
     }
     if constexpr (PAIRED) {                      // the sums of both halves, the first half's first
-      float2* half = reinterpret_cast<float2*>(shown) + warp * 32 + lane;
+      auto half = [&](int which) -> float2& { return reinterpret_cast<float2*>(shown + squares_at(which, warp))[lane]; };
       pair_wait(1 + warp);                       // the other warp has read the last tile's weights
-      half[own * WARPS * 32] = make_float2(squares[0], squares[1]);
+      half(own) = make_float2(squares[0], squares[1]);
       pair_wait(1 + warp);
-      const float2 a = half[0], b = half[WARPS * 32];
+      const float2 a = half(0), b = half(1);
       squares[0] = a.x + b.x;
       squares[1] = a.y + b.y;
     }
