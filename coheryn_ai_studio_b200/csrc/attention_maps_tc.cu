@@ -274,6 +274,16 @@ static_assert(squares_at(1, WARPS - 1) + 16 <= weights_at(0, WARPS - 1) + NT * 3
 #ifndef CO_MAPS_MIN_CTAS
 #define CO_MAPS_MIN_CTAS (PAIRED ? 2 : (DV <= 128 && KROW <= 128) ? 3 : 1)      // the registers of wider heads allow one
 #endif
+// The row tile that starts as the i-th of `tiles`, for all heads and requests: those that see the most keys first.  Without a mask
+// by chunks (or with chunks of less than a row tile) the last ones; with one, the row tiles at the end of a chunk, then those
+// before them, the last chunk's among them as far as it reaches.
+__host__ __device__ inline int tile_in_order(int i, int tiles, int chunk) {
+  if (chunk < BM) return tiles - 1 - i;
+  const int per = chunk / BM, whole = tiles / per, rest = tiles % per, beyond = (per - rest) * whole;    // tiles at places from `rest` on
+  if (i < beyond) return i % whole * per + per - 1 - i / whole;
+  i -= beyond;
+  return i % (whole + 1) * per + rest - 1 - i / (whole + 1);
+}
 __device__ __forceinline__ void pair_wait(int id) { asm volatile("bar.sync %0, 64;" ::"r"(id) : "memory"); }
 __global__ void __launch_bounds__(TW * 32, CO_MAPS_MIN_CTAS) maps_tiles_kernel(MapsArgs A) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -284,15 +294,8 @@ __global__ void __launch_bounds__(TW * 32, CO_MAPS_MIN_CTAS) maps_tiles_kernel(M
   int* tbl = reinterpret_cast<int*>(vs + STAGES * BN * VROW) + SHOWN;    // [table_cache]
   co_pdl_launch_dependents();
   co_pdl_wait();
-  // The row tiles that see the most keys start first, for all heads and requests: the last ones, or with a mask by chunks the
-  // last one of every chunk, then the ones before them.
   const int place = (int)blockIdx.x, others = A.nh * A.requests, tiles = (int)gridDim.x / others;
-  const int r = place % others / A.nh, h = place % A.nh;
-  int tile = tiles - 1 - place / others;
-  if (A.chunk >= BM) {
-    const int per = A.chunk / BM, chunks = tiles / per, i = place / others;
-    tile = i < chunks * per ? i % chunks * per + per - 1 - i / chunks : i;
-  }
+  const int r = place % others / A.nh, h = place % A.nh, tile = tile_in_order(place / others, tiles, A.chunk);
   const int q0 = A.cu_q[r], q_len = A.cu_q[r + 1] - q0, kv_len = A.kv_lens[r];
   if (tile * BM >= q_len || (A.skip_single && q_len == 1)) return;
   const int tid = threadIdx.x, lane = tid & 31, warp = (tid >> 5) % WARPS, own = PAIRED ? (tid >> 5) / WARPS : 0;
@@ -656,6 +659,10 @@ __global__ void __launch_bounds__(128) maps_combine_kernel(MapsArgs A, const flo
 }  // namespace
 
 CO_EXPORT int coheryn_maps_shape(int* dk, int* dv, int* maps) { *dk = DK; *dv = DV; *maps = MAPS; return 0; }
+// The row tiles of a prompt portion in the order in which they start: tile_of[i], i < tiles.
+CO_EXPORT void coheryn_maps_tile_order(int tiles, int chunk, int* tile_of) {
+  for (int i = 0; i < tiles; ++i) tile_of[i] = tile_in_order(i, tiles, chunk);
+}
 CO_EXPORT int coheryn_maps_values_in_keys() { return V_IN_K ? 1 : 0; }
 
 // How the keys a decoded row can see are cut: the keys per split (a multiple of what a CTA's warps take in one round, cut at
