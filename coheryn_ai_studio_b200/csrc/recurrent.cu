@@ -15,8 +15,10 @@
 // of S, each holding a contiguous part of its key channels in registers, so a token costs each thread DK / SPLIT
 // steps and two small shuffle reductions (the column's dot products with k and with q, added in a fixed tree);
 // the per-token vectors (q, k, decays, gates) of a chunk of tokens are staged and prepared in shared memory by
-// the whole CTA.  A token's result depends on the state and the tokens of its own request before it only.  Long runs are
-// taken in chunks instead (delta_chunks.cu, memory_chunks.cu).
+// the whole CTA.  A token's result depends on the state and the tokens of its own request before it only, in an order of
+// operations that is the same however the sequence was cut into steps (the matrix memory's to a last bit, where a long prompt's
+// heads are split over CTAs).  Where the caller allows it long runs are taken in chunks instead (delta_chunks.cu,
+// memory_chunks.cu), whose order of operations begins anew with the run.
 #include "recurrent.cuh"
 
 namespace {
@@ -149,6 +151,19 @@ __global__ void __launch_bounds__(256) head_norm_gate_kernel(HeadOut E, int T, i
   }
   __syncthreads();
   head_out_chunk(E, smem, dv, dv, nt, row0, h);
+}
+
+// n and m of the matrix memory from the side into the state (see HeadOut::nm_next).
+__global__ void memory_nm_commit_kernel(const float* __restrict__ nm, float* __restrict__ state, long state_stride,
+                                        const int* __restrict__ state_slots, const int* __restrict__ cu_q, int heads, int dk, int dv) {
+  co_pdl_launch_dependents();
+  co_pdl_wait();
+  const int r = blockIdx.x, h = blockIdx.y;
+  if (cu_q[r + 1] - cu_q[r] <= 0) return;
+  float* slot = state + (size_t)state_slots[r] * state_stride;
+  const float* from = nm + ((size_t)r * heads + h) * (dk + 1);
+  for (int d = threadIdx.x; d < dk; d += blockDim.x) slot[(size_t)heads * dk * dv + (size_t)h * dk + d] = from[d];
+  if (threadIdx.x == 0) slot[(size_t)heads * dk * dv + (size_t)heads * dk + h] = from[dk];
 }
 
 // ---------------------------------------------------------------------------------
@@ -598,6 +613,157 @@ __global__ void __launch_bounds__(512) matrix_memory_scan_kernel(MemoryIn P, Hea
   }
 }
 
+// For long prompts the normaliser n is kept by every thread for its own part of the key channels (beside its part of S), so
+// that n . q comes out of the token loop like the columns' products and no warp walks the chunk alone first; what is left
+// of the scalar part is the running maximum and the two factors of a token: lf leaves as a, li as b, em as exp(-m).
+__device__ __forceinline__ void memory_factors(float& m, float* li, float* lf, float* em, int nt, int lane) {
+  for (int i = 0; i < nt; ++i) {
+    const float f = lf[i], in = li[i];
+    const float m_new = fmaxf(f + m, in);
+    const float a = expf(f + m - m_new), b = expf(in - m_new);
+    m = m_new;
+    __syncwarp();
+    if (lane == 0) { lf[i] = a; li[i] = b; em[i] = expf(-m); }
+  }
+}
+
+template <typename L, int CP, int SPLIT>
+__device__ __forceinline__ void memory_tokens_n(float (&S)[CP][L::DP], float (&nn)[L::DP], const float* qs, const float* ks, const float* vs,
+                                                const float* li, const float* lf, const float* em, float* os, int nt, int part,
+                                                int col0, int dvp) {
+  constexpr int DP = L::DP, ROW = L::ROW;
+  float4 kc[DP / 4], qc[DP / 4];
+  scan_fetch<DP>(kc, ks + part * L::STRIDE);
+  scan_fetch<DP>(qc, qs + part * L::STRIDE);
+  for (int i = 0; i < nt; ++i) {
+    float4 kn[DP / 4], qn[DP / 4];
+    const int nx = min(i + 1, nt - 1) * ROW + part * L::STRIDE;
+    scan_fetch<DP>(kn, ks + nx); scan_fetch<DP>(qn, qs + nx);
+    const float a = lf[i], b = li[i];
+    float bv[CP], o[CP][2], nq0 = 0.f, nq1 = 0.f;
+#pragma unroll
+    for (int c = 0; c < CP; ++c) { bv[c] = b * vs[i * dvp + col0 + c]; o[c][0] = o[c][1] = 0.f; }
+#pragma unroll
+    for (int d = 0; d < DP / 4; ++d) {
+      const float4 kk = kc[d], qq = qc[d];
+      nn[4 * d] = fmaf(b, kk.x, a * nn[4 * d]); nn[4 * d + 1] = fmaf(b, kk.y, a * nn[4 * d + 1]);
+      nn[4 * d + 2] = fmaf(b, kk.z, a * nn[4 * d + 2]); nn[4 * d + 3] = fmaf(b, kk.w, a * nn[4 * d + 3]);
+      nq0 = fmaf(nn[4 * d], qq.x, nq0); nq1 = fmaf(nn[4 * d + 1], qq.y, nq1);
+      nq0 = fmaf(nn[4 * d + 2], qq.z, nq0); nq1 = fmaf(nn[4 * d + 3], qq.w, nq1);
+#pragma unroll
+      for (int c = 0; c < CP; ++c) {
+        S[c][4 * d] = fmaf(bv[c], kk.x, a * S[c][4 * d]); S[c][4 * d + 1] = fmaf(bv[c], kk.y, a * S[c][4 * d + 1]);
+        S[c][4 * d + 2] = fmaf(bv[c], kk.z, a * S[c][4 * d + 2]); S[c][4 * d + 3] = fmaf(bv[c], kk.w, a * S[c][4 * d + 3]);
+        o[c][0] = fmaf(S[c][4 * d], qq.x, o[c][0]); o[c][1] = fmaf(S[c][4 * d + 1], qq.y, o[c][1]);
+        o[c][0] = fmaf(S[c][4 * d + 2], qq.z, o[c][0]); o[c][1] = fmaf(S[c][4 * d + 3], qq.w, o[c][1]);
+      }
+    }
+    // one division per token, not one per column: the columns take the reciprocal (a last-bit difference from y / den)
+    const float inv = 1.0f / (fmaxf(fabsf(split_sum<SPLIT>(nq0 + nq1)), em[i]) + 1e-6f);
+#pragma unroll
+    for (int c = 0; c < CP; ++c) {
+      const float y = split_sum<SPLIT>(o[c][0] + o[c][1]);
+      if (part == 0) os[i * dvp + col0 + c] = y * inv;
+    }
+#pragma unroll
+    for (int d = 0; d < DP / 4; ++d) { kc[d] = kn[d]; qc[d] = qn[d]; }
+  }
+}
+
+// The matrix memory for long prompts: chunks of 16 tokens staged by asynchronous copies, two deep (what is computed while
+// staging is little here: q times 1 / sqrt(dk) and the two log gates of a token, done when a chunk has landed).
+template <int DK, int CT, int SPLIT, int CP>
+__global__ void __launch_bounds__(512) matrix_memory_scan_pre_kernel(MemoryIn P, HeadOut E) {
+  using L = ScanShape<DK, SPLIT>;
+  constexpr int DP = L::DP, ROW = L::ROW;
+  extern __shared__ __align__(16) float smem[];
+  co_pdl_launch_dependents();
+  co_pdl_wait();
+  const int r = blockIdx.x, h = blockIdx.y;
+  const int part = threadIdx.x % SPLIT, col0 = (threadIdx.x / SPLIT) * CP, d0 = part * DP;
+  const int dk = P.dk, dv = P.dv, dvp = (blockDim.x / SPLIT) * CP;
+  const int colbase = blockIdx.z * dvp;
+  const int start = P.cu_q[r], len = P.cu_q[r + 1] - start;
+  if (len <= 0) return;
+  const int STAGE = 2 * CT * ROW + CT * dvp + 2 * CT;      // floats of one staged chunk: q, k rows, values, the two gates
+  float* os = smem + 2 * STAGE;                            // [CT][dvp]
+  float* den = os + CT * dvp;                              // [CT]
+  float* slot = P.state + (size_t)P.state_slots[r] * P.state_stride;
+  float* S_state = slot + (size_t)h * dk * dv;
+  float* n_state = slot + (size_t)P.heads * dk * dv + (size_t)h * dk;
+  float* m_state = slot + (size_t)P.heads * dk * dv + (size_t)P.heads * dk + h;
+  float S[CP][DP];
+  scan_state_load<CP, DP>(S, S_state, d0, colbase + col0, dk, dv);
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  float nn[DP];                        // this thread's part of the normaliser
+#pragma unroll
+  for (int d = 0; d < DP; ++d) nn[d] = d0 + d < dk ? n_state[d0 + d] : 0.f;
+  float m = warp == 0 ? *m_state : 0.f;
+  const float q_scale = 1.0f / sqrtf((float)dk);
+  const float bi = co_load_any(P.bias_i, P.bias_dtype, h), bf = co_load_any(P.bias_f, P.bias_dtype, h);
+  for (int e = threadIdx.x; e < 2 * STAGE; e += blockDim.x) smem[e] = 0.f;      // the padding of both stages, once
+  __syncthreads();
+  auto stage = [&](int c0, int b) {
+    const int nt = min(CT, len - c0), row0 = start + c0;
+    float* qs = smem + b * STAGE;
+    float* ks = qs + CT * ROW;
+    float* vs = ks + CT * ROW;
+    float* gates = vs + CT * dvp;
+    for (int e = threadIdx.x; e < nt * dk; e += blockDim.x) {
+      const int i = e / dk, d = e % dk;
+      const size_t row = (size_t)(row0 + i);
+      const int o = i * ROW + L::at(d);
+      cp_async4(qs + o, P.q + row * P.ld + (size_t)h * dk + d);
+      cp_async4(ks + o, P.k + row * P.ld + (size_t)h * dk + d);
+    }
+    for (int e = threadIdx.x; e < nt * dvp; e += blockDim.x) {
+      const int i = e / dvp, c = e % dvp;
+      if (colbase + c < dv) cp_async4(vs + e, P.v + (size_t)(row0 + i) * P.ld + (size_t)h * dv + colbase + c);
+    }
+    if (threadIdx.x < nt) {
+      cp_async4(gates + threadIdx.x, P.gi + (size_t)(row0 + threadIdx.x) * P.ld_gate + h);
+      cp_async4(gates + CT + threadIdx.x, P.gf + (size_t)(row0 + threadIdx.x) * P.ld_gate + h);
+    }
+    cp_async_commit_group();
+  };
+  stage(0, 0);
+  int b = 0;
+  for (int c0 = 0; c0 < len; c0 += CT, b ^= 1) {
+    const int nt = min(CT, len - c0), row0 = start + c0;
+    if (c0 + CT < len) { stage(c0 + CT, b ^ 1); cp_async_wait_group<1>(); }
+    else cp_async_wait_group<0>();
+    __syncthreads();
+    float* qs = smem + b * STAGE;
+    float* ks = qs + CT * ROW;
+    float* vs = ks + CT * ROW;
+    float* li = vs + CT * dvp;
+    float* lf = li + CT;
+    for (int e = threadIdx.x; e < nt * dk; e += blockDim.x) qs[(e / dk) * ROW + L::at(e % dk)] *= q_scale;
+    if (threadIdx.x < nt) {
+      li[threadIdx.x] = P.cap * tanhf((li[threadIdx.x] + bi) / P.cap);
+      const float z = P.cap * tanhf((lf[threadIdx.x] + bf) / P.cap);
+      lf[threadIdx.x] = -rc_softplus(-z);
+    }
+    __syncthreads();
+    if (warp == 0) memory_factors(m, li, lf, den, nt, lane);
+    __syncthreads();
+    memory_tokens_n<L, CP, SPLIT>(S, nn, qs, ks, vs, li, lf, den, os, nt, part, col0, dvp);
+    __syncthreads();
+    if (E.raw) raw_out_chunk(E, os, dvp, dv, colbase, nt, row0, h);
+    else head_out_chunk(E, os, dvp, dv, nt, row0, h);
+    __syncthreads();
+  }
+  scan_state_store<CP, DP>(S, S_state, d0, colbase + col0, dk, dv);
+  if (blockIdx.z == 0 && threadIdx.x < SPLIT) {      // the first group of lanes holds the whole of n between them
+    float* n_to = E.nm_next ? E.nm_next + ((size_t)r * P.heads + h) * (dk + 1) : n_state;
+    float* m_to = E.nm_next ? n_to + dk : m_state;
+#pragma unroll
+    for (int d = 0; d < DP; ++d)
+      if (d0 + d < dk) n_to[d0 + d] = nn[d];
+    if (threadIdx.x == 0) *m_to = m;
+  }
+}
+
 // ---------------------------------------------------------------------------------
 // Queries and keys normalised over the WHOLE projection (all heads at once), keys and values written into
 // cache pages: q_out[t] = q / rms(q) * wq, K[slot] = k / rms(k) * wk, V[slot] = v.  A CTA per token.
@@ -747,7 +913,7 @@ CO_EXPORT int coheryn_gated_delta_scan(
   DeltaIn P{q, k, v, ld_qkv, beta, ld_beta, step, ld_step, step_bias, step_bias_dtype, rate_log, rate_log_dtype, state,
             state_stride, cu_q, state_slots, heads, kv_heads, dk, dv, decay_channels};
   HeadOut E{out, out_dtype, ldo, weight, weight_dtype, weight_stride, gate, ldg, eps, out_scale,
-            slices > 1 ? scratch : nullptr, (long)heads * dv, gate_act};
+            slices > 1 ? scratch : nullptr, (long)heads * dv, nullptr, gate_act};
   if (chunked) {
     if (co_delta_chunks(P, E, B, chunks, runs, scratch, stream)) return 1;
     if (!short_runs) return 0;
@@ -772,7 +938,7 @@ CO_EXPORT int coheryn_gated_delta_scan(
       const size_t smem = ((size_t)3 * CT * ROW + (size_t)2 * CT * dvp + CT) * sizeof(float);                  \
       auto kern = gated_delta_scan_kernel<D, CT, SP, CP>;                                                      \
       if (smem > 48 * 1024) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
-      co_launch_ex(true, kern, dim3(B, heads, 1), dim3(threads), smem, stream, P, E, below);                          \
+      co_launch_ex(true, kern, dim3(B, heads, 1), dim3(threads), smem, stream, P, E, below);                   \
     }                                                                                                          \
   }
 #define LAUNCH(D) if (slices == 1 && dv * scan_split(D) > 128 * 16) LAUNCH_CP(D, true) else LAUNCH_CP(D, false)
@@ -787,14 +953,16 @@ CO_EXPORT int coheryn_matrix_memory_scan(
     const float* q, const float* k, const float* v, long ld, const float* gi, const float* gf, long ld_gate,
     const void* bias_i, const void* bias_f, int bias_dtype, float cap, float* state, long state_stride, const int* cu_q,
     const int* state_slots, int B, int heads, int dk, int dv, void* out, int out_dtype, long ldo, const void* weight,
-    int weight_dtype, int weight_stride, const float* gate, long ldg, float eps, float out_scale,
+    int weight_dtype, int weight_stride, const float* gate, long ldg, float eps, float out_scale, int total_tokens,
     float* scratch, long scratch_floats, int chunks, int runs, int short_runs, cudaStream_t stream) {
   if (B <= 0) return 0;
   if (!scan_shape_ok("matrix_memory_scan", heads, dk, dv)) return 1;
   if (!(cap > 0.f)) CO_FAIL("matrix_memory_scan: the gate cap must be positive");
   const bool chunked = chunks > 0 && co_memory_chunks_take(dk, dv) && scratch && scratch_floats >= co_memory_chunk_floats(chunks, heads, dk, dv);
+  const int slices = chunked ? 1 : scan_slices(B, heads, dv, total_tokens, scratch, scratch_floats, (long)B * heads * (dk + 1));
   MemoryIn P{q, k, v, ld, gi, gf, ld_gate, bias_i, bias_f, bias_dtype, cap, state, state_stride, cu_q, state_slots, heads, dk, dv};
-  HeadOut E{out, out_dtype, ldo, weight, weight_dtype, weight_stride, gate, ldg, eps, out_scale, nullptr, 0, 0};
+  HeadOut E{out, out_dtype, ldo, weight, weight_dtype, weight_stride, gate, ldg, eps, out_scale,
+            slices > 1 ? scratch : nullptr, (long)heads * dv, slices > 1 ? scratch + (long)total_tokens * heads * dv : nullptr};
   if (chunked) {
     if (co_memory_chunks(P, E, B, chunks, runs, scratch, stream)) return 1;
     if (!short_runs) return 0;
@@ -803,18 +971,31 @@ CO_EXPORT int coheryn_matrix_memory_scan(
 #define LAUNCH_CP(D, WIDE)                                                                                     \
   {                                                                                                            \
     constexpr int CT = chunk_tokens(D), SP = scan_split(D), CP = scan_columns(D, WIDE), ROW = ScanShape<D, SP>::ROW; \
-    const int threads = ((dv + CP - 1) / CP * SP + 31) / 32 * 32, dvp = threads / SP * CP;                     \
-    const size_t smem = ((size_t)2 * CT * ROW + (size_t)2 * CT * dvp + 3 * CT) * sizeof(float);                \
-    auto kern = matrix_memory_scan_kernel<D, CT, SP, CP>;                                                      \
-    if (smem > 48 * 1024) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);  \
-    co_launch_ex(true, kern, dim3(B, heads, 1), dim3(threads), smem, stream, P, E, below);                     \
+    const int cols = slices > 1 ? SLICE_COLUMNS : dv;                                                          \
+    const int threads = ((cols + CP - 1) / CP * SP + 31) / 32 * 32, dvp = threads / SP * CP;                   \
+    if (slices > 1) {   /* a long prompt: asynchronous staging of 16 tokens, two deep */                        \
+      constexpr int CA = 16;                                                                                   \
+      const size_t smem = ((size_t)2 * (2 * CA * ROW + CA * dvp + 2 * CA) + (size_t)CA * dvp + CA) * sizeof(float); \
+      auto kern = matrix_memory_scan_pre_kernel<D, CA, SP, CP>;                                                \
+      if (smem > 48 * 1024) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
+      co_launch_ex(true, kern, dim3(B, heads, (dv + dvp - 1) / dvp), dim3(threads), smem, stream, P, E);       \
+    } else {                                                                                                   \
+      const size_t smem = ((size_t)2 * CT * ROW + (size_t)2 * CT * dvp + 3 * CT) * sizeof(float);              \
+      auto kern = matrix_memory_scan_kernel<D, CT, SP, CP>;                                                    \
+      if (smem > 48 * 1024) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
+      co_launch_ex(true, kern, dim3(B, heads, 1), dim3(threads), smem, stream, P, E, below);                   \
+    }                                                                                                          \
   }
-#define LAUNCH(D) if (dv * scan_split(D) > 128 * 16) LAUNCH_CP(D, true) else LAUNCH_CP(D, false)
+#define LAUNCH(D) if (slices == 1 && dv * scan_split(D) > 128 * 16) LAUNCH_CP(D, true) else LAUNCH_CP(D, false)
   CO_SCAN_CASES(LAUNCH)
 #undef LAUNCH
 #undef LAUNCH_CP
   CO_CHECK_LAUNCH("matrix_memory_scan");
-  return 0;
+  if (slices == 1) return 0;
+  co_launch(memory_nm_commit_kernel, dim3(B, heads), dim3(128), 0, stream, (const float*)E.nm_next, state, state_stride, state_slots,
+            cu_q, heads, dk, dv);
+  CO_CHECK_LAUNCH("memory_nm_commit");
+  return launch_head_norm_gate(E, total_tokens, heads, dv, stream);
 }
 
 CO_EXPORT int coheryn_qk_norm_kv_write(const float* q, const float* k, const float* v, long ld, const void* wq, const void* wk,

@@ -13,10 +13,12 @@ struct HeadOut {
   int weight_stride;
   const float* gate; long ldg;                 // pre-activations [T, heads * dv]
   float eps, out_scale;
-  // When the columns of a head are split over several CTAs (a long prompt of few requests whose key channels are more than the
-  // chunks take), no CTA sees a whole head: the delta rule's scan then leaves the unnormalised outputs in `raw` [T, heads * dv]
-  // and a second kernel applies norm, weight and gate, in the same order of operations.
+  // When the columns of a head are split over several CTAs (a long prompt of few requests that the scans take: more SMs at work),
+  // no CTA sees a whole head: the scans then leave the unnormalised outputs in `raw` [T, heads * dv] and a second kernel applies
+  // norm, weight and gate, in the same order of operations.  `nm_next`: where the matrix memory's n and m of each (request,
+  // head) wait until every CTA of the head has read the old ones ([B][heads][dk + 1]).
   float* raw; long ldr;
+  float* nm_next;
   int gate_act;                                // what the gate's pre-activation passes: 0 sigmoid, 1 SiLU
 };
 

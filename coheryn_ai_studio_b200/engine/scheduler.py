@@ -18,7 +18,10 @@ allocated on demand:
   (the pool does that by itself), then nothing new is admitted, then the most recently
   admitted running request is preempted: its pages are freed and it goes back to the head
   of the waiting queue with its prompt and the tokens generated so far, to be computed
-  again later.  Sampling state is kept, so its output is the same as without preemption.
+  again later.  Sampling state is kept, so its output is the one without preemption as
+  long as the rows that are computed again give the same logits: to the bit in float32
+  (recurrences that a mixer takes in chunks of a portion's tokens excepted), otherwise up
+  to the rounding of the same sums in another order.
 
 The decisions are taken by the native planner (``csrc/host_engine.cpp``: ``Planner``), which
 works on the cache manager's native book; :class:`Scheduler` is its Python face and keeps the

@@ -1136,13 +1136,14 @@ def short_conv_silu(x: torch.Tensor, taps: torch.Tensor, state: torch.Tensor, st
 
 def gated_delta_scan(q, k, v, beta, step_pre, step_bias, rate_log, state, step, heads: int, kv_heads: int, dk: int, dv: int,
                      out: torch.Tensor, norm_weight: torch.Tensor, gate: torch.Tensor, eps: float, out_scale: float = 1.0,
-                     decay_per_channel: bool = True, gate_activation: str = "sigmoid") -> None:
+                     decay_per_channel: bool = True, gate_activation: str = "sigmoid", in_chunks: bool = True) -> None:
     """The gated delta rule over each request's run of tokens, continued from and left in ``state`` (float32 view
     [slots, heads * dk * dv]), followed by the per-head RMS norm, its weight ([dv], shared by the heads) and the sigmoid
     (or, ``gate_activation = "silu"``, the SiLU) of ``gate``.  q, k [T, kv_heads*dk] and v [T, heads*dv]: float32 with ONE
     row stride (slices of one buffer); beta [T, heads], step_pre [T, heads*dk] (``decay_per_channel``: a decay per head and
     key channel) or [T, heads] (one per head), gate [T, heads*dv]: float32 pre-activations; out [T, heads*dv] in the
-    compute dtype."""
+    compute dtype.  ``in_chunks`` False: every run goes token by token, so that the results do not depend, to the bit, on how a
+    sequence was cut into steps; else long runs go in chunks, which begin where the run begins."""
     _dev(q, k, v, beta, step_pre, step_bias, rate_log, state, out, norm_weight, gate)
     for t, name in ((q, "q"), (k, "k"), (v, "v"), (beta, "beta"), (step_pre, "step"), (state, "state"), (gate, "gate")):
         _f32(t, name)
@@ -1154,7 +1155,7 @@ def gated_delta_scan(q, k, v, beta, step_pre, step_bias, rate_log, state, step, 
     gate_code = {"sigmoid": 0, "silu": 1}[gate_activation]
     assert state.shape[1] == heads * dk * dv and out.shape == (q.shape[0], heads * dv) and out.stride(1) == 1
     lib = recurrent()
-    chunks, runs, rest = _chunked_runs(lib, step, q.shape[0])
+    chunks, runs, rest = _chunked_runs(lib, step, q.shape[0]) if in_chunks else (0, 0, True)
     floats = int(lib.coheryn_delta_chunk_floats(c_int(chunks), c_int(heads), c_int(dk), c_int(dv))) if chunks else 0
     if floats:
         scratch = torch.empty(floats, dtype=torch.float32, device=q.device)
@@ -1171,11 +1172,13 @@ def gated_delta_scan(q, k, v, beta, step_pre, step_bias, rate_log, state, step, 
 
 
 def matrix_memory_scan(q, k, v, gate_i, gate_f, bias_i, bias_f, cap: float, state, step, heads: int, dk: int, dv: int,
-                       out: torch.Tensor, norm_weight: torch.Tensor, gate: torch.Tensor, eps: float, out_scale: float = 1.0) -> None:
+                       out: torch.Tensor, norm_weight: torch.Tensor, gate: torch.Tensor, eps: float, out_scale: float = 1.0,
+                       in_chunks: bool = True) -> None:
     """The stabilised matrix memory over each request's run of tokens, continued from and left in ``state`` (float32
     view [slots, heads * (dk * dv + dk + 1)]: S, n, m), followed by the per-head RMS norm, its weight [heads*dv] and the
     sigmoid of ``gate``.  q, k [T, heads*dk], v [T, heads*dv]: float32 with one row stride; gate_i, gate_f [T, heads] with
-    one row stride; biases [heads]; out [T, heads*dv] in the compute dtype."""
+    one row stride; biases [heads]; out [T, heads*dv] in the compute dtype.  ``in_chunks`` as for ``gated_delta_scan`` (token by
+    token the results are the same to a last bit, where a long portion's heads are split over CTAs)."""
     _dev(q, k, v, gate_i, gate_f, bias_i, bias_f, state, out, norm_weight, gate)
     for t, name in ((q, "q"), (k, "k"), (v, "v"), (gate_i, "gate_i"), (gate_f, "gate_f"), (state, "state"), (gate, "gate")):
         _f32(t, name)
@@ -1186,15 +1189,18 @@ def matrix_memory_scan(q, k, v, gate_i, gate_f, bias_i, bias_f, cap: float, stat
     assert norm_weight.numel() == heads * dv
     assert state.shape[1] == heads * (dk * dv + dk + 1) and out.shape == (q.shape[0], heads * dv) and out.stride(1) == 1
     lib = recurrent()
-    chunks, runs, rest = _chunked_runs(lib, step, q.shape[0])
+    chunks, runs, rest = _chunked_runs(lib, step, q.shape[0]) if in_chunks else (0, 0, True)
     floats = int(lib.coheryn_memory_chunk_floats(c_int(chunks), c_int(heads), c_int(dk), c_int(dv))) if chunks else 0
-    scratch = torch.empty(floats, dtype=torch.float32, device=q.device) if floats else None
+    if floats:
+        scratch = torch.empty(floats, dtype=torch.float32, device=q.device)
+    else:
+        scratch = _scan_scratch(q.shape[0], step.num_requests, heads, dv, step.num_requests * heads * (dk + 1), q.device)
     _check(lib, lib.coheryn_matrix_memory_scan(
         _ptr(q), _ptr(k), _ptr(v), c_long(q.stride(0)), _ptr(gate_i), _ptr(gate_f), c_long(gate_i.stride(0)), _ptr(bias_i),
         _ptr(bias_f), c_int(_code(bias_i)), c_float(cap), _ptr(state), c_long(state.stride(0)), _ptr(step.cu_q),
         _ptr(step.state_slots), c_int(step.num_requests), c_int(heads), c_int(dk), c_int(dv), _ptr(out), c_int(_code(out)),
         c_long(out.stride(0)), _ptr(norm_weight), c_int(_code(norm_weight)), c_int(dv), _ptr(gate), c_long(gate.stride(0)),
-        c_float(eps), c_float(out_scale), _ptr(scratch), c_long(floats),
+        c_float(eps), c_float(out_scale), c_int(q.shape[0]), _ptr(scratch), c_long(scratch.numel() if scratch is not None else 0),
         c_int(chunks if floats else 0), c_int(runs), c_int(1 if rest else 0), _stream()))
 
 

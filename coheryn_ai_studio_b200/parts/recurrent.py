@@ -68,6 +68,13 @@ class _StackedInput:
 class _StateMixer(Mixer):
     output_parts = 1
 
+    @property
+    def in_chunks(self) -> bool:
+        """Whether long runs may go chunk by chunk.  Not in float32: its products give a row the same bits whatever the step's
+        other rows are, and with the scans token by token a sequence has the same bits however load or preemption cut it.  (In
+        bfloat16 the product that runs follows the step's rows anyway.)"""
+        return self.runtime.dtype != torch.float32
+
     def forward(self, x: torch.Tensor, step: StepContext, cache: Optional[LayerCache]) -> torch.Tensor:
         out = torch.empty((1, x.shape[0], self.hidden_size), dtype=torch.float32, device=x.device)
         self.forward_into(x, step, cache, out)
@@ -125,7 +132,7 @@ class MatrixMemory(_StateMixer):
         o = outs[0]
         ops.matrix_memory_scan(st.cut(proj, "q"), st.cut(proj, "k"), st.cut(proj, "v"), st.cut(proj, "i"), st.cut(proj, "f"),
                                self.b_i, self.b_f, self.cap, state, step, self.num_heads, self.dk, self.dv, o, self.norm_w,
-                               st.cut(proj, "g"), self.eps, self.out_scale)
+                               st.cut(proj, "g"), self.eps, self.out_scale, in_chunks=self.in_chunks)
 
 
 class GatedDeltaRule(_StateMixer):
@@ -217,7 +224,7 @@ class GatedDeltaRule(_StateMixer):
         ops.gated_delta_scan(qkv[:, :G * dk], qkv[:, G * dk:2 * G * dk], qkv[:, 2 * G * dk:], st.cut(proj, "b"), step_pre,
                              self.dt_bias, self.rate_log, state[:, :self.memory], step, H, G, dk, dv, o, self.norm_w, gate,
                              self.eps, self.out_scale, decay_per_channel=self.decay == "channel",
-                             gate_activation=self.gate_activation)
+                             gate_activation=self.gate_activation, in_chunks=self.in_chunks)
 
 
 class GatedLinearRecurrence(_StateMixer):

@@ -169,3 +169,36 @@ def test_matrix_memory_in_chunks(lens, heads, dk, dv, cap, open_gate, host):
         want = plain.rms(o, 1e-5).reshape(n, heads * dv) * weight * plain.sigmoid(d["gate"])
         assert np.abs(got[at:at + n] - want).max() <= 1e-3 * max(1.0, np.abs(want).max()), slot
         at += n
+
+
+@pytest.mark.parametrize("kind,dk,dv", [("gated_delta_rule", 64, 128), ("gated_delta_rule", 24, 40), ("matrix_memory", 64, 64), ("matrix_memory", 128, 48)])
+def test_float32_mixers_keep_their_bits_however_a_sequence_is_cut(kind, dk, dv):
+    """A float32 mixer over 200 tokens in one step, in four portions (two of them long enough for chunks), and beside another
+    request: the same outputs and the same state, bit for bit."""
+    from coheryn_ai_studio_b200.config.spec import PartSpec
+    from coheryn_ai_studio_b200.parts.base import MIXERS, LayerCache, Runtime, build_part
+    g = torch.Generator(DEV).manual_seed(dk + dv)
+    params = dict(hidden_size=96, num_heads=2, head_dim=dk, v_head_dim=dv, eps=1e-6)
+    params.update(dict(num_kv_heads=1, conv_taps=4, decay_rank=16, gate_rank=16) if kind == "gated_delta_rule" else dict(gate_cap=15.0))
+    part = build_part(MIXERS, "mixer", PartSpec(kind, params), Runtime(torch.float32, torch.device(DEV)))
+    ranks = {"a1": (16, 96), "a2": (part.decay_size, 16), "g1": (16, 96), "g2": (2 * dv, 16)} if kind == "gated_delta_rule" else {}
+    part.bind({n: torch.randn(ranks.get(n, s.shape), generator=g, device=DEV) * (ranks.get(n, s.shape)[-1] ** -0.5 if len(s.shape) > 1 else 1.0)
+               for n, s in part.tensor_specs().items()})
+    x, other = torch.randn((200, 96), generator=g, device=DEV), torch.randn((120, 96), generator=g, device=DEV)
+    size = part.cache_requirement().shape
+
+    def run(cuts, beside=0):
+        state, outs, at = torch.zeros((2,) + tuple(size), device=DEV), [], 0
+        for n in cuts:
+            rows, lens, slots = x[at:at + n], [n], [1]
+            if beside:
+                rows, lens, slots = torch.cat([other[:beside], rows]), [beside, n], [0, 1]
+            y = part.forward(rows.contiguous(), step_of(lens, slots), LayerCache("state", state=state))
+            outs.append(y[sum(lens) - n:])
+            at += n
+        return torch.cat(outs), state[1]
+
+    want, end = run([200])
+    assert want.shape[0] == 200 and bool(want.isfinite().all()) and float(want.abs().max()) > 0
+    for got, state in (run([64, 1, 70, 65]), run([1, 199]), run([130, 70], beside=120)):
+        assert torch.equal(got, want) and torch.equal(state, end)
