@@ -21,8 +21,8 @@
 // chip could do beside it.  Here the chain is two products of 64 x 128 x 16 per chunk; measured on a B200 (12 heads of 128 x
 // 128, one request of 2,048 tokens) the four kernels take 264 us (70, 36, 100 and 58) in place of 1,150 us for the scan with its preparation.
 //
-// A run of fewer than CHUNK_FROM tokens is left to the scan (recurrent.cu), request by request, so that a row's order of
-// additions depends on its place in its own request's run only.
+// A run of fewer than CHUNK_FROM tokens is left to the scan (recurrent.cu), request by request: of the other requests only
+// whether the step goes in chunks at all (recurrent.cu, coheryn_*_chunks_pay) can reach a row, not its order of additions.
 #include "recurrent.cuh"
 
 namespace {

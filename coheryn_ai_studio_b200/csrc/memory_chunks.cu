@@ -20,8 +20,8 @@
 // element; the rest are products over all chunks at once.  Measured on a B200 (8 heads of 128 x 256, one request of 2,048
 // tokens): 14 + 38 + 16 + 94 us in place of 1,350 us (1,850 with the kernels behind the scan launched ahead and waiting beside it).
 //
-// A run of fewer than CHUNK_FROM tokens is left to the scan (recurrent.cu), request by request, so that a row's order of
-// additions depends on its place in its own request's run only.
+// A run of fewer than CHUNK_FROM tokens is left to the scan (recurrent.cu), request by request: of the other requests only
+// whether the step goes in chunks at all (recurrent.cu, coheryn_*_chunks_pay) can reach a row, not its order of additions.
 #include "recurrent.cuh"
 
 namespace {

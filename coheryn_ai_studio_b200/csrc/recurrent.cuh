@@ -47,8 +47,8 @@ struct MemoryIn {
   int heads, dk, dv;
 };
 
-// Runs of at least CHUNK_FROM tokens go chunk by chunk (delta_chunks.cu, memory_chunks.cu), shorter ones token by token
-// (recurrent.cu), request by request.
+// In a step for which that is faster (coheryn_*_chunks_pay) runs of at least CHUNK_FROM tokens go chunk by chunk (delta_chunks.cu,
+// memory_chunks.cu), shorter ones token by token (recurrent.cu), request by request.
 constexpr int CHUNK_TOKENS = 64, CHUNK_FROM = 48;
 // `chunks` and `runs`: how many chunks and how many such runs the step holds at most (CTAs beyond the last return at once);
 // `scratch`: at least co_*_chunk_floats floats.

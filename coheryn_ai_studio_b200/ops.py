@@ -1102,18 +1102,26 @@ def _scan_scratch(T: int, B: int, heads: int, dv: int, extra: int, device):
     return torch.empty(T * heads * dv + extra, dtype=torch.float32, device=device)
 
 
-def _chunked_runs(lib, step, T: int):
-    """(chunks, runs that are cut into chunks, whether others are left) of a step whose long runs go chunk by chunk.  From the
-    host's copy of the runs' lengths where the step has one, else the most that T tokens of so many requests can be."""
+def _chunked_runs(lib, pay, step, T: int, heads: int, dk: int, dv: int):
+    """(chunks, runs that are cut into chunks, whether others are left) of a step whose long runs go chunk by chunk where ``pay``
+    says that this is faster.  From the host's copy of the runs' lengths where the step has one, else the most that T tokens of
+    so many requests can be."""
     first, size, B = lib.chunk_from, lib.chunk_tokens, step.num_requests
-    if T < first:
+    if T - B + 1 < first:         # no run is as long
         return 0, 0, True
     lens = getattr(step, "q_lens", None)
     if lens is not None and len(lens) == B:
         long = [n for n in lens if n >= first]
-        return sum(-(-n // size) for n in long), len(long), len(long) < B
-    runs = min(B, T // first)
-    return T // size + runs, runs, True
+        if not long:
+            return 0, 0, True
+        chunks, runs, rest, tokens, longest = sum(-(-n // size) for n in long), len(long), len(long) < B, sum(long), max(long)
+        short = max(n for n in lens if n < first) if rest else 0
+    else:
+        runs, longest, tokens, rest, short = min(B, T // first), T - B + 1, T, True, 0
+        chunks = T // size + runs
+    if not pay(c_int(heads), c_int(dk), c_int(dv), c_int(B), c_int(T), c_int(longest), c_int(chunks), c_int(tokens), c_int(short)):
+        return 0, 0, True
+    return chunks, runs, rest
 
 
 def short_conv_silu(x: torch.Tensor, taps: torch.Tensor, state: torch.Tensor, step, update_state: bool = True) -> torch.Tensor:
@@ -1143,7 +1151,7 @@ def gated_delta_scan(q, k, v, beta, step_pre, step_bias, rate_log, state, step, 
     row stride (slices of one buffer); beta [T, heads], step_pre [T, heads*dk] (``decay_per_channel``: a decay per head and
     key channel) or [T, heads] (one per head), gate [T, heads*dv]: float32 pre-activations; out [T, heads*dv] in the
     compute dtype.  ``in_chunks`` False: every run goes token by token, so that the results do not depend, to the bit, on how a
-    sequence was cut into steps; else long runs go in chunks, which begin where the run begins."""
+    sequence was cut into steps; else long runs go in chunks, which begin where the run begins, in steps for which that is faster."""
     _dev(q, k, v, beta, step_pre, step_bias, rate_log, state, out, norm_weight, gate)
     for t, name in ((q, "q"), (k, "k"), (v, "v"), (beta, "beta"), (step_pre, "step"), (state, "state"), (gate, "gate")):
         _f32(t, name)
@@ -1155,7 +1163,7 @@ def gated_delta_scan(q, k, v, beta, step_pre, step_bias, rate_log, state, step, 
     gate_code = {"sigmoid": 0, "silu": 1}[gate_activation]
     assert state.shape[1] == heads * dk * dv and out.shape == (q.shape[0], heads * dv) and out.stride(1) == 1
     lib = recurrent()
-    chunks, runs, rest = _chunked_runs(lib, step, q.shape[0]) if in_chunks else (0, 0, True)
+    chunks, runs, rest = _chunked_runs(lib, lib.coheryn_delta_chunks_pay, step, q.shape[0], heads, dk, dv) if in_chunks else (0, 0, True)
     floats = int(lib.coheryn_delta_chunk_floats(c_int(chunks), c_int(heads), c_int(dk), c_int(dv))) if chunks else 0
     if floats:
         scratch = torch.empty(floats, dtype=torch.float32, device=q.device)
@@ -1189,7 +1197,7 @@ def matrix_memory_scan(q, k, v, gate_i, gate_f, bias_i, bias_f, cap: float, stat
     assert norm_weight.numel() == heads * dv
     assert state.shape[1] == heads * (dk * dv + dk + 1) and out.shape == (q.shape[0], heads * dv) and out.stride(1) == 1
     lib = recurrent()
-    chunks, runs, rest = _chunked_runs(lib, step, q.shape[0]) if in_chunks else (0, 0, True)
+    chunks, runs, rest = _chunked_runs(lib, lib.coheryn_memory_chunks_pay, step, q.shape[0], heads, dk, dv) if in_chunks else (0, 0, True)
     floats = int(lib.coheryn_memory_chunk_floats(c_int(chunks), c_int(heads), c_int(dk), c_int(dv))) if chunks else 0
     if floats:
         scratch = torch.empty(floats, dtype=torch.float32, device=q.device)

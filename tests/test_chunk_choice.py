@@ -1,0 +1,39 @@
+"""Whether a step's long runs go in chunks or token by token (csrc/recurrent.cu, coheryn_*_chunks_pay; no GPU needed): at sizes where
+one form was measured to take a third less time than the other (B200), the choice is the faster one."""
+import types
+
+import pytest
+
+from coheryn_ai_studio_b200 import ops
+
+
+def choice(kind, heads, dk, dv, lens, host=True):
+    lib = ops.recurrent()
+    step = types.SimpleNamespace(num_requests=len(lens), num_tokens=sum(lens))
+    if host:
+        step.q_lens = lens
+    return ops._chunked_runs(lib, getattr(lib, f"coheryn_{kind}_chunks_pay"), step, sum(lens), heads, dk, dv)
+
+
+# us by the scan and in chunks
+@pytest.mark.parametrize("kind,heads,dk,dv,lens,scan,chunks", [
+    ("delta", 12, 128, 128, [48], 54, 89), ("delta", 12, 128, 128, [64], 57, 96), ("delta", 12, 128, 128, [48] * 8, 55, 150),
+    ("delta", 12, 128, 128, [64] * 16, 136, 242), ("delta", 12, 128, 128, [600], 487, 183), ("delta", 12, 64, 128, [48] * 32, 94, 201),
+    ("delta", 16, 64, 64, [96] * 32, 148, 299), ("delta", 16, 64, 64, [192], 158, 68), ("delta", 4, 32, 64, [48] * 128, 47, 188),
+    ("delta", 4, 32, 64, [192] * 4, 129, 67), ("delta", 2, 64, 64, [1] * 64 + [200], 165, 74), ("delta", 12, 128, 128, [1] * 64 + [60] * 3, 120, 211),
+    ("memory", 8, 128, 256, [256] * 32, 1242, 546), ("memory", 8, 128, 256, [192], 141, 92), ("memory", 4, 64, 64, [100], 112, 46),
+    ("memory", 2, 32, 128, [320], 158, 46),
+])
+def test_the_faster_form_is_taken(kind, heads, dk, dv, lens, scan, chunks):
+    got = choice(kind, heads, dk, dv, lens)[0]
+    assert (got > 0) == (chunks < scan), (got, scan, chunks)
+
+
+def test_what_is_cut_into_chunks():
+    assert choice("delta", 12, 128, 128, [1021, 407, 130, 2]) == (16 + 7 + 3, 3, True)
+    assert choice("delta", 12, 128, 128, [1021, 407]) == (16 + 7, 2, False)
+    assert choice("memory", 8, 128, 256, [2048, 47, 48]) == (32 + 1, 2, True)
+    chunks, runs, rest = choice("delta", 12, 128, 128, [1021, 407, 130, 2], host=False)       # the lengths are the device's alone
+    assert chunks >= 26 and runs >= 3 and rest
+    assert choice("delta", 12, 192, 128, [2048]) == (0, 0, True)                              # more key channels than the chunks take
+    assert choice("memory", 8, 128, 256, [1] * 64) == (0, 0, True) and choice("delta", 2, 16, 16, []) == (0, 0, True)
