@@ -12,7 +12,7 @@
 // instructions); the tiles of the next 16 values of k are fetched into registers while the present ones are used.
 // Measured on a B200 (float32, alone, L2 flushed; before: 64 x 64 tiles, 4 x 4 per thread, one buffer): 313 x 17920 x 1536
 // 697 -> 417 us (41 TFLOP/s of 74), 2048 rows 3,593 -> 2,336 us, 313 x 1536 x 8960 830 -> 210 us, one row by 17920 x 1536
-// 183 -> 84 us, one row by 1536 x 8960 955 -> 44 us.
+// 183 -> 84 us, one row by 1536 x 8960 955 -> 44 us; warm, 64 x 256 x 128 10.9 -> 5.9 us.
 #include "common.cuh"
 
 namespace {
@@ -181,41 +181,49 @@ gemm_simt_add_kernel(const float* __restrict__ apart, int stretches, const void*
   store_out(out, m * ldo + n, v, bias, bias_dtype, n, act);
 }
 
-// Tiles by rows: 16 x 64 for a decode step, which is bound by the weight's stream and asks for 64 values of k ahead (16 KB per
-// CTA); 64 x 128 otherwise (128 threads; 128 x 128 would leave more of the last tile idle).
-constexpr int ROWS_FEW = 16;
-constexpr int tile_columns(bool few) { return few ? 64 : 128; }
-
 // Values of k per stretch: a wide weight makes tiles enough for the chip by itself and keeps long stretches (one CTA then
 // needs no second set of sums up to k = 2048); a narrow one is cut finely, so that few rows still fill the chip.
 int stretch_of(int N) { return N >= 4096 ? 2048 : 512; }
 
-// Into how many CTAs the stretches of k go: one each when the tiles alone would leave SMs idle, else one CTA for all.
-int stretches_apart(int M, int N, int K) {
-  const int columns = tile_columns(M <= ROWS_FEW);
-  const long tiles = (long)((N + columns - 1) / columns) * (M <= ROWS_FEW ? 1 : (M + 63) / 64);
+// Tiles: 64 x 128 (128 threads; 128 x 128 would leave more of the last tile idle), or 16 x 64 with 64 values of k at a time (16 KB of
+// the weight per CTA), for a decode step, which is bound by the weight's stream, and where a product is so small that the large
+// tiles leave most SMs idle and each CTA's chain of k is what takes the time: up to about three small tiles per SM, a few more
+// when the sums are short.  Measured on a B200 with the large tiles and with the small ones: 17 x 3584 x 512 (112 small tiles) 38.0 and
+// 16.7 us, 65 x 1536 x 1536 (360) 42 and 36, 130 x 3584 x 512 (504) 42 and 41, 130 x 1536 x 1536 (648) 42 and 63, 2048 x 64 x 64 (128)
+// 10.7 and 4.4, 2048 x 256 x 128 (512) 15.9 and 12.3.  Sums of at most 32 values take 16 of k at a time (64 x 16 x 16: 4.1 and 3.1 us).
+struct Plan { bool few; int rows, columns, apart; };      // tile; into how many CTAs the stretches of k go
+Plan plan_of(int M, int N, int K) {
   const int n = (K + stretch_of(N) - 1) / stretch_of(N);
-  return n > 1 && tiles < 2 * 148 ? n : 1;
+  const long small = (long)((N + 63) / 64) * ((M + 15) / 16) * n;
+  Plan p;
+  p.few = M <= 16 || small <= (K <= 128 ? 592 : 480);
+  p.rows = p.few ? 16 : 64;
+  p.columns = p.few ? 64 : 128;
+  // one CTA each when the tiles alone would leave SMs idle, else one CTA for all
+  const long tiles = (long)((N + p.columns - 1) / p.columns) * ((M + p.rows - 1) / p.rows);
+  p.apart = n > 1 && tiles < 2 * 148 ? n : 1;
+  return p;
 }
 
 template <typename TX, typename TW, typename TO>
 int run(const TX* x, const TW* w, const void* bias, int bias_dtype, TO* out, int M, int N, int K, long ldx, long ldo, int act,
         float* workspace, long floats, int n_split, int k_split, cudaStream_t stream) {
   const bool vec = K % 4 == 0 && k_split % 4 == 0 && ldx % 4 == 0 && (uintptr_t)x % (4 * sizeof(TX)) == 0 && (uintptr_t)w % (4 * sizeof(TW)) == 0;
-  int n = stretches_apart(M, N, K);
+  const Plan p = plan_of(M, N, K);
+  int n = p.apart;
   if (n > 1 || K > stretch_of(N)) n_split = 0;       // the stretches are those of a full row
   if (n > 1 && (!workspace || floats < (long)n * M * N)) n = 1;
   float* apart = n > 1 ? workspace : nullptr;
-  const bool few = M <= ROWS_FEW;
-  const dim3 grid((N + tile_columns(few) - 1) / tile_columns(few), few ? 1 : (M + 63) / 64, n);
+  const dim3 grid((N + p.columns - 1) / p.columns, (M + p.rows - 1) / p.rows, n);
   const int stretch = stretch_of(N);
 #define GO(BM, BN, BK, T, VEC, MULTI)                                                                                       \
   gemm_simt_kernel<TX, TW, TO, BM, BN, BK, T, T, VEC, MULTI><<<grid, (BM / T) * (BN / T), 0, stream>>>(                     \
       x, w, bias, bias_dtype, out, apart, M, N, K, ldx, ldo, act, stretch, n_split, k_split)
-#define BY_ROWS(VEC, MULTI) if (few) GO(16, 64, 64, 4, VEC, MULTI); else GO(64, 128, 16, 8, VEC, MULTI)
-  if (n == 1 && K > stretch) { if (vec) { BY_ROWS(true, true); } else { BY_ROWS(false, true); } }
-  else { if (vec) { BY_ROWS(true, false); } else { BY_ROWS(false, false); } }
-#undef BY_ROWS
+#define BY_TILE(VEC, MULTI) if (p.few) GO(16, 64, 64, 4, VEC, MULTI); else GO(64, 128, 16, 8, VEC, MULTI)
+  if (p.few && K <= 32) { if (vec) GO(16, 64, 16, 4, true, false); else GO(16, 64, 16, 4, false, false); }
+  else if (n == 1 && K > stretch) { if (vec) { BY_TILE(true, true); } else { BY_TILE(false, true); } }
+  else { if (vec) { BY_TILE(true, false); } else { BY_TILE(false, false); } }
+#undef BY_TILE
 #undef GO
   CO_CHECK_LAUNCH("gemm_simt");
   if (n > 1) {
@@ -229,8 +237,14 @@ int run(const TX* x, const TW* w, const void* bias, int bias_dtype, TO* out, int
 
 // The floats of workspace with which a product of this shape shares its stretches of k out over CTAs (0: it does not).
 CO_EXPORT long coheryn_gemm_simt_workspace_floats(int M, int N, int K) {
-  const int n = M > 0 && N > 0 && K > 0 ? stretches_apart(M, N, K) : 1;
+  const int n = M > 0 && N > 0 && K > 0 ? plan_of(M, N, K).apart : 1;
   return n > 1 ? (long)n * M * N : 0;
+}
+
+// How a product of this shape is laid out: rows and columns of a tile, CTAs that its stretches of k go to.
+CO_EXPORT void coheryn_gemm_simt_plan(int M, int N, int K, int* rows, int* columns, int* apart) {
+  const Plan p = plan_of(M, N, K);
+  *rows = p.rows; *columns = p.columns; *apart = p.apart;
 }
 
 // x: [M, K] with row stride ldx; w: [N, K] contiguous; out: [M, N] with row stride ldo.

@@ -51,3 +51,11 @@ def test_block_diagonal_weight(M, rows, cols, N, K):
     out = torch.empty((M, N), device=DEV)
     ops.gemm_simt(x, w, None, out, blocks=(rows, cols))
     assert torch.equal(out, product(x, w, None, torch.float32))
+
+
+# Small products in tiles of 16 x 64 (one and many of them across and down, a rest in each direction), sums of at most 32 values.
+@pytest.mark.parametrize("M,N,K,pad", [(33, 65, 64, 0), (100, 64, 33, 2), (129, 300, 100, 0), (300, 200, 130, 0), (17, 130, 1030, 1), (500, 63, 32, 0),
+                                       (40, 100, 30, 0), (1, 20, 5, 3)])
+@pytest.mark.parametrize("kinds", ["fff", "fbf", "bbf", "bbb"])
+def test_small_products(M, N, K, pad, kinds):
+    test_product_at_the_edges(M, N, K, pad, kinds)
