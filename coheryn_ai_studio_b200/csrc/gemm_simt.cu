@@ -205,6 +205,19 @@ Plan plan_of(int M, int N, int K) {
   return p;
 }
 
+// The sums of the stretches wait in a workspace of [stretch][row][column]: 64 MB at most (it stays in L2, where the adding kernel
+// finds it), so a product of many rows by a long k goes in blocks of that many rows, one after the other; one row tile at least,
+// whose sums are an eighth of the weight's own (float32) bytes.  640 x 3584 x 18944 (37 stretches) would take 339 MB at once.
+int rows_at_once(int apart, int N) {
+  const long rows = (1L << 24) / ((long)apart * N) / 64 * 64;
+  return rows < 64 ? 64 : (int)(rows < (1L << 30) ? rows : 1L << 30);
+}
+long workspace_floats(int M, int N, int apart) {
+  if (apart <= 1) return 0;
+  const int rows = rows_at_once(apart, N);
+  return (long)apart * (M < rows ? M : rows) * N;
+}
+
 template <typename TX, typename TW, typename TO>
 int run(const TX* x, const TW* w, const void* bias, int bias_dtype, TO* out, int M, int N, int K, long ldx, long ldo, int act,
         float* workspace, long floats, int n_split, int k_split, cudaStream_t stream) {
@@ -212,24 +225,27 @@ int run(const TX* x, const TW* w, const void* bias, int bias_dtype, TO* out, int
   const Plan p = plan_of(M, N, K);
   int n = p.apart;
   if (n > 1 || K > stretch_of(N)) n_split = 0;       // the stretches are those of a full row
-  if (n > 1 && (!workspace || floats < (long)n * M * N)) n = 1;
+  if (n > 1 && (!workspace || floats < workspace_floats(M, N, n))) n = 1;
   float* apart = n > 1 ? workspace : nullptr;
-  const dim3 grid((N + p.columns - 1) / p.columns, (M + p.rows - 1) / p.rows, n);
-  const int stretch = stretch_of(N);
+  const int stretch = stretch_of(N), most = n > 1 ? rows_at_once(n, N) : M;
+  for (int m = 0; m < M; m += most, x += (size_t)most * ldx, out += (size_t)most * ldo) {
+    const int rows = M - m < most ? M - m : most;
+    const dim3 grid((N + p.columns - 1) / p.columns, (rows + p.rows - 1) / p.rows, n);
 #define GO(BM, BN, BK, T, VEC, MULTI)                                                                                       \
   gemm_simt_kernel<TX, TW, TO, BM, BN, BK, T, T, VEC, MULTI><<<grid, (BM / T) * (BN / T), 0, stream>>>(                     \
-      x, w, bias, bias_dtype, out, apart, M, N, K, ldx, ldo, act, stretch, n_split, k_split)
+      x, w, bias, bias_dtype, out, apart, rows, N, K, ldx, ldo, act, stretch, n_split, k_split)
 #define BY_TILE(VEC, MULTI) if (p.few) GO(16, 64, 64, 4, VEC, MULTI); else GO(64, 128, 16, 8, VEC, MULTI)
-  if (p.few && K <= 32) { if (vec) GO(16, 64, 16, 4, true, false); else GO(16, 64, 16, 4, false, false); }
-  else if (n == 1 && K > stretch) { if (vec) { BY_TILE(true, true); } else { BY_TILE(false, true); } }
-  else { if (vec) { BY_TILE(true, false); } else { BY_TILE(false, false); } }
+    if (p.few && K <= 32) { if (vec) GO(16, 64, 16, 4, true, false); else GO(16, 64, 16, 4, false, false); }
+    else if (n == 1 && K > stretch) { if (vec) { BY_TILE(true, true); } else { BY_TILE(false, true); } }
+    else { if (vec) { BY_TILE(true, false); } else { BY_TILE(false, false); } }
 #undef BY_TILE
 #undef GO
-  CO_CHECK_LAUNCH("gemm_simt");
-  if (n > 1) {
-    const size_t size = (size_t)M * N;
-    gemm_simt_add_kernel<TO><<<(unsigned)((size + 255) / 256), 256, 0, stream>>>(apart, n, bias, bias_dtype, out, M, N, ldo, act);
-    CO_CHECK_LAUNCH("gemm_simt_add");
+    CO_CHECK_LAUNCH("gemm_simt");
+    if (n > 1) {
+      const size_t size = (size_t)rows * N;
+      gemm_simt_add_kernel<TO><<<(unsigned)((size + 255) / 256), 256, 0, stream>>>(apart, n, bias, bias_dtype, out, rows, N, ldo, act);
+      CO_CHECK_LAUNCH("gemm_simt_add");
+    }
   }
   return 0;
 }
@@ -237,8 +253,7 @@ int run(const TX* x, const TW* w, const void* bias, int bias_dtype, TO* out, int
 
 // The floats of workspace with which a product of this shape shares its stretches of k out over CTAs (0: it does not).
 CO_EXPORT long coheryn_gemm_simt_workspace_floats(int M, int N, int K) {
-  const int n = M > 0 && N > 0 && K > 0 ? plan_of(M, N, K).apart : 1;
-  return n > 1 ? (long)n * M * N : 0;
+  return M > 0 && N > 0 && K > 0 ? workspace_floats(M, N, plan_of(M, N, K).apart) : 0;
 }
 
 // How a product of this shape is laid out: rows and columns of a tile, CTAs that its stretches of k go to.

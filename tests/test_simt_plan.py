@@ -21,3 +21,11 @@ def test_the_faster_tile_is_taken(M, N, K, large, small):
     assert (rows, columns) == ((64, 128) if large < small else (16, 64))
     tiles = -(-M // rows) * -(-N // columns)
     assert apart == 1 or (apart > 1 and tiles < 296)
+
+
+@pytest.mark.parametrize("M,N,K", [(640, 3584, 18944), (300, 3584, 18944), (1100, 1536, 8960), (200, 4095, 30000), (16, 3584, 18944), (1, 100, 1000000)])
+def test_the_workspace_is_bounded(M, N, K):
+    """64 MB, or the sums of one row tile: an eighth of a float32 weight's bytes (the last stretch may be short)."""
+    lib = ops.core()
+    floats = int(lib.coheryn_gemm_simt_workspace_floats(ctypes.c_int(M), ctypes.c_int(N), ctypes.c_int(K)))
+    assert plan(M, N, K)[2] > 1 and 0 < floats <= max(1 << 24, N * (K + 512) // 8)

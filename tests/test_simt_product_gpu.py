@@ -59,3 +59,15 @@ def test_block_diagonal_weight(M, rows, cols, N, K):
 @pytest.mark.parametrize("kinds", ["fff", "fbf", "bbf", "bbb"])
 def test_small_products(M, N, K, pad, kinds):
     test_product_at_the_edges(M, N, K, pad, kinds)
+
+
+def test_rows_in_several_blocks_of_the_workspace():
+    """330 rows whose 37 stretches' sums take the workspace in blocks of 64 and of 192 rows: the bits of the same rows by themselves."""
+    g = torch.Generator(device=DEV).manual_seed(1)
+    for N, K, kinds in ((3584, 18944, torch.bfloat16), (1800, 18900, torch.float32)):
+        x, w = torch.randn((330, K), device=DEV, generator=g), (torch.randn((N, K), device=DEV, generator=g) * 0.1).to(kinds)
+        whole = product(x, w, None, torch.float32)
+        for at, n in ((0, 64), (60, 10), (127, 1), (200, 130)):
+            assert torch.equal(product(x[at:at + n], w, None, torch.float32), whole[at:at + n]), (N, at, n)
+        want = x[300:].double() @ w.double().T
+        assert float((whole[300:].double() - want).norm() / want.norm()) <= 2e-6      # float32 sums of this length are near 1e-7
