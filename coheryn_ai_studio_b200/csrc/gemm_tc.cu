@@ -747,13 +747,17 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
 // 16 KB of weights and at most 16 KB of rows per k-step.  (With rows on the lanes, 128 x 256 tiles and one CTA per tile, groups
 // of about 256 rows were 2.5 tiles of 128 each and an SM pulled 48 KB per k-step.)  Persistent over the tiles, the tiles of a
 // group next to one another, with two accumulators like gemm_tc_pair_kernel, whose barriers these are.  Measured on a B200
-// (2,048 tokens, 4 of 32 choices, 30 experts of 2,048 x 1,024, 7,700 rows): gate/up and down together 209 -> 166 us (580 TFLOP/s).
+// (2,048 tokens, 4 of 32 choices, 30 experts of 2,048 x 1,024, 7,700 rows): gate/up and down together 209 -> 166 us with four
+// epilogue warps; the gate's exponentials were then what a tile took (one warp a scheduler: 2 groups of 3,000 rows by 2,048 x 1,024,
+// gated, 62 us where 128 x 256 tiles took 46, 30 of 100 rows 49 for 40).  With eight: 41 and 38 us, ungated 51 -> 35 and 43 -> 38.
 template <int STAGES>
 struct GroupedSmem {
   static constexpr int A_BYTES = 128 * BK * 2, B_BYTES = 128 * BK * 2, STAGE_BYTES = A_BYTES + B_BYTES;
   static constexpr int FIXED = STAGES * STAGE_BYTES + 1024 /* alignment slack */ + 256 /* barriers */;
 };
 constexpr int GROUP_TILE = 256, GROUP_BOX = 32;      // rows of a tile at most, rows per TMA box
+constexpr int GROUP_EPILOGUE = 8;                    // epilogue warps of a CTA: two per quarter of its features, 32 columns in turn
+constexpr int GROUP_THREADS = 64 + 32 * GROUP_EPILOGUE;
 
 // The tiles in order: group by group, its row tiles, each by all feature tiles.
 struct GroupCursor {
@@ -778,7 +782,7 @@ struct GroupCursor {
 };
 
 template <int STAGES>
-__global__ void __launch_bounds__(192)
+__global__ void __launch_bounds__(GROUP_THREADS)
 gemm_tc_grouped_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_w, const int* __restrict__ group_offsets,
                        int G, int w_rows, void* __restrict__ out, int out_dtype, int N, int K, long ldo, int epilogue,
                        int* __restrict__ status) {
@@ -801,7 +805,7 @@ gemm_tc_grouped_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_c
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < STAGES; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
-    for (int a = 0; a < 2; ++a) { mbar_init(&acc_full[a], 1); mbar_init(&acc_empty[a], 8); }
+    for (int a = 0; a < 2; ++a) { mbar_init(&acc_full[a], 1); mbar_init(&acc_empty[a], 2 * GROUP_EPILOGUE); }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 2) {
@@ -810,7 +814,7 @@ gemm_tc_grouped_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_c
   }
   co_pdl_launch_dependents();
   co_pdl_wait();                              // the offsets and the rows are earlier kernels'
-  for (int i = threadIdx.x; i <= G; i += 192) offsets[i] = group_offsets[i];
+  for (int i = threadIdx.x; i <= G; i += GROUP_THREADS) offsets[i] = group_offsets[i];
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   cluster_sync_all();   // the peer's barriers are initialised before anything is counted on them
@@ -875,7 +879,7 @@ gemm_tc_grouped_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_c
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       const int f = (tile % tiles_f) * 256 + (int)rank * 128 + quarter * 32 + lane;      // this thread's feature
 #pragma unroll 1
-      for (int c0 = 0; c0 < at.rows; c0 += 32) {
+      for (int c0 = (warp - 2) / 4 * 32; c0 < at.rows; c0 += GROUP_EPILOGUE * 8) {
         unsigned r[32];
         tmem_ld32(tmem_base + ((unsigned)(quarter * 32) << 16) + (unsigned)(acc * GROUP_TILE + c0), r);
         if (gated) {
@@ -1187,7 +1191,7 @@ CO_EXPORT int coheryn_gemm_bf16_tc_grouped(const void* x, const void* w, void* o
     CO_FAIL("gemm_bf16_tc_grouped: cuTensorMapEncodeTiled failed (M=%d N=%d K=%d G=%d ldx=%ld)", M, N, K, G, ldx);
   const long most = ((long)M / GROUP_TILE + G) * ((N + 255) / 256);
   const int pairs = (int)(most < slots ? most : slots);
-  cudaError_t le = co_launch_cluster(2, kernel, dim3(2 * pairs), dim3(192), smem, stream, mx, mw, offsets, G, N, out, out_dtype, N, K, ldo,
+  cudaError_t le = co_launch_cluster(2, kernel, dim3(2 * pairs), dim3(GROUP_THREADS), smem, stream, mx, mw, offsets, G, N, out, out_dtype, N, K, ldo,
                                      epilogue, status);
   if (le != cudaSuccess) CO_FAIL("gemm_tc_grouped: launch failed: %s", cudaGetErrorString(le));
   CO_CHECK_LAUNCH("gemm_tc_grouped");
