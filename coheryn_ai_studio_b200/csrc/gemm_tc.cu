@@ -763,12 +763,12 @@ constexpr int GROUP_THREADS = 64 + 32 * GROUP_EPILOGUE;
 struct GroupCursor {
   int g = 0, first = 0;      // group, ordinal of its first row tile
   int row0, rows, cols;      // of the tile found: first row, rows, columns of the instruction
-  __device__ bool find(const int* offsets, int G, int t) {
+  __host__ __device__ bool find(const int* offsets, int G, int t) {
     for (; g < G; ++g) {
       const int n = offsets[g + 1] - offsets[g], tiles = (n + GROUP_TILE - 1) / GROUP_TILE;
       if (t < first + tiles) {
-        // equal tiles while that leaves none empty
-        const int size = tiles <= 8 ? ((n + tiles - 1) / tiles + 31) / 32 * 32 : GROUP_TILE;
+        // equal tiles, in steps of 32 rows: of at most 256, so that n > 256 (tiles - 1) leaves none empty
+        const int size = ((n + tiles - 1) / tiles + 31) / 32 * 32;
         const int at = (t - first) * size;
         row0 = offsets[g] + at;
         rows = min(size, n - at);
@@ -1164,6 +1164,16 @@ CO_EXPORT int coheryn_gemm_bf16_tc(const void* x, const void* w, const void* bia
 // Rows per tile that the caller's lists of row tiles are to have for the grouped product below (it cuts the groups itself).
 CO_EXPORT int coheryn_gemm_tc_grouped_tile_rows() { return BM; }
 
+// The row tiles of groups that begin at offsets[0 .. G] (on the host), as the product below cuts them: their number, and up to `room`
+// of them as (group, first row, rows, columns of the instruction).
+CO_EXPORT int coheryn_gemm_tc_grouped_tiles(const int* offsets, int G, int* tiles, int room) {
+  GroupCursor at;
+  int n = 0;
+  for (; at.find(offsets, G, n); ++n)
+    if (n < room) { tiles[4 * n] = at.g; tiles[4 * n + 1] = at.row0; tiles[4 * n + 2] = at.rows; tiles[4 * n + 3] = at.cols; }
+  return n;
+}
+
 // out[rows of group g] = x[rows of group g] . W_g^T for rows ordered by group: x [M, K] bfloat16 (row stride ldx), w [G, N, K]
 // bfloat16 contiguous, out [M, N] (or [M, N / 2] behind a gated epilogue) bfloat16 or float32; offsets [G + 1] on the device.
 // Rows that belong to no group are not written.
@@ -1179,12 +1189,10 @@ CO_EXPORT int coheryn_gemm_bf16_tc_grouped(const void* x, const void* w, void* o
   auto kernel = gemm_tc_grouped_kernel<STAGES>;
   const size_t smem = GroupedSmem<STAGES>::FIXED + ((size_t)G + 1) * sizeof(int);
   if (smem > 227 * 1024) CO_FAIL("gemm_bf16_tc_grouped: %d groups are too many", G);
-  static int slots = -1;
-  if (slots < 0) {
-    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
-    if (e != cudaSuccess) CO_FAIL("gemm_tc_grouped: %zu bytes of shared memory: %s", smem, cudaGetErrorString(e));
-    slots = pair_slots<256, 6, 2>();       // one CTA per SM as well
-  }
+  // (at every launch: the attribute belongs to the kernel on the current device)
+  cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e != cudaSuccess) CO_FAIL("gemm_tc_grouped: %zu bytes of shared memory: %s", smem, cudaGetErrorString(e));
+  const int slots = pair_slots<256, 6, 2>();       // one CTA per SM as well
   if (slots <= 0) CO_FAIL("gemm_tc_grouped: no pair of CTAs with %zu bytes of shared memory fits the device", smem);
   CUtensorMap mx, mw;
   if (!make_map(&mx, x, M, K, ldx, GROUP_BOX) || !make_map(&mw, w, (long)G * N, K, K, 128))
