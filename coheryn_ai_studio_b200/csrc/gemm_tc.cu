@@ -1161,9 +1161,6 @@ CO_EXPORT int coheryn_gemm_bf16_tc(const void* x, const void* w, const void* bia
 #undef GO
 }
 
-// Rows per tile that the caller's lists of row tiles are to have for the grouped product below (it cuts the groups itself).
-CO_EXPORT int coheryn_gemm_tc_grouped_tile_rows() { return BM; }
-
 // The row tiles of groups that begin at offsets[0 .. G] (on the host), as the product below cuts them: their number, and up to `room`
 // of them as (group, first row, rows, columns of the instruction).
 CO_EXPORT int coheryn_gemm_tc_grouped_tiles(const int* offsets, int G, int* tiles, int room) {

@@ -135,7 +135,7 @@ route_select_kernel(const float* __restrict__ logits, long ld, const void* __res
 
 // ------------------------------------------------------------------------------------------------- sort by expert
 // One CTA.  offsets[E + 1]; row_of[n] (-1 for an identity choice); token_of[row]; tiles: tile_group[], tile_row0[] and
-// n_tiles[0] for row tiles of `bm` rows.
+// n_tiles[0] for row tiles of `bm` rows (tile_group null: no lists).
 __global__ void __launch_bounds__(1024)
 route_sort_kernel(const int* __restrict__ ids, int n, int top, int E, int bm, int* __restrict__ offsets, int* __restrict__ row_of,
                   int* __restrict__ token_of, int* __restrict__ tile_group, int* __restrict__ tile_row0, int* __restrict__ n_tiles) {
@@ -163,10 +163,10 @@ route_sort_kernel(const int* __restrict__ ids, int n, int top, int E, int bm, in
     }
     offsets[E] = at;
     tile0[E] = tiles;
-    n_tiles[0] = tiles;
+    if (tile_group) n_tiles[0] = tiles;
   }
   __syncthreads();
-  for (int e = threadIdx.x; e < E; e += blockDim.x) {
+  for (int e = threadIdx.x; tile_group && e < E; e += blockDim.x) {
     const int first = tile0[e], cnt = tile0[e + 1] - first, base = offsets[e];
     for (int i = 0; i < cnt; ++i) { tile_group[first + i] = e; tile_row0[first + i] = base + i * bm; }
   }
@@ -482,17 +482,16 @@ CO_EXPORT int coheryn_route_select(const float* logits, long ld, const void* cor
 // Rows per tile of the grouped products, by the kernel that will run (both use the same today).
 CO_EXPORT int coheryn_grouped_tile_rows() { return TBM; }
 
-// tile_rows: the rows per tile of the product that will read the lists (0: those of the grouped kernels of this file).
+// The lists of row tiles are those of the grouped kernels of this file; tile_group null: they are left out.
 CO_EXPORT int coheryn_route_sort(const int* ids, int n, int top, int E, int* offsets, int* row_of, int* token_of, int* tile_group,
-                                 int* tile_row0, int* n_tiles, int tile_rows, cudaStream_t stream) {
+                                 int* tile_row0, int* n_tiles, cudaStream_t stream) {
   if (n <= 0) return 0;
-  if (E < 1 || top < 1 || tile_rows < 0) CO_FAIL("route_sort: bad sizes");
-  if (tile_rows == 0) tile_rows = TBM;
+  if (E < 1 || top < 1) CO_FAIL("route_sort: bad sizes");
   static_assert(TBM == SBM, "both grouped kernels take the same row tiles");
   const size_t smem = (size_t)(3 * E + 1) * sizeof(int);
   if (smem > 200 * 1024) CO_FAIL("route_sort: %d experts do not fit in shared memory", E);
   if (smem > 48 * 1024) cudaFuncSetAttribute(route_sort_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  co_launch(route_sort_kernel, dim3(1), dim3(1024), smem, stream, ids, n, top, E, tile_rows, offsets, row_of, token_of, tile_group,
+  co_launch(route_sort_kernel, dim3(1), dim3(1024), smem, stream, ids, n, top, E, TBM, offsets, row_of, token_of, tile_group,
             tile_row0, n_tiles);
   CO_CHECK_LAUNCH("route_sort");
   return 0;

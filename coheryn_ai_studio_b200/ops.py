@@ -1599,32 +1599,34 @@ def route_select(logits: torch.Tensor, correction: Optional[torch.Tensor], n_gro
 
 class RoutedRows:
     """The (token, choice) pairs of a step ordered by expert, as ``route_sort`` leaves them on the device."""
-    __slots__ = ("n", "experts", "offsets", "row_of", "token_of", "tile_group", "tile_row0", "n_tiles", "max_tiles", "tile_rows")
+    __slots__ = ("n", "experts", "offsets", "row_of", "token_of", "wide", "tile_group", "tile_row0", "n_tiles", "max_tiles")
 
 
 def route_sort(ids: torch.Tensor, experts: int, wide_tiles: bool = False) -> RoutedRows:
-    """Order the pairs whose id names one of the first ``experts`` outputs by expert.  ``wide_tiles``: row tiles for
-    ``gemm_bf16_tc_grouped`` instead of ``grouped_linear``; every index of the book is then a valid one (rows that no pair
-    takes name token 0)."""
+    """Order the pairs whose id names one of the first ``experts`` outputs by expert.  ``wide_tiles``: for
+    ``gemm_bf16_tc_grouped``, which cuts the experts' rows itself, instead of ``grouped_linear``, which reads lists of row
+    tiles; every index of the book is then a valid one (rows that no pair takes name token 0)."""
     _dev(ids)
     _i32(ids, "ids")
     T, top = ids.shape
     n = T * top
     lib = routed()
-    bm = int(core().coheryn_gemm_tc_grouped_tile_rows()) if wide_tiles else int(lib.coheryn_grouped_tile_rows())
     r = RoutedRows()
-    r.n, r.experts, r.max_tiles, r.tile_rows = n, experts, n // bm + experts, bm
-    book = (torch.zeros if wide_tiles else torch.empty)(experts + 1 + 2 * n + 2 * r.max_tiles + 1, dtype=torch.int32, device=ids.device)
+    r.n, r.experts, r.wide = n, experts, bool(wide_tiles)
+    r.max_tiles = 0 if wide_tiles else n // int(lib.coheryn_grouped_tile_rows()) + experts
+    book = (torch.zeros if wide_tiles else torch.empty)(experts + 1 + 2 * n + (0 if wide_tiles else 2 * r.max_tiles + 1),
+                                                        dtype=torch.int32, device=ids.device)
     o = 0
     r.offsets = book[o:o + experts + 1]; o += experts + 1
     r.row_of = book[o:o + n]; o += n
     r.token_of = book[o:o + n]; o += n
-    r.tile_group = book[o:o + r.max_tiles]; o += r.max_tiles
-    r.tile_row0 = book[o:o + r.max_tiles]; o += r.max_tiles
-    r.n_tiles = book[o:o + 1]
+    r.tile_group = r.tile_row0 = r.n_tiles = None
+    if not wide_tiles:
+        r.tile_group = book[o:o + r.max_tiles]; o += r.max_tiles
+        r.tile_row0 = book[o:o + r.max_tiles]; o += r.max_tiles
+        r.n_tiles = book[o:o + 1]
     _check(lib, lib.coheryn_route_sort(_ptr(ids), c_int(n), c_int(top), c_int(experts), _ptr(r.offsets), _ptr(r.row_of),
-                                       _ptr(r.token_of), _ptr(r.tile_group), _ptr(r.tile_row0), _ptr(r.n_tiles),
-                                       c_int(bm if wide_tiles else 0), _stream()))
+                                       _ptr(r.token_of), _ptr(r.tile_group), _ptr(r.tile_row0), _ptr(r.n_tiles), _stream()))
     return r
 
 
@@ -1650,7 +1652,7 @@ def gemm_bf16_tc_grouped(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, ro
     assert a.dtype == torch.bfloat16 and w.dtype == torch.bfloat16 and w.is_contiguous() and a.shape == (rows.n, K)
     assert a.stride(1) == 1 and out.stride(1) == 1 and out.shape == (rows.n, N // 2 if epilogue else N) and G == rows.experts
     lib = core()
-    assert rows.tile_rows == int(lib.coheryn_gemm_tc_grouped_tile_rows())
+    assert rows.wide
     _check(lib, lib.coheryn_gemm_bf16_tc_grouped(
         _ptr(a), _ptr(w), _ptr(out), c_int(_code(out)), c_int(rows.n), c_int(N), c_int(K), c_int(G), c_long(a.stride(0)),
         c_long(out.stride(0)), c_int(int(epilogue)), _ptr(rows.offsets), _ptr(tc_status(a.device)), _stream()))
@@ -1673,6 +1675,7 @@ def grouped_linear(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, rows: Op
         _f32(factor, "factor")
         assert factor.stride(1) == 1 and factor.shape[1] == G
     lib = routed()
+    assert rows is None or not rows.wide
     M = a.shape[0] if rows is None else rows.n
     _check(lib, lib.coheryn_grouped_linear(
         _ptr(a), c_int(_code(a)), c_long(a.stride(0)), c_long(a_col), _ptr(w), c_int(_code(w)), c_long(N * K), _ptr(out),
