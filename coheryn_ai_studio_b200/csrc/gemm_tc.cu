@@ -1106,6 +1106,13 @@ static int persistent_width(int M, int N) {
   return best;
 }
 
+// Columns of the persistent kernel's tiles, for a product that the pairs do not take (0: it has no more than one tile per SM, or
+// runs without the persistent kernel).
+CO_EXPORT int coheryn_gemm_tc_persistent_width(int M, int N) {
+  const long tiles_m = ((long)M + BM - 1) / BM;
+  return tile_width(M, N) == 256 && g_stages != 1 && tiles_m * ((N + 255) / 256) > 148 ? persistent_width(M, N) : 0;
+}
+
 // Floats of workspace with which coheryn_gemm_bf16_tc splits K over several CTAs (0: this
 // shape is not split).  Without the workspace the product runs unsplit.
 CO_EXPORT long coheryn_gemm_tc_workspace_floats(int M, int N, int K) {
@@ -1135,11 +1142,11 @@ CO_EXPORT int coheryn_gemm_bf16_tc(const void* x, const void* w, const void* bia
   if (status && pair_suits(M, N))
     return coheryn_gemm_bf16_tc_pair(x, w, bias, bias_dtype, out, out_dtype, M, N, K, ldx, ldo, epilogue, status, stream);
   const int bn = tile_width(M, N);
-  const long tiles_m = (M + BM - 1) / BM;
   int splits = splits_for(M, N, K, bn);
   if (splits > 1 && (!workspace || workspace_floats < (long)splits * M * N)) splits = 1;
-  const bool persistent = bn == 256 && g_stages != 1 && tiles_m * ((N + 255) / 256) > 148;
-  const int width = persistent ? persistent_width(M, N) : bn;
+  const int rounds_width = coheryn_gemm_tc_persistent_width(M, N);
+  const bool persistent = rounds_width > 0;
+  const int width = persistent ? rounds_width : bn;
   CUtensorMap mx, mw;
   if (!make_map(&mx, x, M, K, ldx, BM) || !make_map(&mw, w, N, K, K, width))
     CO_FAIL("gemm_bf16_tc: cuTensorMapEncodeTiled failed (M=%d N=%d K=%d ldx=%ld)", M, N, K, ldx);
