@@ -202,3 +202,42 @@ def test_float32_mixers_keep_their_bits_however_a_sequence_is_cut(kind, dk, dv):
     assert want.shape[0] == 200 and bool(want.isfinite().all()) and float(want.abs().max()) > 0
     for got, state in (run([64, 1, 70, 65]), run([1, 199]), run([130, 70], beside=120)):
         assert torch.equal(got, want) and torch.equal(state, end)
+
+
+@pytest.mark.parametrize("heads,dk,dv", [(2, 24, 200), (1, 128, 256), (3, 64, 72), (1, 192, 80), (2, 256, 130)])
+def test_long_portions_token_by_token(heads, dk, dv):
+    """The scans of long portions, whose heads' columns go to several CTAs (norm and gate in a kernel of their own), and of the
+    short ones between them, continuing each other's state: sizes that chunks take too, and more key channels than they take.  The
+    bounds are those of the scans' own tests."""
+    from coheryn_ai_studio_b200 import ops
+    rng = np.random.default_rng(dv + dk)
+    cuts, eps, cap = [130, 1, 70, 2, 64, 33], 1e-6, 9.0
+    n = sum(cuts)
+    f = lambda *s: rng.normal(size=s)
+    d = dict(delta_inputs(rng, n, heads, 1, dk, dv, True), mq=f(n, heads * dk), mk=f(n, heads * dk), gi=f(n, heads) * 2, gf=f(n, heads) * 2 + 3.0)
+    bias, rate_log, weight, bi, bf, wm = f(heads * dk), f(heads) * 0.5, f(dv), f(heads), f(heads), f(heads * dv)
+    unit = lambda a: a / np.sqrt((a * a).sum(-1, keepdims=True) + 1e-6)
+    decay = np.exp(-np.exp(rate_log)[None, :, None] * plain.softplus(d["step"] + bias).reshape(n, heads, dk))
+    v, per = d["v"].reshape(n, heads, dv), lambda a: a.reshape(n, heads, dk)
+    o = np.stack([plain.gated_delta_rule(unit(d["q"]) * dk ** -0.5, unit(d["k"]), v[:, h], plain.sigmoid(d["beta"][:, h]), decay[:, h])
+                  for h in range(heads)], axis=1)
+    want_d = (plain.rms(o, eps) * weight).reshape(n, heads * dv) * plain.sigmoid(d["gate"])
+    li = cap * np.tanh((d["gi"] + bi) / cap); lf = plain.log_sigmoid(cap * np.tanh((d["gf"] + bf) / cap))
+    o = np.stack([plain.matrix_memory(per(d["mq"])[:, h] * dk ** -0.5, per(d["mk"])[:, h], v[:, h], li[:, h], lf[:, h]) for h in range(heads)], axis=1)
+    want_m = plain.rms(o, eps).reshape(n, heads * dv) * wm * plain.sigmoid(d["gate"])
+    state_d, state_m = torch.zeros((2, heads * dk * dv), device=DEV), torch.zeros((2, heads * (dk * dv + dk + 1)), device=DEV)
+    at = 0
+    for m in cuts:
+        step, cat = step_of([m], [1]), lambda *keys: dev(np.concatenate([d[k][at:at + m] for k in keys], axis=1))
+        out = torch.empty((m, heads * dv), device=DEV)
+        qkv = cat("q", "k", "v")
+        ops.gated_delta_scan(qkv[:, :dk], qkv[:, dk:2 * dk], qkv[:, 2 * dk:], cat("beta"), cat("step"), dev(bias), dev(rate_log), state_d, step,
+                             heads, 1, dk, dv, out, dev(weight), cat("gate"), eps, in_chunks=False)
+        ref = want_d[at:at + m]
+        assert np.abs(out.cpu().numpy() - ref).max() <= 3e-4 * max(1.0, np.abs(ref).max()), ("delta", at, m)
+        qkv, gates, c = cat("mq", "mk", "v"), cat("gi", "gf"), heads * dk
+        ops.matrix_memory_scan(qkv[:, :c], qkv[:, c:2 * c], qkv[:, 2 * c:], gates[:, :heads], gates[:, heads:], dev(bi), dev(bf), cap, state_m, step,
+                               heads, dk, dv, out, dev(wm), cat("gate"), eps, in_chunks=False)
+        ref = want_m[at:at + m]
+        assert np.abs(out.cpu().numpy() - ref).max() <= 1e-3 * max(1.0, np.abs(ref).max()), ("memory", at, m)
+        at += m

@@ -186,9 +186,10 @@ def test_matrix_memory_kernel(heads, dk, dv, cap):
 
 @pytest.mark.parametrize("heads,dk,dv", [(2, 24, 200), (1, 128, 256), (3, 64, 72)])
 def test_scans_of_long_portions_split_a_heads_columns_over_ctas(heads, dk, dv):
-    """One request whose long portions (64 tokens and more) run as several CTAs per head, with norm and gate in a kernel of
-    their own (the delta rule from prepared inputs, staged asynchronously), and whose short portions run the one-CTA kernels:
-    both against the token-by-token recurrences, continuing each other's state."""
+    """One request of long portions (64 tokens and more) and short ones, continuing each other's state, against the token-by-token
+    recurrences.  Token by token a long portion runs as several CTAs per head, with norm and gate in a kernel of their own (the
+    delta rule from prepared inputs, staged asynchronously); here, where chunks are allowed, the form that is estimated to be
+    faster runs, and test_chunked_scans_gpu.py has the same portions token by token."""
     from coheryn_ai_studio_b200 import ops
     rng = np.random.default_rng(dv)
     cuts, eps, cap, groups = [130, 1, 70, 2, 64, 33], 1e-6, 9.0, 1

@@ -71,3 +71,12 @@ def test_rows_in_several_blocks_of_the_workspace():
             assert torch.equal(product(x[at:at + n], w, None, torch.float32), whole[at:at + n]), (N, at, n)
         want = x[300:].double() @ w.double().T
         assert float((whole[300:].double() - want).norm() / want.norm()) <= 2e-6      # float32 sums of this length are near 1e-7
+
+
+# One CTA over several stretches of k (a wide weight): both tiles, with aligned and with unaligned rows.
+@pytest.mark.parametrize("M,N,K,pad", [(600, 4100, 2052, 0), (600, 4100, 2051, 1), (16, 19000, 2052, 4), (5, 18945, 4101, 0)])
+@pytest.mark.parametrize("kinds", ["fff", "fbf", "bbf", "bbb"])
+def test_several_stretches_per_cta(M, N, K, pad, kinds):
+    from coheryn_ai_studio_b200 import ops
+    assert ops._simt_workspace_floats(M, N, K) == 0
+    test_product_at_the_edges(M, N, K, pad, kinds)
