@@ -824,14 +824,17 @@ CO_EXPORT int coheryn_short_conv_silu(const float* x, long ldx, float* y, long l
                                       const int* state_slots, int T, int B, int update_state, cudaStream_t stream) {
   if (T <= 0 || C <= 0) return 0;
   if (n < 1 || n > MAX_TAPS) CO_FAIL("short_conv: 1..%d taps, not %d", MAX_TAPS, n);
-  if (n >= 2 && n <= 4) {
-    const bool vec = C % 4 == 0 && ldx % 4 == 0 && ldy % 4 == 0 && state_stride % 4 == 0 &&
-                     (((uintptr_t)x | (uintptr_t)y | (uintptr_t)state) & 15) == 0;
-    const int across = vec ? (C / 4 + 127) / 128 : (C + 127) / 128;
-    // sixteen tokens per thread (three inputs read again per sixteen) once that leaves a few CTAs per SM, else fewer
+  const bool vec = C % 4 == 0 && ldx % 4 == 0 && ldy % 4 == 0 && state_stride % 4 == 0 &&
+                   (((uintptr_t)x | (uintptr_t)y | (uintptr_t)state) & 15) == 0;
+  const int threads = vec ? C / 4 : C, across = (threads + 127) / 128;
+  // With few channels most of a CTA would idle (24 channels, 2,048 tokens, 2 taps: 4.3 us, 3.4 a thread per element).
+  if (n >= 2 && n <= 4 && 2 * threads >= 128 * across) {
+    // sixteen tokens per thread (three inputs read again per sixteen) once that leaves a few CTAs per SM, else fewer; more where
+    // the grid's second dimension (65,535) would not hold the step
     int per = 16;
     while (per > 1 && (long)across * ((T + per - 1) / per) < 4 * 148) per >>= 1;
-    const dim3 grid(across, (T + per - 1) / per);
+    while ((T - 1) / per + 1 > 65535) per *= 2;
+    const dim3 grid(across, (T - 1) / per + 1);
 #define RUN(N, W)                                                                                                            \
   co_launch(short_conv_silu_run_kernel<N, W>, grid, dim3(128), 0, stream, x, ldx, y, ldy, taps, taps_dtype, C,               \
             (const float*)state, state_stride, token_req, cu_q, state_slots, T, per)

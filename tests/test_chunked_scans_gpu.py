@@ -241,3 +241,26 @@ def test_long_portions_token_by_token(heads, dk, dv):
         ref = want_m[at:at + m]
         assert np.abs(out.cpu().numpy() - ref).max() <= 1e-3 * max(1.0, np.abs(ref).max()), ("memory", at, m)
         at += m
+
+
+@pytest.mark.parametrize("taps,channels,offset", [(2, 256, 0), (3, 260, 4), (2, 65, 0), (3, 129, 1), (4, 24, 0)])
+def test_short_convolution_wide_and_narrow(taps, channels, offset):
+    """Rows by four channels and by one per thread, and too few channels for a CTA."""
+    test_short_convolution_by_runs_of_tokens(taps, channels, offset)
+
+
+def test_short_convolution_of_a_million_tokens():
+    """One run of 2^20 + 50 tokens: more sixteens of tokens than a grid's second dimension holds."""
+    from coheryn_ai_studio_b200 import ops
+    n, channels, taps = (1 << 20) + 50, 65, 3
+    g = torch.Generator(DEV).manual_seed(2)
+    x, w, state = (torch.randn(s, generator=g, device=DEV) for s in ((n, channels), (channels, taps), (1, (taps - 1) * channels)))
+    rows = torch.cat([state.reshape(taps - 1, channels), x])
+    step = types.SimpleNamespace(num_requests=1, num_tokens=n, cu_q=dev([0, n], torch.int32), token_req=torch.zeros(n, dtype=torch.int32, device=DEV),
+                                 state_slots=dev([0], torch.int32), q_lens=[n])
+    y = ops.short_conv_silu(x, w, state, step)
+    for at in (0, 524288, n - 100):
+        s = sum(rows[at + j:at + j + 100].double() * w[:, j].double() for j in range(taps))
+        want = s * torch.sigmoid(s)
+        assert float((y[at:at + 100].double() - want).abs().max()) <= 1e-5 * max(1.0, float(want.abs().max()))
+    assert torch.equal(state.reshape(taps - 1, channels), x[n - taps + 1:])
