@@ -14,6 +14,9 @@
 //   delta_state_kernel   a CTA per (request, head, 16 value channels): chunk after chunk U = T V - W S, S <- E_C S + K^ U;
 //   delta_out_kernel     a CTA per (chunk, head): O = [Q~ | B] [S ; U] and the norm, weight and gate behind it.
 //
+// A value or key that is not finite makes the outputs of its whole chunk so, not only those from its token on (zeros of T and B
+// times it); the state behind it is lost either way.
+//
 // All decays enter as products of the g between two tokens, over at most 16 tokens at a time and then over whole blocks of
 // 16: no quotient and no exponent of a sum, so a decay of any strength is as exact as in the token-by-token scan.
 //

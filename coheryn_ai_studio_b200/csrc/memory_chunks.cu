@@ -12,8 +12,12 @@
 //   memory_carry_kernel   over a run's chunks, element by element: the S_0 and n_0 of every chunk; the last ones are kept;
 //   memory_out_kernel     a CTA per (chunk, head): the outputs and the norm, weight and gate behind them.
 //
-// Every exponent is a difference of float64 sums, so that a weight is as exact however far the gates have summed up, and none
-// is above zero.
+// Every exponent is a difference of float64 sums, so that a weight is as exact however far the gates have summed up.  The maxima
+// m are kept in float32, so an exponent may exceed zero by the rounding of m (3e-5 at m = 1,000): S, n and exp(-m) all use the same
+// rounded m, and what it is off by cancels between numerator and denominator.
+//
+// A value or key that is not finite makes the outputs of its whole chunk so, not only those from its token on: a zero weight times
+// it is not zero.
 //
 // What bounds it: the scan token by token is a chain of dependent multiply-adds and shuffles on a CTA per (head, 64 value
 // channels): 0.65 us per token with 32 of 148 SMs at work.  Here only the carry is a chain, of one multiply-add per chunk and
