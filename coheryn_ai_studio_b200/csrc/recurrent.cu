@@ -895,15 +895,15 @@ CO_EXPORT long coheryn_delta_chunk_floats(int chunks, int heads, int dk, int dv)
 CO_EXPORT long coheryn_memory_chunk_floats(int chunks, int heads, int dk, int dv) {
   return co_memory_chunks_take(dk, dv) ? co_memory_chunk_floats(chunks, heads, dk, dv) : 0;
 }
-// Whether a step's runs of CHUNK_FROM tokens and more (`chunks` chunks, `long_tokens` tokens, the longest of `longest`) are to go in
-// chunks, beside shorter ones of at most `longest_short` tokens, T tokens of B requests in all.  The scan is a chain over the longest
-// run and wants few requests to be slow; the chunks cost four kernels at least, and several times the multiply-adds.  Which is faster is
-// a matter of all these sizes, so both are estimated, in us.  The constants are fitted to the times of both forms on a B200 (1 to 128
-// runs of 48 to 320 tokens, six sizes of heads each): a tenth rms, and of 804 combinations the choice costs more than 15 % in 18 (before, with chunks for every run of 48, that many were 299).  Scan
-// and chunks measured, delta rule: 12 heads of 128 x 128, one run of 64 tokens 58 and 97 us, of 320 199 and 163, 16 of 64 135 and 232,
-// 32 of 256 906 and 897; 4 heads of 32 x 64, one run of 96 tokens 65 and 59, 128 of 48 47 and 188.  Matrix memory: 8 heads of 128 x 256,
-// one run of 64 tokens 59 and 70, of 192 141 and 92, 16 of 64 148 and 132; 2 heads of 32 x 128, 32 of 48 45 and 63.
-// The delta rule's chunks are kept up to a tenth beyond the scan's time.
+// Whether a step's runs of CHUNK_FROM tokens and more (`chunks` chunks, the longest run of `longest` tokens) are to go in chunks; T
+// tokens of B requests in all.  The scan is a chain over the longest run, slow while requests are few; the chunks cost four kernels
+// at least, and several times the multiply-adds.  Which is faster is a matter of all these sizes, so both are estimated, in us.  The
+// constants are fitted to the times of both forms on a B200 (1 to 128 runs of 48 to 320 tokens, six sizes of heads each): a tenth rms,
+// and of 804 combinations the choice costs more than 15 % in 18 (with chunks for every run of 48 that many were 299).  Scan and chunks
+// measured, delta rule: 12 heads of 128 x 128, one run of 64 tokens 58 and 97 us, of 320 199 and 163, 16 of 64 135 and 232, 32 of 256 906
+// and 897; 4 heads of 32 x 64, one run of 96 tokens 65 and 59, 128 of 48 47 and 188.  Matrix memory: 8 heads of 128 x 256, one run of 64
+// tokens 59 and 70, of 192 141 and 92, 16 of 64 148 and 132; 2 heads of 32 x 128, 32 of 48 45 and 63.  The delta rule's chunks are kept up
+// to a tenth beyond the scan's time.
 static float sliced_load(int B, int heads, int dv) { return fmaxf(1.f, (float)((long)B * heads * ((dv + SLICE_COLUMNS - 1) / SLICE_COLUMNS)) / 148.f); }
 static float delta_scan_us(int heads, int dk, int dv, int B, int T, int longest) {
   if (scan_splits(B, heads, dv, T)) return longest * (0.344f + 0.00263f * dk) * sliced_load(B, heads, dv) + 14.f;
@@ -914,18 +914,16 @@ static float memory_scan_us(int heads, int dk, int dv, int B, int T, int longest
   if (scan_splits(B, heads, dv, T)) return longest * (0.41f + 0.00239f * dk) * sliced_load(B, heads, dv) + 13.f;
   return fmaxf(longest * (1.02f + 0.838f * size), (float)T * heads * 0.0195f * powf(size, 0.867f)) - 1.f;
 }
-CO_EXPORT int coheryn_delta_chunks_pay(int heads, int dk, int dv, int B, int T, int longest, int chunks, int long_tokens, int longest_short) {
+CO_EXPORT int coheryn_delta_chunks_pay(int heads, int dk, int dv, int B, int T, int longest, int chunks) {
   if (!co_delta_chunks_take(dk, dv)) return 0;
   const int D = dk <= 64 ? 64 : 128;
-  float us = 24.f + 0.4245f * D + 0.088f * dv + (float)chunks * heads * 0.559f * powf(D * dv / 16384.f, 0.605f);
-  if (longest_short > 0) us += delta_scan_us(heads, dk, dv, 148, T - long_tokens, longest_short);      // (beside chunks no head is split)
+  const float us = 24.f + 0.4245f * D + 0.088f * dv + (float)chunks * heads * 0.559f * powf(D * dv / 16384.f, 0.605f);
   return us <= 1.1f * delta_scan_us(heads, dk, dv, B, T, longest);
 }
-CO_EXPORT int coheryn_memory_chunks_pay(int heads, int dk, int dv, int B, int T, int longest, int chunks, int long_tokens, int longest_short) {
+CO_EXPORT int coheryn_memory_chunks_pay(int heads, int dk, int dv, int B, int T, int longest, int chunks) {
   if (!co_memory_chunks_take(dk, dv)) return 0;
   const float size = dk * dv / 32768.f;
-  float us = 40.f + 17.5f * size + 0.106f * dk + 1.065f * size * ((longest + CHUNK_TOKENS - 1) / CHUNK_TOKENS) + (float)chunks * heads * 0.467f * powf(size, 0.66f);
-  if (longest_short > 0) us += memory_scan_us(heads, dk, dv, 148, T - long_tokens, longest_short);
+  const float us = 40.f + 17.5f * size + 0.106f * dk + 1.065f * size * ((longest + CHUNK_TOKENS - 1) / CHUNK_TOKENS) + (float)chunks * heads * 0.467f * powf(size, 0.66f);
   return us <= memory_scan_us(heads, dk, dv, B, T, longest);
 }
 CO_EXPORT int coheryn_chunk_from() { return CHUNK_FROM; }

@@ -1114,12 +1114,11 @@ def _chunked_runs(lib, pay, step, T: int, heads: int, dk: int, dv: int):
         long = [n for n in lens if n >= first]
         if not long:
             return 0, 0, True
-        chunks, runs, rest, tokens, longest = sum(-(-n // size) for n in long), len(long), len(long) < B, sum(long), max(long)
-        short = max(n for n in lens if n < first) if rest else 0
+        chunks, runs, rest, longest = sum(-(-n // size) for n in long), len(long), len(long) < B, max(long)
     else:
-        runs, longest, tokens, rest, short = min(B, T // first), T - B + 1, T, True, 0
+        runs, longest, rest = min(B, T // first), T - B + 1, True
         chunks = T // size + runs
-    if not pay(c_int(heads), c_int(dk), c_int(dv), c_int(B), c_int(T), c_int(longest), c_int(chunks), c_int(tokens), c_int(short)):
+    if not pay(c_int(heads), c_int(dk), c_int(dv), c_int(B), c_int(T), c_int(longest), c_int(chunks)):
         return 0, 0, True
     return chunks, runs, rest
 

@@ -30,6 +30,8 @@ def test_the_faster_form_is_taken(kind, heads, dk, dv, lens, scan, chunks):
 
 
 def test_what_is_cut_into_chunks():
+    for lens, cut in (([100, 9, 47, 64], 2), ([100], 1), ([64], 1), ([47], 0)):
+        assert choice("delta", 2, 64, 48, lens)[1] == cut
     assert choice("delta", 12, 128, 128, [1021, 407, 130, 2]) == (16 + 7 + 3, 3, True)
     assert choice("delta", 12, 128, 128, [1021, 407]) == (16 + 7, 2, False)
     assert choice("memory", 8, 128, 256, [2048, 47, 48]) == (32 + 1, 2, True)

@@ -84,7 +84,8 @@ def test_gated_delta_rule_in_chunks(lens, heads, groups, dk, dv, channel, act, h
 
 
 def test_a_runs_rows_do_not_depend_on_the_other_runs():
-    """Bit for bit: alone, beside a run that goes chunk by chunk and beside one that goes token by token."""
+    """Bit for bit: alone, beside a run that goes chunk by chunk and beside one that goes token by token (at sizes where each run's
+    own step and the common one take the same form, see test_chunk_choice.py)."""
     rng = np.random.default_rng(5)
     heads, groups, dk, dv = 2, 1, 64, 48
     parts = [delta_inputs(rng, n, heads, groups, dk, dv, True) for n in (100, 9, 47, 64)]
