@@ -1107,7 +1107,7 @@ def _chunked_runs(lib, pay, step, T: int, heads: int, dk: int, dv: int):
     says that this is faster.  From the host's copy of the runs' lengths where the step has one, else the most that T tokens of
     so many requests can be."""
     first, size, B = lib.chunk_from, lib.chunk_tokens, step.num_requests
-    if T - B + 1 < first:         # no run is as long
+    if T < first:
         return 0, 0, True
     lens = getattr(step, "q_lens", None)
     if lens is not None and len(lens) == B:
@@ -1162,12 +1162,13 @@ def gated_delta_scan(q, k, v, beta, step_pre, step_bias, rate_log, state, step, 
     gate_code = {"sigmoid": 0, "silu": 1}[gate_activation]
     assert state.shape[1] == heads * dk * dv and out.shape == (q.shape[0], heads * dv) and out.stride(1) == 1
     lib = recurrent()
-    chunks, runs, rest = _chunked_runs(lib, lib.coheryn_delta_chunks_pay, step, q.shape[0], heads, dk, dv) if in_chunks else (0, 0, True)
-    floats = int(lib.coheryn_delta_chunk_floats(c_int(chunks), c_int(heads), c_int(dk), c_int(dv))) if chunks else 0
-    if floats:
-        scratch = torch.empty(floats, dtype=torch.float32, device=q.device)
+    T, B, chunks, runs, rest = q.shape[0], step.num_requests, 0, 0, True
+    if in_chunks and T - B + 1 >= lib.chunk_from:      # (else no run is as long)
+        chunks, runs, rest = _chunked_runs(lib, lib.coheryn_delta_chunks_pay, step, T, heads, dk, dv)
+    if chunks:
+        scratch = torch.empty(int(lib.coheryn_delta_chunk_floats(c_int(chunks), c_int(heads), c_int(dk), c_int(dv))), dtype=torch.float32, device=q.device)
     else:
-        scratch = _scan_scratch(q.shape[0], step.num_requests, heads, dv, q.shape[0] * (2 * kv_heads * dk + heads * dk + heads), q.device)
+        scratch = _scan_scratch(T, B, heads, dv, T * (2 * kv_heads * dk + heads * dk + heads), q.device)
     _check(lib, lib.coheryn_gated_delta_scan(
         _ptr(q), _ptr(k), _ptr(v), c_long(q.stride(0)), _ptr(beta), c_long(beta.stride(0)), _ptr(step_pre),
         c_long(step_pre.stride(0)), _ptr(step_bias), c_int(_code(step_bias)), _ptr(rate_log), c_int(_code(rate_log)),
@@ -1175,7 +1176,7 @@ def gated_delta_scan(q, k, v, beta, step_pre, step_bias, rate_log, state, step, 
         c_int(heads), c_int(kv_heads), c_int(dk), c_int(dv), _ptr(out), c_int(_code(out)), c_long(out.stride(0)),
         _ptr(norm_weight), c_int(_code(norm_weight)), c_int(0), _ptr(gate), c_long(gate.stride(0)), c_float(eps),
         c_float(out_scale), c_int(q.shape[0]), _ptr(scratch), c_long(scratch.numel() if scratch is not None else 0),
-        c_int(dc), c_int(gate_code), c_int(chunks if floats else 0), c_int(runs), c_int(1 if rest else 0), _stream()))
+        c_int(dc), c_int(gate_code), c_int(chunks), c_int(runs), c_int(1 if rest else 0), _stream()))
 
 
 def matrix_memory_scan(q, k, v, gate_i, gate_f, bias_i, bias_f, cap: float, state, step, heads: int, dk: int, dv: int,
@@ -1196,19 +1197,20 @@ def matrix_memory_scan(q, k, v, gate_i, gate_f, bias_i, bias_f, cap: float, stat
     assert norm_weight.numel() == heads * dv
     assert state.shape[1] == heads * (dk * dv + dk + 1) and out.shape == (q.shape[0], heads * dv) and out.stride(1) == 1
     lib = recurrent()
-    chunks, runs, rest = _chunked_runs(lib, lib.coheryn_memory_chunks_pay, step, q.shape[0], heads, dk, dv) if in_chunks else (0, 0, True)
-    floats = int(lib.coheryn_memory_chunk_floats(c_int(chunks), c_int(heads), c_int(dk), c_int(dv))) if chunks else 0
-    if floats:
-        scratch = torch.empty(floats, dtype=torch.float32, device=q.device)
+    T, B, chunks, runs, rest = q.shape[0], step.num_requests, 0, 0, True
+    if in_chunks and T - B + 1 >= lib.chunk_from:
+        chunks, runs, rest = _chunked_runs(lib, lib.coheryn_memory_chunks_pay, step, T, heads, dk, dv)
+    if chunks:
+        scratch = torch.empty(int(lib.coheryn_memory_chunk_floats(c_int(chunks), c_int(heads), c_int(dk), c_int(dv))), dtype=torch.float32, device=q.device)
     else:
-        scratch = _scan_scratch(q.shape[0], step.num_requests, heads, dv, step.num_requests * heads * (dk + 1), q.device)
+        scratch = _scan_scratch(T, B, heads, dv, B * heads * (dk + 1), q.device)
     _check(lib, lib.coheryn_matrix_memory_scan(
         _ptr(q), _ptr(k), _ptr(v), c_long(q.stride(0)), _ptr(gate_i), _ptr(gate_f), c_long(gate_i.stride(0)), _ptr(bias_i),
         _ptr(bias_f), c_int(_code(bias_i)), c_float(cap), _ptr(state), c_long(state.stride(0)), _ptr(step.cu_q),
         _ptr(step.state_slots), c_int(step.num_requests), c_int(heads), c_int(dk), c_int(dv), _ptr(out), c_int(_code(out)),
         c_long(out.stride(0)), _ptr(norm_weight), c_int(_code(norm_weight)), c_int(dv), _ptr(gate), c_long(gate.stride(0)),
         c_float(eps), c_float(out_scale), c_int(q.shape[0]), _ptr(scratch), c_long(scratch.numel() if scratch is not None else 0),
-        c_int(chunks if floats else 0), c_int(runs), c_int(1 if rest else 0), _stream()))
+        c_int(chunks), c_int(runs), c_int(1 if rest else 0), _stream()))
 
 
 def qk_norm_kv_write(q, k, v, q_weight, k_weight, eps: float, slots, k_cache, v_cache, num_heads: int, num_kv_heads: int,

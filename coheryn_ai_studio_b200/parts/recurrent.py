@@ -68,12 +68,12 @@ class _StackedInput:
 class _StateMixer(Mixer):
     output_parts = 1
 
-    @property
-    def in_chunks(self) -> bool:
-        """Whether long runs may go chunk by chunk.  Not in float32: its products give a row the same bits whatever the step's
-        other rows are, and with the scans token by token a sequence has the same bits however load or preemption cut it.  (In
-        bfloat16 the product that runs follows the step's rows anyway.)"""
-        return self.runtime.dtype != torch.float32
+    def __init__(self, runtime: Runtime):
+        super().__init__(runtime)
+        # Whether long runs may go chunk by chunk.  Not in float32: its products give a row the same bits whatever the step's other
+        # rows are, and with the scans token by token a sequence has the same bits however load or preemption cut it.  (In bfloat16
+        # the product that runs follows the step's rows anyway.)
+        self.in_chunks = runtime.dtype != torch.float32
 
     def forward(self, x: torch.Tensor, step: StepContext, cache: Optional[LayerCache]) -> torch.Tensor:
         out = torch.empty((1, x.shape[0], self.hidden_size), dtype=torch.float32, device=x.device)
