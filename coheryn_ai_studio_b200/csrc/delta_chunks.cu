@@ -120,7 +120,7 @@ constexpr int CW = 64, CP = CW + 4;      // channels of a pass, pitch of its til
 constexpr size_t CHUNK_SMEM = sizeof(float) * (3 * CH * CP + 4 * CW + 4 * CH + 2 * CH * 17);
 
 template <int DK>
-__global__ void __launch_bounds__(THREADS, 3) delta_chunk_kernel(DeltaIn P, int B, float* __restrict__ scratch, int dvp) {
+__global__ void __launch_bounds__(THREADS, 3) delta_chunk_kernel(DeltaIn P, int B, int base, float* __restrict__ scratch, int dvp) {
   constexpr int PASSES = DK / CW;
   extern __shared__ __align__(16) float sm[];
   float* Qs = sm;                       // [64][CP] q, then q E
@@ -138,7 +138,7 @@ __global__ void __launch_bounds__(THREADS, 3) delta_chunk_kernel(DeltaIn P, int 
   co_pdl_wait();
   const int h = blockIdx.y, dk = P.dk;
   Run R;
-  if (!find_run(P.cu_q, B, blockIdx.x, false, R)) return;
+  if (!find_run(P.cu_q, B, base + blockIdx.x, false, R)) return;
   const int row0 = R.start + R.chunk * CH, nt = min(CH, R.len - R.chunk * CH);
   const int g = h / (P.heads / P.kv_heads);
   const float rate = expf(co_load_any(P.rate_log, P.rate_log_dtype, h));
@@ -324,7 +324,7 @@ template <int DK>
 constexpr size_t solve_smem() { return sizeof(float) * (2 * CH * NP + CH * (DK + 4) + CH + 3 * BL * BL); }
 
 template <int DK>
-__global__ void __launch_bounds__(THREADS, 3) delta_solve_kernel(DeltaIn P, int B, float* __restrict__ scratch, int dvp) {
+__global__ void __launch_bounds__(THREADS, 3) delta_solve_kernel(DeltaIn P, int B, int base, float* __restrict__ scratch, int dvp) {
   constexpr int DKP = DK + 4, TC = DK / 32;
   extern __shared__ __align__(16) float sm[];
   float* Nm = sm;                       // [t][s] beta_t A_ts, s < t
@@ -337,7 +337,7 @@ __global__ void __launch_bounds__(THREADS, 3) delta_solve_kernel(DeltaIn P, int 
   co_pdl_wait();
   const int h = blockIdx.y, dv = P.dv;
   Run R;
-  if (!find_run(P.cu_q, B, blockIdx.x, false, R)) return;
+  if (!find_run(P.cu_q, B, base + blockIdx.x, false, R)) return;
   const int row0 = R.start + R.chunk * CH, nt = min(CH, R.len - R.chunk * CH);
   const Piece<DK> out(scratch, (size_t)blockIdx.x * P.heads + h, dvp);
 #pragma unroll
@@ -440,7 +440,7 @@ constexpr int STATE_THREADS = 512;
 __device__ __forceinline__ int slot_of(int row) { return row ^ ((row >> 2) & 1); }
 
 template <int DK>
-__global__ void __launch_bounds__(STATE_THREADS, 1) delta_state_kernel(DeltaIn P, int B, float* __restrict__ scratch, int dvp) {
+__global__ void __launch_bounds__(STATE_THREADS, 1) delta_state_kernel(DeltaIn P, int B, int base, int count, float* __restrict__ scratch, int dvp) {
   constexpr int STAGE = 2 * CH * DK + CH * VS + DK;
   constexpr int DG = DK / 32, KG = 16 / DG;     // the update: warps over groups of 32 key channels, and over tokens
   extern __shared__ __align__(16) float sm[];
@@ -453,10 +453,12 @@ __global__ void __launch_bounds__(STATE_THREADS, 1) delta_state_kernel(DeltaIn P
   const int h = blockIdx.y, c0 = blockIdx.x * VS, dk = P.dk, dv = P.dv;
   Run R;
   if (!find_run(P.cu_q, B, blockIdx.z, true, R)) return;
-  const int chunks = (R.len + CH - 1) / CH;
+  // the run's chunks among the `count` that are worked on, from `base` on
+  const int from = max(0, base - R.first), to = min((R.len + CH - 1) / CH, base + count - R.first);
+  if (from >= to) return;
   float* state = P.state + (size_t)P.state_slots[R.r] * P.state_stride + (size_t)h * dk * dv;
   auto stage = [&](int c) {
-    const Piece<DK> in(scratch, (size_t)(R.first + c) * P.heads + h, dvp);
+    const Piece<DK> in(scratch, (size_t)(R.first + c - base) * P.heads + h, dvp);
     float* to = sm + (c & 1) * STAGE;
 #pragma unroll 4
     for (int e = tid; e < 2 * CH * DK / 4; e += STATE_THREADS) cp16(to + 4 * e, in.wt + 4 * e);      // W^T and K^ are neighbours
@@ -464,21 +466,21 @@ __global__ void __launch_bounds__(STATE_THREADS, 1) delta_state_kernel(DeltaIn P
     if (tid < DK / 4) cp16(to + 2 * CH * DK + CH * VS + 4 * tid, in.dec + 4 * tid);
     cp_commit();
   };
-  stage(0);
+  stage(from);
   for (int e = tid; e < DK * VS; e += STATE_THREADS) {
     const int d = e / VS, c = c0 + e % VS;
     S[e] = d < dk && c < dv ? state[(size_t)d * dv + c] : 0.f;
   }
   const int la = lane >> 2, lb = 4 * (lane & 3);
-  for (int c = 0; c < chunks; ++c) {
-    if (c + 1 < chunks) { stage(c + 1); cp_wait<1>(); }
+  for (int c = from; c < to; ++c) {
+    if (c + 1 < to) { stage(c + 1); cp_wait<1>(); }
     else cp_wait<0>();
     __syncthreads();
     const float* wt = sm + (c & 1) * STAGE;
     const float* kh = wt + CH * DK;
     const float* uv = kh + CH * DK;
     const float* dec = uv + CH * VS;
-    const Piece<DK> out(scratch, (size_t)(R.first + c) * P.heads + h, dvp);
+    const Piece<DK> out(scratch, (size_t)(R.first + c - base) * P.heads + h, dvp);
     for (int e = tid; e < DK * VS / 4; e += STATE_THREADS) st4(out.s + (size_t)(e >> 2) * dvp + c0 + 4 * (e & 3), ld4(S + 4 * e));
     {
       const int t = 32 * (warp & 1) + 4 * la, slice = warp >> 1;
@@ -554,7 +556,7 @@ size_t out_smem(int dvp) {
 }
 
 template <int DK, int TC>
-__global__ void __launch_bounds__(THREADS) delta_out_kernel(DeltaIn P, HeadOut E, int B, float* __restrict__ scratch, int dvp) {
+__global__ void __launch_bounds__(THREADS) delta_out_kernel(DeltaIn P, HeadOut E, int B, int base, float* __restrict__ scratch, int dvp) {
   constexpr int W = 32 * TC, SL = 32, STAGE = SL * (CH + W), SLICES = (DK + CH) / SL;
   extern __shared__ __align__(16) float sm[];
   float* os = dvp <= W ? sm : sm + 2 * STAGE;   // [64][dvp + 4]
@@ -563,7 +565,7 @@ __global__ void __launch_bounds__(THREADS) delta_out_kernel(DeltaIn P, HeadOut E
   co_pdl_wait();
   const int h = blockIdx.y;
   Run R;
-  if (!find_run(P.cu_q, B, blockIdx.x, false, R)) return;
+  if (!find_run(P.cu_q, B, base + blockIdx.x, false, R)) return;
   const int row0 = R.start + R.chunk * CH, nt = min(CH, R.len - R.chunk * CH);
   const Piece<DK> in(scratch, (size_t)blockIdx.x * P.heads + h, dvp);
   const int la = lane >> 2, col = warp * 4 * TC + (lane & 3) * TC;
@@ -612,21 +614,24 @@ int padded(int dv) { return (dv + VS - 1) / VS * VS; }
 
 template <int DK>
 int launch(const DeltaIn& P, const HeadOut& E, int B, int chunks, int runs, float* scratch, cudaStream_t stream) {
-  const int dvp = padded(P.dv);
-  cudaFuncSetAttribute(delta_chunk_kernel<DK>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)CHUNK_SMEM);
-  co_launch(delta_chunk_kernel<DK>, dim3(chunks, P.heads), dim3(THREADS), CHUNK_SMEM, stream, P, B, scratch, dvp);
-  CO_CHECK_LAUNCH("delta_chunk");
-  cudaFuncSetAttribute(delta_solve_kernel<DK>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)solve_smem<DK>());
-  co_launch(delta_solve_kernel<DK>, dim3(chunks, P.heads), dim3(THREADS), solve_smem<DK>(), stream, P, B, scratch, dvp);
-  CO_CHECK_LAUNCH("delta_solve");
-  cudaFuncSetAttribute(delta_state_kernel<DK>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)state_smem<DK>());
-  co_launch(delta_state_kernel<DK>, dim3(dvp / VS, P.heads, runs), dim3(STATE_THREADS), state_smem<DK>(), stream, P, B, scratch, dvp);
-  CO_CHECK_LAUNCH("delta_state");
+  const int dvp = padded(P.dv), at_once = chunks_at_once(P.heads * Piece<DK>::floats(dvp));
   auto out = dvp <= 64 ? delta_out_kernel<DK, 2> : delta_out_kernel<DK, 4>;
   const size_t smem = dvp <= 64 ? out_smem<2>(dvp) : out_smem<4>(dvp);
+  cudaFuncSetAttribute(delta_chunk_kernel<DK>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)CHUNK_SMEM);
+  cudaFuncSetAttribute(delta_solve_kernel<DK>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)solve_smem<DK>());
+  cudaFuncSetAttribute(delta_state_kernel<DK>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)state_smem<DK>());
   cudaFuncSetAttribute(out, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  co_launch(out, dim3(chunks, P.heads), dim3(THREADS), smem, stream, P, E, B, scratch, dvp);
-  CO_CHECK_LAUNCH("delta_out");
+  for (int base = 0; base < chunks; base += at_once) {
+    const int count = chunks - base < at_once ? chunks - base : at_once;
+    co_launch(delta_chunk_kernel<DK>, dim3(count, P.heads), dim3(THREADS), CHUNK_SMEM, stream, P, B, base, scratch, dvp);
+    CO_CHECK_LAUNCH("delta_chunk");
+    co_launch(delta_solve_kernel<DK>, dim3(count, P.heads), dim3(THREADS), solve_smem<DK>(), stream, P, B, base, scratch, dvp);
+    CO_CHECK_LAUNCH("delta_solve");
+    co_launch(delta_state_kernel<DK>, dim3(dvp / VS, P.heads, runs), dim3(STATE_THREADS), state_smem<DK>(), stream, P, B, base, count, scratch, dvp);
+    CO_CHECK_LAUNCH("delta_state");
+    co_launch(out, dim3(count, P.heads), dim3(THREADS), smem, stream, P, E, B, base, scratch, dvp);
+    CO_CHECK_LAUNCH("delta_out");
+  }
   return 0;
 }
 
@@ -636,8 +641,9 @@ int launch(const DeltaIn& P, const HeadOut& E, int B, int chunks, int runs, floa
 bool co_delta_chunks_take(int dk, int dv) { return dk >= 1 && dk <= 128 && dv >= 1 && dv <= 256; }
 
 long co_delta_chunk_floats(int chunks, int heads, int dk, int dv) {
-  const size_t each = dk <= 64 ? Piece<64>::floats(padded(dv)) : Piece<128>::floats(padded(dv));
-  return (long)((size_t)chunks * heads * each);
+  const size_t each = heads * (dk <= 64 ? Piece<64>::floats(padded(dv)) : Piece<128>::floats(padded(dv)));
+  const int at_once = chunks_at_once(each);
+  return (long)((size_t)(chunks < at_once ? chunks : at_once) * each);
 }
 
 int co_delta_chunks(const DeltaIn& P, const HeadOut& E, int B, int chunks, int runs, float* scratch, cudaStream_t stream) {

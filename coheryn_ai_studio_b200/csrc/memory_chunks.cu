@@ -74,15 +74,17 @@ struct Area {
 // another is the running maximum alone, a chain of one step per chunk that one thread walks between the two passes (a warp per
 // head that walked the chunks from beginning to end took 30 us for 32 of them).
 constexpr int GATE_WARPS = 16;
-__global__ void __launch_bounds__(32 * GATE_WARPS) memory_gates_kernel(MemoryIn P, int B, Area A) {
+__global__ void __launch_bounds__(32 * GATE_WARPS) memory_gates_kernel(MemoryIn P, int B, int base, int count, Area A) {
   co_pdl_launch_dependents();
   co_pdl_wait();
   const int h = blockIdx.y, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   Run R;
   if (!find_run(P.cu_q, B, blockIdx.x, true, R)) return;
+  // the run's chunks among the `count` that are worked on, from `base` on
+  const int from = max(0, base - R.first), to = min((R.len + CH - 1) / CH, base + count - R.first), first = R.first - base;
+  if (from >= to) return;
   float* m_state = P.state + (size_t)P.state_slots[R.r] * P.state_stride + (size_t)P.heads * P.dk * P.dv + (size_t)P.heads * P.dk + h;
   const float bi = co_load_any(P.bias_i, P.bias_dtype, h), bf = co_load_any(P.bias_f, P.bias_dtype, h);
-  const int chunks = (R.len + CH - 1) / CH;
   // the largest i_s - F_s up to and with this lane's tokens
   auto best_of = [&](const double (&F)[2], const float (&li)[2], int nt, double (&best)[2]) {
     const double p0 = 2 * lane < nt ? (double)li[0] - F[0] : -1e300, p1 = fmax(p0, 2 * lane + 1 < nt ? (double)li[1] - F[1] : -1e300);
@@ -96,7 +98,7 @@ __global__ void __launch_bounds__(32 * GATE_WARPS) memory_gates_kernel(MemoryIn 
     best[0] = fmax(lane ? before : -1e300, p0);
     best[1] = x;
   };
-  for (int c = warp; c < chunks; c += GATE_WARPS) {
+  for (int c = from + warp; c < to; c += GATE_WARPS) {
     const int nt = min(CH, R.len - c * CH);
     float li[2];
     double F[2];
@@ -118,7 +120,7 @@ __global__ void __launch_bounds__(32 * GATE_WARPS) memory_gates_kernel(MemoryIn 
     F[1] = x;
     double best[2];
     best_of(F, li, nt, best);
-    const size_t at = (size_t)(R.first + c) * P.heads + h;
+    const size_t at = (size_t)(first + c) * P.heads + h;
 #pragma unroll
     for (int u = 0; u < 2; ++u) { A.f[at * CH + 2 * lane + u] = F[u]; A.i[at * CH + 2 * lane + u] = li[u]; }
     if (lane == 31) {
@@ -129,19 +131,19 @@ __global__ void __launch_bounds__(32 * GATE_WARPS) memory_gates_kernel(MemoryIn 
   __syncthreads();
   if (threadIdx.x == 0) {
     float m0 = *m_state;
-    for (int c0 = 0; c0 < chunks; c0 += 8) {
+    for (int c0 = from; c0 < to; c0 += 8) {
       double best[8], end[8];
 #pragma unroll
       for (int i = 0; i < 8; ++i)
-        if (c0 + i < chunks) {
-          const float* p = A.m0 + ((size_t)(R.first + c0 + i) * P.heads + h) * 4;
+        if (c0 + i < to) {
+          const float* p = A.m0 + ((size_t)(first + c0 + i) * P.heads + h) * 4;
           best[i] = *reinterpret_cast<const double*>(p);
           end[i] = *reinterpret_cast<const double*>(p + 2);
         }
 #pragma unroll
       for (int i = 0; i < 8; ++i)
-        if (c0 + i < chunks) {
-          float* p = A.m0 + ((size_t)(R.first + c0 + i) * P.heads + h) * 4;
+        if (c0 + i < to) {
+          float* p = A.m0 + ((size_t)(first + c0 + i) * P.heads + h) * 4;
           const float m1 = (float)(end[i] + fmax((double)m0, best[i]));
           p[0] = m0; p[1] = m1;
           m0 = m1;
@@ -150,8 +152,8 @@ __global__ void __launch_bounds__(32 * GATE_WARPS) memory_gates_kernel(MemoryIn 
     *m_state = m0;
   }
   __syncthreads();
-  for (int c = warp; c < chunks; c += GATE_WARPS) {
-    const size_t at = (size_t)(R.first + c) * P.heads + h;
+  for (int c = from + warp; c < to; c += GATE_WARPS) {
+    const size_t at = (size_t)(first + c) * P.heads + h;
     const double F[2] = {A.f[at * CH + 2 * lane], A.f[at * CH + 2 * lane + 1]};
     const float li[2] = {A.i[at * CH + 2 * lane], A.i[at * CH + 2 * lane + 1]};
     const double m0 = (double)A.m0[at * 4];
@@ -187,7 +189,7 @@ __device__ __forceinline__ void zero(float (&acc)[8][TC]) {
 __device__ __forceinline__ int row_of(int i, int la) { return (i < 4 ? 0 : 32) + 4 * la + (i & 3); }
 
 // grid (chunks, heads, ceil(dk / 64) * ceil(dvp / 128)), 256 threads.
-__global__ void __launch_bounds__(256) memory_sum_kernel(MemoryIn P, int B, Area A) {
+__global__ void __launch_bounds__(256) memory_sum_kernel(MemoryIn P, int B, int base, Area A) {
   extern __shared__ __align__(16) float sm[];
   float* Ks = sm;                    // [64 tokens][64 channels], weighted
   float* Vs = Ks + CH * 64;          // [64 tokens][128]
@@ -196,7 +198,7 @@ __global__ void __launch_bounds__(256) memory_sum_kernel(MemoryIn P, int B, Area
   co_pdl_wait();
   const int h = blockIdx.y, dk = P.dk, dv = P.dv, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   Run R;
-  if (!find_run(P.cu_q, B, blockIdx.x, false, R)) return;
+  if (!find_run(P.cu_q, B, base + blockIdx.x, false, R)) return;
   const int nv = (A.dvp + 127) / 128, d0 = (blockIdx.z / nv) * 64, c0 = (blockIdx.z % nv) * 128;
   const int row0 = R.start + R.chunk * CH, nt = min(CH, R.len - R.chunk * CH);
   const size_t at = (size_t)blockIdx.x * P.heads + h;
@@ -236,7 +238,7 @@ __global__ void __launch_bounds__(256) memory_sum_kernel(MemoryIn P, int B, Area
 
 // grid (ceil(size / 1024), heads, runs), 256 threads of four neighbouring elements each; the chunks ahead are requested eight at
 // a time.
-__global__ void __launch_bounds__(256) memory_carry_kernel(MemoryIn P, int B, Area A) {
+__global__ void __launch_bounds__(256) memory_carry_kernel(MemoryIn P, int B, int base, int count, Area A) {
   co_pdl_launch_dependents();
   co_pdl_wait();
   const int h = blockIdx.y, dk = P.dk, dv = P.dv;
@@ -244,7 +246,9 @@ __global__ void __launch_bounds__(256) memory_carry_kernel(MemoryIn P, int B, Ar
   if (!find_run(P.cu_q, B, blockIdx.z, true, R)) return;
   const size_t e = ((size_t)blockIdx.x * 256 + threadIdx.x) * 4;
   if (e >= A.size) return;
-  const int chunks = (R.len + CH - 1) / CH, d = (int)(e / A.dvp), c = (int)(e % A.dvp);
+  const int from = max(0, base - R.first), chunks = min((R.len + CH - 1) / CH, base + count - R.first) - from;      // of the run, among those worked on
+  if (chunks <= 0) return;
+  const int d = (int)(e / A.dvp), c = (int)(e % A.dvp);
   float* slot = P.state + (size_t)P.state_slots[R.r] * P.state_stride;
   float* st = d < dk ? slot + ((size_t)h * dk + d) * dv + c : slot + (size_t)P.heads * dk * dv + (size_t)h * dk + (e - (size_t)dk * A.dvp);
   const int left = d < dk ? dv - c : dk - (int)(e - (size_t)dk * A.dvp);      // entries of the state from here on
@@ -252,8 +256,8 @@ __global__ void __launch_bounds__(256) memory_carry_kernel(MemoryIn P, int B, Ar
 #pragma unroll
   for (int j = 0; j < 4; ++j) s[j] = j < left ? st[j] : 0.f;
   const size_t step = (size_t)P.heads * A.size;
-  float* p = A.s + ((size_t)R.first * P.heads + h) * A.size + e;
-  const float* g = A.m0 + ((size_t)R.first * P.heads + h) * 4;
+  float* p = A.s + ((size_t)(R.first - base + from) * P.heads + h) * A.size + e;
+  const float* g = A.m0 + ((size_t)(R.first - base + from) * P.heads + h) * 4;
   constexpr int AHEAD = 8;
   for (int i0 = 0; i0 < chunks; i0 += AHEAD) {
     float4 x[AHEAD];
@@ -290,7 +294,7 @@ size_t out_smem(int W, int dk, int dvp) {
 }
 
 template <int W>
-__global__ void __launch_bounds__(2 * W, 512 / W) memory_out_kernel(MemoryIn P, HeadOut E, int B, Area A, int first_floats) {
+__global__ void __launch_bounds__(2 * W, 512 / W) memory_out_kernel(MemoryIn P, HeadOut E, int B, int base, Area A, int first_floats) {
   constexpr int THREADS = 2 * W;
   extern __shared__ __align__(16) float sm[];
   const int dk = P.dk, dv = P.dv, dvp = A.dvp, dkp = (dk + SLICE - 1) / SLICE * SLICE;
@@ -305,7 +309,7 @@ __global__ void __launch_bounds__(2 * W, 512 / W) memory_out_kernel(MemoryIn P, 
   co_pdl_wait();
   const int h = blockIdx.y;
   Run R;
-  if (!find_run(P.cu_q, B, blockIdx.x, false, R)) return;
+  if (!find_run(P.cu_q, B, base + blockIdx.x, false, R)) return;
   const int row0 = R.start + R.chunk * CH, nt = min(CH, R.len - R.chunk * CH);
   const size_t at = (size_t)blockIdx.x * P.heads + h;
   const float q_scale = 1.0f / sqrtf((float)dk);
@@ -425,26 +429,34 @@ int padded(int dv) { return (dv + 15) / 16 * 16; }
 
 bool co_memory_chunks_take(int dk, int dv) { return dk >= 1 && dk <= 256 && dv >= 1 && dv <= 256; }
 
-long co_memory_chunk_floats(int chunks, int heads, int dk, int dv) { return (long)Area::floats(chunks, heads, dk, padded(dv)); }
+static int memory_chunks_at_once(int heads, int dk, int dv) { return chunks_at_once(Area::floats(1, heads, dk, padded(dv))); }
+
+long co_memory_chunk_floats(int chunks, int heads, int dk, int dv) {
+  const int at_once = memory_chunks_at_once(heads, dk, dv);
+  return (long)Area::floats(chunks < at_once ? chunks : at_once, heads, dk, padded(dv));
+}
 
 int co_memory_chunks(const MemoryIn& P, const HeadOut& E, int B, int chunks, int runs, float* scratch, cudaStream_t stream) {
-  const int dvp = padded(P.dv);
-  const Area A(scratch, chunks, P.heads, P.dk, dvp);
-  co_launch(memory_gates_kernel, dim3(runs, P.heads), dim3(32 * GATE_WARPS), 0, stream, P, B, A);
-  CO_CHECK_LAUNCH("memory_gates");
+  const int dvp = padded(P.dv), at_once = memory_chunks_at_once(P.heads, P.dk, P.dv);
   const size_t sum_smem = sizeof(float) * (CH * 64 + CH * 128 + CH);
   cudaFuncSetAttribute(memory_sum_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sum_smem);
-  co_launch(memory_sum_kernel, dim3(chunks, P.heads, ((P.dk + 63) / 64) * ((dvp + 127) / 128)), dim3(256), sum_smem, stream, P, B, A);
-  CO_CHECK_LAUNCH("memory_sum");
-  co_launch(memory_carry_kernel, dim3((unsigned)((A.size + 1023) / 1024), P.heads, runs), dim3(256), 0, stream, P, B, A);
-  CO_CHECK_LAUNCH("memory_carry");
   const int W = dvp <= 128 ? 128 : 256;
   const size_t smem = out_smem(W, P.dk, dvp);
   const int dkp = (P.dk + SLICE - 1) / SLICE * SLICE;
   const int first = (int)(smem / sizeof(float)) - (dkp * TP + CH * TP + 8 * CH);
   auto out = W == 128 ? memory_out_kernel<128> : memory_out_kernel<256>;
   cudaFuncSetAttribute(out, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  co_launch(out, dim3(chunks, P.heads), dim3(2 * W), smem, stream, P, E, B, A, first);
-  CO_CHECK_LAUNCH("memory_out");
+  for (int base = 0; base < chunks; base += at_once) {
+    const int count = chunks - base < at_once ? chunks - base : at_once;
+    const Area A(scratch, count, P.heads, P.dk, dvp);
+    co_launch(memory_gates_kernel, dim3(runs, P.heads), dim3(32 * GATE_WARPS), 0, stream, P, B, base, count, A);
+    CO_CHECK_LAUNCH("memory_gates");
+    co_launch(memory_sum_kernel, dim3(count, P.heads, ((P.dk + 63) / 64) * ((dvp + 127) / 128)), dim3(256), sum_smem, stream, P, B, base, A);
+    CO_CHECK_LAUNCH("memory_sum");
+    co_launch(memory_carry_kernel, dim3((unsigned)((A.size + 1023) / 1024), P.heads, runs), dim3(256), 0, stream, P, B, base, count, A);
+    CO_CHECK_LAUNCH("memory_carry");
+    co_launch(out, dim3(count, P.heads), dim3(2 * W), smem, stream, P, E, B, base, A, first);
+    CO_CHECK_LAUNCH("memory_out");
+  }
   return 0;
 }

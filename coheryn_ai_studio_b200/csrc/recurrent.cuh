@@ -52,6 +52,9 @@ struct MemoryIn {
 constexpr int CHUNK_TOKENS = 64, CHUNK_FROM = 48;
 // `chunks` and `runs`: how many chunks and how many such runs the step holds at most (CTAs beyond the last return at once);
 // `scratch`: at least co_*_chunk_floats floats.
+// The scratch of a step of many chunks is bounded: the kernels work on as many chunks at a time as 256 MB hold (`each` floats per
+// chunk), one after the other; a run's state goes from one to the next through its slot, as it does from step to step.
+constexpr int chunks_at_once(size_t each) { return each >= (1u << 26) ? 1 : (int)((1u << 26) / each); }
 bool co_delta_chunks_take(int dk, int dv);
 long co_delta_chunk_floats(int chunks, int heads, int dk, int dv);
 int co_delta_chunks(const DeltaIn& P, const HeadOut& E, int B, int chunks, int runs, float* scratch, cudaStream_t stream);

@@ -1396,7 +1396,8 @@ def attention_maps(q: torch.Tensor, out: torch.Tensor, k_cache: torch.Tensor, v_
     assert k_cache.dtype == q.dtype and out.dtype == q.dtype and v_cache.dtype == q.dtype
     q_lens = getattr(step, "q_lens", None)
     # what the tensor-core kernels keep in shared memory: 64 query rows, two tiles of 32 key rows (and of value rows when
-    # those are rows of their own), up to 4,096 block-table entries; values wider than 256 channels go in chunks
+    # those are rows of their own; a third one and 16 KB more where two warps share a row tile's rows, whose heads are so narrow
+    # that this fits in any case), up to 4,096 block-table entries; values wider than 256 channels go in chunks
     tc_smem = 2 * (128 * (maps * dk + 8) + (0 if values_in_keys else 64 * (dv + 8))) + 16384
     fast = (MAPS_TC and not force_simple and q.dtype == torch.bfloat16 and dk % 16 == 0 and dv % 16 == 0 and 16 <= dk <= 1024
             and 16 <= dv <= 1024 and tc_smem <= 227 * 1024 and not (head_norm and dv > 256)

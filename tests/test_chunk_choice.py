@@ -39,3 +39,14 @@ def test_what_is_cut_into_chunks():
     assert chunks >= 26 and runs >= 3 and rest
     assert choice("delta", 12, 192, 128, [2048]) == (0, 0, True)                              # more key channels than the chunks take
     assert choice("memory", 8, 128, 256, [1] * 64) == (0, 0, True) and choice("delta", 2, 16, 16, []) == (0, 0, True)
+
+
+def test_the_chunks_scratch_is_bounded():
+    """256 MB whatever the step, and what the chunks need below that."""
+    import ctypes
+    lib = ops.recurrent()
+    for f, heads, dk, dv in ((lib.coheryn_delta_chunk_floats, 16, 128, 128), (lib.coheryn_delta_chunk_floats, 2, 20, 30),
+                             (lib.coheryn_memory_chunk_floats, 8, 128, 256), (lib.coheryn_memory_chunk_floats, 64, 256, 256)):
+        floats = [int(f(*(ctypes.c_int(x) for x in (chunks, heads, dk, dv)))) for chunks in (1, 2, 10000)]
+        assert floats[1] == 2 * floats[0] or floats[1] == floats[0] > 1 << 25
+        assert floats[2] <= 1 << 26 and floats[2] >= (1 << 26) - floats[0] or floats[2] == 10000 * floats[0]

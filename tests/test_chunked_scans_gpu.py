@@ -265,3 +265,33 @@ def test_short_convolution_of_a_million_tokens():
         want = s * torch.sigmoid(s)
         assert float((y[at:at + 100].double() - want).abs().max()) <= 1e-5 * max(1.0, float(want.abs().max()))
     assert torch.equal(state.reshape(taps - 1, channels), x[n - taps + 1:])
+
+
+@pytest.mark.parametrize("kind,heads,dk,dv,lens", [("delta", 16, 128, 128, [4000, 70, 3000]), ("memory", 8, 128, 256, [9000, 70, 9000])])
+def test_more_chunks_than_the_scratch_holds(kind, heads, dk, dv, lens):
+    """A step whose chunks' scratch would pass its bound goes in several groups of chunks, the last run's state from one to the next:
+    the same bits as each long run alone, which fits at once."""
+    from coheryn_ai_studio_b200 import ops
+    g, n = torch.Generator(DEV).manual_seed(3), sum(lens)
+    f = lambda *s: torch.randn(s, generator=g, device=DEV)
+    size = heads * (dk * dv + (dk + 1 if kind == "memory" else 0))
+    qkv, step_pre, pair, gate, weight = f(n, heads * (2 * dk + dv)), f(n, heads * dk), f(n, 2 * heads), f(n, heads * dv), f(heads * dv)
+    bias, small, c = f(heads * dk), f(2 * heads), heads * dk
+
+    def run(a, b, lens):
+        rows, out = slice(a, b), torch.empty((b - a, heads * dv), device=DEV)
+        state, step = torch.zeros((len(lens), size), device=DEV), step_of(lens, list(range(len(lens))))
+        q, k, v = qkv[rows, :c], qkv[rows, c:2 * c], qkv[rows, 2 * c:]
+        if kind == "delta":
+            ops.gated_delta_scan(q, k, v, pair[rows, :heads], step_pre[rows], bias, small[:heads].contiguous(), state, step, heads, heads, dk, dv, out,
+                                 weight[:dv].contiguous(), gate[rows], 1e-5)
+        else:
+            ops.matrix_memory_scan(q, k, v, pair[rows, :heads], pair[rows, heads:], small[:heads].contiguous(), small[heads:].contiguous(), 15.0, state,
+                                   step, heads, dk, dv, out, weight, gate[rows], 1e-5)
+        return out, state
+
+    both, state = run(0, n, lens)
+    for i in (0, 2):
+        a = sum(lens[:i])
+        alone, end = run(a, a + lens[i], [lens[i]])
+        assert torch.equal(alone, both[a:a + lens[i]]) and torch.equal(end[0], state[i]) and bool(alone.isfinite().all())
