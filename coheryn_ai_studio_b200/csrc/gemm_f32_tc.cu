@@ -1,0 +1,414 @@
+// out[M, N] = x[M, K] . W[N, K]^T (+ bias) of float32 operands to float32's accuracy on the 5th-generation tensor cores.
+//
+// Every float32 value is the exact sum of three bfloat16 ones, v = v0 + v1 + v2 (each the rest's nearest: 8 + 8 + 8 bits), and a
+// product of two bfloat16 values is exact in the accumulator.  Of the nine products of terms the six with i + j <= 2 are formed; the
+// three left out are below 2^-25 of |x w|, half of what rounding one product would cost.  The accumulator in tensor memory only
+// ever holds 64 values of k, the small products first and x0 w0 last, and is then added to sums in registers with ordinary
+// float32 additions: its own rounding (which truncates) touches the large products four times per 64 values, and a sum of K
+// values has K / 64 roundings in place of the FMA chain's K.  Measured against float64: below.
+//
+// The operands swap places as in gemm_tc_few.cu: 128 output features sit on the lanes, BT tokens on the columns.  The tokens'
+// three terms are written once by a small kernel and come by TMA; W is read once from memory in float32 and split on its way:
+//
+//   warp 0       producer: W boxes of 128 x 32 floats (a ring of three stages of 64 k, fetched before the wait for the predecessor),
+//                x terms (two stages; from 96 tokens on a term is fetched again as soon as its last product is formed)
+//   warp 1       issues 24 tcgen05.mma per stage: A = W's terms in TENSOR MEMORY, B = x's terms in shared memory
+//   warps 2-5    split: a thread reads its feature's 64 values, writes 3 x 32 columns of bfloat16 pairs to tensor memory
+//   warps 6-13   add a stage's accumulator (two of them in tensor memory) to their sums, and the epilogue
+//
+// What bounds it: the tensor cores' operand W from tensor memory and the gaps between stages.  A product with A in tensor memory takes
+// 70 cycles at 16 tokens and 93 at 160 (80 would be the matrix pipe's rate), 24 of them a stage, and about 400 cycles pass until the
+// next stage's first; shared memory moves 248 KB a stage (W's terms there as well: 480 KB) and the split takes 2,000 cycles of one
+// warp beside it.  Measured on a B200 (alone, L2 flushed, with the two small kernels; before: the CUDA cores, gemm_simt.cu):
+// 313 x 17920 x 1536 417 -> 116 us, 313 x 1536 x 8960 216 -> 79, 313 x 1536 x 1536 77 -> 28, 2048 x 17920 x 1536 2,518 -> 701, one row by
+// 17920 x 1536 84 -> 47.  Error against float64 (2-norm, relative): 0.8e-7 to 1.2e-7 where the FMA chain has 2.8e-7 to 5.0e-7.
+//
+// A row's result does not depend on the other rows: K is cut into slices by the weight's shape alone, a slice's sum goes to a
+// workspace (where there is more than one) and the slices are added in order.  A result that is not finite is formed again from the
+// operands themselves (an infinity has no finite rest, so the terms' products would make it a NaN).
+// Every wait is bounded: on expiry the kernel records an error code and winds down.
+#include "tc_common.cuh"
+
+namespace {
+
+constexpr int F_ROWS = 128;                      // features per tile
+constexpr int W_STAGES = 3, X_STAGES = 2;
+constexpr int W_BYTES = F_ROWS * BK * 4;         // two boxes of 128 rows x 128 bytes
+constexpr int TERM_COLS = BK / 2;                // a term's columns in tensor memory: two k each
+
+template <int BT>
+struct F32Tile {
+  static constexpr int X_TERM = BT * BK * 2, X_BYTES = 3 * X_TERM;
+  static constexpr int SMEM = W_STAGES * W_BYTES + X_STAGES * X_BYTES + 1024 /* alignment */ + 256 /* barriers */;
+  static constexpr int A_AT = 2 * BT, COLS_USED = A_AT + 2 * 3 * TERM_COLS;
+  static constexpr int COLS = COLS_USED <= 256 ? 256 : 512;
+  static constexpr bool BY_TERM = BT > 64;      // whether x's terms come and go one by one
+  static constexpr int HALVES = BT >= 32 ? 2 : 1, PART = BT / HALVES;       // columns of an adding warp
+  static_assert(COLS_USED <= 512 && PART % 16 == 0, "tensor memory");
+};
+
+// v0 + v1 + v2 = v for a pair of neighbouring values, as packed bfloat16 pairs (the first value in the low half): v0 and v1 the
+// nearest (halves away from zero) of the value and of the rest, v2 what is left, which has at most eight bits.  Integer operations: the
+// conversion instructions go through the narrow pipe of the special functions, which three per pair would keep busy for a third of the time.
+__device__ __forceinline__ void split3(float a, float b, unsigned& t0, unsigned& t1, unsigned& t2) {
+  const unsigned a0 = (__float_as_uint(a) + 0x8000u) & 0xffff0000u, b0 = (__float_as_uint(b) + 0x8000u) & 0xffff0000u;
+  a -= __uint_as_float(a0);
+  b -= __uint_as_float(b0);
+  const unsigned a1 = (__float_as_uint(a) + 0x8000u) & 0xffff0000u, b1 = (__float_as_uint(b) + 0x8000u) & 0xffff0000u;
+  t0 = __byte_perm(a0, b0, 0x7632);
+  t1 = __byte_perm(a1, b1, 0x7632);
+  t2 = __byte_perm(__float_as_uint(a - __uint_as_float(a1)), __float_as_uint(b - __uint_as_float(b1)), 0x7632);
+}
+
+// The three terms of x as [3][M][pitch] bfloat16, pitch = K rounded up to eight; a thread takes eight values of a row.
+template <bool VEC>
+__global__ void __launch_bounds__(256) split_rows_kernel(const float* __restrict__ x, long ldx, int M, int K, int pitch, uint4* __restrict__ terms) {
+  co_pdl_launch_dependents();
+  co_pdl_wait();
+  const int chunks = pitch / 8;
+  const long n = (long)M * chunks;
+  for (long i = (long)blockIdx.x * 256 + threadIdx.x; i < n; i += (long)gridDim.x * 256) {
+    const long m = i / chunks;
+    const int k = (int)(i - m * chunks) * 8;
+    const float* p = x + m * ldx + k;
+    float v[8];
+    if (VEC && k + 8 <= K) {
+      const float4 a = *reinterpret_cast<const float4*>(p), b = *reinterpret_cast<const float4*>(p + 4);
+      v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w; v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
+    } else {
+#pragma unroll
+      for (int j = 0; j < 8; ++j) v[j] = k + j < K ? p[j] : 0.f;
+    }
+    uint4 t[3];
+    split3(v[0], v[1], t[0].x, t[1].x, t[2].x);
+    split3(v[2], v[3], t[0].y, t[1].y, t[2].y);
+    split3(v[4], v[5], t[0].z, t[1].z, t[2].z);
+    split3(v[6], v[7], t[0].w, t[1].w, t[2].w);
+#pragma unroll
+    for (int j = 0; j < 3; ++j) terms[j * n + i] = t[j];
+  }
+}
+
+// A warp forms the products of the lanes in `bad` (lane l: feature n_first + l) with one row of x over [k0, k1) anew.
+__device__ __noinline__ float sum_again(unsigned bad, const float* __restrict__ x, const float* __restrict__ w, int n_first, int K, int k0, int k1) {
+  const int lane = threadIdx.x & 31;
+  float mine = 0.f;
+  while (bad) {
+    const int l = __ffs(bad) - 1;
+    bad &= bad - 1;
+    const float* row = w + (size_t)(n_first + l) * K;
+    float s = 0.f;
+    for (int k = k0 + lane; k < k1; k += 32) s = fmaf(x[k], row[k], s);
+    s = co_warp_sum(s);
+    if (lane == l) mine = s;
+  }
+  return mine;
+}
+
+struct F32Args {
+  const float* x; const float* w; const void* bias; float* out; float* apart;      // apart: [slice][M][N] (absent: one slice)
+  int bias_dtype, M, N, K, per_slice;      // stages of 64 k per slice
+  long ldx, ldo;
+  int* status;
+};
+
+template <int BT>
+__global__ void __launch_bounds__(448, 1)
+gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x, const F32Args P) {
+  using S = F32Tile<BT>;
+  extern __shared__ unsigned char smem_raw[];
+  unsigned char* ws = (unsigned char*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+  unsigned char* xs = ws + W_STAGES * W_BYTES;
+  unsigned long long* w_full = (unsigned long long*)(xs + X_STAGES * S::X_BYTES);
+  unsigned long long* w_free = w_full + W_STAGES;
+  unsigned long long* x_full = w_free + W_STAGES;       // [stage][term]
+  unsigned long long* x_free = x_full + 2 * 3;          // [stage][term]; of term 0: all products are formed, W's terms are free and the sums stand
+  unsigned long long* a_full = x_free + 2 * 3;          // W's terms stand in tensor memory
+  unsigned long long* acc_free = a_full + 2;            // the sums have been read
+  unsigned* tmem_slot = (unsigned*)(acc_free + 2);
+  static_assert((2 * W_STAGES + 16) * 8 + 4 <= 256, "barriers fit their slot");
+
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int n0 = blockIdx.x * F_ROWS, m0 = blockIdx.y * BT;
+  const int first = blockIdx.z * P.per_slice;
+  const int stages = min(P.per_slice, (P.K + BK - 1) / BK - first);
+
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < W_STAGES; ++s) { mbar_init(&w_full[s], 1); mbar_init(&w_free[s], 4); }
+    for (int s = 0; s < 6; ++s) { mbar_init(&x_full[s], 1); mbar_init(&x_free[s], 1); }
+    for (int s = 0; s < 2; ++s) { mbar_init(&a_full[s], 4); mbar_init(&acc_free[s], 4 * S::HALVES); }
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (warp == 2) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "n"(S::COLS) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  const unsigned tmem = *tmem_slot;
+  co_pdl_launch_dependents();
+
+  if (warp == 0) {
+    if (lane == 0) {
+      auto fetch_w = [&](int kt) {
+        const int s = kt % W_STAGES;
+        unsigned char* to = ws + s * W_BYTES;
+        mbar_expect_tx(&w_full[s], W_BYTES);      // (the map counts in halves of a float)
+        tma_load_2d(to, &map_w, (first + kt) * 2 * BK, n0, &w_full[s]);
+        tma_load_2d(to + W_BYTES / 2, &map_w, (first + kt) * 2 * BK + BK, n0, &w_full[s]);
+      };
+      for (int kt = 0; kt < W_STAGES && kt < stages; ++kt) fetch_w(kt);
+      co_pdl_wait();
+      for (int kt = 0; kt < stages; ++kt) {
+        const int b = kt & 1;
+        bool ok = true;
+        for (int t = 2; t >= 0 && ok; --t) {      // in the order in which the products let go of them
+          const int at = 3 * b + (S::BY_TERM ? t : 0);
+          if (S::BY_TERM || t == 2) {
+            ok = kt < 2 || mbar_wait(&x_free[at], ((kt >> 1) - 1) & 1);
+            if (!ok) break;
+            mbar_expect_tx(&x_full[at], S::BY_TERM ? S::X_TERM : S::X_BYTES);
+          }
+          tma_load_3d(xs + b * S::X_BYTES + t * S::X_TERM, &map_x, (first + kt) * BK, m0, t, &x_full[at]);
+        }
+        if (!ok) { atomicExch(P.status, 11); break; }
+        const int next = kt + W_STAGES - 1;       // freed when stage kt - 1 was split
+        if (kt >= 1 && next < stages) {
+          if (!mbar_wait(&w_free[next % W_STAGES], (next / W_STAGES - 1) & 1)) { atomicExch(P.status, 11); break; }
+          fetch_w(next);
+        }
+      }
+    }
+  } else if (warp == 1) {
+    if (lane == 0) {
+      constexpr unsigned idesc = umma_idesc(F_ROWS, BT);
+      for (int kt = 0; kt < stages; ++kt) {
+        const int b = kt & 1;
+        bool ok = mbar_wait(&a_full[b], (kt >> 1) & 1) && (kt < 2 || mbar_wait(&acc_free[b], ((kt >> 1) - 1) & 1));
+        const unsigned acc = tmem + b * BT, terms = tmem + S::A_AT + b * 3 * TERM_COLS;
+        const unsigned char* x = xs + b * S::X_BYTES;
+        // small products before large ones as far as x2 and x1 can be let go early: what fetches them again takes as long as a stage's products
+        constexpr int XT[6] = {2, 1, 1, 0, 0, 0}, WT[6] = {0, 1, 0, 2, 1, 0};
+#pragma unroll
+        for (int p = 0; p < 6; ++p) {
+          if (p == 0 || (S::BY_TERM && XT[p] != XT[p - 1])) {
+            ok = ok && mbar_wait(&x_full[3 * b + (S::BY_TERM ? XT[p] : 0)], (kt >> 1) & 1);
+            if (!ok) break;
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+          }
+          const unsigned long long db = umma_desc(x + XT[p] * S::X_TERM);
+#pragma unroll
+          for (int k = 0; k < BK / UMMA_K; ++k)
+            umma_bf16_a_tmem(acc, terms + WT[p] * TERM_COLS + k * (UMMA_K / 2), db + 2 * k, idesc, (p | k) != 0);
+          if (p == 5 || (S::BY_TERM && XT[p] != XT[p + 1])) umma_commit(&x_free[3 * b + XT[p]]);
+        }
+        if (!ok) { atomicExch(P.status, 12); break; }
+      }
+    }
+  } else if (warp < 6) {
+    const int quarter = warp & 3, row = quarter * 32 + lane;
+    for (int kt = 0; kt < stages; ++kt) {
+      const int s = kt % W_STAGES, b = kt & 1;
+      bool ok = mbar_wait(&w_full[s], (kt / W_STAGES) & 1);
+      const unsigned char* from = ws + s * W_BYTES + row * 128;
+      unsigned t0[32], t1[32], t2[32];
+#pragma unroll
+      for (int h = 0; h < 2; ++h)
+#pragma unroll
+        for (int c = 0; c < 8; ++c) {
+          const float4 v = *reinterpret_cast<const float4*>(from + h * (W_BYTES / 2) + ((c ^ (row & 7)) << 4));
+          const int at = h * 16 + 2 * c;
+          split3(v.x, v.y, t0[at], t1[at], t2[at]);
+          split3(v.z, v.w, t0[at + 1], t1[at + 1], t2[at + 1]);
+        }
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&w_free[s]);
+      if (kt >= 2) ok = ok && mbar_wait(&x_free[3 * b], ((kt >> 1) - 1) & 1);
+      ok = __all_sync(0xffffffffu, ok);
+      if (!ok) { if (lane == 0) atomicExch(P.status, 14); break; }
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      const unsigned to = tmem + ((unsigned)(quarter * 32) << 16) + S::A_AT + b * 3 * TERM_COLS;
+      tmem_st32(to, t0);
+      tmem_st32(to + TERM_COLS, t1);
+      tmem_st32(to + 2 * TERM_COLS, t2);
+      tmem_wait_st();
+      asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&a_full[b]);
+    }
+  } else if (warp < 6 + 4 * S::HALVES) {
+    const int quarter = warp & 3, half = (warp - 6) >> 2;
+    const int n_first = n0 + quarter * 32, n = n_first + lane, c0 = half * S::PART;
+    float sum[S::PART];
+#pragma unroll
+    for (int j = 0; j < S::PART; ++j) sum[j] = 0.f;
+    bool ok = true;
+    for (int kt = 0; kt < stages; ++kt) {
+      const int b = kt & 1;
+      ok = __all_sync(0xffffffffu, mbar_wait(&x_free[3 * b], (kt >> 1) & 1));
+      if (!ok) { if (lane == 0) atomicExch(P.status, 13); break; }
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      const unsigned from = tmem + ((unsigned)(quarter * 32) << 16) + b * BT + c0;
+#pragma unroll
+      for (int c = 0; c < S::PART; c += 16) {
+        unsigned r[16];
+        tmem_ld16(from + c, r);
+#pragma unroll
+        for (int j = 0; j < 16; ++j) sum[c + j] += __uint_as_float(r[j]);
+      }
+      asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&acc_free[b]);
+    }
+    if (ok) {
+      co_pdl_wait();      // out and the workspace may still be read by the predecessor; x is read where a result is not finite
+      const int k0 = first * BK, k1 = min(P.K, (first + stages) * BK);
+      const float bias = n < P.N && P.bias && !P.apart ? co_load_any(P.bias, P.bias_dtype, n) : 0.f;
+      float* to = P.apart ? P.apart + ((size_t)blockIdx.z * P.M) * P.N + n : P.out + n;
+      const long ld = P.apart ? P.N : P.ldo;
+      // (few instructions per column: code that runs once comes from memory, and at ten times the length it took as long as the products)
+      const int rows = min(S::PART, P.M - m0 - c0);
+      float* at = to + (long)(m0 + c0) * ld;
+      unsigned largest = 0;
+#pragma unroll
+      for (int j = 0; j < S::PART; ++j) {
+        largest = max(largest, __float_as_uint(sum[j]) & 0x7fffffffu);
+        if (j < rows && n < P.N) at[j * ld] = sum[j] + bias;
+      }
+      if (__any_sync(0xffffffffu, n < P.N && largest >= 0x7f800000u)) {
+        for (int j = 0; j < rows; ++j) {
+          const unsigned bad = __ballot_sync(0xffffffffu, n < P.N && !(fabsf(n < P.N ? at[j * ld] : 0.f) < INFINITY));
+          if (!bad) continue;
+          const float again = sum_again(bad, P.x + (m0 + c0 + j) * P.ldx, P.w, n_first, P.K, k0, k1);
+          if (bad >> lane & 1) at[j * ld] = again + bias;
+        }
+      }
+    }
+  }
+
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  if (warp == 2) {
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "n"(S::COLS) : "memory");
+  }
+}
+
+// The slices' sums, added in order, with what the product's own epilogue does; a thread takes four columns where N allows.
+template <int V>
+__global__ void __launch_bounds__(256)
+add_slices_kernel(const float* __restrict__ apart, int slices, const void* __restrict__ bias, int bias_dtype, float* __restrict__ out,
+                  int M, int N, long ldo, int act) {
+  co_pdl_launch_dependents();
+  co_pdl_wait();
+  const size_t size = (size_t)M * N, e = ((size_t)blockIdx.x * 256 + threadIdx.x) * V;
+  if (e >= size) return;
+  float v[V];
+#pragma unroll
+  for (int i = 0; i < V; ++i) v[i] = 0.f;
+#pragma unroll 4
+  for (int s = 0; s < slices; ++s) {
+    float t[V];
+    if (V == 4) *reinterpret_cast<float4*>(t) = *reinterpret_cast<const float4*>(apart + s * size + e);
+    else t[0] = apart[s * size + e];
+#pragma unroll
+    for (int i = 0; i < V; ++i) v[i] += t[i];
+  }
+  const size_t m = e / N;
+  const int n = (int)(e - m * N);
+#pragma unroll
+  for (int i = 0; i < V; ++i) {
+    float y = v[i];
+    if (bias) y += co_load_any(bias, bias_dtype, n + i);
+    out[m * ldo + n + i] = act ? co_gelu(y) : y;
+  }
+}
+
+// Slices of K: about one CTA per SM at few rows, at least four stages each; a function of the weight's shape alone.
+int slices_of(int N, int K) {
+  const int tiles = (N + F_ROWS - 1) / F_ROWS, k_tiles = (K + BK - 1) / BK;
+  if (tiles >= 100) return 1;
+  int s = (148 + tiles / 2) / tiles;
+  if (s > k_tiles / 4) s = k_tiles / 4;
+  if (s < 2) return 1;
+  const int per = (k_tiles + s - 1) / s;
+  return (k_tiles + per - 1) / per;
+}
+int pitch_of(int K) { return (K + 7) / 8 * 8; }
+constexpr int BT_MOST = 160;
+// Rows that are worked on at a time: their terms (6 bytes a value) and their slices' sums take 128 MB at most (the slices' sums then
+// about stay in L2, where the adding kernel finds them), one tile of rows at least.
+int rows_at_once(int M, int N, int K) {
+  const int slices = slices_of(N, K);
+  const double each = 6.0 * pitch_of(K) + 4.0 * slices * N;
+  const double rows = floor((double)(128 << 20) / each / BT_MOST) * BT_MOST;
+  return rows < BT_MOST ? (M < BT_MOST ? M : BT_MOST) : (rows < M ? (int)rows : M);
+}
+long terms_floats(long rows, int K) { return (3 * rows * pitch_of(K) / 2 + 63) / 64 * 64; }
+
+template <int BT>
+int launch(const CUtensorMap& mw, const CUtensorMap& mx, const F32Args& P, int slices, cudaStream_t stream) {
+  auto kernel = gemm_f32_tc_kernel<BT>;
+  cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, F32Tile<BT>::SMEM);
+  if (e != cudaSuccess) CO_FAIL("gemm_f32_tc: %d bytes of shared memory: %s", F32Tile<BT>::SMEM, cudaGetErrorString(e));
+  e = co_launch(kernel, dim3((P.N + F_ROWS - 1) / F_ROWS, (P.M + BT - 1) / BT, slices), dim3(448), F32Tile<BT>::SMEM, stream, mw, mx, P);
+  if (e != cudaSuccess) CO_FAIL("gemm_f32_tc: launch failed: %s", cudaGetErrorString(e));
+  CO_CHECK_LAUNCH("gemm_f32_tc");
+  return 0;
+}
+}  // namespace
+
+// Whether the kernel takes a weight of this shape (a function of the shape alone, so that all rows of a product go the same way):
+// rows of 16-byte multiples, and large enough that a tile of 128 features and stages of 64 k pay.
+CO_EXPORT int coheryn_gemm_f32_tc_takes(int N, int K) { return N >= 128 && K >= 256 && K % 4 == 0; }
+
+// Floats of workspace (16-byte aligned) that a product with this activation needs.
+CO_EXPORT long coheryn_gemm_f32_tc_workspace_floats(int M, int N, int K, int act) {
+  if (M <= 0 || N <= 0 || K <= 0) return 0;
+  const int rows = rows_at_once(M, N, K), slices = slices_of(N, K);
+  return terms_floats(rows, K) + (slices > 1 || act ? (long)slices * rows * N : 0);
+}
+
+// x: [M, K] with row stride ldx; w: [N, K] contiguous, 16-byte aligned; out: [M, N] with row stride ldo; all float32.
+// act 0: the (biased) product; CO_ACT_GELU: its exact GELU.  status: device word that receives 11..14 if a bounded wait ran out.
+CO_EXPORT int coheryn_gemm_f32_tc(const float* x, const float* w, const void* bias, int bias_dtype, float* out, int M, int N, int K,
+                                  long ldx, long ldo, int act, int* status, float* workspace, long floats, cudaStream_t stream) {
+  if (M <= 0 || N <= 0) return 0;
+  if (!coheryn_gemm_f32_tc_takes(N, K)) CO_FAIL("gemm_f32_tc: a weight of %d x %d is not taken", N, K);
+  if (act != 0 && act != CO_ACT_GELU) CO_FAIL("gemm_f32_tc: unknown activation %d", act);
+  if (((uintptr_t)w & 15) || ((uintptr_t)workspace & 15)) CO_FAIL("gemm_f32_tc: the weight and the workspace must be 16-byte aligned");
+  if (!workspace || floats < coheryn_gemm_f32_tc_workspace_floats(M, N, K, act)) CO_FAIL("gemm_f32_tc: the workspace of %ld floats is too small", floats);
+  const int slices = slices_of(N, K), pitch = pitch_of(K), most = rows_at_once(M, N, K);
+  const bool apart = slices > 1 || act != 0;      // what follows the sums is the adding kernel's
+  CUtensorMap mw, mx;
+  if (!make_map(&mw, w, N, 2L * K, 2L * K, F_ROWS)) CO_FAIL("gemm_f32_tc: cuTensorMapEncodeTiled failed (N=%d K=%d)", N, K);
+  for (int m = 0; m < M; m += most, x += (size_t)most * ldx, out += (size_t)most * ldo) {
+    const int rows = M - m < most ? M - m : most;
+    // tiles of tokens as even as tiles of at most 160 allow
+    const int tiles = (rows + BT_MOST - 1) / BT_MOST, each = (rows + tiles - 1) / tiles;
+    const int bt = each <= 16 ? 16 : each <= 32 ? 32 : (each + 31) / 32 * 32;
+    const cuuint64_t dims[3] = {(cuuint64_t)K, (cuuint64_t)rows, 3}, strides[2] = {(cuuint64_t)pitch * 2, (cuuint64_t)pitch * 2 * rows};
+    const cuuint32_t box[3] = {(cuuint32_t)BK, (cuuint32_t)bt, 1};
+    if (!make_map_nd(&mx, workspace, 3, dims, strides, box)) CO_FAIL("gemm_f32_tc: cuTensorMapEncodeTiled failed (M=%d K=%d)", rows, K);
+    const long chunks = (long)rows * (pitch / 8);
+    const unsigned blocks = (unsigned)((chunks + 255) / 256 < 148 * 8 ? (chunks + 255) / 256 : 148 * 8);
+    const bool vec = ldx % 4 == 0 && !((uintptr_t)x & 15);
+    co_launch(vec ? split_rows_kernel<true> : split_rows_kernel<false>, dim3(blocks), dim3(256), 0, stream, x, ldx, rows, K, pitch, (uint4*)workspace);
+    CO_CHECK_LAUNCH("split_rows");
+    const F32Args P = {x, w, bias, out, apart ? workspace + terms_floats(most, K) : nullptr, bias_dtype, rows, N, K,
+                       ((K + BK - 1) / BK + slices - 1) / slices, ldx, ldo, status};
+    const int rc = bt == 16 ? launch<16>(mw, mx, P, slices, stream) : bt == 32 ? launch<32>(mw, mx, P, slices, stream)
+                 : bt == 64 ? launch<64>(mw, mx, P, slices, stream) : bt == 96 ? launch<96>(mw, mx, P, slices, stream)
+                 : bt == 128 ? launch<128>(mw, mx, P, slices, stream) : launch<160>(mw, mx, P, slices, stream);
+    if (rc) return rc;
+    if (apart) {
+      const bool four = N % 4 == 0;
+      const size_t n = (size_t)rows * N / (four ? 4 : 1);
+      co_launch(four ? add_slices_kernel<4> : add_slices_kernel<1>, dim3((unsigned)((n + 255) / 256)), dim3(256), 0, stream, P.apart, slices, bias,
+                bias_dtype, out, rows, N, ldo, act);
+      CO_CHECK_LAUNCH("add_slices");
+    }
+  }
+  return 0;
+}

@@ -45,6 +45,7 @@ def core():
         lib.coheryn_argmax_scratch_slots.restype = ctypes.c_long
         lib.coheryn_gemm_tc_workspace_floats.restype = ctypes.c_long
         lib.coheryn_gemm_simt_workspace_floats.restype = ctypes.c_long
+        lib.coheryn_gemm_f32_tc_workspace_floats.restype = ctypes.c_long
         _core = lib
     return _core
 
@@ -494,6 +495,38 @@ def gemm_simt(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor], ou
         c_int(blocks[0] if blocks else 0), c_int(blocks[1] if blocks else 0), _stream()))
 
 
+@functools.lru_cache(maxsize=4096)
+def _f32_tc_workspace_floats(M: int, N: int, K: int, act: int) -> int:
+    """0: the tensor-core kernel does not take such a weight (its shape alone decides, so all rows go the same way)."""
+    lib = core()
+    if not lib.coheryn_gemm_f32_tc_takes(c_int(N), c_int(K)):
+        return 0
+    return int(lib.coheryn_gemm_f32_tc_workspace_floats(c_int(M), c_int(N), c_int(K), c_int(act)))
+
+
+def gemm_f32(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor], out: torch.Tensor, act: int = 0) -> None:
+    """out = x @ w.T (+ bias), passed through ``act``, to float32's accuracy: float32 operands on the tensor cores as exact sums
+    of three bfloat16 terms (csrc/gemm_f32_tc.cu) where the weight's shape pays, everything else on the CUDA cores
+    (``gemm_simt``).  A row's bits do not depend on the other rows."""
+    M, K = x.shape
+    N = w.shape[0]
+    floats = 0
+    if M and x.dtype == w.dtype == out.dtype == torch.float32 and w.data_ptr() % 16 == 0:
+        floats = _f32_tc_workspace_floats(M, N, K, act)
+    if not floats:
+        return gemm_simt(x, w, bias, out, act)
+    _dev(x, w, bias, out)
+    assert w.shape == (N, K) and w.is_contiguous() and out.shape == (M, N)
+    assert x.stride(1) == 1 and out.stride(1) == 1
+    if bias is not None:
+        assert bias.shape == (N,) and bias.is_contiguous()
+    lib = core()
+    workspace = torch.empty(floats, dtype=torch.float32, device=x.device)
+    _check(lib, lib.coheryn_gemm_f32_tc(
+        _ptr(x), _ptr(w), _ptr(bias), c_int(_code(bias) if bias is not None else F32), _ptr(out), c_int(M), c_int(N), c_int(K),
+        c_long(x.stride(0)), c_long(out.stride(0)), c_int(act), _ptr(tc_status(x.device)), _ptr(workspace), c_long(floats), _stream()))
+
+
 def attention_simple(q: torch.Tensor, out: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor,
                      block_tables: torch.Tensor, token_req: torch.Tensor, positions: torch.Tensor,
                      num_heads: int, num_kv_heads: int, head_dim: int, page_size: int,
@@ -782,8 +815,8 @@ def _small_ok(x, w) -> bool:
 def linear(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor] = None,
            out_dtype: Optional[torch.dtype] = None, out: Optional[torch.Tensor] = None,
            partial_ok: bool = False, activation: Optional[str] = None) -> torch.Tensor:
-    """y = x @ w.T (+ bias), float32 accumulation.  float32 operands use FMA on the CUDA
-    cores (no reduced-precision tensor mode); bfloat16 operands use the tensor-core
+    """y = x @ w.T (+ bias), float32 accumulation.  float32 operands keep float32's
+    accuracy (``gemm_f32``: no reduced-precision tensor mode); bfloat16 operands use the tensor-core
     kernels where the shape allows and the FMA kernel otherwise.  With ``partial_ok`` the
     result may come as a float32 stack [splits, M, N] of partial sums whose addition is left
     to the consumer (``add_rmsnorm`` takes such a stack as its delta).  ``activation``: y passes this function (a name of
@@ -808,7 +841,7 @@ def linear(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor] = None
     elif _tc_ok(x, w):
         gemm_bf16_tc(x, w, bias, out, epilogue=act)
     else:
-        gemm_simt(x, w, bias, out, act)
+        gemm_f32(x, w, bias, out, act)
     return out
 
 
@@ -1069,7 +1102,7 @@ def gated_linear(x: torch.Tensor, w_gate_up: torch.Tensor, activation: str = "si
         gemm_bf16_tc(x, w_gate_up, None, out, gated=code)
         return out
     gu = torch.empty((M, 2 * I), dtype=x.dtype, device=x.device)
-    gemm_simt(x, w_gate_up, None, gu)
+    gemm_f32(x, w_gate_up, None, gu)
     silu_mul(gu, out, code, float(param or 0.0))
     return out
 
