@@ -810,11 +810,6 @@ qk_norm_kv_write_kernel(const float* __restrict__ q, const float* __restrict__ k
 }
 
 constexpr int chunk_tokens(int DK) { return DK <= 128 ? 32 : 16; }
-// Lanes per group of columns and columns per group.  The more lanes share a column, the fewer steps a token costs
-// each of them (the recurrence is a chain of dependent steps, and that chain is what bounds a long prompt): sixteen
-// from 128 key channels on, eight from 64, four below.  Four columns per group (two for narrow heads); a head of more
-// than 128 value channels takes twice as many so that the CTA stays within 512 threads.
-constexpr int scan_split(int DK) { return DK >= 128 ? 16 : (DK >= 64 ? 8 : 4); }
 constexpr int scan_columns(int DK, bool wide) { return (DK >= 64 ? 4 : 2) * (wide ? 2 : 1); }
 
 }  // namespace
@@ -855,11 +850,6 @@ CO_EXPORT int coheryn_short_conv_silu(const float* x, long ldx, float* y, long l
   }
   return 0;
 }
-
-#define CO_SCAN_CASES(LAUNCH)                                                                   \
-  if (dk <= 16) { LAUNCH(16) } else if (dk <= 32) { LAUNCH(32) } else if (dk <= 48) { LAUNCH(48) } \
-  else if (dk <= 64) { LAUNCH(64) } else if (dk <= 96) { LAUNCH(96) } else if (dk <= 128) { LAUNCH(128) } \
-  else if (dk <= 192) { LAUNCH(192) } else { LAUNCH(256) }
 
 // Into how many CTAs the columns of a head are split: one (the scan's own epilogue normalises whole heads) unless the
 // step is a long prompt of few requests, where a CTA per head would leave most SMs idle; then 64 columns per CTA, the
@@ -942,13 +932,15 @@ CO_EXPORT int coheryn_gated_delta_scan(
   if (gate_act != 0 && gate_act != 1) CO_FAIL("gated_delta_scan: unknown gate activation %d", gate_act);
   const long ld_prep = (long)2 * kv_heads * dk + (long)heads * dk + heads;     // per token: q, k, decays, beta
   const bool chunked = chunks > 0 && co_delta_chunks_take(dk, dv) && scratch && scratch_floats >= co_delta_chunk_floats(chunks, heads, dk, dv);
-  const int slices = chunked ? 1 : scan_slices(B, heads, dv, total_tokens, scratch, scratch_floats, (long)total_tokens * ld_prep);
+  const bool one = !chunked && total_tokens <= B && co_one_token_takes(dk, dv, state, state_stride);      // (almost) every run is one token
+  const int slices = chunked || one ? 1 : scan_slices(B, heads, dv, total_tokens, scratch, scratch_floats, (long)total_tokens * ld_prep);
   float* prep = slices > 1 ? scratch + (long)total_tokens * heads * dv : nullptr;
   if (kv_heads < 1 || heads % kv_heads) CO_FAIL("gated_delta_scan: %d heads do not group over %d q/k heads", heads, kv_heads);
   DeltaIn P{q, k, v, ld_qkv, beta, ld_beta, step, ld_step, step_bias, step_bias_dtype, rate_log, rate_log_dtype, state,
             state_stride, cu_q, state_slots, heads, kv_heads, dk, dv, decay_channels};
   HeadOut E{out, out_dtype, ldo, weight, weight_dtype, weight_stride, gate, ldg, eps, out_scale,
             slices > 1 ? scratch : nullptr, (long)heads * dv, nullptr, gate_act};
+  if (one) return co_delta_one(P, E, B, stream);
   if (chunked) {
     if (co_delta_chunks(P, E, B, chunks, runs, scratch, stream)) return 1;
     if (!short_runs) return 0;
@@ -994,10 +986,12 @@ CO_EXPORT int coheryn_matrix_memory_scan(
   if (!scan_shape_ok("matrix_memory_scan", heads, dk, dv)) return 1;
   if (!(cap > 0.f)) CO_FAIL("matrix_memory_scan: the gate cap must be positive");
   const bool chunked = chunks > 0 && co_memory_chunks_take(dk, dv) && scratch && scratch_floats >= co_memory_chunk_floats(chunks, heads, dk, dv);
-  const int slices = chunked ? 1 : scan_slices(B, heads, dv, total_tokens, scratch, scratch_floats, (long)B * heads * (dk + 1));
+  const bool one = !chunked && total_tokens <= B && co_one_token_takes(dk, dv, state, state_stride);      // (almost) every run is one token
+  const int slices = chunked || one ? 1 : scan_slices(B, heads, dv, total_tokens, scratch, scratch_floats, (long)B * heads * (dk + 1));
   MemoryIn P{q, k, v, ld, gi, gf, ld_gate, bias_i, bias_f, bias_dtype, cap, state, state_stride, cu_q, state_slots, heads, dk, dv};
   HeadOut E{out, out_dtype, ldo, weight, weight_dtype, weight_stride, gate, ldg, eps, out_scale,
             slices > 1 ? scratch : nullptr, (long)heads * dv, slices > 1 ? scratch + (long)total_tokens * heads * dv : nullptr};
+  if (one) return co_memory_one(P, E, B, stream);
   if (chunked) {
     if (co_memory_chunks(P, E, B, chunks, runs, scratch, stream)) return 1;
     if (!short_runs) return 0;

@@ -62,6 +62,22 @@ bool co_memory_chunks_take(int dk, int dv);
 long co_memory_chunk_floats(int chunks, int heads, int dk, int dv);
 int co_memory_chunks(const MemoryIn& P, const HeadOut& E, int B, int chunks, int runs, float* scratch, cudaStream_t stream);
 
+// Lanes per group of columns and columns per group.  The more lanes share a column, the fewer steps a token costs
+// each of them (the recurrence is a chain of dependent steps, and that chain is what bounds a long prompt): sixteen
+// from 128 key channels on, eight from 64, four below.  Four columns per group (two for narrow heads); a head of more
+// than 128 value channels takes twice as many so that the CTA stays within 512 threads.
+constexpr int scan_split(int DK) { return DK >= 128 ? 16 : (DK >= 64 ? 8 : 4); }
+// The key channels that the scans are built for, the smallest that hold `dk`.
+#define CO_SCAN_CASES(LAUNCH)                                                                   \
+  if (dk <= 16) { LAUNCH(16) } else if (dk <= 32) { LAUNCH(32) } else if (dk <= 48) { LAUNCH(48) } \
+  else if (dk <= 64) { LAUNCH(64) } else if (dk <= 96) { LAUNCH(96) } else if (dk <= 128) { LAUNCH(128) } \
+  else if (dk <= 192) { LAUNCH(192) } else { LAUNCH(256) }
+
+// Steps in which every request brings one token (recurrent_one.cu): the same bits as the scans.
+bool co_one_token_takes(int dk, int dv, const float* state, long stride);
+int co_delta_one(const DeltaIn& P, const HeadOut& E, int B, cudaStream_t stream);
+int co_memory_one(const MemoryIn& P, const HeadOut& E, int B, cudaStream_t stream);
+
 namespace {
 
 __device__ __forceinline__ float rc_sigmoid(float z) { return 1.0f / (1.0f + expf(-z)); }
