@@ -16,9 +16,7 @@
 // Temporaries live in one scratch area that the caller provides (its size is asked for with
 // dry_run = 1); the block's output (bfloat16 [T, H], or a float32 stack of partial sums
 // [splits, T, H] that the next norm adds) goes where the caller says, its kind being part of the plan.
-#include "common.cuh"
-
-#include <cstdint>
+#include "block_routes.h"
 
 extern "C" {
 int coheryn_add_rmsnorm(float* resid, const void* delta, int delta_dtype, const int* rows, const void* weight, int wdtype,
@@ -32,22 +30,12 @@ int coheryn_rope_kv_write_parts(const float* parts, int splits, long split_strid
 int coheryn_rope_kv_write(void* qkv, int dtype, const int* positions, const float* cos_sin, const int* slots, void* k_cache,
                           void* v_cache, int T, int nh, int nkv, int hd, int rot, int page_size, int write_kv,
                           cudaStream_t stream);
-int coheryn_gemm_bf16_small(const void* x, const void* w, const void* bias, int bias_dtype, void* out, int out_dtype, int M,
-                            int N, int K, long ldx, long ldo, int epilogue, cudaStream_t stream);
 int coheryn_qkv_rope_bf16_small(const void* x, const void* w, const void* bias, int bias_dtype, void* q_out, long ldq,
                                 const int* positions, const float* cos_sin, const int* slots, void* k_cache, void* v_cache,
                                 int M, int K, long ldx, int nh, int nkv, int hd, int page_size, cudaStream_t stream);
-long coheryn_gemm_tc_workspace_floats(int M, int N, int K);
-int coheryn_gemm_bf16_tc(const void* x, const void* w, const void* bias, int bias_dtype, void* out, int out_dtype, int M,
-                         int N, int K, long ldx, long ldo, int epilogue, int* status, float* workspace,
-                         long workspace_floats, cudaStream_t stream);
 int coheryn_gemm_tc_parts_count(int M, int N, int K);
 int coheryn_gemm_bf16_tc_parts(const void* x, const void* w, float* parts, int M, int N, int K, long ldx, int* status,
                                cudaStream_t stream);
-int coheryn_gemm_tc_few_splits(int N, int K);
-int coheryn_gemm_bf16_tc_few(const void* x, const void* w, const void* bias, int bias_dtype, void* out, int out_dtype, int M,
-                             int N, int K, long ldx, long ldo, int epilogue, int* status, float* workspace,
-                             long workspace_floats, int defer, cudaStream_t stream);
 }
 
 // Entry points of the attention library of the layer's head size (a library of its own).
@@ -87,13 +75,6 @@ struct CoBlockStep {
   const int* q_lens;      // on the host: tokens of every request (null: not counted)
 };
 
-// ops.py's thresholds, as they stand when the step is run.
-struct CoBlockTuning {
-  long small_weight_elements, few_large_weight, attn_oproj_merge_bytes;
-  int few_m, few_defer_m, few_head_m, small_m, small_m_short, defer_min_k, defer_min_k_wide;
-  int qkv_rope_m, qkv_parts_m, qkv_parts_few_from, attn_oproj_m;
-};
-
 // What the block's output is: kind 1 = bfloat16 [T, H]; 2 = float32 [splits, T, H].
 // The rest says which way each step of the block goes (tests compare it with ops.py's predicates):
 // qkv_route 1 = rotation in the product's epilogue, 2 = K slices of the few-rows product added by the
@@ -108,64 +89,6 @@ struct CoBlockPlan {
 
 #define CO_BLOCK_UNSUPPORTED 3    // nothing was launched: run the parts one by one
 #define CO_BLOCK_ATTENTION_FAILED 2   // the message is the attention library's
-
-namespace {
-
-enum Route { R_NONE = 0, R_FEW, R_FEW_DEFER, R_SMALL, R_TC };
-
-inline bool aligned16(const void* p) { return ((uintptr_t)p & 15) == 0; }
-
-struct Router {
-  const CoBlockTuning& t;
-  bool operands_ok(int K, long ldx, const void* x, const void* w) const {
-    return K % 8 == 0 && ldx % 8 == 0 && aligned16(x) && aligned16(w);
-  }
-  bool few_shape_ok(int M, int K, long ldx, const void* x, const void* w, int limit) const {
-    return 0 < M && M <= limit && operands_ok(K, ldx, x, w);
-  }
-  bool few_ok(int M, int N, int K, long ldx, const void* x, const void* w) const {
-    const int limit = (long)N * K >= t.few_large_weight ? t.few_head_m : t.few_m;
-    return few_shape_ok(M, K, ldx, x, w, limit) && coheryn_gemm_tc_few_splits(N, K) == 1;
-  }
-  bool small_ok(int M, int N, int K, long ldx, const void* x, const void* w) const {
-    return ((0 < M && M <= t.small_m) || (0 < M && M <= t.small_m_short && (long)N * K <= t.small_weight_elements)) &&
-           operands_ok(K, ldx, x, w);
-  }
-  bool tc_ok(int M, int K, long ldx, const void* x, const void* w) const {
-    return M > t.small_m && operands_ok(K, ldx, x, w);
-  }
-  // ops.linear: the route of y = x w^T and, for R_FEW_DEFER, the number of K slices.
-  Route linear(int M, int N, int K, long ldx, const void* x, const void* w, bool partial_ok, int* splits) const {
-    *splits = 1;
-    if (partial_ok && M > 0 && K >= (M > t.small_m_short ? t.defer_min_k_wide : t.defer_min_k) &&
-        few_shape_ok(M, K, ldx, x, w, t.few_defer_m)) {
-      const int s = coheryn_gemm_tc_few_splits(N, K);
-      if (s > 1) {
-        *splits = s;
-        return R_FEW_DEFER;
-      }
-    }
-    if (few_ok(M, N, K, ldx, x, w)) return R_FEW;
-    if (small_ok(M, N, K, ldx, x, w)) return R_SMALL;
-    if (tc_ok(M, K, ldx, x, w)) return R_TC;
-    return R_NONE;
-  }
-};
-
-struct Arena {
-  char* base;
-  size_t off;
-  void* workspace = nullptr;      // one area for the K slices of whichever many-rows product is running
-  long workspace_floats = 0;
-  void* take(size_t bytes) {
-    off = (off + 255) & ~(size_t)255;
-    void* p = base ? (void*)(base + off) : nullptr;
-    off += bytes;
-    return p;
-  }
-};
-
-}  // namespace
 
 namespace {
 

@@ -30,7 +30,7 @@ BASE_FLAGS = ["-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC", "-Xcompil
 # The core library: everything that is not specialised by a compile-time size.
 CORE_SOURCES = ["runtime.cu", "elementwise.cu", "gemm_simt.cu", "attention_simple.cu",
                 "sampling.cu", "gemm_bf16_small.cu", "gemm_tc.cu", "gemm_tc_few.cu", "gemm_f32_tc.cu", "seeded_fill.cu", "selftest.cu",
-                "block_runner.cu", "stream_ops.cu"]
+                "block_runner.cu", "mixer_runner.cu", "stream_ops.cu"]
 ROUTED_SOURCES = ["routed.cu", "runtime.cu"]
 RECURRENT_SOURCES = ["recurrent.cu", "recurrent_one.cu", "delta_chunks.cu", "memory_chunks.cu", "runtime.cu"]
 VARIANT_SOURCES = ["attention_variants.cu", "runtime.cu"]

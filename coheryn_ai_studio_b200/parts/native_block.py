@@ -42,6 +42,13 @@ class CoBlockTuning(ctypes.Structure):
                                      "defer_min_k_wide", "qkv_rope_m", "qkv_parts_m", "qkv_parts_few_from", "attn_oproj_m")]
 
 
+def block_tuning() -> CoBlockTuning:
+    """The thresholds of ``ops`` as they stand."""
+    return CoBlockTuning(ops.SMALL_WEIGHT_ELEMENTS, ops.FEW_LARGE_WEIGHT, ops.ATTN_OPROJ_MERGE_BYTES, ops.FEW_M, ops.FEW_DEFER_M,
+                         ops.FEW_HEAD_M, ops.SMALL_M, ops.SMALL_M_SHORT, ops.DEFER_MIN_K, ops.DEFER_MIN_K_WIDE, ops.QKV_ROPE_M,
+                         ops.QKV_PARTS_M, ops.QKV_PARTS_FEW_FROM, ops.ATTN_OPROJ_M)
+
+
 class CoBlockPlan(ctypes.Structure):
     _fields_ = [("scratch_bytes", c_long), ("out_kind", c_int), ("out_splits", c_int)] + \
                [(n, c_int) for n in ("qkv_route", "qkv_parts", "qkv_linear", "merged", "o_route", "gate_route", "down_route")]
@@ -116,10 +123,7 @@ class StepNative:
                                 ops.tc_status(device).data_ptr(), ops._stream().value or 0, step.num_tokens, n,
                                 shortest, longest, step.max_kv_len, 1 if step.prior_positions_settled else 0,
                                 ctypes.addressof(self.q_lens) if self.q_lens is not None else None)
-        self.tuning = CoBlockTuning(ops.SMALL_WEIGHT_ELEMENTS, ops.FEW_LARGE_WEIGHT, ops.ATTN_OPROJ_MERGE_BYTES, ops.FEW_M,
-                                    ops.FEW_DEFER_M, ops.FEW_HEAD_M, ops.SMALL_M, ops.SMALL_M_SHORT, ops.DEFER_MIN_K,
-                                    ops.DEFER_MIN_K_WIDE, ops.QKV_ROPE_M, ops.QKV_PARTS_M, ops.QKV_PARTS_FEW_FROM,
-                                    ops.ATTN_OPROJ_M)
+        self.tuning = block_tuning()
         self.step_ref, self.tuning_ref = ctypes.addressof(self.step), ctypes.addressof(self.tuning)
         self.groups = {}
         self.plans = {}

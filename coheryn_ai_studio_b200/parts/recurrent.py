@@ -45,6 +45,7 @@ from .. import ops
 from ..config.spec import PartSpec
 from ..weights.spec import TensorSpec
 from .base import MIXERS, POSITIONS, FixedState, LayerCache, Mixer, NormedSum, Runtime, StepContext, build_part, register_mixer
+from .native_mixer import NativeMixer
 
 
 class _StackedInput:
@@ -74,6 +75,15 @@ class _StateMixer(Mixer):
         # rows are, and with the scans token by token a sequence has the same bits however load or preemption cut it.  (In bfloat16
         # the product that runs follows the step's rows anyway.)
         self.in_chunks = runtime.dtype != torch.float32
+        self.native = None      # the whole mixer by one call into the library: made when the weights are bound
+
+    def _bind_native(self, memory: bool, names, **fields_and_tensors) -> None:
+        """``names``: the fields that hold tensors."""
+        self.native = None
+        if self.runtime.dtype == torch.bfloat16 and self.w_o.is_cuda:
+            tensors = {n: fields_and_tensors.pop(n) for n in names}
+            self.native = NativeMixer.build(dict(fields_and_tensors, width=self.hidden_size, heads=self.num_heads, dk=self.dk, dv=self.dv,
+                                                 eps=self.eps, out_scale=self.out_scale, in_chunks=int(self.in_chunks)), tensors, memory)
 
     def forward(self, x: torch.Tensor, step: StepContext, cache: Optional[LayerCache]) -> torch.Tensor:
         out = torch.empty((1, x.shape[0], self.hidden_size), dtype=torch.float32, device=x.device)
@@ -116,11 +126,17 @@ class MatrixMemory(_StateMixer):
         self.w_o, self.norm_w = tensors["o"], tensors["norm"]
         dt = torch.float32 if torch.float32 in (tensors["i.b"].dtype, tensors["f.b"].dtype) else tensors["i.b"].dtype
         self.b_i, self.b_f = tensors["i.b"].to(dt).contiguous(), tensors["f.b"].to(dt).contiguous()
+        at = {n: r[0] for n, r in self.stacked.ranges.items()}
+        self._bind_native(True, ("w_in", "w_o", "bias_a", "bias_b", "norm_w"), w_in=self.stacked.weight, w_o=self.w_o, bias_a=self.b_i, bias_b=self.b_f,
+                          norm_w=self.norm_w, cap=self.cap, columns=self.stacked.weight.shape[0], kv_heads=self.num_heads, at_q=at["q"],
+                          at_k=at["k"], at_v=at["v"], at_g=at["g"], at_a=at["i"], at_b=at["f"])
 
     def output_weights(self):
         return [self.w_o]
 
     def forward_into(self, x: torch.Tensor, step: StepContext, cache: Optional[LayerCache], out: torch.Tensor) -> None:
+        if self.native is not None and ops.NATIVE_BLOCK and self.native.run(x, step, self._state_of(cache), None, out[0]):
+            return
         o = torch.empty((x.shape[0], self.num_heads * self.dv), dtype=self.runtime.dtype, device=x.device)
         self.forward_open(x, step, cache, [o])
         ops.linear(o, self.w_o, out=out[0])
@@ -128,6 +144,8 @@ class MatrixMemory(_StateMixer):
     def forward_open(self, x: torch.Tensor, step: StepContext, cache: Optional[LayerCache], outs) -> None:
         """The activations in front of the output product (normalised, gated, weighted) into ``outs[0]``."""
         state = self._state_of(cache)
+        if self.native is not None and ops.NATIVE_BLOCK and self.native.run(x, step, state, outs[0], None):
+            return
         st, proj = self.stacked, self.stacked.project(x)
         o = outs[0]
         ops.matrix_memory_scan(st.cut(proj, "q"), st.cut(proj, "k"), st.cut(proj, "v"), st.cut(proj, "i"), st.cut(proj, "f"),
@@ -187,7 +205,8 @@ class GatedDeltaRule(_StateMixer):
         self.rate_log, self.dt_bias, self.norm_w = tensors["A_log"], tensors["dt_bias"], tensors["norm"]
         if not self.low_rank:
             self.stacked = _StackedInput([(n, tensors[n]) for n in ("q", "k", "v", "b", "a", "g")])
-            self.w_second = None
+            self.w_second, self.second_blocks = None, (0, 0)
+            self._bind_native_delta("a", "g")
             return
         if tensors["a1"].shape[0] != tensors["a2"].shape[1] or tensors["g1"].shape[0] != tensors["g2"].shape[1]:
             raise ValueError("the two steps of a low-rank projection do not fit each other")
@@ -199,17 +218,32 @@ class GatedDeltaRule(_StateMixer):
         both[:a2.shape[0], :a2.shape[1]] = a2
         both[a2.shape[0]:, a2.shape[1]:] = g2
         self.w_second, self.second_blocks = both.contiguous(), tuple(a2.shape)
+        self._bind_native_delta("a1", "g1")
+
+    def _bind_native_delta(self, step_name: str, gate_name: str) -> None:
+        at = {n: r[0] for n, r in self.stacked.ranges.items()}
+        second = tuple(self.w_second.shape) if self.w_second is not None else (0, 0)
+        self._bind_native(False, ("w_in", "w_second", "w_o", "conv_w", "bias_a", "bias_b", "norm_w"), w_in=self.stacked.weight, w_second=self.w_second,
+                          w_o=self.w_o, conv_w=self.conv_w, bias_a=self.dt_bias, bias_b=self.rate_log, norm_w=self.norm_w,
+                          columns=self.stacked.weight.shape[0], kv_heads=self.num_kv_heads, taps=self.taps,
+                          decay_channels=self.dk if self.decay == "channel" else 1, gate_act=1 if self.gate_activation == "silu" else 0,
+                          at_q=at["q"], at_k=at["k"], at_v=at["v"], at_b=at["b"], at_a=at[step_name], at_g=at[gate_name],
+                          second_n=second[0], second_k=second[1], second_rows=self.second_blocks[0], second_columns=self.second_blocks[1])
 
     def output_weights(self):
         return [self.w_o]
 
     def forward_into(self, x: torch.Tensor, step: StepContext, cache: Optional[LayerCache], out: torch.Tensor) -> None:
+        if self.native is not None and ops.NATIVE_BLOCK and self.native.run(x, step, self._state_of(cache), None, out[0]):
+            return
         o = torch.empty((x.shape[0], self.num_heads * self.dv), dtype=self.runtime.dtype, device=x.device)
         self.forward_open(x, step, cache, [o])
         ops.linear(o, self.w_o, out=out[0])
 
     def forward_open(self, x: torch.Tensor, step: StepContext, cache: Optional[LayerCache], outs) -> None:
         state = self._state_of(cache)
+        if self.native is not None and ops.NATIVE_BLOCK and self.native.run(x, step, state, outs[0], None):
+            return
         st, proj = self.stacked, self.stacked.project(x)
         G, H, dk, dv = self.num_kv_heads, self.num_heads, self.dk, self.dv
         qkv = ops.short_conv_silu(st.cut(proj, "q", "v"), self.conv_w, state[:, self.memory:], step)
