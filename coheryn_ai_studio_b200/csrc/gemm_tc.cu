@@ -566,20 +566,25 @@ __device__ __forceinline__ void mbar_arrive_cluster(unsigned bar_cluster_addr) {
   asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar_cluster_addr) : "memory");
 }
 
+// Eight epilogue warps per CTA, two per quarter of its rows, that take the chunks of columns in turn.  With four (a warp a scheduler)
+// the gate's exponentials and divisions took longer than the 24 k-steps of the next tile at K = 1,536: measured on a B200, 2048 x 17920 x
+// 1536 gated 108 -> 85 us (ungated 82), 1873 rows 120 -> 84, 1024 rows 68 -> 45.
+constexpr int PAIR_EPILOGUE = 8, PAIR_THREADS = 64 + 32 * PAIR_EPILOGUE;
+
 template <int BN, int STAGES, int ACCS>
 struct PairSmem {
   static constexpr int A_BYTES = BM * BK * 2;
   static constexpr int B_BYTES = (BN / 2) * BK * 2;
   static constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
   // Staging chunks per epilogue warp: two where shared memory allows, else one.
-  static constexpr int SBUF = STAGES * STAGE_BYTES + STAGING_BYTES + 1024 + 256 + ACCS * BN * 4 <= 227 * 1024 ? 2 : 1;
-  static constexpr int STAGING = SBUF * 4 * 4096;
-  static constexpr int TOTAL = STAGES * STAGE_BYTES + STAGING + 1024 /* alignment slack */ + 256 /* barriers */ + ACCS * BN * 4 /* bias */;
+  static constexpr int SBUF = STAGES * STAGE_BYTES + 2 * PAIR_EPILOGUE * 4096 + 1024 + 256 + BN * 4 <= 227 * 1024 ? 2 : 1;
+  static constexpr int STAGING = SBUF * PAIR_EPILOGUE * 4096;
+  static constexpr int TOTAL = STAGES * STAGE_BYTES + STAGING + 1024 /* alignment slack */ + 256 /* barriers */ + BN * 4 /* bias */;
   static_assert(TOTAL <= 227 * 1024, "stages, staging area and barriers fit shared memory");
 };
 
 template <int BN, int STAGES, int ACCS>
-__global__ void __launch_bounds__(192)
+__global__ void __launch_bounds__(PAIR_THREADS)
 gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_w,
                     const __grid_constant__ CUtensorMap map_out, int tma_out,
                     const void* __restrict__ bias, int bias_dtype, void* __restrict__ out, int out_dtype,
@@ -587,13 +592,13 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
   using S = PairSmem<BN, STAGES, ACCS>;
   extern __shared__ unsigned char smem_raw[];
   unsigned char* tiles = (unsigned char*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
-  unsigned char* staging = tiles + STAGES * S::STAGE_BYTES;      // [4 warps][SBUF][4 KB], 1024-byte aligned
+  unsigned char* staging = tiles + STAGES * S::STAGE_BYTES;      // [warps][SBUF][4 KB], 1024-byte aligned
   unsigned long long* full = (unsigned long long*)(staging + S::STAGING);
   unsigned long long* empty = full + STAGES;
   unsigned long long* acc_full = empty + STAGES;      // [ACCS]
   unsigned long long* acc_empty = acc_full + ACCS;    // [ACCS]
   unsigned* tmem_slot = (unsigned*)(acc_empty + ACCS);
-  float* bias_s = (float*)(staging + S::STAGING + 256);   // [ACCS][BN]
+  float* bias_s = (float*)(staging + S::STAGING + 256);   // [BN]
   static_assert(2 * STAGES * 8 + 2 * ACCS * 8 + 4 <= 256, "barriers fit their slot");
   static_assert(ACCS * BN <= 512 && BN % 128 == 0 && BN <= 256, "accumulators fit tensor memory, chunks of 128 divide them");
   static_assert(S::STAGE_BYTES % 1024 == 0, "the staging area stays 1024-byte aligned");
@@ -609,7 +614,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < STAGES; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
-    for (int a = 0; a < ACCS; ++a) { mbar_init(&acc_full[a], 1); mbar_init(&acc_empty[a], 8); }
+    for (int a = 0; a < ACCS; ++a) { mbar_init(&acc_full[a], 1); mbar_init(&acc_empty[a], 2 * PAIR_EPILOGUE); }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 2) {   // the same warp of both CTAs allocates (and frees) the pair's columns
@@ -678,17 +683,17 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
       }
     }
   } else {
-    const int quarter = warp & 3;
+    const int quarter = warp & 3, turn = (warp - 2) >> 2;
     int j = 0, chunk = 0;
     co_pdl_wait();   // out may still be in use by the predecessor
     for (int tile = pair; tile < num_tiles; tile += pairs, ++j) {
       const int acc = j % ACCS;
       const int m0 = (tile % tiles_m) * PM + (int)rank * BM, n0 = (tile / tiles_m) * BN;
       const int row = m0 + quarter * 32 + lane;
-      float* bias_t = bias_s + acc * BN;
       if (bias) {
-        for (int i = threadIdx.x - 64; i < BN; i += 128) bias_t[i] = n0 + i < N ? co_load_any(bias, bias_dtype, n0 + i) : 0.f;
-        asm volatile("bar.sync 1, 128;" ::: "memory");
+        if (j) asm volatile("bar.sync 1, %0;" ::"n"(32 * PAIR_EPILOGUE) : "memory");      // the last tile's has been read
+        for (int i = threadIdx.x - 64; i < BN; i += 32 * PAIR_EPILOGUE) bias_s[i] = n0 + i < N ? co_load_any(bias, bias_dtype, n0 + i) : 0.f;
+        asm volatile("bar.sync 1, %0;" ::"n"(32 * PAIR_EPILOGUE) : "memory");
       }
       if (!mbar_wait(&acc_full[acc], (unsigned)(j / ACCS) & 1)) {
         if (lane == 0) atomicExch(status, 13);
@@ -699,24 +704,24 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
         const int gated = co_gate_word(epilogue), act = co_plain_act(epilogue);
         const int step = gated ? 128 : 64;
 #pragma unroll 1
-        for (int c0 = 0; c0 < BN; c0 += step, ++chunk) {
+        for (int c0 = turn * step; c0 < BN; c0 += 2 * step, ++chunk) {
           if (n0 + c0 >= N) break;
           if (chunk >= S::SBUF) {   // the chunk that used this staging buffer has left it
             if (lane == 0) tma_store_wait_read<S::SBUF - 1>();
             __syncwarp();
           }
           store_chunk_tma(tmem_base + ((unsigned)(quarter * 32) << 16) + (unsigned)(acc * BN + c0),
-                          bias && !gated ? bias_t + c0 : nullptr, gated, act,
-                          staging + (quarter * S::SBUF + chunk % S::SBUF) * 4096, &map_out,
+                          bias && !gated ? bias_s + c0 : nullptr, gated, act,
+                          staging + ((warp - 2) * S::SBUF + chunk % S::SBUF) * 4096, &map_out,
                           gated ? (n0 + c0) >> 1 : n0 + c0, m0 + quarter * 32, lane);
         }
       } else {
 #pragma unroll 1
-        for (int c0 = 0; c0 < BN; c0 += 32) {
+        for (int c0 = 32 * turn; c0 < BN; c0 += 64) {
           if (n0 + c0 >= N) break;
           unsigned r[32];
           tmem_ld32(tmem_base + ((unsigned)(quarter * 32) << 16) + (unsigned)(acc * BN + c0), r);
-          if (row < M) store_piece(r, row, n0 + c0, bias ? bias_t + c0 : nullptr, out, out_dtype, N, ldo, epilogue);
+          if (row < M) store_piece(r, row, n0 + c0, bias ? bias_s + c0 : nullptr, out, out_dtype, N, ldo, epilogue);
         }
       }
       // This warp has read its part of the accumulator: tell the leader's MMA issuer.
@@ -1004,7 +1009,7 @@ int pair_slots() {
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(sms > 1 ? (sms & ~1) : 2);
-    cfg.blockDim = dim3(192);
+    cfg.blockDim = dim3(PAIR_THREADS);
     cfg.dynamicSmemBytes = smem;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -1032,7 +1037,7 @@ int launch_tc_pair(const CUtensorMap& mx, const CUtensorMap& mw, const void* bia
   const int pairs = (int)(tiles < slots ? tiles : slots);
   CUtensorMap mo = mx;
   const int tma_out = make_out_map(&mo, out, out_dtype, M, co_gate_word(epilogue) != EPI_PLAIN ? N / 2 : N, ldo) ? 1 : 0;
-  cudaError_t le = co_launch_cluster(2, kernel, dim3(2 * pairs), dim3(192), (size_t)smem, stream, mx, mw, mo, tma_out, bias, bias_dtype,
+  cudaError_t le = co_launch_cluster(2, kernel, dim3(2 * pairs), dim3(PAIR_THREADS), (size_t)smem, stream, mx, mw, mo, tma_out, bias, bias_dtype,
                                      out, out_dtype, M, N, K, ldo, epilogue, status);
   if (le != cudaSuccess) CO_FAIL("gemm_tc_pair: launch failed: %s", cudaGetErrorString(le));
   CO_CHECK_LAUNCH("gemm_tc_pair");
