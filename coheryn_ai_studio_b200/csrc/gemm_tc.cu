@@ -9,7 +9,7 @@
 //            issues the two TMA loads (x tile 128 x 64, W tile BN x 64);
 //   warp 1   MMA issuer: waits for a full stage, issues four m128 nBN k16 MMAs, and lets
 //            tcgen05.commit release the stage (and, after the last step, signal the epilogue);
-//   warps 2-5 epilogue: each reads its 32 lanes of the accumulator, applies bias or the gate
+//   warps 2-9 epilogue: each reads its 32 lanes of the accumulator, applies bias or the gate
 //            and converts.  bfloat16 output goes 64 columns at a time into a swizzled 4 KB
 //            staging buffer in shared memory (the stages are free by then) and leaves as a
 //            32 x 64 box through a TMA store, two boxes in flight per warp; float32 output
@@ -23,6 +23,11 @@ namespace {
 
 constexpr int BM = 128;          // tokens per tile = TMEM lanes
 constexpr int EPI_PLAIN = 0, EPI_GATED_SILU = 1;
+// Eight epilogue warps per CTA, two per quarter of its rows, that take the chunks of columns in turn.  With four (a warp a scheduler)
+// the gate's exponentials and divisions took longer than the 24 k-steps of the next tile at K = 1,536: measured on a B200, 2048 x 17920 x
+// 1536 gated by the pairs 108 -> 85 us (ungated 82), 1873 rows 120 -> 84, 1024 rows 68 -> 45; 800 rows by the
+// persistent kernel 55 -> 49, 513 rows 43 -> 38; 200 rows, one tile per CTA, 22.7 -> 18.7.  (Ungated products: no change.)
+constexpr int EPI_WARPS = 8, EPI_THREADS = 64 + 32 * EPI_WARPS;
 
 template <int BN, int STAGES>
 struct Smem {
@@ -80,10 +85,9 @@ __device__ __forceinline__ void store_chunk_tma(unsigned tmem_chunk, const float
     tma_store_commit();
   }
 }
-constexpr int STAGING_BYTES = 4 * 2 * 4096;   // four epilogue warps, two chunks each
 
 template <int BN, int STAGES>
-__global__ void __launch_bounds__(192)
+__global__ void __launch_bounds__(EPI_THREADS)
 gemm_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_w,
                const __grid_constant__ CUtensorMap map_out, int tma_out,
                const void* __restrict__ bias, int bias_dtype, void* __restrict__ out, int out_dtype, int M, int N,
@@ -159,12 +163,12 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
       umma_commit(accum_full);                  // arrives when every MMA issued so far is complete
     }
   } else {
-    // Epilogue warps 2..5: TMEM lane quarter = warp % 4.
-    const int quarter = warp & 3;
+    // Epilogue warps 2..9: TMEM lane quarter = warp % 4, two warps per quarter that take the chunks of columns in turn.
+    const int quarter = warp & 3, turn = (warp - 2) >> 2;
     const int row = m0 + quarter * 32 + lane;
     if (bias) {   // the tile's slice of the bias, once, while the main loop runs
-      for (int i = threadIdx.x - 64; i < BN; i += 128) bias_s[i] = n0 + i < N ? co_load_any(bias, bias_dtype, n0 + i) : 0.f;
-      asm volatile("bar.sync 1, 128;" ::: "memory");
+      for (int i = threadIdx.x - 64; i < BN; i += 32 * EPI_WARPS) bias_s[i] = n0 + i < N ? co_load_any(bias, bias_dtype, n0 + i) : 0.f;
+      asm volatile("bar.sync 1, %0;" ::"n"(32 * EPI_WARPS) : "memory");
     }
     co_pdl_wait();   // out (and the split workspace) may still be in use by the predecessor
     const bool waited = mbar_wait(accum_full, 0);
@@ -175,10 +179,11 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
       // stages are free and serve as the staging area (two 4 KB chunks per warp).
       const int gated = co_gate_word(epilogue), act = co_plain_act(epilogue);   // 0, or the gate's word; 0, or a plain activation
       const int step = gated ? 128 : 64;
-      unsigned char* stage = tiles + quarter * 8192;
+      unsigned char* stage = tiles + (warp - 2) * 8192;
+      static_assert(EPI_WARPS * 8192 <= STAGES * S::STAGE_BYTES, "the stages hold the staging area");
       int chunk = 0;
 #pragma unroll 1
-      for (int c0 = 0; c0 < BN; c0 += step, ++chunk) {
+      for (int c0 = turn * step; c0 < BN; c0 += 2 * step, ++chunk) {
         if (n0 + c0 >= N) break;
         if (chunk >= 2) {
           if (lane == 0) tma_store_wait_read<1>();
@@ -190,7 +195,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
       if (lane == 0) tma_store_wait_all();
     } else if (waited) {
 #pragma unroll 1
-      for (int c0 = 0; c0 < BN; c0 += 32) {
+      for (int c0 = 32 * turn; c0 < BN; c0 += 64) {
         if (n0 + c0 >= N) break;
         unsigned r[32];
         tmem_ld32(tmem_base + ((unsigned)(quarter * 32) << 16) + (unsigned)c0, r);
@@ -390,7 +395,7 @@ __global__ void splitk_reduce_kernel(const float* __restrict__ partial, int spli
 // let the epilogue of one tile run while the MMAs of the next are issued; the shared-memory
 // stages and their barriers simply keep cycling across tiles.
 template <int BN, int STAGES>
-__global__ void __launch_bounds__(192)
+__global__ void __launch_bounds__(EPI_THREADS)
 gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_w,
                           const void* __restrict__ bias, int bias_dtype, void* __restrict__ out, int out_dtype,
                           int M, int N, int K, long ldo, int epilogue, int* __restrict__ status) {
@@ -414,7 +419,7 @@ gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_x, const __gri
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < STAGES; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
-    for (int a = 0; a < 2; ++a) { mbar_init(&acc_full[a], 1); mbar_init(&acc_empty[a], 4); }
+    for (int a = 0; a < 2; ++a) { mbar_init(&acc_full[a], 1); mbar_init(&acc_empty[a], EPI_WARPS); }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 2) {
@@ -481,7 +486,7 @@ gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_x, const __gri
       }
     }
   } else {
-    const int quarter = warp & 3;
+    const int quarter = warp & 3, turn = (warp - 2) >> 2;
     int j = 0;
     co_pdl_wait();   // out may still be in use by the predecessor
     for (int tile = blockIdx.x; tile < num_tiles; tile += gridDim.x, ++j) {
@@ -490,8 +495,8 @@ gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_x, const __gri
       const int row = m0 + quarter * 32 + lane;
       float* bias_t = bias_s + acc * BN;
       if (bias) {
-        for (int i = threadIdx.x - 64; i < BN; i += 128) bias_t[i] = n0 + i < N ? co_load_any(bias, bias_dtype, n0 + i) : 0.f;
-        asm volatile("bar.sync 1, 128;" ::: "memory");
+        for (int i = threadIdx.x - 64; i < BN; i += 32 * EPI_WARPS) bias_t[i] = n0 + i < N ? co_load_any(bias, bias_dtype, n0 + i) : 0.f;
+        asm volatile("bar.sync 1, %0;" ::"n"(32 * EPI_WARPS) : "memory");
       }
       if (!mbar_wait(&acc_full[acc], (unsigned)(j >> 1) & 1)) {
         if (lane == 0) atomicExch(status, 13);
@@ -499,7 +504,7 @@ gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_x, const __gri
       }
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 #pragma unroll 1
-      for (int c0 = 0; c0 < BN; c0 += 32) {
+      for (int c0 = 32 * turn; c0 < BN; c0 += 64) {
         if (n0 + c0 >= N) break;
         unsigned r[32];
         tmem_ld32(tmem_base + ((unsigned)(quarter * 32) << 16) + (unsigned)(acc * BN + c0), r);
@@ -531,7 +536,7 @@ gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_x, const __gri
 //                 the peer's TMA loads complete on it (cp.async.bulk.tensor ... cta_group::2);
 //   empty[s]      in each CTA: the leader's tcgen05.commit arrives on both (multicast);
 //   acc_full[a]   in each CTA: likewise, after a tile's last MMA;
-//   acc_empty[a]  in the leader: the eight epilogue warps of both CTAs arrive on it.
+//   acc_empty[a]  in the leader: the epilogue warps of both CTAs arrive on it.
 // The pair walks the tiles t = pair, pair + pairs, ... (row tiles fastest) with two accumulators.
 __device__ __forceinline__ unsigned cluster_ctarank() { unsigned r; asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r)); return r; }
 __device__ __forceinline__ unsigned map_to_cta(const void* local, unsigned rank) {
@@ -566,25 +571,20 @@ __device__ __forceinline__ void mbar_arrive_cluster(unsigned bar_cluster_addr) {
   asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar_cluster_addr) : "memory");
 }
 
-// Eight epilogue warps per CTA, two per quarter of its rows, that take the chunks of columns in turn.  With four (a warp a scheduler)
-// the gate's exponentials and divisions took longer than the 24 k-steps of the next tile at K = 1,536: measured on a B200, 2048 x 17920 x
-// 1536 gated 108 -> 85 us (ungated 82), 1873 rows 120 -> 84, 1024 rows 68 -> 45.
-constexpr int PAIR_EPILOGUE = 8, PAIR_THREADS = 64 + 32 * PAIR_EPILOGUE;
-
 template <int BN, int STAGES, int ACCS>
 struct PairSmem {
   static constexpr int A_BYTES = BM * BK * 2;
   static constexpr int B_BYTES = (BN / 2) * BK * 2;
   static constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
   // Staging chunks per epilogue warp: two where shared memory allows, else one.
-  static constexpr int SBUF = STAGES * STAGE_BYTES + 2 * PAIR_EPILOGUE * 4096 + 1024 + 256 + BN * 4 <= 227 * 1024 ? 2 : 1;
-  static constexpr int STAGING = SBUF * PAIR_EPILOGUE * 4096;
+  static constexpr int SBUF = STAGES * STAGE_BYTES + 2 * EPI_WARPS * 4096 + 1024 + 256 + BN * 4 <= 227 * 1024 ? 2 : 1;
+  static constexpr int STAGING = SBUF * EPI_WARPS * 4096;
   static constexpr int TOTAL = STAGES * STAGE_BYTES + STAGING + 1024 /* alignment slack */ + 256 /* barriers */ + BN * 4 /* bias */;
   static_assert(TOTAL <= 227 * 1024, "stages, staging area and barriers fit shared memory");
 };
 
 template <int BN, int STAGES, int ACCS>
-__global__ void __launch_bounds__(PAIR_THREADS)
+__global__ void __launch_bounds__(EPI_THREADS)
 gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_w,
                     const __grid_constant__ CUtensorMap map_out, int tma_out,
                     const void* __restrict__ bias, int bias_dtype, void* __restrict__ out, int out_dtype,
@@ -614,7 +614,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < STAGES; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
-    for (int a = 0; a < ACCS; ++a) { mbar_init(&acc_full[a], 1); mbar_init(&acc_empty[a], 2 * PAIR_EPILOGUE); }
+    for (int a = 0; a < ACCS; ++a) { mbar_init(&acc_full[a], 1); mbar_init(&acc_empty[a], 2 * EPI_WARPS); }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 2) {   // the same warp of both CTAs allocates (and frees) the pair's columns
@@ -691,9 +691,9 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
       const int m0 = (tile % tiles_m) * PM + (int)rank * BM, n0 = (tile / tiles_m) * BN;
       const int row = m0 + quarter * 32 + lane;
       if (bias) {
-        if (j) asm volatile("bar.sync 1, %0;" ::"n"(32 * PAIR_EPILOGUE) : "memory");      // the last tile's has been read
-        for (int i = threadIdx.x - 64; i < BN; i += 32 * PAIR_EPILOGUE) bias_s[i] = n0 + i < N ? co_load_any(bias, bias_dtype, n0 + i) : 0.f;
-        asm volatile("bar.sync 1, %0;" ::"n"(32 * PAIR_EPILOGUE) : "memory");
+        if (j) asm volatile("bar.sync 1, %0;" ::"n"(32 * EPI_WARPS) : "memory");      // the last tile's has been read
+        for (int i = threadIdx.x - 64; i < BN; i += 32 * EPI_WARPS) bias_s[i] = n0 + i < N ? co_load_any(bias, bias_dtype, n0 + i) : 0.f;
+        asm volatile("bar.sync 1, %0;" ::"n"(32 * EPI_WARPS) : "memory");
       }
       if (!mbar_wait(&acc_full[acc], (unsigned)(j / ACCS) & 1)) {
         if (lane == 0) atomicExch(status, 13);
@@ -958,7 +958,7 @@ int launch_tc(const CUtensorMap& mx, const CUtensorMap& mw, const void* bias, in
   const int k_per_split = partial ? (k_tiles + splits - 1) / splits : k_tiles;
   const int used = partial ? (k_tiles + k_per_split - 1) / k_per_split : 1;    // no split is left empty
   dim3 grid((N + BN - 1) / BN, (M + BM - 1) / BM, used);
-  cudaError_t le = co_launch(kernel, grid, dim3(192), (size_t)smem, stream, mx, mw, mo, tma_out, bias, bias_dtype, out, out_dtype, M, N,
+  cudaError_t le = co_launch(kernel, grid, dim3(EPI_THREADS), (size_t)smem, stream, mx, mw, mo, tma_out, bias, bias_dtype, out, out_dtype, M, N,
                              K, ldo, epilogue, status, used > 1 ? partial : (float*)nullptr, k_per_split);
   if (le != cudaSuccess) CO_FAIL("gemm_tc: launch failed: %s", cudaGetErrorString(le));
   CO_CHECK_LAUNCH("gemm_tc");
@@ -989,7 +989,7 @@ int launch_tc_persistent(const CUtensorMap& mx, const CUtensorMap& mw, const voi
   }
   const long tiles = (long)((N + BN - 1) / BN) * ((M + BM - 1) / BM);
   const int grid = (int)(tiles < sms ? tiles : sms);
-  cudaError_t le = co_launch(kernel, dim3(grid), dim3(192), (size_t)smem, stream, mx, mw, bias, bias_dtype, out,
+  cudaError_t le = co_launch(kernel, dim3(grid), dim3(EPI_THREADS), (size_t)smem, stream, mx, mw, bias, bias_dtype, out,
                              out_dtype, M, N, K, ldo, epilogue, status);
   if (le != cudaSuccess) CO_FAIL("gemm_tc: launch failed: %s", cudaGetErrorString(le));
   CO_CHECK_LAUNCH("gemm_tc_persistent");
@@ -1009,7 +1009,7 @@ int pair_slots() {
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(sms > 1 ? (sms & ~1) : 2);
-    cfg.blockDim = dim3(PAIR_THREADS);
+    cfg.blockDim = dim3(EPI_THREADS);
     cfg.dynamicSmemBytes = smem;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -1037,7 +1037,7 @@ int launch_tc_pair(const CUtensorMap& mx, const CUtensorMap& mw, const void* bia
   const int pairs = (int)(tiles < slots ? tiles : slots);
   CUtensorMap mo = mx;
   const int tma_out = make_out_map(&mo, out, out_dtype, M, co_gate_word(epilogue) != EPI_PLAIN ? N / 2 : N, ldo) ? 1 : 0;
-  cudaError_t le = co_launch_cluster(2, kernel, dim3(2 * pairs), dim3(PAIR_THREADS), (size_t)smem, stream, mx, mw, mo, tma_out, bias, bias_dtype,
+  cudaError_t le = co_launch_cluster(2, kernel, dim3(2 * pairs), dim3(EPI_THREADS), (size_t)smem, stream, mx, mw, mo, tma_out, bias, bias_dtype,
                                      out, out_dtype, M, N, K, ldo, epilogue, status);
   if (le != cudaSuccess) CO_FAIL("gemm_tc_pair: launch failed: %s", cudaGetErrorString(le));
   CO_CHECK_LAUNCH("gemm_tc_pair");
