@@ -32,7 +32,7 @@ CORE_SOURCES = ["runtime.cu", "elementwise.cu", "gemm_simt.cu", "attention_simpl
                 "sampling.cu", "gemm_bf16_small.cu", "gemm_tc.cu", "gemm_tc_few.cu", "gemm_f32_tc.cu", "seeded_fill.cu", "selftest.cu",
                 "block_runner.cu", "mixer_runner.cu", "stream_ops.cu"]
 ROUTED_SOURCES = ["routed.cu", "runtime.cu"]
-RECURRENT_SOURCES = ["recurrent.cu", "recurrent_one.cu", "delta_chunks.cu", "memory_chunks.cu", "runtime.cu"]
+RECURRENT_SOURCES = ["recurrent.cu", "recurrent_one.cu", "delta_chunks.cu", "memory_chunks.cu", "memory_chunks_tc.cu", "runtime.cu"]
 VARIANT_SOURCES = ["attention_variants.cu", "runtime.cu"]
 LINEAR_RECURRENCE_SOURCES = ["linear_recurrence.cu", "runtime.cu"]
 LINEAR_ATTENTION_SOURCES = ["linear_attention.cu", "runtime.cu"]

@@ -47,19 +47,6 @@ struct F32Tile {
   static_assert(COLS_USED <= 512 && PART % 16 == 0, "tensor memory");
 };
 
-// v0 + v1 + v2 = v for a pair of neighbouring values, as packed bfloat16 pairs (the first value in the low half): v0 and v1 the
-// nearest (halves away from zero) of the value and of the rest, v2 what is left, which has at most eight bits.  Integer operations: the
-// conversion instructions go through the narrow pipe of the special functions, which three per pair would keep busy for a third of the time.
-__device__ __forceinline__ void split3(float a, float b, unsigned& t0, unsigned& t1, unsigned& t2) {
-  const unsigned a0 = (__float_as_uint(a) + 0x8000u) & 0xffff0000u, b0 = (__float_as_uint(b) + 0x8000u) & 0xffff0000u;
-  a -= __uint_as_float(a0);
-  b -= __uint_as_float(b0);
-  const unsigned a1 = (__float_as_uint(a) + 0x8000u) & 0xffff0000u, b1 = (__float_as_uint(b) + 0x8000u) & 0xffff0000u;
-  t0 = __byte_perm(a0, b0, 0x7632);
-  t1 = __byte_perm(a1, b1, 0x7632);
-  t2 = __byte_perm(__float_as_uint(a - __uint_as_float(a1)), __float_as_uint(b - __uint_as_float(b1)), 0x7632);
-}
-
 // The three terms of x as [3][M][pitch] bfloat16, pitch = K rounded up to eight; a thread takes eight values of a row.
 template <bool VEC>
 __global__ void __launch_bounds__(256) split_rows_kernel(const float* __restrict__ x, long ldx, int M, int K, int pitch, uint4* __restrict__ terms) {

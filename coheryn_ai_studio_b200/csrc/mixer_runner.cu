@@ -29,7 +29,8 @@ typedef int (*co_memory_fn)(const float* q, const float* k, const float* v, long
                             const void* bias_i, const void* bias_f, int bias_dtype, float cap, float* state, long state_stride,
                             const int* cu_q, const int* state_slots, int B, int heads, int dk, int dv, void* out, int out_dtype, long ldo,
                             const void* weight, int weight_dtype, int weight_stride, const float* gate, long ldg, float eps, float out_scale,
-                            int total_tokens, float* scratch, long scratch_floats, int chunks, int runs, int short_runs, cudaStream_t stream);
+                            int total_tokens, float* scratch, long scratch_floats, int chunks, int runs, int short_runs, int* status,
+                            cudaStream_t stream);
 typedef long (*co_chunk_floats_fn)(int chunks, int heads, int dk, int dv);
 typedef int (*co_chunks_pay_fn)(int heads, int dk, int dv, int B, int T, int longest, int chunks);
 
@@ -135,7 +136,7 @@ int mixer_pass(const CoMixerLayer& L, const CoMixerStep& S, const CoBlockTuning&
     float* area = floats ? (float*)A.take((size_t)floats * 4) : nullptr;
     RUN_RECURRENT(L.memory(proj + L.at_q, proj + L.at_k, proj + L.at_v, L.columns, proj + L.at_a, proj + L.at_b, L.columns, L.bias_a, L.bias_b,
                            L.bias_a_dtype, L.cap, state, state_stride, S.cu_q, S.state_slots, B, H, dk, dv, o, CO_BF16, ldo, L.norm_w, L.norm_dtype,
-                           dv, proj + L.at_g, L.columns, L.eps, L.out_scale, T, area, floats, r.chunks, r.runs, r.rest, S.stream));
+                           dv, proj + L.at_g, L.columns, L.eps, L.out_scale, T, area, floats, r.chunks, r.runs, r.rest, S.tc_status, S.stream));
   } else {
     const int G = L.kv_heads, C = 2 * G * dk + H * dv;
     float* qkv = (float*)A.take((size_t)T * C * 4);

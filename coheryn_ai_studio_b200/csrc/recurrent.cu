@@ -981,7 +981,8 @@ CO_EXPORT int coheryn_matrix_memory_scan(
     const void* bias_i, const void* bias_f, int bias_dtype, float cap, float* state, long state_stride, const int* cu_q,
     const int* state_slots, int B, int heads, int dk, int dv, void* out, int out_dtype, long ldo, const void* weight,
     int weight_dtype, int weight_stride, const float* gate, long ldg, float eps, float out_scale, int total_tokens,
-    float* scratch, long scratch_floats, int chunks, int runs, int short_runs, cudaStream_t stream) {
+    float* scratch, long scratch_floats, int chunks, int runs, int short_runs, int* status,
+    cudaStream_t stream) {
   if (B <= 0) return 0;
   if (!scan_shape_ok("matrix_memory_scan", heads, dk, dv)) return 1;
   if (!(cap > 0.f)) CO_FAIL("matrix_memory_scan: the gate cap must be positive");
@@ -993,7 +994,8 @@ CO_EXPORT int coheryn_matrix_memory_scan(
             slices > 1 ? scratch : nullptr, (long)heads * dv, slices > 1 ? scratch + (long)total_tokens * heads * dv : nullptr};
   if (one) return co_memory_one(P, E, B, stream);
   if (chunked) {
-    if (co_memory_chunks(P, E, B, chunks, runs, scratch, stream)) return 1;
+    if (!status) CO_FAIL("matrix_memory_scan: runs in chunks need a status word");
+    if (co_memory_chunks(P, E, B, chunks, runs, scratch, status, stream)) return 1;
     if (!short_runs) return 0;
   }
   const int below = chunked ? CHUNK_FROM : 0x7fffffff;

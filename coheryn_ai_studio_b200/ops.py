@@ -1243,7 +1243,7 @@ def matrix_memory_scan(q, k, v, gate_i, gate_f, bias_i, bias_f, cap: float, stat
         _ptr(step.state_slots), c_int(step.num_requests), c_int(heads), c_int(dk), c_int(dv), _ptr(out), c_int(_code(out)),
         c_long(out.stride(0)), _ptr(norm_weight), c_int(_code(norm_weight)), c_int(dv), _ptr(gate), c_long(gate.stride(0)),
         c_float(eps), c_float(out_scale), c_int(q.shape[0]), _ptr(scratch), c_long(scratch.numel() if scratch is not None else 0),
-        c_int(chunks), c_int(runs), c_int(1 if rest else 0), _stream()))
+        c_int(chunks), c_int(runs), c_int(1 if rest else 0), _ptr(tc_status(q.device)), _stream()))
 
 
 def qk_norm_kv_write(q, k, v, q_weight, k_weight, eps: float, slots, k_cache, v_cache, num_heads: int, num_kv_heads: int,
