@@ -134,7 +134,6 @@ __global__ void __launch_bounds__(THREADS, 3) delta_chunk_kernel(DeltaIn P, int 
   float* As = iks + CH;                 // [64][17] the sums of A inside the blocks, of B
   float* Bs = As + CH * 17;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  co_pdl_launch_dependents();
   co_pdl_wait();
   const int h = blockIdx.y, dk = P.dk;
   Run R;
@@ -333,7 +332,6 @@ __global__ void __launch_bounds__(THREADS, 3) delta_solve_kernel(DeltaIn P, int 
   float* betas = Ys + CH * DKP;         // [64]
   float* Ms = betas + CH;               // [3][16][16]
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  co_pdl_launch_dependents();
   co_pdl_wait();
   const int h = blockIdx.y, dv = P.dv;
   Run R;
@@ -448,7 +446,6 @@ __global__ void __launch_bounds__(STATE_THREADS, 1) delta_state_kernel(DeltaIn P
   float* U = S + DK * VS;                       // [64][16]
   float* part = U + CH * VS;                    // [8][64][16], then [KG][DK][16]
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  co_pdl_launch_dependents();
   co_pdl_wait();
   const int h = blockIdx.y, c0 = blockIdx.x * VS, dk = P.dk, dv = P.dv;
   Run R;
@@ -561,7 +558,6 @@ __global__ void __launch_bounds__(THREADS) delta_out_kernel(DeltaIn P, HeadOut E
   extern __shared__ __align__(16) float sm[];
   float* os = dvp <= W ? sm : sm + 2 * STAGE;   // [64][dvp + 4]
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  co_pdl_launch_dependents();
   co_pdl_wait();
   const int h = blockIdx.y;
   Run R;

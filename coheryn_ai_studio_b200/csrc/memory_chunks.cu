@@ -38,7 +38,6 @@ __device__ __forceinline__ void st4(float* p, float4 v) { *reinterpret_cast<floa
 // head that walked the chunks from beginning to end took 30 us for 32 of them).
 constexpr int GATE_WARPS = 16;
 __global__ void __launch_bounds__(32 * GATE_WARPS) memory_gates_kernel(MemoryIn P, int B, int base, int count, Area A) {
-  co_pdl_launch_dependents();
   co_pdl_wait();
   const int h = blockIdx.y, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   Run R;
@@ -130,7 +129,6 @@ __global__ void __launch_bounds__(32 * GATE_WARPS) memory_gates_kernel(MemoryIn 
 // grid (ceil(size / 1024), heads, runs), 256 threads of four neighbouring elements each; the chunks ahead are requested eight at
 // a time.
 __global__ void __launch_bounds__(256) memory_carry_kernel(MemoryIn P, int B, int base, int count, Area A) {
-  co_pdl_launch_dependents();
   co_pdl_wait();
   const int h = blockIdx.y, dk = P.dk, dv = P.dv;
   Run R;

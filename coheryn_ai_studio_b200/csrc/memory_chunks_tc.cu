@@ -129,7 +129,6 @@ __global__ void __launch_bounds__(32 * (4 * HALVES + 1)) memory_sum_tc_kernel(Me
   unsigned char* ks = (unsigned char*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);      // [3][2][64 tokens][64 channels]
   co_pdl_wait();
   const unsigned tmem = begin(bars, WORKERS, COLUMNS);
-  co_pdl_launch_dependents();      // behind the allocation, as below
   const int h = blockIdx.y, dk = P.dk, dv = P.dv, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   Run R;
   if (!find_run(P.cu_q, B, base + blockIdx.x, false, R)) { end(tmem, COLUMNS); return; }
@@ -278,7 +277,6 @@ __global__ void __launch_bounds__(32 * (4 * HALVES + 1)) memory_out_tc_kernel(Me
   unsigned char* ps = first + blocks * 3 * TILE;            // behind q's tiles
   float* gates = scores + CH * (CH + 4);                    // [token][dvp]
   const unsigned tmem = begin(bars, WORKERS, 512);
-  co_pdl_launch_dependents();      // behind the allocation: a successor's CTA that took the columns first would wait for this kernel's end
   co_pdl_wait();
   const int h = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   Run R;

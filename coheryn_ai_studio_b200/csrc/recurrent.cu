@@ -61,7 +61,6 @@ short_conv_silu_run_kernel(const float* __restrict__ x, long ldx, float* __restr
                            int taps_dtype, int C, const float* __restrict__ state, long state_stride,
                            const int* __restrict__ token_req, const int* __restrict__ cu_q, const int* __restrict__ state_slots, int T, int per) {
   const int c = (blockIdx.x * 128 + threadIdx.x) * W;
-  co_pdl_launch_dependents();
   float w[N][W];
   if (c < C) {
 #pragma unroll
@@ -114,7 +113,6 @@ short_conv_silu_run_kernel(const float* __restrict__ x, long ldx, float* __restr
 __global__ void short_conv_state_kernel(const float* __restrict__ x, long ldx, int n, int C, float* __restrict__ state,
                                         long state_stride, const int* __restrict__ cu_q,
                                         const int* __restrict__ state_slots, int B) {
-  co_pdl_launch_dependents();
   co_pdl_wait();
   const size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= (size_t)B * C) return;
@@ -295,7 +293,6 @@ __global__ void __launch_bounds__(512) gated_delta_scan_kernel(DeltaIn P, HeadOu
   using L = ScanShape<DK, SPLIT>;
   constexpr int DP = L::DP, ROW = L::ROW;
   extern __shared__ __align__(16) float smem[];
-  co_pdl_launch_dependents();
   co_pdl_wait();
   const int r = blockIdx.x, h = blockIdx.y;
   const int part = threadIdx.x % SPLIT, col0 = (threadIdx.x / SPLIT) * CP, d0 = part * DP;
@@ -407,7 +404,6 @@ __global__ void __launch_bounds__(512) gated_delta_scan_pre_kernel(DeltaIn P, He
   using L = ScanShape<DK, SPLIT>;
   constexpr int DP = L::DP, ROW = L::ROW;
   extern __shared__ __align__(16) float smem[];
-  co_pdl_launch_dependents();
   co_pdl_wait();
   const int r = blockIdx.x, h = blockIdx.y;
   const int part = threadIdx.x % SPLIT, col0 = (threadIdx.x / SPLIT) * CP, d0 = part * DP;
@@ -543,7 +539,6 @@ __global__ void __launch_bounds__(512) matrix_memory_scan_kernel(MemoryIn P, Hea
   using L = ScanShape<DK, SPLIT>;
   constexpr int DP = L::DP, ROW = L::ROW;
   extern __shared__ __align__(16) float smem[];
-  co_pdl_launch_dependents();
   co_pdl_wait();
   const int r = blockIdx.x, h = blockIdx.y;
   const int part = threadIdx.x % SPLIT, col0 = (threadIdx.x / SPLIT) * CP, d0 = part * DP;
@@ -677,7 +672,6 @@ __global__ void __launch_bounds__(512) matrix_memory_scan_pre_kernel(MemoryIn P,
   using L = ScanShape<DK, SPLIT>;
   constexpr int DP = L::DP, ROW = L::ROW;
   extern __shared__ __align__(16) float smem[];
-  co_pdl_launch_dependents();
   co_pdl_wait();
   const int r = blockIdx.x, h = blockIdx.y;
   const int part = threadIdx.x % SPLIT, col0 = (threadIdx.x / SPLIT) * CP, d0 = part * DP;

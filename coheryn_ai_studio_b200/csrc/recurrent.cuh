@@ -63,6 +63,13 @@ long co_memory_chunk_floats(int chunks, int heads, int dk, int dv);
 // `status`: device word that receives a code if a bounded wait for the tensor cores ran out.
 int co_memory_chunks(const MemoryIn& P, const HeadOut& E, int B, int chunks, int runs, float* scratch, int* status, cudaStream_t stream);
 
+// No co_pdl_launch_dependents() in the kernels of the scans and chunks and in the convolution in front of them: a successor that is
+// launched ahead only sits beside them, and its early CTAs take SMs out of turn (several of them on one SM where another stands empty).
+// Their successors start when they end.  Measured on a B200, whole mixers, launched ahead and not: delta rule, 16 heads of 64 x 64,
+// runs of 9, 3, 263 and 217 tokens 163 and 131 us, 12 heads of 128 x 128, one run of 360 196 and 184, of 2,048 402 and 393; matrix
+// memory, 8 heads of 128 x 256, runs of 400, 30 and 7 207 and 188.  Steps of a token per request (recurrent_one.cu) are too short for
+// that and launch ahead.
+
 // Lanes per group of columns and columns per group.  The more lanes share a column, the fewer steps a token costs
 // each of them (the recurrence is a chain of dependent steps, and that chain is what bounds a long prompt): sixteen
 // from 128 key channels on, eight from 64, four below.  Four columns per group (two for narrow heads); a head of more
