@@ -99,6 +99,7 @@ struct F32Args {
   int* status;
 };
 
+// (Its successor starts at its end: launched ahead, the block of 512 tokens of 1536 x 8960 took 324 us in place of 316.)
 template <int BT>
 __global__ void __launch_bounds__(448, 1)
 gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x, const F32Args P) {
@@ -134,7 +135,6 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const unsigned tmem = *tmem_slot;
-  co_pdl_launch_dependents();
 
   if (warp == 0) {
     if (lane == 0) {
