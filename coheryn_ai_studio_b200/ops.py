@@ -1127,6 +1127,15 @@ def _f32(t: torch.Tensor, name: str) -> None:
         raise KernelError(f"{name} must be float32 with contiguous rows")
 
 
+def _step_fits(step, T: int) -> None:
+    """The step's arrays must cover its requests and tokens: the kernels read them by those counts alone."""
+    if step.cu_q.numel() <= step.num_requests or step.state_slots.numel() < step.num_requests:
+        raise KernelError(f"the step's arrays do not cover its {step.num_requests} requests")
+    token_req = getattr(step, "token_req", None)
+    if token_req is not None and token_req.numel() < T:
+        raise KernelError(f"the step's array of requests does not cover {T} tokens")
+
+
 def _scan_scratch(T: int, B: int, heads: int, dv: int, extra: int, device):
     """Scratch for a scan that may split the columns of its heads over several CTAs (a long prompt of few requests; the
     library decides by the same numbers): the unnormalised outputs, then ``extra`` floats.  None when it will not."""
@@ -1161,7 +1170,7 @@ def short_conv_silu(x: torch.Tensor, taps: torch.Tensor, state: torch.Tensor, st
     step's first token come from ``state`` (a float32 view [slots, (n-1) * C] whose rows may be strided), which then
     receives the last n-1 inputs.  ``x`` float32 [T, C] (a column slice is fine); returns float32 [T, C]."""
     _dev(x, taps, state, step.token_req, step.cu_q, step.state_slots)
-    _f32(x, "x"); _f32(state, "state")
+    _f32(x, "x"); _f32(state, "state"); _step_fits(step, x.shape[0])
     T, C = x.shape
     n = taps.shape[1]
     assert taps.shape == (C, n) and taps.is_contiguous() and state.shape[1] == (n - 1) * C
@@ -1187,6 +1196,7 @@ def gated_delta_scan(q, k, v, beta, step_pre, step_bias, rate_log, state, step, 
     _dev(q, k, v, beta, step_pre, step_bias, rate_log, state, out, norm_weight, gate)
     for t, name in ((q, "q"), (k, "k"), (v, "v"), (beta, "beta"), (step_pre, "step"), (state, "state"), (gate, "gate")):
         _f32(t, name)
+    _step_fits(step, q.shape[0])
     assert q.stride(0) == k.stride(0) == v.stride(0)
     assert q.shape[1] == kv_heads * dk and k.shape[1] == kv_heads * dk and v.shape[1] == heads * dv
     dc = dk if decay_per_channel else 1
@@ -1223,6 +1233,7 @@ def matrix_memory_scan(q, k, v, gate_i, gate_f, bias_i, bias_f, cap: float, stat
     _dev(q, k, v, gate_i, gate_f, bias_i, bias_f, state, out, norm_weight, gate)
     for t, name in ((q, "q"), (k, "k"), (v, "v"), (gate_i, "gate_i"), (gate_f, "gate_f"), (state, "state"), (gate, "gate")):
         _f32(t, name)
+    _step_fits(step, q.shape[0])
     assert q.stride(0) == k.stride(0) == v.stride(0) and gate_i.stride(0) == gate_f.stride(0)
     assert q.shape[1] == heads * dk and k.shape[1] == heads * dk and v.shape[1] == heads * dv
     assert gate_i.shape[1] == heads and gate_f.shape[1] == heads and gate.shape[1] == heads * dv

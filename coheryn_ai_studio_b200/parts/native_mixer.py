@@ -50,14 +50,23 @@ def _entry_point():
     return _entry
 
 
-def _i32(*tensors) -> bool:
-    return all(t is not None and t.dtype == torch.int32 and t.is_cuda and t.is_contiguous() for t in tensors)
+def _i32(device, *sized) -> bool:
+    """Whether every (tensor, entries it must have) is a contiguous int32 tensor on ``device``."""
+    return all(t is not None and t.dtype == torch.int32 and t.device == device and t.is_contiguous() and t.numel() >= n for t, n in sized)
+
+
+def shapes_fit(specs, tensors) -> bool:
+    """Whether every tensor has the shape that its specification names (-1: any size).  The library takes sizes from the part's
+    description alone, so a tensor of another size must not reach it."""
+    return all(t.dim() == len(specs[n].shape) and all(want in (-1, got) for want, got in zip(specs[n].shape, t.shape))
+               for n, t in tensors.items() if n in specs)
 
 
 class NativeMixer:
-    """``fields``: what ``CoMixerLayer`` holds beside the pointers; ``tensors``: its tensors by field (kept alive here)."""
+    """``fields``: what ``CoMixerLayer`` holds beside the pointers; ``tensors``: its tensors by field (kept alive here);
+    ``state_width``: floats of a request's state."""
 
-    def __init__(self, fields: dict, tensors: dict, memory: bool):
+    def __init__(self, fields: dict, tensors: dict, memory: bool, state_width: int):
         lib = ops.recurrent()
         fn = lambda f: ctypes.cast(f, c_void_p).value
         code = lambda t: ops._code(t) if t is not None else ops.F32
@@ -68,31 +77,38 @@ class NativeMixer:
                                   chunks_pay=fn(lib.coheryn_memory_chunks_pay if memory else lib.coheryn_delta_chunks_pay),
                                   chunk_from=lib.chunk_from, chunk_tokens=lib.chunk_tokens, conv_dtype=code(tensors.get("conv_w")),
                                   bias_a_dtype=code(tensors["bias_a"]), bias_b_dtype=code(tensors["bias_b"]), norm_dtype=code(tensors["norm_w"]))
-        self.tensors, self.lib = tensors, lib
+        self.tensors, self.lib, self.device, self.state_width = tensors, lib, tensors["w_in"].device, state_width
         self.layer_ref = ctypes.addressof(self.layer)
 
     @classmethod
-    def build(cls, fields: dict, tensors: dict, memory: bool) -> Optional["NativeMixer"]:
-        """None when a tensor is not as the library's sequence takes it."""
+    def build(cls, fields: dict, tensors: dict, memory: bool, state_width: int) -> Optional["NativeMixer"]:
+        """None when a tensor is not as the library's sequence takes it (its shapes are the caller's to check: ``shapes_fit``)."""
+        if len({t.device for t in tensors.values() if t is not None}) != 1:
+            return None
         matrices = [tensors[n] for n in ("w_in", "w_second", "w_o") if tensors.get(n) is not None]
         if any(not t.is_cuda or t.dtype != torch.bfloat16 or not t.is_contiguous() for t in matrices):
             return None
         vectors = [tensors[n] for n in ("conv_w", "bias_a", "bias_b", "norm_w") if tensors.get(n) is not None]
         if any(not t.is_cuda or t.dtype not in (torch.bfloat16, torch.float32) or not t.is_contiguous() for t in vectors):
             return None
-        return cls(fields, tensors, memory)
+        return cls(fields, tensors, memory, state_width)
 
     def run(self, x: torch.Tensor, step, state: torch.Tensor, opened: Optional[torch.Tensor], out: Optional[torch.Tensor]) -> bool:
         """The mixer on ``x``, continued from and left in ``state``: the activations in front of the output product into ``opened``
-        (bfloat16) and / or the output into ``out`` (float32 [T, width])."""
+        (bfloat16) and / or the output into ``out`` (float32 [T, width]).  Everything is compared with the part's sizes first; what does
+        not fit is left to the part's own path, whose operations check it again and raise."""
         L, T, B = self.layer, x.shape[0], step.num_requests
         width = L.heads * L.dv
-        if (x.dtype != torch.bfloat16 or not x.is_cuda or x.shape[1] != L.width or x.stride(1) != 1 or state.dtype != torch.float32
-                or state.stride(1) != 1 or not _i32(getattr(step, "token_req", None), step.cu_q, step.state_slots)):
+        if x.dtype != torch.bfloat16 or x.device != self.device or x.dim() != 2 or x.shape[1] != L.width or x.stride(1) != 1:
             return False
-        if opened is not None and (opened.dtype != torch.bfloat16 or opened.shape != (T, width) or opened.stride(1) != 1):
+        if (state.dtype != torch.float32 or state.device != self.device or state.dim() != 2 or state.shape[1] != self.state_width
+                or state.stride(1) != 1):
             return False
-        if out is not None and (out.dtype != torch.float32 or out.shape != (T, L.width) or not out.is_contiguous()):
+        if not _i32(self.device, (getattr(step, "token_req", None), T), (step.cu_q, B + 1), (step.state_slots, B)):
+            return False
+        if opened is not None and (opened.dtype != torch.bfloat16 or opened.device != self.device or opened.shape != (T, width) or opened.stride(1) != 1):
+            return False
+        if out is not None and (out.dtype != torch.float32 or out.device != self.device or out.shape != (T, L.width) or not out.is_contiguous()):
             return False
         lens = None
         if L.in_chunks and T - B + 1 >= L.chunk_from:      # (else no run is as long)

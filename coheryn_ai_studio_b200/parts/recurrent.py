@@ -45,7 +45,7 @@ from .. import ops
 from ..config.spec import PartSpec
 from ..weights.spec import TensorSpec
 from .base import MIXERS, POSITIONS, FixedState, LayerCache, Mixer, NormedSum, Runtime, StepContext, build_part, register_mixer
-from .native_mixer import NativeMixer
+from .native_mixer import NativeMixer, shapes_fit
 
 
 class _StackedInput:
@@ -77,13 +77,13 @@ class _StateMixer(Mixer):
         self.in_chunks = runtime.dtype != torch.float32
         self.native = None      # the whole mixer by one call into the library: made when the weights are bound
 
-    def _bind_native(self, memory: bool, names, **fields_and_tensors) -> None:
-        """``names``: the fields that hold tensors."""
+    def _bind_native(self, bound, memory: bool, names, **fields_and_tensors) -> None:
+        """``bound``: the part's tensors as they were handed to it; ``names``: the fields that hold tensors."""
         self.native = None
-        if self.runtime.dtype == torch.bfloat16 and self.w_o.is_cuda:
+        if self.runtime.dtype == torch.bfloat16 and self.w_o.is_cuda and shapes_fit(self.tensor_specs(), bound):
             tensors = {n: fields_and_tensors.pop(n) for n in names}
             self.native = NativeMixer.build(dict(fields_and_tensors, width=self.hidden_size, heads=self.num_heads, dk=self.dk, dv=self.dv,
-                                                 eps=self.eps, out_scale=self.out_scale, in_chunks=int(self.in_chunks)), tensors, memory)
+                                                 eps=self.eps, out_scale=self.out_scale, in_chunks=int(self.in_chunks)), tensors, memory, self.cache_requirement().shape[0])
 
     def forward(self, x: torch.Tensor, step: StepContext, cache: Optional[LayerCache]) -> torch.Tensor:
         out = torch.empty((1, x.shape[0], self.hidden_size), dtype=torch.float32, device=x.device)
@@ -127,7 +127,7 @@ class MatrixMemory(_StateMixer):
         dt = torch.float32 if torch.float32 in (tensors["i.b"].dtype, tensors["f.b"].dtype) else tensors["i.b"].dtype
         self.b_i, self.b_f = tensors["i.b"].to(dt).contiguous(), tensors["f.b"].to(dt).contiguous()
         at = {n: r[0] for n, r in self.stacked.ranges.items()}
-        self._bind_native(True, ("w_in", "w_o", "bias_a", "bias_b", "norm_w"), w_in=self.stacked.weight, w_o=self.w_o, bias_a=self.b_i, bias_b=self.b_f,
+        self._bind_native(tensors, True, ("w_in", "w_o", "bias_a", "bias_b", "norm_w"), w_in=self.stacked.weight, w_o=self.w_o, bias_a=self.b_i, bias_b=self.b_f,
                           norm_w=self.norm_w, cap=self.cap, columns=self.stacked.weight.shape[0], kv_heads=self.num_heads, at_q=at["q"],
                           at_k=at["k"], at_v=at["v"], at_g=at["g"], at_a=at["i"], at_b=at["f"])
 
@@ -206,7 +206,7 @@ class GatedDeltaRule(_StateMixer):
         if not self.low_rank:
             self.stacked = _StackedInput([(n, tensors[n]) for n in ("q", "k", "v", "b", "a", "g")])
             self.w_second, self.second_blocks = None, (0, 0)
-            self._bind_native_delta("a", "g")
+            self._bind_native_delta(tensors, "a", "g")
             return
         if tensors["a1"].shape[0] != tensors["a2"].shape[1] or tensors["g1"].shape[0] != tensors["g2"].shape[1]:
             raise ValueError("the two steps of a low-rank projection do not fit each other")
@@ -218,12 +218,12 @@ class GatedDeltaRule(_StateMixer):
         both[:a2.shape[0], :a2.shape[1]] = a2
         both[a2.shape[0]:, a2.shape[1]:] = g2
         self.w_second, self.second_blocks = both.contiguous(), tuple(a2.shape)
-        self._bind_native_delta("a1", "g1")
+        self._bind_native_delta(tensors, "a1", "g1")
 
-    def _bind_native_delta(self, step_name: str, gate_name: str) -> None:
+    def _bind_native_delta(self, bound, step_name: str, gate_name: str) -> None:
         at = {n: r[0] for n, r in self.stacked.ranges.items()}
         second = tuple(self.w_second.shape) if self.w_second is not None else (0, 0)
-        self._bind_native(False, ("w_in", "w_second", "w_o", "conv_w", "bias_a", "bias_b", "norm_w"), w_in=self.stacked.weight, w_second=self.w_second,
+        self._bind_native(bound, False, ("w_in", "w_second", "w_o", "conv_w", "bias_a", "bias_b", "norm_w"), w_in=self.stacked.weight, w_second=self.w_second,
                           w_o=self.w_o, conv_w=self.conv_w, bias_a=self.dt_bias, bias_b=self.rate_log, norm_w=self.norm_w,
                           columns=self.stacked.weight.shape[0], kv_heads=self.num_kv_heads, taps=self.taps,
                           decay_channels=self.dk if self.decay == "channel" else 1, gate_act=1 if self.gate_activation == "silu" else 0,
