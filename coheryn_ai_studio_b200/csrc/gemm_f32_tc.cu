@@ -10,7 +10,7 @@
 // The operands swap places as in gemm_tc_few.cu: 128 output features sit on the lanes, BT tokens on the columns.  The tokens'
 // three terms are written once by a small kernel and come by TMA; W is read once from memory in float32 and split on its way:
 //
-//   warp 0       producer: W boxes of 128 x 32 floats (a ring of three stages of 64 k, fetched before the wait for the predecessor),
+//   warp 0       producer: W boxes of 128 x 32 floats (a ring of three stages of 64 k, fetched before the wait for the kernel that makes x's terms),
 //                x terms (two stages; from 96 tokens on a term is fetched again as soon as its last product is formed)
 //   warp 1       issues 24 tcgen05.mma per stage: A = W's terms in TENSOR MEMORY, B = x's terms in shared memory
 //   warps 2-5    split: a thread reads its feature's 64 values, writes 3 x 32 columns of bfloat16 pairs to tensor memory
@@ -48,10 +48,12 @@ struct F32Tile {
 };
 
 // The three terms of x as [3][M][pitch] bfloat16, pitch = K rounded up to eight; a thread takes eight values of a row.
+// Its successor, the product, fetches W before it waits for this kernel.  W may be the result of a kernel before this one, so that
+// this kernel lets the product start only when what came before it is complete.
 template <bool VEC>
 __global__ void __launch_bounds__(256) split_rows_kernel(const float* __restrict__ x, long ldx, int M, int K, int pitch, uint4* __restrict__ terms) {
-  co_pdl_launch_dependents();
   co_pdl_wait();
+  co_pdl_launch_dependents();
   const int chunks = pitch / 8;
   const long n = (long)M * chunks;
   for (long i = (long)blockIdx.x * 256 + threadIdx.x; i < n; i += (long)gridDim.x * 256) {

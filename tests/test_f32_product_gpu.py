@@ -75,6 +75,23 @@ def test_values_that_are_not_finite(M, N):
     assert bool(((got == want) | want.isnan() | ((got - want).abs() <= 1e-4 * (1.0 + want.abs()))).all())
 
 
+def test_a_weight_that_the_kernel_before_writes():
+    """The weight is fetched ahead, but not ahead of the kernel in front that is still writing it (and lets its successors start early)."""
+    from coheryn_ai_studio_b200 import ops
+    N, K = 12928, 1536
+    x, gate_up, _ = operands(24, N, 2 * K)
+    x, w, want = x[:, :K].contiguous(), torch.empty((N, K), device=DEV), torch.empty((N, K), device=DEV)
+    code = ops.gated_epilogue_word("silu", None)
+    ops.silu_mul(gate_up, want, code, 0.0)
+    torch.cuda.synchronize()
+    want = product(x, want)
+    torch.cuda.synchronize()
+    for _ in range(10):
+        w.zero_()
+        ops.silu_mul(gate_up, w, code, 0.0)
+        assert torch.equal(product(x, w), want)
+
+
 def test_which_products_it_takes():
     from coheryn_ai_studio_b200 import ops
     for M, N, K, taken in ((1, 128, 256, True), (5, 127, 256, False), (5, 128, 255, False), (5, 128, 252, False), (2000, 4000, 258, False)):
