@@ -8,7 +8,8 @@
 // another, are read from memory lane by lane, 128 bytes a warp, split in registers and written to TENSOR MEMORY as the operand A, 64
 // values of k at a time, while the tensor cores work on the 64 before; nothing of them passes through shared memory.  The other operand's
 // terms (q, the weighted scores, the weighted keys) stand in shared memory in the 128-byte swizzle.  The scores k q^T are formed the
-// same way with the keys of the chunk on 64 of the lanes.
+// same way with the keys of the chunk on 64 of the lanes.  The tensor cores' accumulator, which cuts instead of rounding, holds 64 values
+// of k at most: the sums over more key channels are added up by the threads, with ordinary float32 additions.
 //
 // What bounds it: the chain of a CTA, which has an SM's tensor memory to itself.  A chunk's 60 MMAs take 5 us of it; the rest is the
 // splits (the conversions to bfloat16 run at a quarter of the rate), the weights of the scores, and the norm and gate of the rows, one
@@ -226,6 +227,20 @@ __device__ __forceinline__ void tmem_ld4(unsigned taddr, unsigned (&r)[4]) {
   asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 }
 
+// Sixteen columns of this thread's lane are added to sixteen others.
+__device__ __forceinline__ void columns_add(unsigned to, unsigned from) {
+  unsigned x[16], y[16];
+  tmem_ld16(to, x);
+  tmem_ld16(from, y);
+#pragma unroll
+  for (int j = 0; j < 16; ++j) x[j] = __float_as_uint(__uint_as_float(x[j]) + __uint_as_float(y[j]));
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};"
+      :: "r"(to), "r"(x[0]), "r"(x[1]), "r"(x[2]), "r"(x[3]), "r"(x[4]), "r"(x[5]), "r"(x[6]), "r"(x[7]), "r"(x[8]), "r"(x[9]), "r"(x[10]), "r"(x[11]),
+         "r"(x[12]), "r"(x[13]), "r"(x[14]), "r"(x[15]) : "memory");
+  tmem_wait_st();
+}
+
 // Norm, weight and gate of the finished rows [64][pitch] of a head (head_out_chunk with four rows of a warp side by side, their gates
 // and the head's weight in shared memory).  The code is small on purpose: each warp passes it once.
 template <class To>
@@ -264,6 +279,8 @@ __device__ __forceinline__ void rows_out(const HeadOut& E, To* out, const float*
 template <int HALVES>
 __global__ void __launch_bounds__(32 * (4 * HALVES + 1)) memory_out_tc_kernel(MemoryIn P, HeadOut E, int B, int base, Area A, int key_bytes, int* status) {
   constexpr int WORKERS = 4 * HALVES, THREADS = 32 * WORKERS;
+  // D_P: the scores, 64 columns per block of 64 key channels (the others' columns are free again when the products with S_0 begin).
+  // D_S: the sum of S_0's blocks; D_V: the products with one block from the second on, then with the values.
   constexpr int D_P = 0, D_S = 64, D_V = D_S + 64 * HALVES, A_AT = D_V + 64 * HALVES;
   static_assert(A_AT + HALVES * A_COLS <= 512, "tensor memory");
   extern __shared__ unsigned char smem_raw[];
@@ -321,7 +338,7 @@ __global__ void __launch_bounds__(32 * (4 * HALVES + 1)) memory_out_tc_kernel(Me
             for (int p = 0; p < 6; ++p) {
               const unsigned long long da = umma_desc(ks + (block * 3 + PAIR_A[p]) * TILE), db = umma_desc(first + (block * 3 + PAIR_B[p]) * TILE);
 #pragma unroll
-              for (int k = 0; k < 4; ++k) umma_bf16(tmem + D_P, da + 2 * k, db + 2 * k, idesc, block || (p | k));
+              for (int k = 0; k < 4; ++k) umma_bf16(tmem + D_P + 64 * block, da + 2 * k, db + 2 * k, idesc, (p | k) != 0);
             }
         } else {
           const bool values = b == blocks + 1;
@@ -332,8 +349,8 @@ __global__ void __launch_bounds__(32 * (4 * HALVES + 1)) memory_out_tc_kernel(Me
               const unsigned long long db = umma_desc(tile + PAIR_B[p] * TILE);
 #pragma unroll
               for (int k = 0; k < 4; ++k)
-                umma_bf16_a_tmem(tmem + (values ? D_V : D_S) + 64 * half, tmem + A_AT + half * A_COLS + PAIR_A[p] * TERM_COLS + 8 * k, db + 2 * k, idesc,
-                                 (!values && b > 1) || (p | k));
+                umma_bf16_a_tmem(tmem + (b == 1 ? D_S : D_V) + 64 * half, tmem + A_AT + half * A_COLS + PAIR_A[p] * TERM_COLS + 8 * k, db + 2 * k, idesc,
+                                 (p | k) != 0);
             }
         }
         umma_commit(&bars.done);
@@ -400,6 +417,14 @@ __global__ void __launch_bounds__(32 * (4 * HALVES + 1)) memory_out_tc_kernel(Me
       // the products with the block before have been formed when its columns are written
       ok = __all_sync(0xffffffffu, mbar_wait(&bars.done, (b - 1) & 1)) && ok;
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      if (b == 1) {       // the blocks' scores are added
+        if (quarter < 2)
+          for (int block = 1; block < blocks; ++block)
+#pragma unroll 1
+            for (int t = half * (CH / HALVES); t < (half + 1) * (CH / HALVES); t += 16) columns_add(lanes + D_P + t, lanes + D_P + 64 * block + t);
+      } else if (b > 2)   // the block before is added to the sum
+#pragma unroll 1
+        for (int j = 64 * half; j < 64 * half + 64; j += 16) columns_add(lanes + D_S + j, lanes + D_V + j);
       put_terms(terms, t0, t1, t2);
       __syncwarp();
       if (lane == 0) mbar_arrive(&bars.a_full);

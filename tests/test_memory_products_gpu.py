@@ -60,3 +60,52 @@ def test_products_at_the_edges_of_their_tiles(dk, dv, lens, dtype, scale):
     bound = bound + (2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -21) * np.abs(want) + 1e-37
     got = out.double().cpu().numpy().reshape(n, heads, dv)
     assert (np.abs(got - want) <= bound).all(), (np.abs(got - want) / bound).max()
+
+
+@pytest.mark.parametrize("dk,dv", [(64, 128), (128, 256), (200, 72), (256, 128)])
+def test_error_no_larger_than_that_of_multiply_adds(dk, dv):
+    """A chunk's outputs against float64: no further off than the same products by the FMA kernel, whatever the number of key channels."""
+    from coheryn_ai_studio_b200 import ops
+    H, T, lib = 4, 64, ops.recurrent()
+    g = torch.Generator(device=DEV).manual_seed(dk)
+    f = lambda *s: torch.randn(s, device=DEV, generator=g)
+    q, k, v, gates, state = f(T, H * dk), f(T, H * dk), f(T, H * dv), f(T, 2 * H), f(1, H * (dk * dv + dk + 1))
+    gates[:, :H] -= 2.0
+    gates[:, H:] += 4.5
+    state[:, -H:] = 0.0
+    first, qkv, out, zero = state[0].clone(), torch.cat([q, k, v], dim=1), torch.empty((T, H * dv), device=DEV), torch.zeros(H, device=DEV)
+    pays = lib.coheryn_memory_chunks_pay
+    try:
+        lib.coheryn_memory_chunks_pay = lambda *a: 1
+        ops.matrix_memory_scan(qkv[:, :H * dk], qkv[:, H * dk:2 * H * dk], qkv[:, 2 * H * dk:], gates[:, :H], gates[:, H:], zero, zero, 15.0, state,
+                               step_of([T], [0], True), H, dk, dv, out, torch.ones(H * dv, device=DEV), torch.full((T, H * dv), 40.0, device=DEV), 1e-6)
+    finally:
+        lib.coheryn_memory_chunks_pay = pays
+    cap = lambda z: 15.0 * torch.tanh(z.double() / 15.0)
+    i, F = cap(gates[:, :H]), torch.nn.functional.logsigmoid(cap(gates[:, H:])).cumsum(0)
+    errors = [0.0, 0.0, 0.0]
+    for h in range(H):
+        rows = lambda x, d: x[:, h * d:(h + 1) * d].contiguous()
+        qh, kh, vh = rows(q, dk), rows(k, dk), rows(v, dv)
+        S, n = first[h * dk * dv:(h + 1) * dk * dv].view(dk, dv), first[H * dk * dv + h * dk:H * dk * dv + (h + 1) * dk]
+        each = F[:, h, None] - F[None, :, h] + i[None, :, h]
+        each.masked_fill_(torch.ones(T, T, device=DEV).triu(1).bool(), -float("inf"))
+        m = torch.maximum(each.max(1).values, F[:, h])
+        w, a = (each - m[:, None]).exp(), (F[:, h] - m).exp()
+
+        def outputs(product, dtype):
+            s = product((qh.to(dtype) * dk ** -0.5), kh.to(dtype)) * w.to(dtype)
+            den = torch.maximum((a.to(dtype) * (qh.to(dtype) * dk ** -0.5 * n.to(dtype)).sum(1) + s.sum(1)).abs(), (-m).exp().to(dtype)) + 1e-6
+            o = (a[:, None].to(dtype) * product(qh.to(dtype) * dk ** -0.5, S.T.contiguous().to(dtype)) + product(s, vh.T.contiguous().to(dtype))) / den[:, None]
+            return (o.double() / (o.double().square().mean(1, keepdim=True) + 1e-6).sqrt())
+
+        def fma(x, y):
+            got = torch.empty((x.shape[0], y.shape[0]), device=DEV)
+            ops.gemm_simt(x.contiguous(), y, None, got)
+            return got
+
+        want = outputs(lambda x, y: x @ y.T, torch.float64)
+        for e, got in enumerate((rows(out, dv).double(), outputs(fma, torch.float32))):
+            errors[e] += float((got - want).square().sum())
+        errors[2] += float(want.square().sum())
+    assert errors[0] <= errors[1], [(e / errors[2]) ** 0.5 for e in errors[:2]]
