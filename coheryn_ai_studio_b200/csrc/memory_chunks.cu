@@ -12,7 +12,7 @@
 //   memory_carry_kernel   over a run's chunks, element by element: the S_0 and n_0 of every chunk; the last ones are kept;
 //   memory_out_tc_kernel  (memory_chunks_tc.cu) the outputs and the norm, weight and gate behind them.
 //
-// Every exponent is a difference of float64 sums, so that a weight is as exact however far the gates have summed up.  The maxima
+// Every exponent is a difference of float64 sums, rounded once, so that a weight is as exact however far the gates have summed up.  The maxima
 // m are kept in float32, so an exponent may exceed zero by the rounding of m (3e-5 at m = 1,000): S, n and exp(-m) all use the same
 // rounded m, and what it is off by cancels between numerator and denominator.
 //

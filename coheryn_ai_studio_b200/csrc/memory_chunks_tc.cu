@@ -213,15 +213,6 @@ inline size_t larger(size_t a, size_t b) { return ((a > b ? a : b) + 1023) / 102
 size_t out_tc_keys(int dk, int dvp) { return larger((size_t)q_tiles(dk) * 3 * TILE, (size_t)CH * (CH + 4) * 4 + (size_t)CH * dvp * 4); }
 size_t out_tc_smem(int dk, int dvp) { return 1024 + out_tc_keys(dk, dvp) + larger((size_t)(q_tiles(dk) + 1) * 3 * TILE, (size_t)CH * (dvp + 4) * 4); }
 
-// A float64 as the sum of two float32.
-struct Two { float hi, lo; };
-__device__ __forceinline__ Two two(double x) { const float h = (float)x; return {h, (float)(x - (double)h)}; }
-// a + b, rounded once (almost): the rounding of the high parts' sum is formed exactly and added with the low parts.
-__device__ __forceinline__ float add(const Two& a, const Two& b) {
-  const float s = a.hi + b.hi, t = s - a.hi;
-  return s + (((a.hi - (s - t)) + (b.hi - t)) + (a.lo + b.lo));
-}
-
 __device__ __forceinline__ void tmem_ld4(unsigned taddr, unsigned (&r)[4]) {
   asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(taddr));
   asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
@@ -285,7 +276,7 @@ __global__ void __launch_bounds__(32 * (4 * HALVES + 1)) memory_out_tc_kernel(Me
   static_assert(A_AT + HALVES * A_COLS <= 512, "tensor memory");
   extern __shared__ unsigned char smem_raw[];
   __shared__ Bars bars;
-  __shared__ Two down[CH], up[CH];           // F_t - m_t, i_s - F_s
+  __shared__ double down[CH], up[CH];        // F_t - m_t, i_s - F_s
   __shared__ float ms[CH], as[CH], dens[CH], sums[4][CH], weight[256];
   unsigned char* ks = (unsigned char*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);      // the keys' tiles [block][3], then:
   float* scores = (float*)ks;                               // [s][CH + 1]
@@ -303,8 +294,8 @@ __global__ void __launch_bounds__(32 * (4 * HALVES + 1)) memory_out_tc_kernel(Me
   if (tid < CH) {
     const double f = A.f[at * CH + tid];
     const float m = A.m[at * CH + tid];
-    down[tid] = two(f - (double)m);
-    up[tid] = two((double)A.i[at * CH + tid] - f);
+    down[tid] = f - (double)m;
+    up[tid] = (double)A.i[at * CH + tid] - f;
     ms[tid] = m;
     as[tid] = expf((float)(f + (double)A.m0[at * 4] - (double)m));
   }
@@ -386,7 +377,7 @@ __global__ void __launch_bounds__(32 * (4 * HALVES + 1)) memory_out_tc_kernel(Me
       if (values && quarter < 2) {
         // The weighted scores: lane s of the first two quarters, half of the tokens t for each half of the warps.
         const int s = quarter * 32 + lane;
-        const Two mine = up[s];
+        const double mine = up[s];
 #pragma unroll 1
         for (int t = half * (CH / HALVES); t < (half + 1) * (CH / HALVES); t += 4) {
           unsigned r[4];
@@ -396,7 +387,7 @@ __global__ void __launch_bounds__(32 * (4 * HALVES + 1)) memory_out_tc_kernel(Me
             float x[2];
 #pragma unroll
             for (int i = 0; i < 2; ++i) {
-              x[i] = s <= t + j + i && t + j + i < nt ? __uint_as_float(r[j + i]) * expf(add(down[t + j + i], mine)) : 0.f;
+              x[i] = s <= t + j + i && t + j + i < nt ? __uint_as_float(r[j + i]) * expf((float)(down[t + j + i] + mine)) : 0.f;
               scores[s * (CH + 1) + t + j + i] = x[i];
             }
             unsigned y[3];
