@@ -12,10 +12,10 @@
 // of k at most: the sums over more key channels are added up by the threads, with ordinary float32 additions.
 //
 // What bounds it: the chain of a CTA, which has an SM's tensor memory to itself.  A chunk's 60 MMAs take 5 us of it; the rest is the
-// splits (the conversions to bfloat16 run at a quarter of the rate), the weights of the scores, and the norm and gate of the rows, one
-// after another.  A warp passes each piece of code a few times only, so the loops are kept small (unrolled further they wait for
-// instructions: 87 us), and the gate's quotient is formed without a division's branch (80 -> 65 us).  Measured on a B200 (8 heads of
-// 128 x 256, one request of 2,048 tokens): sums 24 us, outputs 65 us; the same products in multiply-adds took 38 and 94.
+// splits (a dozen integer and float32 operations a value), the weights of the scores, and the norm and gate of the rows, one after
+// another.  A warp passes each piece of code a few times only, so the loops are kept small (unrolled further they wait for
+// instructions: 87 us for the outputs).  Measured on a B200 (8 heads of 128 x 256, one request of 2,048 tokens, all four kernels with
+// L2 flushed): 169 us with the products in float32 multiply-adds, 137 now, 7 of which are the gates' divisions.
 //
 // Every wait is for the CTA's own products and is bounded: on expiry the kernel records an error code and winds down.
 #include "tc_common.cuh"
@@ -259,7 +259,7 @@ __device__ __forceinline__ void rows_out(const HeadOut& E, To* out, const float*
       const float w = weight[c];
 #pragma unroll
       for (int u = 0; u < 4; ++u) {
-        const float z = gates[(i + u) * ldg + c], g = swish ? z * rc_sigmoid_many(z) : rc_sigmoid_many(z);
+        const float z = gates[(i + u) * ldg + c], g = swish ? z * rc_sigmoid(z) : rc_sigmoid(z);
         if (i + u < nt) to[(size_t)u * E.ldo + c] = (To)(os[(i + u) * pitch + c] * inv[u] * w * g * E.out_scale);
       }
     }

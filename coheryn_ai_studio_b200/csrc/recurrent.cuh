@@ -89,15 +89,6 @@ int co_memory_one(const MemoryIn& P, const HeadOut& E, int B, cudaStream_t strea
 namespace {
 
 __device__ __forceinline__ float rc_sigmoid(float z) { return 1.0f / (1.0f + expf(-z)); }
-// The same value for loops over many elements: 1.0f / x is a division with a branch for its rare cases, 90 cycles a warp where this
-// takes 15.  The quotient is the hardware's estimate (1 ulp) and one Newton step, r + r (1 - d r), for d from 1 to 6e37; beyond, where
-// the quotient is under 1.7e-38, it is 0.
-__device__ __forceinline__ float rc_sigmoid_many(float z) {
-  const float e = expf(-z), d = 1.0f + e;
-  float r;
-  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(d));
-  return e > 6e37f ? 0.f : fmaf(r, fmaf(-d, r, 1.0f), r);
-}
 __device__ __forceinline__ float rc_softplus(float z) { return fmaxf(z, 0.f) + log1pf(expf(-fabsf(z))); }
 __device__ __forceinline__ void rc_store(void* out, int dtype, size_t i, float v) {
   if (dtype == CO_BF16) ((__nv_bfloat16*)out)[i] = __float2bfloat16_rn(v);
