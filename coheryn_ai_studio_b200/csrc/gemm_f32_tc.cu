@@ -1,10 +1,10 @@
 // out[M, N] = x[M, K] . W[N, K]^T (+ bias) of float32 operands to float32's accuracy on the 5th-generation tensor cores.
 //
-// Every float32 value is the exact sum of three bfloat16 ones, v = v0 + v1 + v2 (each the rest's nearest: 8 + 8 + 8 bits), and a
-// product of two bfloat16 values is exact in the accumulator.  Of the nine products of terms the six with i + j <= 2 are formed; the
-// three left out are below 2^-25 of |x w|, half of what rounding one product would cost.  The accumulator in tensor memory only
-// ever holds 64 values of k, the small products first and x0 w0 last, and is then added to sums in registers with ordinary
-// float32 additions: its own rounding (which truncates) touches the large products four times per 64 values, and a sum of K
+// Every float32 value from 2^-110 up is the exact sum of three bfloat16 ones, v = v0 + v1 + v2 (each the rest's nearest: 8 + 8 + 8 bits),
+// and a product of two bfloat16 values is exact in the accumulator.  Of the nine products of terms the six with i + j <= 2 are formed; of
+// the three left out two are below 2^-25 of |x w| each and one below 2^-33: together what rounding one product may cost.  The accumulator
+// in tensor memory only ever holds 64 values of k, the small products first and x0 w0 last, and is then added to sums in registers with
+// ordinary float32 additions: its own rounding (which truncates) touches the large products four times per 64 values, and a sum of K
 // values has K / 64 roundings in place of the FMA chain's K.  Measured against float64: below.
 //
 // The operands swap places as in gemm_tc_few.cu: 128 output features sit on the lanes, BT tokens on the columns.  The tokens'
@@ -24,8 +24,12 @@
 // 17920 x 1536 84 -> 47.  Error against float64 (2-norm, relative): 0.8e-7 to 1.2e-7 where the FMA chain has 2.8e-7 to 5.0e-7.
 //
 // A row's result does not depend on the other rows: K is cut into slices by the weight's shape alone, a slice's sum goes to a
-// workspace (where there is more than one) and the slices are added in order.  A result that is not finite is formed again from the
-// operands themselves (an infinity has no finite rest, so the terms' products would make it a NaN).
+// workspace (where there is more than one) and the slices are added in order.  Two kinds of results are formed again from the operands
+// themselves, by float32 multiply-adds: one that is not finite (an infinity has no finite rest, so the terms' products would make it a
+// NaN), and one so small that the bits which the split of operands under 2^-110 cuts off may count in it.  For the second the largest
+// magnitude of the row and of the feature are kept: with operands of ordinary size beside the small ones nothing is formed again (an
+// activation of 1e-34 leaves its row's results alone: 313 x 1536 x 8960 with one in every row 71 us, with none 69 to 73).  Where all of
+// x is that small they are all formed again, in 3.8 ms.  Results in float32's subnormal range are good to a unit of 2^-149 per value of k.
 // Every wait is bounded: on expiry the kernel records an error code and winds down.
 #include "tc_common.cuh"
 
@@ -47,34 +51,54 @@ struct F32Tile {
   static_assert(COLS_USED <= 512 && PART % 16 == 0, "tensor memory");
 };
 
-// The three terms of x as [3][M][pitch] bfloat16, pitch = K rounded up to eight; a thread takes eight values of a row.
+// What the epilogue has to know of an operand's row: its largest magnitude, and whether the terms are short of some value's bits.
+struct RowInfo { float largest; unsigned cut; };
+
+// The three terms of x as [3][M][pitch] bfloat16, pitch = K rounded up to eight, and each row's RowInfo.  A CTA takes a row at a
+// time, a thread eight values.
 // Its successor, the product, fetches W before it waits for this kernel.  W may be the result of a kernel before this one, so that
 // this kernel lets the product start only when what came before it is complete.
 template <bool VEC>
-__global__ void __launch_bounds__(256) split_rows_kernel(const float* __restrict__ x, long ldx, int M, int K, int pitch, uint4* __restrict__ terms) {
+__global__ void __launch_bounds__(256) split_rows_kernel(const float* __restrict__ x, long ldx, int M, int K, int pitch, uint4* __restrict__ terms,
+                                                         RowInfo* __restrict__ info) {
+  __shared__ unsigned largest_of[8], cut_of[8];
   co_pdl_wait();
   co_pdl_launch_dependents();
-  const int chunks = pitch / 8;
+  const int chunks = pitch / 8, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const long n = (long)M * chunks;
-  for (long i = (long)blockIdx.x * 256 + threadIdx.x; i < n; i += (long)gridDim.x * 256) {
-    const long m = i / chunks;
-    const int k = (int)(i - m * chunks) * 8;
-    const float* p = x + m * ldx + k;
-    float v[8];
-    if (VEC && k + 8 <= K) {
-      const float4 a = *reinterpret_cast<const float4*>(p), b = *reinterpret_cast<const float4*>(p + 4);
-      v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w; v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
-    } else {
+  for (int m = blockIdx.x; m < M; m += gridDim.x) {
+    unsigned largest = 0, cut = 0;
+    for (int c = threadIdx.x; c < chunks; c += 256) {
+      const int k = 8 * c;
+      const float* p = x + m * ldx + k;
+      float v[8];
+      if (VEC && k + 8 <= K) {
+        const float4 a = *reinterpret_cast<const float4*>(p), b = *reinterpret_cast<const float4*>(p + 4);
+        v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w; v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
+      } else {
 #pragma unroll
-      for (int j = 0; j < 8; ++j) v[j] = k + j < K ? p[j] : 0.f;
+        for (int j = 0; j < 8; ++j) v[j] = k + j < K ? p[j] : 0.f;
+      }
+#pragma unroll
+      for (int j = 0; j < 8; ++j) largest = max(largest, __float_as_uint(v[j]) & 0x7fffffffu);
+      uint4 t[3];
+      split3(v[0], v[1], t[0].x, t[1].x, t[2].x, cut);
+      split3(v[2], v[3], t[0].y, t[1].y, t[2].y, cut);
+      split3(v[4], v[5], t[0].z, t[1].z, t[2].z, cut);
+      split3(v[6], v[7], t[0].w, t[1].w, t[2].w, cut);
+#pragma unroll
+      for (int j = 0; j < 3; ++j) terms[j * n + (long)m * chunks + c] = t[j];
     }
-    uint4 t[3];
-    split3(v[0], v[1], t[0].x, t[1].x, t[2].x);
-    split3(v[2], v[3], t[0].y, t[1].y, t[2].y);
-    split3(v[4], v[5], t[0].z, t[1].z, t[2].z);
-    split3(v[6], v[7], t[0].w, t[1].w, t[2].w);
+    largest = __reduce_max_sync(0xffffffffu, largest);
+    cut = __reduce_or_sync(0xffffffffu, cut);
+    if (lane == 0) { largest_of[warp] = largest; cut_of[warp] = cut; }
+    __syncthreads();
+    if (threadIdx.x == 0) {
 #pragma unroll
-    for (int j = 0; j < 3; ++j) terms[j * n + i] = t[j];
+      for (int w = 1; w < 8; ++w) { largest = max(largest, largest_of[w]); cut |= cut_of[w]; }
+      info[m] = {__uint_as_float(largest), cut & 0xffffu};
+    }
+    __syncthreads();
   }
 }
 
@@ -98,6 +122,7 @@ struct F32Args {
   const float* x; const float* w; const void* bias; float* out; float* apart;      // apart: [slice][M][N] (absent: one slice)
   int bias_dtype, M, N, K, per_slice;      // stages of 64 k per slice
   long ldx, ldo;
+  const RowInfo* info;                     // of x's rows
   int* status;
 };
 
@@ -107,6 +132,7 @@ __global__ void __launch_bounds__(448, 1)
 gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x, const F32Args P) {
   using S = F32Tile<BT>;
   extern __shared__ unsigned char smem_raw[];
+  __shared__ RowInfo w_info[F_ROWS];                    // of W's rows, as far as this CTA's k go
   unsigned char* ws = (unsigned char*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   unsigned char* xs = ws + W_STAGES * W_BYTES;
   unsigned long long* w_full = (unsigned long long*)(xs + X_STAGES * S::X_BYTES);
@@ -117,6 +143,7 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
   unsigned long long* acc_free = a_full + 2;            // the sums have been read
   unsigned* tmem_slot = (unsigned*)(acc_free + 2);
   static_assert((2 * W_STAGES + 16) * 8 + 4 <= 256, "barriers fit their slot");
+  constexpr int INFO_THREADS = 128 + 128 * S::HALVES;
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int n0 = blockIdx.x * F_ROWS, m0 = blockIdx.y * BT;
@@ -197,6 +224,8 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
     }
   } else if (warp < 6) {
     const int quarter = warp & 3, row = quarter * 32 + lane;
+    unsigned cut = 0;
+    float largest = 0.f;
     for (int kt = 0; kt < stages; ++kt) {
       const int s = kt % W_STAGES, b = kt & 1;
       bool ok = mbar_wait(&w_full[s], (kt / W_STAGES) & 1);
@@ -208,8 +237,9 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
         for (int c = 0; c < 8; ++c) {
           const float4 v = *reinterpret_cast<const float4*>(from + h * (W_BYTES / 2) + ((c ^ (row & 7)) << 4));
           const int at = h * 16 + 2 * c;
-          split3(v.x, v.y, t0[at], t1[at], t2[at]);
-          split3(v.z, v.w, t0[at + 1], t1[at + 1], t2[at + 1]);
+          split3(v.x, v.y, t0[at], t1[at], t2[at], cut);
+          split3(v.z, v.w, t0[at + 1], t1[at + 1], t2[at + 1], cut);
+          largest = fmaxf(fmaxf(largest, fmaxf(fabsf(v.x), fabsf(v.y))), fmaxf(fabsf(v.z), fabsf(v.w)));
         }
       __syncwarp();
       if (lane == 0) mbar_arrive(&w_free[s]);
@@ -226,6 +256,8 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
       __syncwarp();
       if (lane == 0) mbar_arrive(&a_full[b]);
     }
+    w_info[row] = {largest, cut & 0xffffu};
+    asm volatile("bar.arrive 1, %0;" ::"n"(INFO_THREADS) : "memory");
   } else if (warp < 6 + 4 * S::HALVES) {
     const int quarter = warp & 3, half = (warp - 6) >> 2;
     const int n_first = n0 + quarter * 32, n = n_first + lane, c0 = half * S::PART;
@@ -233,6 +265,15 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
 #pragma unroll
     for (int j = 0; j < S::PART; ++j) sum[j] = 0.f;
     bool ok = true;
+    co_pdl_wait();      // whether a row of x in this warp's columns was cut (and before the results are written: the predecessor may read there)
+    unsigned x_cut = 0, x_largest = 0;
+    for (int j = lane; j < S::PART && m0 + c0 + j < P.M; j += 32) {
+      const RowInfo x = P.info[m0 + c0 + j];
+      x_cut |= x.cut;
+      x_largest = max(x_largest, __float_as_uint(x.largest));
+    }
+    x_cut = __any_sync(0xffffffffu, x_cut != 0);
+    x_largest = __reduce_max_sync(0xffffffffu, x_largest);
     for (int kt = 0; kt < stages; ++kt) {
       const int b = kt & 1;
       ok = __all_sync(0xffffffffu, mbar_wait(&x_free[3 * b], (kt >> 1) & 1));
@@ -250,8 +291,8 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
       __syncwarp();
       if (lane == 0) mbar_arrive(&acc_free[b]);
     }
+    asm volatile("bar.sync 1, %0;" ::"n"(INFO_THREADS) : "memory");      // W's rows have been looked at
     if (ok) {
-      co_pdl_wait();      // out and the workspace may still be read by the predecessor; x is read where a result is not finite
       const int k0 = first * BK, k1 = min(P.K, (first + stages) * BK);
       const float bias = n < P.N && P.bias && !P.apart ? co_load_any(P.bias, P.bias_dtype, n) : 0.f;
       float* to = P.apart ? P.apart + ((size_t)blockIdx.z * P.M) * P.N + n : P.out + n;
@@ -259,18 +300,36 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
       // (few instructions per column: code that runs once comes from memory, and at ten times the length it took as long as the products)
       const int rows = min(S::PART, P.M - m0 - c0);
       float* at = to + (long)(m0 + c0) * ld;
-      unsigned largest = 0;
+      unsigned largest = 0, smallest = 0x7fffffffu;
 #pragma unroll
       for (int j = 0; j < S::PART; ++j) {
-        largest = max(largest, __float_as_uint(sum[j]) & 0x7fffffffu);
+        const unsigned size = __float_as_uint(sum[j]) & 0x7fffffffu;
+        largest = max(largest, size);
+        if (j < rows) smallest = min(smallest, size);
         if (j < rows && n < P.N) at[j * ld] = sum[j] + bias;
       }
-      if (__any_sync(0xffffffffu, n < P.N && largest >= 0x7f800000u)) {
+      // less than 2^-133 of every value that was cut, times the other operand: a result of 2^25 times that is right to its last bit
+      const RowInfo w = w_info[quarter * 32 + lane];
+      const float unit = (float)(k1 - k0) * 0x1p-108f;
+      const float most = unit * ((x_cut ? w.largest : 0.f) + (w.cut ? __uint_as_float(x_largest) : 0.f));
+      if (__any_sync(0xffffffffu, n < P.N && (largest >= 0x7f800000u || __uint_as_float(smallest) < most))) {
+        unsigned again[(S::PART + 31) / 32] = {};
+#pragma unroll
+        for (int j = 0; j < S::PART; ++j)
+          if (j < rows) {
+            const RowInfo x = P.info[m0 + c0 + j];
+            const float least = unit * ((x.cut ? w.largest : 0.f) + (w.cut ? x.largest : 0.f)), size = fabsf(sum[j]);
+            if (n < P.N && (!(size < INFINITY) || size < least)) again[j / 32] |= 1u << (j % 32);
+          }
+#pragma unroll 1
         for (int j = 0; j < rows; ++j) {
-          const unsigned bad = __ballot_sync(0xffffffffu, n < P.N && !(fabsf(n < P.N ? at[j * ld] : 0.f) < INFINITY));
+          unsigned word = again[0];
+#pragma unroll
+          for (int i = 1; i < (S::PART + 31) / 32; ++i) word = j / 32 == i ? again[i] : word;
+          const unsigned bad = __ballot_sync(0xffffffffu, word >> (j % 32) & 1);
           if (!bad) continue;
-          const float again = sum_again(bad, P.x + (m0 + c0 + j) * P.ldx, P.w, n_first, P.K, k0, k1);
-          if (bad >> lane & 1) at[j * ld] = again + bias;
+          const float y = sum_again(bad, P.x + (m0 + c0 + j) * P.ldx, P.w, n_first, P.K, k0, k1);
+          if (bad >> lane & 1) at[j * ld] = y + bias;
         }
       }
     }
@@ -334,7 +393,7 @@ int rows_at_once(int M, int N, int K) {
   const double rows = floor((double)(128 << 20) / each / BT_MOST) * BT_MOST;
   return rows < BT_MOST ? (M < BT_MOST ? M : BT_MOST) : (rows < M ? (int)rows : M);
 }
-long terms_floats(long rows, int K) { return (3 * rows * pitch_of(K) / 2 + 63) / 64 * 64; }
+long terms_floats(long rows, int K) { return (3 * rows * pitch_of(K) / 2 + 2 * rows + 63) / 64 * 64; }      // and the rows' RowInfo
 
 template <int BT>
 int launch(const CUtensorMap& mw, const CUtensorMap& mx, const F32Args& P, int slices, cudaStream_t stream) {
@@ -381,12 +440,13 @@ CO_EXPORT int coheryn_gemm_f32_tc(const float* x, const float* w, const void* bi
     const cuuint32_t box[3] = {(cuuint32_t)BK, (cuuint32_t)bt, 1};
     if (!make_map_nd(&mx, workspace, 3, dims, strides, box)) CO_FAIL("gemm_f32_tc: cuTensorMapEncodeTiled failed (M=%d K=%d)", rows, K);
     const long chunks = (long)rows * (pitch / 8);
-    const unsigned blocks = (unsigned)((chunks + 255) / 256 < 148 * 8 ? (chunks + 255) / 256 : 148 * 8);
+    RowInfo* info = reinterpret_cast<RowInfo*>((uint4*)workspace + 3 * chunks);
     const bool vec = ldx % 4 == 0 && !((uintptr_t)x & 15);
-    co_launch(vec ? split_rows_kernel<true> : split_rows_kernel<false>, dim3(blocks), dim3(256), 0, stream, x, ldx, rows, K, pitch, (uint4*)workspace);
+    co_launch(vec ? split_rows_kernel<true> : split_rows_kernel<false>, dim3(rows < 148 * 8 ? rows : 148 * 8), dim3(256), 0, stream, x, ldx, rows, K, pitch,
+              (uint4*)workspace, info);
     CO_CHECK_LAUNCH("split_rows");
     const F32Args P = {x, w, bias, out, apart ? workspace + terms_floats(most, K) : nullptr, bias_dtype, rows, N, K,
-                       ((K + BK - 1) / BK + slices - 1) / slices, ldx, ldo, status};
+                       ((K + BK - 1) / BK + slices - 1) / slices, ldx, ldo, info, status};
     const int rc = bt == 16 ? launch<16>(mw, mx, P, slices, stream) : bt == 32 ? launch<32>(mw, mx, P, slices, stream)
                  : bt == 64 ? launch<64>(mw, mx, P, slices, stream) : bt == 96 ? launch<96>(mw, mx, P, slices, stream)
                  : bt == 128 ? launch<128>(mw, mx, P, slices, stream) : launch<160>(mw, mx, P, slices, stream);

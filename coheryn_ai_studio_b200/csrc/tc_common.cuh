@@ -163,14 +163,22 @@ __device__ __forceinline__ void mbar_arrive(unsigned long long* bar) {
 // v0 + v1 + v2 = v for a pair of neighbouring values, as packed bfloat16 pairs (the first value in the low half): v0 and v1 the
 // nearest (halves away from zero) of the value and of the rest, v2 what is left, which has at most eight bits.  Integer operations: the
 // conversion instructions go through the narrow pipe of the special functions, which three per pair would keep busy for a third of the time.
-__device__ __forceinline__ void split3(float a, float b, unsigned& t0, unsigned& t1, unsigned& t2) {
+// The sum is exact for zero and from 2^-110 up.  Below, bits of v2 can lie under bfloat16's smallest number, 2^-133, and are cut off (less
+// than 2^-133 of a value): `cut` then gets a bit in its low half.
+__device__ __forceinline__ void split3(float a, float b, unsigned& t0, unsigned& t1, unsigned& t2, unsigned& cut) {
   const unsigned a0 = (__float_as_uint(a) + 0x8000u) & 0xffff0000u, b0 = (__float_as_uint(b) + 0x8000u) & 0xffff0000u;
   a -= __uint_as_float(a0);
   b -= __uint_as_float(b0);
   const unsigned a1 = (__float_as_uint(a) + 0x8000u) & 0xffff0000u, b1 = (__float_as_uint(b) + 0x8000u) & 0xffff0000u;
   t0 = __byte_perm(a0, b0, 0x7632);
   t1 = __byte_perm(a1, b1, 0x7632);
-  t2 = __byte_perm(__float_as_uint(a - __uint_as_float(a1)), __float_as_uint(b - __uint_as_float(b1)), 0x7632);
+  const unsigned a2 = __float_as_uint(a - __uint_as_float(a1)), b2 = __float_as_uint(b - __uint_as_float(b1));
+  t2 = __byte_perm(a2, b2, 0x7632);
+  cut |= a2 | b2;
+}
+__device__ __forceinline__ void split3(float a, float b, unsigned& t0, unsigned& t1, unsigned& t2) {
+  unsigned cut = 0;
+  split3(a, b, t0, t1, t2, cut);
 }
 
 typedef CUresult (*EncodeTiled)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,

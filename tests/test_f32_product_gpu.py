@@ -75,6 +75,26 @@ def test_values_that_are_not_finite(M, N):
     assert bool(((got == want) | want.isnan() | ((got - want).abs() <= 1e-4 * (1.0 + want.abs()))).all())
 
 
+@pytest.mark.parametrize("M,N,K", [(24, 256, 512), (90, 300, 324), (170, 13000, 260), (20, 1536, 2304)])
+@pytest.mark.parametrize("ex,ew", [(-100, 0), (-108, 20), (-114, 100), (0, -118), (-124, 120), (118, -135), (-140, 100), (-70, -60)])
+def test_operands_under_the_terms_range(M, N, K, ex, ew):
+    """Bits that lie under the terms' smallest number count where the other operand is large: the error is the FMA product's at most, and
+    a few units of float32's own smallest number where the results come down to it."""
+    from coheryn_ai_studio_b200 import ops
+    x, w, bias = operands(M, N, K)
+    x, w = (x.double() * 2.0 ** ex).float(), (w.double() * 2.0 ** ew).float()
+    want, fma, got = x.double() @ w.double().T, torch.empty((M, N), device=DEV), product(x, w)
+    ops.gemm_simt(x, w, None, fma)
+    error, room = float((got.double() - want).norm()), K * 2.0 ** -149 * (M * N) ** 0.5      # one unit for every value of k
+    assert error <= max(float((fma.double() - want).norm()), room)
+    # the same beside operands of ordinary size: in some rows, in some features, at some k
+    small, x, w = (x, w), torch.randn(M, K, device=DEV), torch.randn(N, K, device=DEV)
+    x[::3], w[::5], x[:, ::7], w[:, 1::7] = small[0][::3], small[1][::5], small[0][:, ::7], small[1][:, 1::7]
+    want, got = x.double() @ w.double().T, product(x, w, bias).double() - bias.double()
+    size = x.double().abs() @ w.double().abs().T + bias.double().abs()
+    assert bool(((got - want).abs() <= (K + 2) * 2.0 ** -24 * size + K * 2.0 ** -149).all())
+
+
 def test_a_weight_that_the_kernel_before_writes():
     """The weight is fetched ahead, but not ahead of the kernel in front that is still writing it (and lets its successors start early)."""
     from coheryn_ai_studio_b200 import ops
