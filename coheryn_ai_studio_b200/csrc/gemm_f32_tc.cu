@@ -373,10 +373,11 @@ add_slices_kernel(const float* __restrict__ apart, int slices, const void* __res
   }
 }
 
-// Slices of K: about one CTA per SM at few rows, at least four stages each; a function of the weight's shape alone.
+// Slices of K: about one CTA per SM at few rows, at least four stages each; a function of the weight's shape alone.  Measured on a B200 (us
+// at 1, 313 and 2,048 rows, back to back): 1536 x 8960 for 100, 148 (here), 220 and 296 CTAs 28 / 78 / 399, 22 / 64 / 404, 29 / 74 / 486 and
+// 26 / 84 / 541; 1024 x 1024 with at least two, four (here) and eight stages 8.4 / 15 / 84, 9.9 / 17 / 50 and 14 / 23 / 47.
 int slices_of(int N, int K) {
   const int tiles = (N + F_ROWS - 1) / F_ROWS, k_tiles = (K + BK - 1) / BK;
-  if (tiles >= 100) return 1;
   int s = (148 + tiles / 2) / tiles;
   if (s > k_tiles / 4) s = k_tiles / 4;
   if (s < 2) return 1;
@@ -385,11 +386,12 @@ int slices_of(int N, int K) {
 }
 int pitch_of(int K) { return (K + 7) / 8 * 8; }
 constexpr int BT_MOST = 160;
-// Rows that are worked on at a time: their terms (6 bytes a value) and their slices' sums take 128 MB at most (the slices' sums then
-// about stay in L2, where the adding kernel finds them), one tile of rows at least.
-int rows_at_once(int M, int N, int K) {
+// Rows that are worked on at a time: their terms (6 bytes a value) and, where there are any, their slices' sums take 128 MB at most (the
+// slices' sums then about stay in L2, where the adding kernel finds them), one tile of rows at least.  Measured on a B200 with 32, 64 and
+// 128 MB: 2048 x 4096 x 4096 (five slices) 751, 530 and 453 us, 2048 x 1536 x 8960 (twelve) 454, 404 and 400.
+int rows_at_once(int M, int N, int K, int act) {
   const int slices = slices_of(N, K);
-  const double each = 6.0 * pitch_of(K) + 4.0 * slices * N;
+  const double each = 6.0 * pitch_of(K) + 8.0 + (slices > 1 || act ? 4.0 * slices * N : 0.0);
   const double rows = floor((double)(128 << 20) / each / BT_MOST) * BT_MOST;
   return rows < BT_MOST ? (M < BT_MOST ? M : BT_MOST) : (rows < M ? (int)rows : M);
 }
@@ -407,14 +409,19 @@ int launch(const CUtensorMap& mw, const CUtensorMap& mx, const F32Args& P, int s
 }
 }  // namespace
 
-// Whether the kernel takes a weight of this shape (a function of the shape alone, so that all rows of a product go the same way):
-// rows of 16-byte multiples, and large enough that a tile of 128 features and stages of 64 k pay.
+// Whether the kernel takes a weight of this shape: rows of 16-byte multiples, a tile of 128 features and a few stages of 64 k.
 CO_EXPORT int coheryn_gemm_f32_tc_takes(int N, int K) { return N >= 128 && K >= 256 && K % 4 == 0; }
+// Whether it is the faster one for this weight, whatever the rows (a function of the shape alone, so that all rows of a product go the
+// same way).  Its two or three launches and its start lie against one or two launches of the FMA kernel.  Measured on a B200 from 1 to 1,500
+// rows, back to back, this one's us and the FMA kernel's: 128 x 256 one row 8.4 and 8.4, 313 rows 14 and 9.1; 256 x 448 9 to 11 against 14 up
+// to 64 rows, then 18 against 14 at 313; 1024 x 256 12 and 9.1 at 128 rows, 16 and 36 at 1,500; 4096 x 256 8.4 and 8.7 at one row, 12 and 24
+// at 128; 128 x 512 9.7 and 15 at one row, 16 and 16 at 700, 192 x 512 the same; from there on it is ahead everywhere.
+CO_EXPORT int coheryn_gemm_f32_tc_pays(int N, int K) { return coheryn_gemm_f32_tc_takes(N, K) && (K >= 512 || N >= 4096); }
 
 // Floats of workspace (16-byte aligned) that a product with this activation needs.
 CO_EXPORT long coheryn_gemm_f32_tc_workspace_floats(int M, int N, int K, int act) {
   if (M <= 0 || N <= 0 || K <= 0) return 0;
-  const int rows = rows_at_once(M, N, K), slices = slices_of(N, K);
+  const int rows = rows_at_once(M, N, K, act), slices = slices_of(N, K);
   return terms_floats(rows, K) + (slices > 1 || act ? (long)slices * rows * N : 0);
 }
 
@@ -427,7 +434,7 @@ CO_EXPORT int coheryn_gemm_f32_tc(const float* x, const float* w, const void* bi
   if (act != 0 && act != CO_ACT_GELU) CO_FAIL("gemm_f32_tc: unknown activation %d", act);
   if (((uintptr_t)w & 15) || ((uintptr_t)workspace & 15)) CO_FAIL("gemm_f32_tc: the weight and the workspace must be 16-byte aligned");
   if (!workspace || floats < coheryn_gemm_f32_tc_workspace_floats(M, N, K, act)) CO_FAIL("gemm_f32_tc: the workspace of %ld floats is too small", floats);
-  const int slices = slices_of(N, K), pitch = pitch_of(K), most = rows_at_once(M, N, K);
+  const int slices = slices_of(N, K), pitch = pitch_of(K), most = rows_at_once(M, N, K, act);
   const bool apart = slices > 1 || act != 0;      // what follows the sums is the adding kernel's
   CUtensorMap mw, mx;
   if (!make_map(&mw, w, N, 2L * K, 2L * K, F_ROWS)) CO_FAIL("gemm_f32_tc: cuTensorMapEncodeTiled failed (N=%d K=%d)", N, K);

@@ -497,30 +497,41 @@ def gemm_simt(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor], ou
 
 @functools.lru_cache(maxsize=4096)
 def _f32_tc_workspace_floats(M: int, N: int, K: int, act: int) -> int:
-    """0: the tensor-core kernel does not take such a weight (its shape alone decides, so all rows go the same way)."""
+    """0: the tensor-core kernel does not take such a weight."""
     lib = core()
     if not lib.coheryn_gemm_f32_tc_takes(c_int(N), c_int(K)):
         return 0
     return int(lib.coheryn_gemm_f32_tc_workspace_floats(c_int(M), c_int(N), c_int(K), c_int(act)))
 
 
+@functools.lru_cache(maxsize=4096)
+def _f32_tc_pays(N: int, K: int) -> bool:
+    return bool(core().coheryn_gemm_f32_tc_pays(c_int(N), c_int(K)))
+
+
 def gemm_f32(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor], out: torch.Tensor, act: int = 0) -> None:
-    """out = x @ w.T (+ bias), passed through ``act``, to float32's accuracy: float32 operands on the tensor cores as exact sums
-    of three bfloat16 terms (csrc/gemm_f32_tc.cu) where the weight's shape pays, everything else on the CUDA cores
-    (``gemm_simt``).  A row's bits do not depend on the other rows."""
+    """out = x @ w.T (+ bias), passed through ``act``, to float32's accuracy: float32 operands on the tensor cores
+    (``gemm_f32_tc``) where the weight's shape pays, everything else on the CUDA cores (``gemm_simt``).  The weight's shape
+    alone decides, so all rows go the same way and a row's bits do not depend on the other rows."""
+    if (x.shape[0] and x.dtype == w.dtype == out.dtype == torch.float32 and w.data_ptr() % 16 == 0
+            and _f32_tc_pays(w.shape[0], x.shape[1])):
+        gemm_f32_tc(x, w, bias, out, act)
+    else:
+        gemm_simt(x, w, bias, out, act)
+
+
+def gemm_f32_tc(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor], out: torch.Tensor, act: int = 0) -> None:
+    """The float32 product on the tensor cores, operands as exact sums of three bfloat16 terms (csrc/gemm_f32_tc.cu)."""
+    _dev(x, w, bias, out)
     M, K = x.shape
     N = w.shape[0]
-    floats = 0
-    if M and x.dtype == w.dtype == out.dtype == torch.float32 and w.data_ptr() % 16 == 0:
-        floats = _f32_tc_workspace_floats(M, N, K, act)
-    if not floats:
-        return gemm_simt(x, w, bias, out, act)
-    _dev(x, w, bias, out)
+    assert x.dtype == w.dtype == out.dtype == torch.float32
     assert w.shape == (N, K) and w.is_contiguous() and out.shape == (M, N)
     assert x.stride(1) == 1 and out.stride(1) == 1
     if bias is not None:
         assert bias.shape == (N,) and bias.is_contiguous()
     lib = core()
+    floats = _f32_tc_workspace_floats(M, N, K, act)
     workspace = torch.empty(floats, dtype=torch.float32, device=x.device)
     _check(lib, lib.coheryn_gemm_f32_tc(
         _ptr(x), _ptr(w), _ptr(bias), c_int(_code(bias) if bias is not None else F32), _ptr(out), c_int(M), c_int(N), c_int(K),

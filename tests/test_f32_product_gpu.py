@@ -11,7 +11,7 @@ def product(x, w, bias=None, act=0):
     from coheryn_ai_studio_b200 import ops
     out = torch.full((x.shape[0], w.shape[0] + 3), float("nan"), device=DEV)[:, :w.shape[0]]
     assert ops._f32_tc_workspace_floats(x.shape[0], w.shape[0], w.shape[1], act) > 0
-    ops.gemm_f32(x, w, bias, out, act)
+    ops.gemm_f32_tc(x, w, bias, out, act)
     return out
 
 
