@@ -88,8 +88,12 @@ __device__ __forceinline__ void store_chunk_tma(unsigned tmem_chunk, const float
 
 // No co_pdl_launch_dependents() in this file: these kernels fill the SMs, so a successor that is launched ahead finds no good places,
 // and what it takes early (several of its CTAs on the first SM that is free) it keeps.  Successors start at the end, their launch still
-// hidden.  Measured on a B200, launched ahead and not: a block of 437 rows of 1536 x 8960 (two prompts, 22 decodes) 161 and 140 us, 64
-// decodes 105 and 100, routed experts of 2,048 tokens 200 and 193.  (The few-rows kernel, bound by its stream of weights, launches ahead.)
+// hidden.  Measured on a B200, whole blocks with the successors launched ahead and not, 1.5B layer sizes: 17, 24, 40 and 64 decoding
+// requests 67.3 / 66.9, 71.4 / 71.4, 78 / 78 and 90 / 85 us, prompts of 33, 200, 513 and 1,500 tokens 84 / 76, 118 / 105, 146 / 142 and
+// 197 / 192, 403 tokens over 1,024 beside 37 decodes 175 / 154; 7B: 32 and 64 decodes 147 / 140 and 183 / 184, prompts of 200 and 513 205 / 197
+// and 320 / 307; routed experts of 2,048 tokens 200 / 193.  Launched ahead when the products are formed, or by the kernel that adds the
+// slices alone: between the two.  Only products back to back, as no model runs them, lose 0.3 to 1 us each (1536 x 1536 by 313
+// rows 15.5 and 16.6).  (The few-rows kernel, bound by its stream of weights, launches ahead.)
 template <int BN, int STAGES>
 __global__ void __launch_bounds__(EPI_THREADS)
 gemm_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_w,
