@@ -11,11 +11,14 @@
 // same way with the keys of the chunk on 64 of the lanes.  The tensor cores' accumulator, which cuts instead of rounding, holds 64 values
 // of k at most: the sums over more key channels are added up by the threads, with ordinary float32 additions.
 //
-// What bounds it: the chain of a CTA, which has an SM's tensor memory to itself.  A chunk's 60 MMAs take 5 us of it; the rest is the
-// splits (a dozen integer and float32 operations a value), the weights of the scores, and the norm and gate of the rows, one after
-// another.  A warp passes each piece of code a few times only, so the loops are kept small (unrolled further they wait for
-// instructions: 87 us for the outputs).  Measured on a B200 (8 heads of 128 x 256, one request of 2,048 tokens, all four kernels with
-// L2 flushed): 169 us with the products in float32 multiply-adds, 137 now, 7 of which are the gates' divisions.
+// What bounds it: the chain of a CTA.  A chunk's 60 MMAs take 5 us of it; the rest is the splits (a dozen integer and float32 operations
+// a value), the weights of the scores, and the norm and gate of the rows, one after another.  With more than 128 value channels a CTA has
+// an SM's tensor memory to itself; with fewer it takes half of it and two CTAs share an SM (with one, steps of many chunks of narrow
+// heads were slower than by multiply-adds: 8 heads of 64 x 128, three requests of 1,024 tokens 120 us by multiply-adds, 144, and 120 now).  A warp passes
+// each piece of code a few times only, so the loops are kept small (unrolled further they wait for instructions: 87 us for the outputs).
+// Measured on a B200, all four kernels with L2 flushed, by multiply-adds and now: 8 heads of 128 x 256, one request of 2,048 tokens 167 and
+// 135 us, 7 of them the gates' divisions; 8 heads of 128 x 128, 32 requests of 128 222 and 176; the worst, 2 heads of 32 x 128 and 128
+// requests of 80, 108 and 128.
 //
 // Every wait is for the CTA's own products and is bounded: on expiry the kernel records an error code and winds down.
 #include "tc_common.cuh"
@@ -205,17 +208,20 @@ __global__ void __launch_bounds__(32 * (4 * HALVES + 1)) memory_sum_tc_kernel(Me
   end(tmem, COLUMNS);
 }
 
-// Shared memory of the output kernel: the keys' terms per 64 key channels, later the scores and the gates; and behind them q's terms and
-// the weighted scores' terms, later the finished rows.  (The keys are an operand of 128 rows: what lies behind a tile's 64 is read too,
-// for lanes that nobody reads.)
+// Shared memory of the output kernel, two areas.  First the keys' terms per 64 key channels; when the scores are formed, the scores and,
+// behind them, with up to 128 value channels the weighted scores' terms and at the end the gates over both (two CTAs fit an SM up to 128
+// key channels), with more the gates.  Second q's terms and, with more than 128 value channels, the weighted scores' terms; at the end the
+// finished rows.  (The keys are an operand of 128 rows: what lies behind a tile's 64 is read too, for lanes that nobody reads.)
+constexpr int SCORES = CH * (CH + 4) * 4;
+static_assert(SCORES % 1024 == 0, "what lies behind the scores is a tile");
 __host__ __device__ inline int q_tiles(int dk) { return (dk + 63) / 64; }
 inline size_t larger(size_t a, size_t b) { return ((a > b ? a : b) + 1023) / 1024 * 1024; }
-size_t out_tc_keys(int dk, int dvp) { return larger((size_t)q_tiles(dk) * 3 * TILE, (size_t)CH * (CH + 4) * 4 + (size_t)CH * dvp * 4); }
-size_t out_tc_smem(int dk, int dvp) { return 1024 + out_tc_keys(dk, dvp) + larger((size_t)(q_tiles(dk) + 1) * 3 * TILE, (size_t)CH * (dvp + 4) * 4); }
-
-__device__ __forceinline__ void tmem_ld4(unsigned taddr, unsigned (&r)[4]) {
-  asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(taddr));
-  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+size_t out_tc_keys(int dk, int dv, int dvp) {
+  const size_t keys = (size_t)q_tiles(dk) * 3 * TILE, gates = (size_t)CH * dvp * 4;
+  return dv <= 128 ? larger(keys, larger(SCORES + 3 * TILE, gates)) : larger(keys, SCORES + gates);
+}
+size_t out_tc_smem(int dk, int dv, int dvp) {
+  return 1024 + out_tc_keys(dk, dv, dvp) + larger((size_t)(q_tiles(dk) + (dv <= 128 ? 0 : 1)) * 3 * TILE, (size_t)CH * (dvp + 4) * 4);
 }
 
 // Sixteen columns of this thread's lane are added to sixteen others.
@@ -268,12 +274,12 @@ __device__ __forceinline__ void rows_out(const HeadOut& E, To* out, const float*
 
 // grid (chunks, heads), 4 HALVES + 1 warps.
 template <int HALVES>
-__global__ void __launch_bounds__(32 * (4 * HALVES + 1)) memory_out_tc_kernel(MemoryIn P, HeadOut E, int B, int base, Area A, int key_bytes, int* status) {
+__global__ void __launch_bounds__(32 * (4 * HALVES + 1), 3 - HALVES) memory_out_tc_kernel(MemoryIn P, HeadOut E, int B, int base, Area A, int key_bytes, int* status) {
   constexpr int WORKERS = 4 * HALVES, THREADS = 32 * WORKERS;
-  // D_P: the scores, 64 columns per block of 64 key channels (the others' columns are free again when the products with S_0 begin).
+  // D_P: the scores, 64 columns per block of 64 key channels, until they are taken out in front of the products with S_0.
   // D_S: the sum of S_0's blocks; D_V: the products with one block from the second on, then with the values.
-  constexpr int D_P = 0, D_S = 64, D_V = D_S + 64 * HALVES, A_AT = D_V + 64 * HALVES;
-  static_assert(A_AT + HALVES * A_COLS <= 512, "tensor memory");
+  constexpr int D_P = 0, D_V = 0, D_S = 64 * HALVES, A_AT = 2 * 64 * HALVES, COLUMNS = HALVES == 1 ? 256 : 512;
+  static_assert(A_AT + HALVES * A_COLS <= COLUMNS, "tensor memory");
   extern __shared__ unsigned char smem_raw[];
   __shared__ Bars bars;
   __shared__ double down[CH], up[CH];        // F_t - m_t, i_s - F_s
@@ -282,13 +288,13 @@ __global__ void __launch_bounds__(32 * (4 * HALVES + 1)) memory_out_tc_kernel(Me
   float* scores = (float*)ks;                               // [s][CH + 1]
   unsigned char* first = ks + key_bytes;                    // q's tiles [block][3], later the finished rows
   const int dk = P.dk, dv = P.dv, dvp = A.dvp, blocks = q_tiles(dk);
-  unsigned char* ps = first + blocks * 3 * TILE;            // behind q's tiles
-  float* gates = scores + CH * (CH + 4);                    // [token][dvp]
-  const unsigned tmem = begin(bars, WORKERS, 512);
+  unsigned char* ps = HALVES == 1 ? ks + SCORES : first + blocks * 3 * TILE;
+  float* gates = (float*)(HALVES == 1 ? ks : ks + SCORES);  // [token][dvp]
+  const unsigned tmem = begin(bars, WORKERS, COLUMNS);
   co_pdl_wait();
   const int h = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   Run R;
-  if (!find_run(P.cu_q, B, base + blockIdx.x, false, R)) { end(tmem, 512); return; }
+  if (!find_run(P.cu_q, B, base + blockIdx.x, false, R)) { end(tmem, COLUMNS); return; }
   const int row0 = R.start + R.chunk * CH, nt = min(CH, R.len - R.chunk * CH);
   const size_t at = (size_t)blockIdx.x * P.heads + h;
   if (tid < CH) {
@@ -368,6 +374,19 @@ __global__ void __launch_bounds__(32 * (4 * HALVES + 1)) memory_out_tc_kernel(Me
     fence_proxy_async();
     __syncwarp();
     if (lane == 0) mbar_arrive(&bars.a_full);
+    auto fetch_gates = [&]() {
+      const float* from = E.gate + (size_t)row0 * E.ldg + (size_t)h * dv;
+      const bool vec = dv % 4 == 0 && E.ldg % 4 == 0 && ((uintptr_t)E.gate & 15) == 0;
+      const int per = vec ? dv / 4 : dv;
+#pragma unroll 1
+      for (int t = warp; t < nt; t += WORKERS)
+#pragma unroll 1
+        for (int e = lane; e < per; e += 32) {
+          if (vec) cp16(gates + t * dvp + 4 * e, from + (size_t)t * E.ldg + 4 * e);
+          else cp4(gates + t * dvp + e, from + (size_t)t * E.ldg + e);
+        }
+      cp_commit();
+    };
     bool ok = true;
     // The blocks of A, one copy of the code for all: S_0's rows, then the values.
 #pragma unroll 1
@@ -378,17 +397,16 @@ __global__ void __launch_bounds__(32 * (4 * HALVES + 1)) memory_out_tc_kernel(Me
         // The weighted scores: lane s of the first two quarters, half of the tokens t for each half of the warps.
         const int s = quarter * 32 + lane;
         const double mine = up[s];
+        float* score = scores + s * (CH + 1);
 #pragma unroll 1
         for (int t = half * (CH / HALVES); t < (half + 1) * (CH / HALVES); t += 4) {
-          unsigned r[4];
-          tmem_ld4(lanes + D_P + t, r);
 #pragma unroll
           for (int j = 0; j < 4; j += 2) {
             float x[2];
 #pragma unroll
             for (int i = 0; i < 2; ++i) {
-              x[i] = s <= t + j + i && t + j + i < nt ? __uint_as_float(r[j + i]) * expf((float)(down[t + j + i] + mine)) : 0.f;
-              scores[s * (CH + 1) + t + j + i] = x[i];
+              x[i] = s <= t + j + i && t + j + i < nt ? score[t + j + i] * expf((float)(down[t + j + i] + mine)) : 0.f;
+              score[t + j + i] = x[i];
             }
             unsigned y[3];
             split3(x[0], x[1], y[0], y[1], y[2]);
@@ -408,30 +426,29 @@ __global__ void __launch_bounds__(32 * (4 * HALVES + 1)) memory_out_tc_kernel(Me
       // the products with the block before have been formed when its columns are written
       ok = __all_sync(0xffffffffu, mbar_wait(&bars.done, (b - 1) & 1)) && ok;
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      if (b == 1) {       // the blocks' scores are added
+      if (b == 1) {       // the scores, added over the blocks, go to where the keys were
         if (quarter < 2)
-          for (int block = 1; block < blocks; ++block)
 #pragma unroll 1
-            for (int t = half * (CH / HALVES); t < (half + 1) * (CH / HALVES); t += 16) columns_add(lanes + D_P + t, lanes + D_P + 64 * block + t);
+          for (int t = half * (CH / HALVES); t < (half + 1) * (CH / HALVES); t += 16) {
+            float* score = scores + (quarter * 32 + lane) * (CH + 1) + t;
+            unsigned x[16];
+            tmem_ld16(lanes + D_P + t, x);
+#pragma unroll
+            for (int j = 0; j < 16; ++j) score[j] = __uint_as_float(x[j]);
+#pragma unroll 1
+            for (int block = 1; block < blocks; ++block) {
+              tmem_ld16(lanes + D_P + 64 * block + t, x);
+#pragma unroll
+              for (int j = 0; j < 16; ++j) score[j] += __uint_as_float(x[j]);
+            }
+          }
       } else if (b > 2)   // the block before is added to the sum
 #pragma unroll 1
         for (int j = 64 * half; j < 64 * half + 64; j += 16) columns_add(lanes + D_S + j, lanes + D_V + j);
       put_terms(terms, t0, t1, t2);
       __syncwarp();
       if (lane == 0) mbar_arrive(&bars.a_full);
-      if (b == 1) {      // the keys' tiles have been read: the gates come in their place
-        const float* from = E.gate + (size_t)row0 * E.ldg + (size_t)h * dv;
-        const bool vec = dv % 4 == 0 && E.ldg % 4 == 0 && ((uintptr_t)E.gate & 15) == 0;
-        const int per = vec ? dv / 4 : dv;
-#pragma unroll 1
-        for (int t = warp; t < nt; t += WORKERS)
-#pragma unroll 1
-          for (int e = lane; e < per; e += 32) {
-            if (vec) cp16(gates + t * dvp + 4 * e, from + (size_t)t * E.ldg + 4 * e);
-            else cp4(gates + t * dvp + e, from + (size_t)t * E.ldg + e);
-          }
-        cp_commit();
-      }
+      if (HALVES == 2 && b == 1) fetch_gates();      // the keys' tiles have been read: there is room
     }
     workers_meet<THREADS>();       // the scores stand
     // n_t . q_t, and with it the denominators
@@ -461,7 +478,8 @@ __global__ void __launch_bounds__(32 * (4 * HALVES + 1)) memory_out_tc_kernel(Me
     ok = __all_sync(0xffffffffu, mbar_wait(&bars.done, (blocks + 1) & 1)) && ok;
     if (!ok && lane == 0) atomicExch(status, 13);
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    workers_meet<THREADS>();       // the denominators stand, nobody reads the tiles any more
+    workers_meet<THREADS>();       // the denominators stand, nobody reads the tiles and scores any more
+    if (HALVES == 1) fetch_gates();
     float* rows = (float*)first;
 #pragma unroll 1
     for (int j0 = 0; j0 < CH; j0 += 16) {
@@ -478,7 +496,7 @@ __global__ void __launch_bounds__(32 * (4 * HALVES + 1)) memory_out_tc_kernel(Me
   __syncthreads();
   if (E.out_dtype == CO_BF16) rows_out(E, (__nv_bfloat16*)E.out + (size_t)h * dv, (float*)first, dvp + 4, gates, dvp, weight, dv, nt, row0);
   else rows_out(E, (float*)E.out + (size_t)h * dv, (float*)first, dvp + 4, gates, dvp, weight, dv, nt, row0);
-  end(tmem, 512);
+  end(tmem, COLUMNS);
 }
 
 }  // namespace
@@ -492,10 +510,10 @@ int co_memory_sum_tc(const MemoryIn& P, int B, int base, int count, const Area& 
   return 0;
 }
 int co_memory_out_tc(const MemoryIn& P, const HeadOut& E, int B, int base, int count, const Area& A, int* status, cudaStream_t stream) {
-  const size_t smem = out_tc_smem(P.dk, A.dvp);
+  const size_t smem = out_tc_smem(P.dk, P.dv, A.dvp);
   auto kernel = P.dv <= 128 ? memory_out_tc_kernel<1> : memory_out_tc_kernel<2>;
   cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  co_launch(kernel, dim3(count, P.heads), dim3(P.dv <= 128 ? 160 : 288), smem, stream, P, E, B, base, A, (int)out_tc_keys(P.dk, A.dvp), status);
+  co_launch(kernel, dim3(count, P.heads), dim3(P.dv <= 128 ? 160 : 288), smem, stream, P, E, B, base, A, (int)out_tc_keys(P.dk, P.dv, A.dvp), status);
   CO_CHECK_LAUNCH("memory_out_tc");
   return 0;
 }
