@@ -882,33 +882,33 @@ CO_EXPORT long coheryn_memory_chunk_floats(int chunks, int heads, int dk, int dv
 // Whether a step's runs of CHUNK_FROM tokens and more (`chunks` chunks, the longest run of `longest` tokens) are to go in chunks; T
 // tokens of B requests in all.  The scan is a chain over the longest run, slow while requests are few; the chunks cost four kernels
 // at least, and several times the multiply-adds.  Which is faster is a matter of all these sizes, so both are estimated, in us.  The
-// constants are fitted to the times of both forms on a B200 (1 to 128 runs of 48 to 320 tokens, six sizes of heads each): a tenth rms,
-// and of 804 combinations the choice costs more than 15 % in 18 (with chunks for every run of 48 that many were 299).  Scan and chunks
-// measured, delta rule: 12 heads of 128 x 128, one run of 64 tokens 58 and 97 us, of 320 199 and 163, 16 of 64 135 and 232, 32 of 256 906
-// and 897; 4 heads of 32 x 64, one run of 96 tokens 65 and 59, 128 of 48 47 and 188.  Matrix memory: 8 heads of 128 x 256, one run of 64
-// tokens 59 and 70, of 192 141 and 92, 16 of 64 148 and 132; 2 heads of 32 x 128, 32 of 48 45 and 63.  The delta rule's chunks are kept up
-// to a tenth beyond the scan's time.
+// constants are fitted to the times of both forms on a B200 (1 to 128 runs of 48 to 2,048 tokens, alone and beside single tokens; six sizes of
+// heads for the delta rule, seven for the matrix memory): a tenth to a fifth rms, and the choice costs more than 15 % in 21 of 780 and 2 of
+// 910 steps.  Scan and chunks measured, delta rule: 12 heads of 128 x 128, one run of 64 tokens 65 and 105 us, of 192 136 and 112, 16 of 64
+// 180 and 194, 32 of 256 993 and 875; 4 heads of 32 x 64, one run of 96 tokens 115 and 68, 128 of 48 74 and 177.  Matrix memory: 8 heads of
+// 128 x 256, one run of 64 tokens 71 and 65, of 192 155 and 65, 16 of 64 184 and 85; 2 heads of 32 x 128, 32 of 48 68 and 56, 128 of 96 135
+// and 128.
 static float sliced_load(int B, int heads, int dv) { return fmaxf(1.f, (float)((long)B * heads * ((dv + SLICE_COLUMNS - 1) / SLICE_COLUMNS)) / 148.f); }
 static float delta_scan_us(int heads, int dk, int dv, int B, int T, int longest) {
-  if (scan_splits(B, heads, dv, T)) return longest * (0.344f + 0.00263f * dk) * sliced_load(B, heads, dv) + 14.f;
-  return 5.f + fmaxf(longest * (0.478f + 0.00238f * dk + 0.00197f * dv), (float)T * heads * 0.009f * powf(dk * dv / 16384.f, 0.82f));
+  if (scan_splits(B, heads, dv, T)) return longest * (0.319f + 0.00231f * dk) * sliced_load(B, heads, dv) + 25.7f;
+  return 11.8f + fmaxf(longest * (1.067f + 0.00117f * dk + 0.00117f * dv), (float)T * heads * 0.00981f * powf(dk * dv / 16384.f, 0.729f));
 }
 static float memory_scan_us(int heads, int dk, int dv, int B, int T, int longest) {
   const float size = dk * dv / 32768.f;
-  if (scan_splits(B, heads, dv, T)) return longest * (0.41f + 0.00239f * dk) * sliced_load(B, heads, dv) + 13.f;
-  return fmaxf(longest * (1.02f + 0.838f * size), (float)T * heads * 0.0195f * powf(size, 0.867f)) - 1.f;
+  if (scan_splits(B, heads, dv, T)) return longest * (0.339f + 0.00337f * dk) * sliced_load(B, heads, dv) + 21.6f;
+  return 9.8f + fmaxf(longest * (1.247f + 1.366f * size), (float)T * heads * 0.0249f * powf(size, 0.937f));
 }
 CO_EXPORT int coheryn_delta_chunks_pay(int heads, int dk, int dv, int B, int T, int longest, int chunks) {
   if (!co_delta_chunks_take(dk, dv)) return 0;
   const int D = dk <= 64 ? 64 : 128;
-  const float us = 24.f + 0.4245f * D + 0.088f * dv + (float)chunks * heads * 0.559f * powf(D * dv / 16384.f, 0.605f);
-  return us <= 1.1f * delta_scan_us(heads, dk, dv, B, T, longest);
+  const float us = 30.8f + 0.2767f * D + 0.202f * dv + (float)chunks * heads * 0.484f * powf(D * dv / 16384.f, 0.605f);
+  return us <= delta_scan_us(heads, dk, dv, B, T, longest);
 }
 CO_EXPORT int coheryn_memory_chunks_pay(int heads, int dk, int dv, int B, int T, int longest, int chunks) {
   if (!co_memory_chunks_take(dk, dv)) return 0;
   const float size = dk * dv / 32768.f;
-  const float us = 40.f + 17.5f * size + 0.106f * dk + 1.065f * size * ((longest + CHUNK_TOKENS - 1) / CHUNK_TOKENS) + (float)chunks * heads * 0.467f * powf(size, 0.66f);
-  return us <= memory_scan_us(heads, dk, dv, B, T, longest);
+  const float us = 53.5f + 2.9f * size + 0.0097f * dk + 0.125f * size * ((longest + CHUNK_TOKENS - 1) / CHUNK_TOKENS) + (float)chunks * heads * 0.379f * powf(size, 0.63f);
+  return us <= 1.05f * memory_scan_us(heads, dk, dv, B, T, longest);
 }
 CO_EXPORT int coheryn_chunk_from() { return CHUNK_FROM; }
 CO_EXPORT int coheryn_chunk_tokens() { return CHUNK_TOKENS; }
