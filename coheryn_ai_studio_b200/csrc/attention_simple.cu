@@ -1,13 +1,14 @@
-// Causal (optionally windowed) grouped-query attention over cache pages, written for
-// clarity: one block per (token, query head), float32 arithmetic throughout.  It is
-// the attention of the true 32-bit path and the any-shape reference of the bfloat16
-// tensor-core kernels.
+// Causal (optionally windowed) grouped-query attention over cache pages, float32
+// arithmetic throughout.  It is the attention of the true 32-bit path and the any-shape
+// reference of the bfloat16 tensor-core kernels.  A block takes a token and several query
+// heads of a group (attention_group_kernel) or, for shapes that allow no vector loads, one
+// head (attention_simple_kernel).
 //
 // For token t of request r at position p the keys are positions first..p of r's cache,
 // first = max(0, p - window + 1) with a window, else 0; the cache already holds the
-// keys that this step wrote.  Four warps each run an online softmax over the keys
-// k = first + warp, first + warp + 4, ...; their (max, sum, accumulator) triples are
-// merged in warp order.  The result therefore depends only on (p, first), never on
+// keys that this step wrote.  The block's W warps (eight, or four for one head) each run an
+// online softmax over the keys k = first + warp, first + warp + W, ...; their (max, sum,
+// accumulator) triples are merged in warp order.  The result therefore depends only on (p, first), never on
 // how the step was cut or batched.
 //
 // What bounds it: with a block per (token, query head), the reads of the same keys and values by every head of a group (1 KB a key and

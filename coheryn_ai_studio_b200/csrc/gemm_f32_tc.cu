@@ -16,12 +16,12 @@
 //   warps 2-5    split: a thread reads its feature's 64 values, writes 3 x 32 columns of bfloat16 pairs to tensor memory
 //   warps 6-13   add a stage's accumulator (two of them in tensor memory) to their sums, and the epilogue
 //
-// What bounds it: the tensor cores' operand W from tensor memory and the gaps between stages.  A product with A in tensor memory takes
-// 70 cycles at 16 tokens and 93 at 160 (80 would be the matrix pipe's rate), 24 of them a stage, and about 400 cycles pass until the
-// next stage's first; shared memory moves 248 KB a stage (W's terms there as well: 480 KB) and the split takes 2,000 cycles of one
-// warp beside it.  Measured on a B200 (alone, L2 flushed, with the two small kernels; before: the CUDA cores, gemm_simt.cu):
-// 313 x 17920 x 1536 417 -> 116 us, 313 x 1536 x 8960 216 -> 79, 313 x 1536 x 1536 77 -> 28, 2048 x 17920 x 1536 2,518 -> 701, one row by
-// 17920 x 1536 84 -> 47.  Error against float64 (2-norm, relative): 0.8e-7 to 1.2e-7 where the FMA chain has 2.8e-7 to 5.0e-7.
+// What bounds it: the chain of a CTA's stages (W's tile, its split, the products, the sums) with one CTA per SM.  The profiler's counters:
+// 313 x 17920 x 1536 keeps the tensor pipe 55 % busy, the integer pipe of the split 25 % and DRAM 27 %; one row by 17920 x 1536 DRAM 39 %
+// and the integer pipe 30 %.  (With W's terms in shared memory as well that would move 480 KB a stage in place of 248.)  Measured on a B200
+// (alone, L2 flushed, with the two small kernels; before: the CUDA cores, gemm_simt.cu): 313 x 17920 x 1536 417 -> 105 us, 313 x 1536 x 8960
+// 216 -> 73, 313 x 1536 x 1536 77 -> 24, 2048 x 17920 x 1536 2,518 -> 632, one row by 17920 x 1536 84 -> 40.  Error against float64
+// (2-norm, relative): 0.8e-7 to 1.2e-7 where the FMA chain has 2.8e-7 to 5.0e-7.
 //
 // A row's result does not depend on the other rows: K is cut into slices by the weight's shape alone, a slice's sum goes to a
 // workspace (where there is more than one) and the slices are added in order.  Two kinds of results are formed again from the operands

@@ -26,7 +26,10 @@ constexpr int EPI_PLAIN = 0, EPI_GATED_SILU = 1;
 // Eight epilogue warps per CTA, two per quarter of its rows, that take the chunks of columns in turn.  With four (a warp a scheduler)
 // the gate's exponentials and divisions took longer than the 24 k-steps of the next tile at K = 1,536: measured on a B200, 2048 x 17920 x
 // 1536 gated by the pairs 108 -> 85 us (ungated 82), 1873 rows 120 -> 84, 1024 rows 68 -> 45; 800 rows by the
-// persistent kernel 55 -> 49, 513 rows 43 -> 38; 200 rows, one tile per CTA, 22.7 -> 18.7.  (Ungated products: no change.)
+// persistent kernel 55 -> 49, 513 rows 43 -> 38; 200 rows, one tile per CTA, 22.7 -> 18.7.  (Ungated products: no change.)  When SiLU was
+// the only gate, four warps took 84 us for the first of these; with the activation chosen at run time for every pair they took 108.
+// A gated tile of 128 columns is one chunk, so that the second four of its warps have nothing to do there: 128 rows of 256 x 1536 8.7 us
+// with four warps and with eight.
 constexpr int EPI_WARPS = 8, EPI_THREADS = 64 + 32 * EPI_WARPS;
 
 template <int BN, int STAGES>

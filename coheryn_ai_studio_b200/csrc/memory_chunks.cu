@@ -16,13 +16,14 @@
 // m are kept in float32, so an exponent may exceed zero by the rounding of m (3e-5 at m = 1,000): S, n and exp(-m) all use the same
 // rounded m, and what it is off by cancels between numerator and denominator.
 //
-// A value or key that is not finite makes the outputs of its whole chunk so, not only those from its token on: a zero weight times
-// it is not zero.
+// A value, key, query or state that is not finite makes the outputs of its whole chunk so (of the head's value channels it reaches), not
+// only those from its token on: a zero weight times it is not zero.  The products split every operand into three bfloat16 terms: one
+// of 3.39e38 and more counts as not finite, and of one under 2^-110 up to 2^-133 is cut off, which the norm's eps hides.
 //
 // What bounds it: the scan token by token is a chain of dependent multiply-adds and shuffles on a CTA per (head, 64 value
 // channels): 0.65 us per token with 32 of 148 SMs at work.  Here only the carry is a chain, of one multiply-add per chunk and
 // element; the rest are products over all chunks at once.  Measured on a B200 (8 heads of 128 x 256, one request of 2,048
-// tokens): 14 + 24 + 16 + 65 us in place of 1,350 us (1,850 with the kernels behind the scan launched ahead and waiting beside it).
+// tokens, L2 flushed): 135 us in place of 1,377 (by the profiler's clock, one kernel at a time from cold caches, 15 + 31 + 26 + 80).
 //
 // A run of fewer than CHUNK_FROM tokens is left to the scan (recurrent.cu), request by request: of the other requests only
 // whether the step goes in chunks at all (recurrent.cu, coheryn_*_chunks_pay) can reach a row, not its order of additions.

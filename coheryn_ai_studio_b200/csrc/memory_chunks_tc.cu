@@ -1,5 +1,7 @@
 // The two products of the chunked matrix memory (memory_chunks.cu) on the 5th-generation tensor cores, to float32's accuracy: every
-// float32 operand is the exact sum of three bfloat16 terms, and the six products of terms i + j <= 2 are formed (as in gemm_f32_tc.cu).
+// float32 operand is the sum of three bfloat16 terms (tc_common.cuh, split3), and the six products of terms i + j <= 2 are formed (as in
+// gemm_f32_tc.cu).  Error of the outputs against float64 (2-norm, relative) 1.3e-7 to 1.5e-7 from 64 to 256 key channels, by float32
+// multiply-adds 2.0e-7 to 3.3e-7; of the state 1.2e-7 to 1.6e-7 and 1.5e-7 to 1.7e-7.
 //
 //   memory_sum_tc_kernel   a CTA per (chunk, head, 128 key channels): what the chunk adds to S and n;
 //   memory_out_tc_kernel   a CTA per (chunk, head): scores, outputs, and the norm, weight and gate behind them.

@@ -641,8 +641,9 @@ def describe_status(code: int) -> str:
     if code in STATUS_MESSAGES:
         return STATUS_MESSAGES[code]
     if 11 <= code <= 39:
-        return (f"a kernel gave up a bounded wait and left its output unfinished (code {code}: 11-13 tensor-core product: "
-                "producer, MMA issuer, epilogue; 19 self-test; 31-39 prompt attention: 31 producer, 32-36 MMA issuer, "
+        return (f"a kernel gave up a bounded wait and left its output unfinished (code {code}: 11-14 tensor-core product: "
+                "producer, MMA issuer, epilogue, split of float32 operands; 12 and 13 also the matrix memory in chunks: MMA issuer, the "
+                "others; 19 self-test; 31-39 prompt attention: 31 producer, 32-36 MMA issuer, "
                 "37-39 softmax)")
     return f"device status {code}"
 
