@@ -109,3 +109,74 @@ def test_error_no_larger_than_that_of_multiply_adds(dk, dv):
             errors[e] += float((got - want).square().sum())
         errors[2] += float(want.square().sum())
     assert errors[0] <= errors[1], [(e / errors[2]) ** 0.5 for e in errors[:2]]
+
+
+@pytest.mark.parametrize("dk,dv", [(64, 128), (96, 200)])
+@pytest.mark.parametrize("where,value", [("v", float("nan")), ("k", float("inf")), ("q", float("nan")), ("state", float("-inf")), ("v", 3.4e38)])
+def test_values_that_are_not_finite_stay_in_their_chunks(dk, dv, where, value):
+    """A bad value reaches its head's chunk and, through the state, the later ones; other heads, requests and earlier chunks keep their bits."""
+    from coheryn_ai_studio_b200 import ops
+    H, lens, lib = 3, [150, 70], ops.recurrent()
+    T = sum(lens)
+    g = torch.Generator(device=DEV).manual_seed(dk)
+    f = lambda *s: torch.randn(s, device=DEV, generator=g)
+    clean, gates, gate, first, zero = f(T, H * (2 * dk + dv)), f(T, 2 * H), f(T, H * dv), f(2, H * (dk * dv + dk + 1)), torch.zeros(H, device=DEV)
+    first[:, -H:] = 0.0
+    pays, got = lib.coheryn_memory_chunks_pay, []
+    try:
+        lib.coheryn_memory_chunks_pay = lambda *a: 1
+        for bad in (False, True):
+            qkv, state, out = clean.clone(), first.clone(), torch.empty((T, H * dv), device=DEV)
+            if bad:      # head 1 of the first request; token 70 is the second chunk's
+                at = {"q": dk + 5, "k": H * dk + dk + 5, "v": 2 * H * dk + dv + 7}
+                if where == "state":
+                    state[0, dk * dv + 3 * dv + 7] = value
+                else:
+                    qkv[70, at[where]] = value
+            ops.matrix_memory_scan(qkv[:, :H * dk], qkv[:, H * dk:2 * H * dk], qkv[:, 2 * H * dk:], gates[:, :H], gates[:, H:], zero, zero, 15.0, state,
+                                   step_of(lens, [0, 1], True), H, dk, dv, out, torch.ones(H * dv, device=DEV), gate, 1e-5)
+            got.append((out.view(T, H, dv), state))
+    finally:
+        lib.coheryn_memory_chunks_pay = pays
+    ops.check_tc_status(DEV)
+    (want, want_state), (out, state) = got
+    assert torch.isfinite(want).all() and torch.isfinite(want_state).all()
+    assert torch.equal(out[:, 0], want[:, 0]) and torch.equal(out[:, 2], want[:, 2]) and torch.equal(out[150:], want[150:])
+    assert torch.equal(state[1], want_state[1])
+    start = 0 if where == "state" else 64
+    assert torch.equal(out[:start, 1], want[:start, 1])
+    assert not torch.isfinite(out[70, 1]).all()
+    if where != "q":      # the norm over the value channels takes it to all of them, the state to the chunks behind
+        assert not torch.isfinite(out[130:150, 1]).any() and not torch.isfinite(state[0]).all()
+    else:
+        assert torch.isfinite(out[128:150, 1]).all() and torch.equal(state[0], want_state[0])
+
+
+@pytest.mark.parametrize("what", ["v", "state", "k"])
+def test_operands_under_the_terms_range(what):
+    """Operands under 2^-110: a result is off by 2^-133 of each at most, times the other operand."""
+    from coheryn_ai_studio_b200 import ops
+    H, T, dk, dv, lib = 2, 64, 64, 128, ops.recurrent()
+    g = torch.Generator(device=DEV).manual_seed(5)
+    f = lambda *s: torch.randn(s, device=DEV, generator=g)
+    q, k, v, state = f(T, H * dk), f(T, H * dk), f(T, H * dv), f(1, H * (dk * dv + dk + 1))
+    state[:, H * dk * dv:] = 0.0
+    for name, t in (("v", v), ("k", k), ("state", state)):
+        if name == what or (name == "state" and what != "state") or (name == "v" and what == "state"):
+            t.mul_(2.0 ** -124 if name == what else 0.0)
+    first, qkv, zero, out = state.clone(), torch.cat([q, k, v], dim=1), torch.zeros(H, device=DEV), torch.empty((T, H * dv), device=DEV)
+    pays = lib.coheryn_memory_chunks_pay
+    try:
+        lib.coheryn_memory_chunks_pay = lambda *a: 1      # the gates are open: log f = 0 to 1e-6, log i = 0
+        ops.matrix_memory_scan(qkv[:, :H * dk], qkv[:, H * dk:2 * H * dk], qkv[:, 2 * H * dk:], torch.zeros(T, H, device=DEV),
+                               torch.full((T, H), 1e4, device=DEV), zero, zero, 15.0, state, step_of([T], [0], True), H, dk, dv, out,
+                               torch.ones(H * dv, device=DEV), torch.full((T, H * dv), 40.0, device=DEV), 1e-6)
+    finally:
+        lib.coheryn_memory_chunks_pay = pays
+    for h in range(H):
+        S, kh, vh = first[0, h * dk * dv:(h + 1) * dk * dv].view(dk, dv).double(), k[:, h * dk:(h + 1) * dk].double(), v[:, h * dv:(h + 1) * dv].double()
+        want, got = S + kh.T @ vh, state[0, h * dk * dv:(h + 1) * dk * dv].view(dk, dv).double()
+        # the gates and float32's sums as everywhere; what the split cuts off
+        bound = (T + 32) * 2.0 ** -23 * (S.abs() + kh.abs().T @ vh.abs()) + 2.0 ** -133 * (kh.abs().sum(0)[:, None] + vh.abs().sum(0)[None, :])
+        assert bool(((got - want).abs() <= bound).all())
+    assert bool(torch.isfinite(out).all()) and float(out.abs().max()) < 1e-25      # (the norm's eps is larger than any of these)
