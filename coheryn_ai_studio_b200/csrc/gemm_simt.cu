@@ -1,6 +1,6 @@
 // out[M, N] = x[M, K] . W[N, K]^T (+ bias[N]) with float32 FMA accumulation on the CUDA
-// cores: the matrix product of the true 32-bit path (no reduced-precision tensor mode),
-// and the any-shape reference for the bfloat16 tensor-core kernels.
+// cores: the matrix product of the true 32-bit path where a weight is small, unaligned or of
+// another type (else gemm_f32_tc.cu), and the any-shape reference for the tensor-core kernels.
 //
 // An output element is the sum, in ascending order, of the sums over stretches of values of k, each of them accumulated in
 // ascending order from zero.  The length of a stretch follows from the weight's shape; neither the tile of a launch nor
